@@ -177,7 +177,6 @@ int run_kpm1d(Operator* op, int64_t NC, int64_t NR, int64_t NH, const void* psi_
   if (lr) KPMGB_TRY(ws.bra.ensure(slot));
   // scales: column factors of the ket and the bra, and their products
   KPMGB_TRY(ws.scales.ensure((size_t)(3 * NR + 2) * sizeof(double)));
-  KPMGB_TRY(ws.partials.ensure(step_partials_bytes(op->csr, NH, (int)NR, precision)));
   KPMGB_TRY(ensure_sync(op, s));
   char* slots = ws.slots.as<char>();
   void* sl[2] = {slots, slots + slot};
@@ -264,18 +263,12 @@ int run_kpm1d(Operator* op, int64_t NC, int64_t NR, int64_t NH, const void* psi_
       t.H = &op->csr;
       t.NH = NH;
       t.NR = (int)NR;
-      t.mu = mu;
-      t.mom_scale = mom_scale;
-      t.sync = ws.sync.as<unsigned>();
-      t.partials = ws.partials.ptr;
-      t.partials_bytes = ws.partials.bytes;
       t.bra = lr ? ws.bra.ptr : nullptr;
       t.x = sl[0];
       t.y = sl[1];
       t.dot = lr ? DOT_LR2 : DOT_DOUBLING;
-      t.mom = MOM_STORE;
       int v = 1, sh = 0;
-      KPMGB_TRY(tune_step(t, precision, s, &v, &sh));
+      KPMGB_TRY(tune_step(t, precision, ws.partials, s, &v, &sh));
       it = op->tuned.emplace(tkey, std::make_pair(v, sh)).first;
       tune_cache_put(pkey, std::to_string(v) + "," + std::to_string(sh));
     }
@@ -285,62 +278,25 @@ int run_kpm1d(Operator* op, int64_t NC, int64_t NR, int64_t NH, const void* psi_
   // The recurrence proper: NC/2 (doubling) or NC-1 (bra/ket) step launches.
   // With use_graph on a non-legacy stream it is captured once into a CUDA
   // graph and replayed while sizes, options and device pointers repeat.
-  auto recurrence = [&]() -> int {
   StepArgs a;
   a.H = &op->csr;
   a.NH = NH;
   a.NR = (int)NR;
-  a.mu = mu;
-  a.mom_scale = mom_scale;
-  a.sync = ws.sync.as<unsigned>();
-  a.partials = ws.partials.ptr;
-  a.partials_bytes = ws.partials.bytes;
   a.bra = lr ? ws.bra.ptr : nullptr;
   a.variant = chosen_variant;
   a.shape = chosen_shape;
   a.paired = paired;
-  // alpha_1 = H alpha_0 with mu_0, mu_1 (src/moment.jl:440-449, :521-527)
-  a.x = sl[0];
-  a.z = nullptr;
-  a.y = sl[1];
-  a.alpha = 1.0;
-  a.beta = 0.0;
-  a.dot = lr ? DOT_LR2 : DOT_DOUBLING;
-  a.mom = MOM_STORE;
-  a.i0 = 0;
-  KPMGB_TRY(launch_step(a, precision, s));
-  int ip = 1, ipp = 0;
-  a.alpha = 2.0;
-  a.beta = -1.0;
-  if (!lr) {
-    const bool check = o && o->stability_check;
-    for (int64_t n = 2; n <= NC / 2; ++n) {
-      // alpha_n = 2 H alpha_{n-1} - alpha_{n-2} in place; doubling moments
-      // mu_{2n-2}, mu_{2n-1} (src/moment.jl:460-487)
-      a.x = sl[ip];
-      a.z = sl[ipp];
-      a.y = sl[ipp];
-      a.dot = DOT_DOUBLING;
-      a.mom = MOM_DOUBLING;
-      a.i0 = 2 * n - 2;
-      a.growth_limit = check ? 2.25 : 0.0;
-      KPMGB_TRY(launch_step(a, precision, s));
-      std::swap(ip, ipp);
-    }
-  } else {
-    for (int64_t n = 2; n < NC; ++n) {
-      // full recurrence, mu_n = <psil|alpha_n> (src/moment.jl:540-549)
-      a.x = sl[ip];
-      a.z = sl[ipp];
-      a.y = sl[ipp];
-      a.dot = DOT_LR1;
-      a.mom = MOM_STORE;
-      a.i0 = n;
-      KPMGB_TRY(launch_step(a, precision, s));
-      std::swap(ip, ipp);
-    }
-  }
-  return KPMGB_OK;
+  size_t held = 0;
+  KPMGB_TRY(recurrence_scratch_bytes(a, precision, NC, lr, &held));
+  KPMGB_TRY(ws.partials.ensure(std::max(ws.partials.bytes, held)));
+  a.partials = ws.partials.ptr;
+  MomentArgs m;
+  m.mu = mu;
+  m.scale = mom_scale;
+  m.growth_limit = !lr && o && o->stability_check ? 2.25 : 0.0;
+  m.status = ws.sync.as<unsigned>() + 1;
+  auto recurrence = [&]() -> int {
+    return launch_recurrence(a, precision, NC, lr, sl, held, m, s);
   };
   const bool graph = o && o->use_graph && s != nullptr && s != cudaStreamLegacy &&
                      s != cudaStreamPerThread;
@@ -456,7 +412,6 @@ int run_kpm2d(Operator* H, Operator* Ja, Operator* Jb, int64_t NC, int64_t NR, i
   // scales, then the per-vector maxima of the L and R blocks (column pairs)
   const size_t scale_bytes = (size_t)(2 * NR + 8) * sizeof(double);
   KPMGB_TRY(ws.scales.ensure(scale_bytes + (size_t)(KLa + KRa) * sizeof(unsigned)));
-  KPMGB_TRY(ws.partials.ensure(step_partials_bytes(H->csr, NH, (int)NR, precision)));
   const size_t cs = contract_scratch_bytes(K, (int)KRa, (int)KLa, precision, opt.contraction);
   KPMGB_TRY(ws.gemm.ensure(cs));
   KPMGB_TRY(ensure_sync(H, s));
@@ -512,9 +467,6 @@ int run_kpm2d(Operator* H, Operator* Ja, Operator* Jb, int64_t NC, int64_t NR, i
     a.y = y;
     a.alpha = alpha;
     a.beta = beta;
-    a.sync = ws.sync.as<unsigned>();
-    a.partials = ws.partials.ptr;
-    a.partials_bytes = ws.partials.bytes;
     a.colpair = colpair;
     a.vmax = vmax;
     return launch_step(a, precision, s);

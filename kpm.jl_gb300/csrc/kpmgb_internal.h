@@ -172,9 +172,19 @@ enum DotMode : int {
 };
 
 enum MomentMode : int {
-  MOM_NONE = 0,
   MOM_STORE = 1,     // mu[i0 + d] = d_d                        (d = 0..ND-1)
   MOM_DOUBLING = 2,  // mu[i0] = 2 d0 - mu[0], mu[i0+1] = 2 d1 - mu[1]
+};
+
+// Where the moments of a run of steps go: step q of the run writes the
+// moments i0 + q ND .. of every column, [NC][NR].
+struct MomentArgs {
+  double2* mu = nullptr;
+  int mom = MOM_STORE;
+  int64_t i0 = 0;
+  const double* scale = nullptr;  // per-column factor applied to the dots, or null
+  double growth_limit = 0.0;      // > 0 (MOM_DOUBLING): flag if d0 > growth_limit * mu[0]
+  unsigned* status = nullptr;
 };
 
 // One application of the recurrence y = alpha * H x + beta * z to a row-major
@@ -190,16 +200,10 @@ struct StepArgs {
   double beta = 0.0;
   const void* bra = nullptr;
   int dot = DOT_NONE;
-  int mom = MOM_NONE;
-  int64_t i0 = 0;            // moment index written by this step
-  double2* mu = nullptr;     // device moments [NC][NR]
-  const double* mom_scale = nullptr;  // per-column factor applied to the dots
-  double growth_limit = 0.0; // >0: flag if <x|x> > growth_limit * mu[0] (doubling)
-  unsigned* sync = nullptr;  // ticket counter + status word
+  void* partials = nullptr;   // per-block sums of the dots (step_partials_bytes;
+                              // unused for DOT_NONE), see launch_finish_moments
   unsigned* vmax = nullptr;  // column-pair steps: the largest |y| high part
                              // (float bits, atomicMax; zeroed by the caller)
-  void* partials = nullptr;
-  size_t partials_bytes = 0;  // 0: capacity not checked
   int variant = 0;           // 0 auto, 1 register-gather kernel, 9 padded-row kernel
   int shape = 0;             // lanes-per-row * 10 + columns-per-lane of the
                              // register-gather kernel; 0 = automatic
@@ -227,10 +231,21 @@ bool colpair_step_applies(const DeviceCSR& H, int NR);
 // Autotuning: times every (variant, shape) candidate of the step `a` (which
 // must not write its own inputs: y aliasing neither x nor z) with CUDA events
 // on `s`, after one warm launch each, and returns the fastest in
-// *variant / *shape.  Synchronises `s`.
-int tune_step(const StepArgs& a, int precision, cudaStream_t s, int* variant, int* shape);
-// Bytes of partial-sum scratch that launch_step needs for this shape.
-size_t step_partials_bytes(const DeviceCSR& H, int64_t NH, int NR, int precision);
+// *variant / *shape.  The candidates' dots go to `partials` and are dropped.
+// Synchronises `s`.
+int tune_step(const StepArgs& a, int precision, DevBuf& partials, cudaStream_t s, int* variant,
+              int* shape);
+// Bytes of per-block sums that the step `a` writes (0 without dots).
+int step_partials_bytes(const StepArgs& a, int precision, size_t* bytes);
+// A kpm_1d recurrence from slot[0] (slot[1] is overwritten): NC/2 doubling
+// steps, or NC - 1 bra/ket steps (lr), with all moments into m.mu.  `a` names
+// the operator, sizes, kernel and bra; a.partials holds `held` bytes, between
+// the two counts of recurrence_scratch_bytes (*least at least, the returned
+// count for the fewest finishing launches).
+int launch_recurrence(StepArgs a, int precision, int64_t NC, bool lr, void* const (&slot)[2],
+                      size_t held, MomentArgs m, cudaStream_t s);
+int recurrence_scratch_bytes(const StepArgs& a, int precision, int64_t NC, bool lr,
+                             size_t* bytes, size_t* least = nullptr);
 
 // Column-major (NH x NR, complex double) -> row-major slot, converting to the
 // working precision.  For KPMGB_PREC_FF each column is also multiplied by a

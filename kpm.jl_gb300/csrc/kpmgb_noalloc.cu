@@ -125,7 +125,12 @@ extern "C" int kpmgb_kpm1d_noalloc(int64_t NH, const int32_t* rowptr, const int3
   H.val = reinterpret_cast<double2*>(const_cast<double*>(val));
   H.is_real = 0;
   const size_t slot = (size_t)NH * NR * sizeof(double2);
-  const size_t part = step_partials_bytes(H, NH, (int)NR, KPMGB_PREC_FP64);
+  StepArgs a;
+  a.H = &H;
+  a.NH = NH;
+  a.NR = (int)NR;
+  size_t most = 0, part = 0;
+  KPMGB_TRY(recurrence_scratch_bytes(a, KPMGB_PREC_FP64, NC, false, &most, &part));
   const size_t need = kSyncBytes + 2 * align256(slot) + align256(part);
   if (need > kNoAllocScratchBytes)
     return fail(KPMGB_ERR_ARGUMENT,
@@ -139,37 +144,15 @@ extern "C" int kpmgb_kpm1d_noalloc(int64_t NH, const int32_t* rowptr, const int3
   unsigned* sync = reinterpret_cast<unsigned*>(b);
   void* sl[2] = {b + kSyncBytes, b + kSyncBytes + align256(slot)};
   void* partials = b + kSyncBytes + 2 * align256(slot);
-  // the ticket counter and the status word must start at zero
+  // the status word must start at zero
   KPMGB_CUDA(cudaMemsetAsync(sync, 0, kSyncBytes, s));
   KPMGB_TRY(launch_load_block(psi, sl[0], NH, (int)NR, KPMGB_PREC_FP64, nullptr, false, s));
-  StepArgs a;
-  a.H = &H;
-  a.NH = NH;
-  a.NR = (int)NR;
-  a.mu = reinterpret_cast<double2*>(mu_all);
-  a.sync = sync;
   a.partials = partials;
-  a.partials_bytes = part;  // the step kernels check their grid against it
-  a.x = sl[0];
-  a.y = sl[1];
-  a.alpha = 1.0;
-  a.beta = 0.0;
-  a.dot = DOT_DOUBLING;
-  a.mom = MOM_STORE;
-  a.i0 = 0;
-  KPMGB_TRY(launch_step(a, KPMGB_PREC_FP64, s));
-  int ip = 1, ipp = 0;
-  a.alpha = 2.0;
-  a.beta = -1.0;
-  for (int64_t n = 2; n <= NC / 2; ++n) {
-    a.x = sl[ip];
-    a.z = sl[ipp];
-    a.y = sl[ipp];
-    a.mom = MOM_DOUBLING;
-    a.i0 = 2 * n - 2;
-    KPMGB_TRY(launch_step(a, KPMGB_PREC_FP64, s));
-    std::swap(ip, ipp);
-  }
+  MomentArgs m;
+  m.mu = reinterpret_cast<double2*>(mu_all);
+  m.status = sync + 1;
+  const size_t room = kNoAllocScratchBytes - kSyncBytes - 2 * align256(slot);
+  KPMGB_TRY(launch_recurrence(a, KPMGB_PREC_FP64, NC, false, sl, std::min(most, room), m, s));
   unsigned status = 0;
   KPMGB_CUDA(cudaMemcpyAsync(&status, sync + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
   KPMGB_CUDA(cudaStreamSynchronize(s));

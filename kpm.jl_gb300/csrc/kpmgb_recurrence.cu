@@ -15,7 +15,8 @@
 //
 // Reductions are deterministic: warp shuffles, then a fixed-order sum over the
 // warps of a block, per-block partials in global memory, and a fixed-order
-// sum over blocks performed by the last block to finish (ticket counter).
+// sum over blocks by k_finish_moments, one launch for the steps whose
+// partials the scratch buffer holds.
 // The grid size is a pure function of the problem shape, so two identical
 // calls give bitwise-identical moments.
 #include <cuda_runtime.h>
@@ -225,35 +226,6 @@ int grid_packed(const PackedStep& ps, int64_t NH) {
 
 }  // namespace
 
-size_t step_partials_bytes(const DeviceCSR& H, int64_t NH, int NR, int precision) {
-  size_t worst = 0;
-  const int W = cols_per_launch();
-  for (int c0 = 0; c0 < NR; c0 += W) {
-    const int ncols = std::min(W, NR - c0);
-    for (const Shape& c : candidate_shapes(ncols))
-      for (int dot : {DOT_DOUBLING, DOT_LR2, DOT_LR1}) {
-        KernelFn fn = select_kernel(c, precision, dot, H.is_real != 0);
-        const int G = grid_for(fn, NH, c.lpr);
-        worst = std::max(worst, (size_t)G * 2 * ncols * sizeof(double2));
-      }
-    if (precision == KPMGB_PREC_FF) {
-      for (int dot : {DOT_DOUBLING, DOT_LR2, DOT_LR1}) {
-        if (KernelFn fe = select_kernel_ffe(ncols, dot, H.is_real != 0))
-          worst = std::max(worst, (size_t)grid_for(fe, NH, ffe_lanes(ncols)) * 2 * ncols *
-                                      sizeof(double2));
-        if (KernelFn fr = select_kernel_ffr(ncols, dot, H.is_real != 0, H.max_row_nnz, H.ell_w))
-          worst = std::max(worst, (size_t)grid_for(fr, NH, 32) * 2 * ncols * sizeof(double2));
-        if (KernelFn fc = select_kernel_ffc(ncols, dot, H.is_real != 0, H.ell_w, H.max_row_nnz))
-          worst = std::max(worst, (size_t)grid_for(fc, NH, ffc_lanes(ncols)) * 2 * ncols *
-                                      sizeof(double2));
-      }
-      const PackedStep ps = select_packed_step(ncols, H.is_real != 0, H.max_row_nnz, H.ell_w);
-      if (ps.fn) worst = std::max(worst, (size_t)grid_packed(ps, NH) * 2 * ncols * sizeof(double2));
-    }
-  }
-  return worst;
-}
-
 bool colpair_step_applies(const DeviceCSR& H, int NR) {
   return NR <= cols_per_launch() &&
          select_kernel_ffcp(NR, H.is_real != 0, H.ell_w, H.max_row_nnz) != nullptr;
@@ -264,18 +236,214 @@ bool packed_step_applies(const DeviceCSR& H, int NR) {
          select_kernel_ffpk(NR, H.is_real != 0, H.max_row_nnz, H.ell_w) != nullptr;
 }
 
+namespace {
+
+// The kernel of the step `a` for a launch of ncols columns, with its grid.
+struct StepChoice {
+  KernelFn fn = nullptr;
+  int grid = 0;
+  int threads = kThreads;
+  size_t smem = 0;
+};
+
+int choose_step(const StepArgs& a, int precision, int ncols, StepChoice* out) {
+  const DeviceCSR& H = *a.H;
+  auto take = [&](KernelFn fn, int lpr) {
+    *out = StepChoice{fn, grid_for(fn, a.NH, lpr)};
+    return KPMGB_OK;
+  };
+  const bool real = H.is_real != 0;
+  // Automatic selection for real operators with 33..64 columns per launch:
+  // the row-streaming kernel when rows hold at most 8 nonzeros (measured on
+  // GB300, 3D Anderson L=128, NR=64: 61.6% of the HBM roofline), else the
+  // padded-row kernel (43.5%; the CSR register-gather kernel 35.3%).
+  // Elsewhere the CSR kernel measured faster: complex Haldane 256x256,
+  // NR=16, kpm_2d 183 ms against 189 ms (exact-length last chunk); the
+  // L2-resident 2D Anderson L=64, NR=12, 7.4 ms against 8.3 ms per call
+  // (4 lanes x 3 columns against 16 x 1).
+  if (a.colpair) {
+    // the call keeps its vectors in the column-pair layout: only the
+    // column-pair kernel reads them
+    KernelFn fq = precision == KPMGB_PREC_FF && a.dot == DOT_NONE
+                      ? select_kernel_ffcp(ncols, real, H.ell_w, H.max_row_nnz)
+                      : nullptr;
+    if (!fq) return fail(KPMGB_ERR_CUDA, "internal: column-pair layout without its kernel");
+    return take(fq, ncols / 2);
+  }
+  if (a.paired) {
+    // the call keeps its vectors in the paired layout: only the packed
+    // kernel reads them
+    const PackedStep ps = precision == KPMGB_PREC_FF && a.dot == DOT_DOUBLING
+                              ? select_packed_step(ncols, real, H.max_row_nnz, H.ell_w)
+                              : PackedStep{};
+    if (!ps.fn) return fail(KPMGB_ERR_CUDA, "internal: paired layout without the packed kernel");
+    *out = StepChoice{ps.fn, grid_packed(ps, a.NH), ps.threads, ps.smem};
+    return KPMGB_OK;
+  }
+  if (a.variant == 11 && precision != KPMGB_PREC_FF)
+    return fail(KPMGB_ERR_ARGUMENT, "the row-streaming kernel is float-float only");
+  if (precision == KPMGB_PREC_FF && (a.variant == 11 || a.variant == 0)) {
+    if (KernelFn fr = select_kernel_ffr(ncols, a.dot, real, H.max_row_nnz, H.ell_w))
+      return take(fr, 32);
+    KernelFn fc = H.ell_w > 0 && (kStreamingComplex || a.variant == 11)
+                      ? select_kernel_ffc(ncols, a.dot, real, H.ell_w, H.max_row_nnz)
+                      : nullptr;
+    if (fc) return take(fc, ffc_lanes(ncols));
+    if (a.variant == 11)
+      return fail(KPMGB_ERR_ARGUMENT,
+                  "the row-streaming kernels serve float-float steps of real operators with "
+                  "33..64 columns and rows of 5..8 nonzeros, and of complex operators with "
+                  "9..32 columns and rows of 5..12 nonzeros");
+  }
+  const bool auto_padded =
+      a.variant == 0 && H.ell_w > 0 && ((real && ncols > 32) || padded_complex());
+  if (precision == KPMGB_PREC_FF && (a.variant == 9 || auto_padded)) {
+    KernelFn fe = H.ell_w > 0 ? select_kernel_ffe(ncols, a.dot, real) : nullptr;
+    if (fe) return take(fe, ffe_lanes(ncols));
+    if (a.variant == 9)
+      return fail(KPMGB_ERR_ARGUMENT, "the padded-row kernel serves float-float steps with 5..64 "
+                                      "columns and rows of at most 16 nonzeros");
+  }
+  const Shape sh = shape_for(a, ncols);
+  return take(select_kernel(sh, precision, a.dot, real), sh.lpr);
+}
+
+int num_dots(int dot) { return dot == DOT_NONE ? 0 : (dot == DOT_LR1 ? 1 : 2); }
+
+size_t partials_count(const StepArgs& a, const StepChoice& c, int ncols) {
+  return (size_t)c.grid * num_dots(a.dot) * ncols;
+}
+
+// A block adds the per-block sums of one step for up to 32 of its entries
+// (dot, column): the blocks in P interleaved parts of 4 accumulators each,
+// then the parts, always in the same order.
+struct FinishParams {
+  const double2* partials;
+  int64_t stride;  // double2 elements from step to step
+  int G;           // blocks per step
+  int nd, ncols, c0, ld;
+  MomentArgs m;
+};
+
+__global__ void __launch_bounds__(256) k_finish_moments(FinishParams f) {
+  __shared__ double2 part[256];
+  const int ne = f.nd * f.ncols;
+  const int e0 = blockIdx.y * 32;
+  const int E = min(32, ne - e0);
+  const int P = 256 / E;
+  const int q = threadIdx.x / E, e = threadIdx.x % E;
+  const double2* src = f.partials + (int64_t)blockIdx.x * f.stride + e0 + e;
+  if (q < P) {
+    double2 a[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) a[k] = make_double2(0.0, 0.0);
+    for (int b = q; b < f.G; b += 4 * P) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (b + k * P < f.G) {
+          const double2 v = src[(int64_t)(b + k * P) * ne];
+          a[k].x += v.x;
+          a[k].y += v.y;
+        }
+    }
+    part[threadIdx.x] = make_double2((a[0].x + a[1].x) + (a[2].x + a[3].x),
+                                     (a[0].y + a[1].y) + (a[2].y + a[3].y));
+  }
+  for (int w = 128; w > 0; w >>= 1) {
+    __syncthreads();
+    if (q < w && q + w < P) {
+      part[threadIdx.x].x += part[threadIdx.x + w * E].x;
+      part[threadIdx.x].y += part[threadIdx.x + w * E].y;
+    }
+  }
+  if (q != 0) return;
+  double2 s = part[e];
+  const int k = (e0 + e) / f.ncols;
+  const int cc = f.c0 + (e0 + e) % f.ncols;
+  if (f.m.scale) {
+    s.x *= f.m.scale[cc];
+    s.y *= f.m.scale[cc];
+  }
+  if (f.m.mom == MOM_DOUBLING) {
+    const double2 base = f.m.mu[(size_t)k * f.ld + cc];
+    if (k == 0 && f.m.growth_limit > 0.0 && !(s.x <= f.m.growth_limit * base.x))
+      atomicOr(f.m.status, (unsigned)STATUS_GROWTH);
+    s.x = 2.0 * s.x - base.x;
+    s.y = 2.0 * s.y - base.y;
+  }
+  f.m.mu[(size_t)(f.m.i0 + (int64_t)blockIdx.x * f.nd + k) * f.ld + cc] = s;
+  if (!isfinite(s.x) || !isfinite(s.y)) atomicOr(f.m.status, (unsigned)STATUS_NONFINITE);
+}
+
+}  // namespace
+
+int step_partials_bytes(const StepArgs& a, int precision, size_t* bytes) {
+  *bytes = 0;
+  const int W = cols_per_launch();
+  for (int c0 = 0; c0 < a.NR; c0 += W) {
+    const int ncols = std::min(W, a.NR - c0);
+    StepChoice c;
+    KPMGB_TRY(choose_step(a, precision, ncols, &c));
+    *bytes += partials_count(a, c, ncols) * sizeof(double2);
+  }
+  return KPMGB_OK;
+}
+
+namespace {
+
+// Adds the per-block sums of nsteps steps like `a` (consecutive runs of
+// step_partials_bytes at a.partials) in a fixed order and writes their moments.
+int launch_finish_moments(const StepArgs& a, int precision, int nsteps, const MomentArgs& m,
+                          cudaStream_t s) {
+  size_t bytes = 0;
+  KPMGB_TRY(step_partials_bytes(a, precision, &bytes));
+  FinishParams f;
+  f.partials = static_cast<const double2*>(a.partials);
+  f.stride = (int64_t)(bytes / sizeof(double2));
+  f.nd = num_dots(a.dot);
+  f.ld = a.NR;
+  f.m = m;
+  const int W = cols_per_launch();
+  for (int c0 = 0; c0 < a.NR; c0 += W) {
+    f.c0 = c0;
+    f.ncols = std::min(W, a.NR - c0);
+    StepChoice c;
+    KPMGB_TRY(choose_step(a, precision, f.ncols, &c));
+    f.G = c.grid;
+    k_finish_moments<<<dim3((unsigned)nsteps, (unsigned)((f.nd * f.ncols + 31) / 32)), 256, 0,
+                       s>>>(f);
+    KPMGB_LAUNCHED();
+    f.partials += partials_count(a, c, f.ncols);
+  }
+  return KPMGB_OK;
+}
+
+// The later steps of a recurrence: the doubling dots, or the one bra dot.
+StepArgs later_step(StepArgs a, bool lr) {
+  a.dot = lr ? DOT_LR1 : DOT_DOUBLING;
+  a.alpha = 2.0;
+  a.beta = -1.0;
+  return a;
+}
+
+int64_t later_steps(int64_t NC, bool lr) { return lr ? NC - 2 : NC / 2 - 1; }
+
+}  // namespace
+
 int launch_step(const StepArgs& a, int precision, cudaStream_t s) {
   const DeviceCSR& H = *a.H;
-  if (precision == KPMGB_PREC_FF) {
-    const double al = std::fabs(a.alpha);
-    int e = 0;
-    const double m = std::frexp(al, &e);
-    if (!(m == 0.5) || !(a.beta == 0.0 || a.beta == 1.0 || a.beta == -1.0))
-      return fail(KPMGB_ERR_ARGUMENT,
-                  "float-float recurrence supports alpha = +-2^k and beta in {-1, 0, 1}");
-    if (!H.val_ff) return fail(KPMGB_ERR_ARGUMENT, "operator has no float-float values");
-  }
+  const double al = std::fabs(a.alpha);
+  int e = 0;
+  const double m = std::frexp(al, &e);
+  if (!(m == 0.5) || !(a.beta == 0.0 || a.beta == -1.0))
+    return fail(KPMGB_ERR_ARGUMENT,
+                "the recurrence step supports alpha = +-2^k and beta in {-1, 0}");
+  if (precision == KPMGB_PREC_FF && !H.val_ff)
+    return fail(KPMGB_ERR_ARGUMENT, "operator has no float-float values");
   const int W = cols_per_launch();
+  double2* partials = static_cast<double2*>(a.partials);
+  if (a.dot != DOT_NONE && !partials)
+    return fail(KPMGB_ERR_CUDA, "internal: a step with dots needs its partial sums");
   for (int c0 = 0; c0 < a.NR; c0 += W) {
     KParams p;
     p.rowptr = H.rowptr;
@@ -291,95 +459,87 @@ int launch_step(const StepArgs& a, int precision, cudaStream_t s) {
     p.y = a.y;
     p.bra = a.bra;
     p.alpha = a.alpha;
-    p.beta = a.beta;
-    p.mom = a.mom;
-    p.i0 = a.i0;
-    p.mu = a.mu;
-    p.mom_scale = a.mom_scale;
-    p.growth_limit = a.growth_limit;
-    p.sync = a.sync;
+    p.partials = partials;
     p.vmax = a.vmax;
-    p.partials = static_cast<double2*>(a.partials);
-    p.partials_cap = (int64_t)(a.partials_bytes / sizeof(double2));
     p.ell_col = H.ell_col;
     p.ell_val = H.ell_val;
     p.ell_w = H.ell_w;
     p.alpha_f = (float)a.alpha;
-    p.beta_mode = a.beta == 0.0 ? 0 : (a.beta > 0.0 ? 1 : -1);
-    // Automatic selection for real operators with 33..64 columns per launch:
-    // the row-streaming kernel when rows hold at most 8 nonzeros (measured on
-    // GB300, 3D Anderson L=128, NR=64: 61.6% of the HBM roofline), else the
-    // padded-row kernel (43.5%; the CSR register-gather kernel 35.3%).
-    // Elsewhere the CSR kernel measured faster: complex Haldane 256x256,
-    // NR=16, kpm_2d 183 ms against 189 ms (exact-length last chunk); the
-    // L2-resident 2D Anderson L=64, NR=12, 7.4 ms against 8.3 ms per call
-    // (4 lanes x 3 columns against 16 x 1).
-    if (a.colpair) {
-      // the call keeps its vectors in the column-pair layout: only the
-      // column-pair kernel reads them
-      KernelFn fq = precision == KPMGB_PREC_FF && a.dot == DOT_NONE
-                        ? select_kernel_ffcp(p.ncols, H.is_real != 0, H.ell_w, H.max_row_nnz)
-                        : nullptr;
-      if (!fq) return fail(KPMGB_ERR_CUDA, "internal: column-pair layout without its kernel");
-      KPMGB_TRY(launch_step_kernel(fq, grid_for(fq, a.NH, p.ncols / 2), s, p));
-      continue;
-    }
-    if (a.paired) {
-      // the call keeps its vectors in the paired layout: only the packed
-      // kernel reads them
-      const PackedStep ps =
-          precision == KPMGB_PREC_FF && a.dot == DOT_DOUBLING
-              ? select_packed_step(p.ncols, H.is_real != 0, H.max_row_nnz, H.ell_w)
-              : PackedStep{};
-      if (!ps.fn) return fail(KPMGB_ERR_CUDA, "internal: paired layout without the packed kernel");
-      KPMGB_TRY(launch_step_kernel(ps.fn, grid_packed(ps, a.NH), s, p, ps.threads, ps.smem));
-      continue;
-    }
-    if (a.variant == 11 && precision != KPMGB_PREC_FF)
-      return fail(KPMGB_ERR_ARGUMENT, "the row-streaming kernel is float-float only");
-    if (precision == KPMGB_PREC_FF && (a.variant == 11 || a.variant == 0)) {
-      KernelFn fr = select_kernel_ffr(p.ncols, a.dot, H.is_real != 0, H.max_row_nnz, H.ell_w);
-      if (fr) {
-        KPMGB_TRY(launch_step_kernel(fr, grid_for(fr, a.NH, 32), s, p));
-        continue;
-      }
-      KernelFn fc = H.ell_w > 0 && kStreamingComplex
-                        ? select_kernel_ffc(p.ncols, a.dot, H.is_real != 0, H.ell_w, H.max_row_nnz)
-                        : nullptr;
-      if (a.variant == 11 && !fc && H.ell_w > 0)
-        fc = select_kernel_ffc(p.ncols, a.dot, H.is_real != 0, H.ell_w, H.max_row_nnz);
-      if (fc) {
-        KPMGB_TRY(launch_step_kernel(fc, grid_for(fc, a.NH, ffc_lanes(p.ncols)), s, p));
-        continue;
-      }
-      if (a.variant == 11)
-        return fail(KPMGB_ERR_ARGUMENT,
-                    "the row-streaming kernels serve float-float steps of real operators with "
-                    "33..64 columns and rows of 5..8 nonzeros, and of complex operators with "
-                    "9..32 columns and rows of 5..12 nonzeros");
-    }
-    const bool auto_padded = a.variant == 0 && H.ell_w > 0 &&
-                             ((H.is_real && p.ncols > 32) || padded_complex());
-    if (precision == KPMGB_PREC_FF && (a.variant == 9 || auto_padded)) {
-      KernelFn fe = H.ell_w > 0 ? select_kernel_ffe(p.ncols, a.dot, H.is_real != 0) : nullptr;
-      if (fe || a.variant == 9) {
-        if (!fe)
-          return fail(KPMGB_ERR_ARGUMENT,
-                      "the padded-row kernel serves float-float steps with 5..64 columns "
-                      "and rows of at most 16 nonzeros");
-        KPMGB_TRY(launch_step_kernel(fe, grid_for(fe, a.NH, ffe_lanes(p.ncols)), s, p));
-        continue;
-      }
-    }
-    const Shape sh = shape_for(a, p.ncols);
-    KernelFn fn = select_kernel(sh, precision, a.dot, H.is_real != 0);
-    const int G = grid_for(fn, a.NH, sh.lpr);
-    KPMGB_TRY(launch_step_kernel(fn, G, s, p));
+    p.beta_mode = a.beta == 0.0 ? 0 : -1;
+    StepChoice c;
+    KPMGB_TRY(choose_step(a, precision, p.ncols, &c));
+    KPMGB_TRY(launch_step_kernel(c.fn, c.grid, s, p, c.threads, c.smem));
+    if (partials) partials += partials_count(a, c, p.ncols);
   }
   return KPMGB_OK;
 }
 
-int tune_step(const StepArgs& a0, int precision, cudaStream_t s, int* variant, int* shape) {
+int recurrence_scratch_bytes(const StepArgs& a0, int precision, int64_t NC, bool lr,
+                             size_t* bytes, size_t* least) {
+  // 32 MiB of block sums stay in L2 and cover 25 steps of the widest grids
+  // and hundreds of the narrow ones, so that the finishing launch (a few us)
+  // costs well under 1% of the steps it serves
+  constexpr size_t kHeldBytes = size_t(32) << 20;
+  StepArgs a = a0;
+  a.dot = lr ? DOT_LR2 : DOT_DOUBLING;
+  size_t first = 0, step = 0;
+  KPMGB_TRY(step_partials_bytes(a, precision, &first));
+  KPMGB_TRY(step_partials_bytes(later_step(a, lr), precision, &step));
+  const size_t n = (size_t)std::max<int64_t>(1, later_steps(NC, lr));
+  *bytes = std::max(first, step * std::max<size_t>(1, std::min(n, kHeldBytes / step)));
+  if (least) *least = std::max(first, step);
+  return KPMGB_OK;
+}
+
+int launch_recurrence(StepArgs a, int precision, int64_t NC, bool lr, void* const (&slot)[2],
+                      size_t held, MomentArgs m, cudaStream_t s) {
+  // alpha_1 = H alpha_0 with mu_0, mu_1 (src/moment.jl:440-449, :521-527)
+  a.dot = lr ? DOT_LR2 : DOT_DOUBLING;
+  a.x = slot[0];
+  a.z = nullptr;
+  a.y = slot[1];
+  a.alpha = 1.0;
+  a.beta = 0.0;
+  KPMGB_TRY(launch_step(a, precision, s));
+  const double growth = m.growth_limit;
+  m.mom = MOM_STORE;
+  m.i0 = 0;
+  m.growth_limit = 0.0;
+  KPMGB_TRY(launch_finish_moments(a, precision, 1, m, s));
+  // alpha_n = 2 H alpha_{n-1} - alpha_{n-2} in place: doubling moments
+  // mu_{2n-2}, mu_{2n-1} (src/moment.jl:460-487), or mu_n = <psil|alpha_n>
+  // (src/moment.jl:540-549)
+  const int64_t later = later_steps(NC, lr);
+  if (later < 1) return KPMGB_OK;
+  StepArgs b = later_step(a, lr);
+  char* const base = static_cast<char*>(a.partials);
+  size_t step_bytes = 0;
+  KPMGB_TRY(step_partials_bytes(b, precision, &step_bytes));
+  const int64_t hold = std::max<int64_t>(1, std::min<int64_t>(later, (int64_t)(held / step_bytes)));
+  m.mom = lr ? MOM_STORE : MOM_DOUBLING;
+  m.i0 = 2;
+  m.growth_limit = growth;
+  int ip = 1;
+  int64_t n = 0;
+  for (int64_t i = 0; i < later; ++i) {
+    b.partials = base + n * step_bytes;
+    b.x = slot[ip];
+    b.z = slot[ip ^ 1];
+    b.y = slot[ip ^ 1];
+    KPMGB_TRY(launch_step(b, precision, s));
+    ip ^= 1;
+    if (++n == hold || i + 1 == later) {
+      b.partials = base;
+      KPMGB_TRY(launch_finish_moments(b, precision, (int)n, m, s));
+      m.i0 += n * (lr ? 1 : 2);
+      n = 0;
+    }
+  }
+  return KPMGB_OK;
+}
+
+int tune_step(const StepArgs& a0, int precision, DevBuf& partials, cudaStream_t s, int* variant,
+              int* shape) {
   *variant = 1;
   *shape = 0;
   if (a0.NR > kMaxCols) return KPMGB_OK;  // several column batches: keep the default
@@ -408,6 +568,13 @@ int tune_step(const StepArgs& a0, int precision, cudaStream_t s, int* variant, i
     StepArgs a = a0;
     a.variant = c.variant;
     a.shape = c.shape;
+    size_t bytes = 0;
+    if (step_partials_bytes(a, precision, &bytes) != KPMGB_OK ||
+        partials.ensure(std::max(bytes, partials.bytes)) != KPMGB_OK) {
+      clear_error();
+      continue;
+    }
+    a.partials = partials.ptr;
     if (launch_step(a, precision, s) != KPMGB_OK) {
       clear_error();
       continue;

@@ -103,20 +103,13 @@ struct KParams {
   const void* z;
   void* y;
   const void* bra;
-  double alpha, beta;
-  int mom;
-  int64_t i0;
-  double2* mu;
-  const double* mom_scale;
-  double growth_limit;
-  unsigned* sync;
-  double2* partials;
-  int64_t partials_cap;  // capacity in double2 elements (0: unchecked)
+  double alpha;          // +-2^k
+  double2* partials;     // [block][dots][ncols] sums of this launch (null: none)
   // fixed-width padded rows (k_step_ffe): NH x ell_w columns / values
   const int* ell_col;
   const void* ell_val;
   int ell_w;
-  // alpha as a float and the sign of beta (0, 1, -1), set on the host so that
+  // alpha as a float and beta (0 or -1), set on the host so that
   // the float-float kernels execute no FP64 instruction per row
   float alpha_f;
   int beta_mode;
@@ -131,121 +124,151 @@ struct NDots {
 };
 
 // ------------------------------------------------------------------ reduction
-// Sum per-lane dot accumulators over the grid and write the moments.
-// NW warps per block (all of them reach this point; warps that own no rows
-// pass zero accumulators).
-template <int ND, int LPR, int CPL, int NW = kWarps>
-__device__ __forceinline__ void reduce_finalize(double2 (&d)[ND > 0 ? ND : 1][CPL],
-                                                const KParams& p) {
-  constexpr int THREADS = NW * 32;
-  if constexpr (ND == 0) {
-    return;
-  } else {
-    __shared__ double2 red[NW][ND][LPR * CPL];
-    __shared__ double2 tmp[THREADS];  // the last block's part sums
-    __shared__ unsigned s_ticket;
-    const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
+// Every block stores its sums of the dots at partials[block][dot][column];
+// k_finish_moments (kpmgb_recurrence.cu) adds the blocks of many steps at
+// once.  A step that added its blocks itself, in the block that finished
+// last, spent ~20 us on that block's serial FP64 additions (two FP64
+// additions per clock and SM: 304 blocks x 128 entries, or 1216 x 16) while
+// the other SMs idled: NH = 13824, NR = 64 float-float 44.8 us per step.
+
+// Butterfly over the lane offsets 16 .. LPR of V values per lane in which the
+// lanes of a pair each take half of the values, so that a level costs half of
+// the additions of the one before (an FP64 addition occupies an SM's FP64
+// pipe for 16 clocks per warp).  Afterwards value base + i, i < count, of the
+// lane's column is v[i]; add(a, b) merges.
+template <int V, int LPR, int OFF = 16, bool MORE = (OFF >= LPR)>
+struct Fold {  // values per lane afterwards
+  static constexpr int count = Fold<(V > 1 && V % 2 == 0 ? V / 2 : V), LPR, OFF / 2>::count;
+};
+template <int V, int LPR, int OFF>
+struct Fold<V, LPR, OFF, false> {
+  static constexpr int count = V;
+};
+
+template <int V, int LPR, typename T, typename Shfl, typename Add>
+__device__ __forceinline__ int lane_fold(T (&v)[V], int lane, Shfl shfl, Add add) {
+  int base = 0, cnt = V;
 #pragma unroll
-    for (int off = LPR; off < 32; off <<= 1) {
+  for (int off = 16; off >= LPR; off >>= 1) {
+    if (cnt > 1 && cnt % 2 == 0) {
+      const int h = cnt / 2;
+      const bool up = (lane & off) != 0;
 #pragma unroll
-      for (int k = 0; k < ND; ++k)
-#pragma unroll
-        for (int c = 0; c < CPL; ++c) {
-          d[k][c].x += __shfl_xor_sync(0xffffffffu, d[k][c].x, off);
-          d[k][c].y += __shfl_xor_sync(0xffffffffu, d[k][c].y, off);
+      for (int i = 0; i < V / 2; ++i)
+        if (i < h) {
+          const T keep = up ? v[i + h] : v[i];
+          const T send = up ? v[i] : v[i + h];
+          v[i] = add(keep, shfl(send, off));
         }
+      base += up ? h : 0;
+      cnt = h;
+    } else {
+#pragma unroll
+      for (int i = 0; i < V; ++i)
+        if (i < cnt) v[i] = add(v[i], shfl(v[i], off));
     }
-    if (lane < LPR) {
-#pragma unroll
-      for (int k = 0; k < ND; ++k)
-#pragma unroll
-        for (int c = 0; c < CPL; ++c) red[warp][k][lane + c * LPR] = d[k][c];
-    }
-    __syncthreads();
-    const int NE = ND * p.ncols;
-    // the partial sums of every block must fit the scratch buffer
-    if (p.partials_cap > 0 && (int64_t)gridDim.x * NE > p.partials_cap) {
-      if (threadIdx.x == 0 && blockIdx.x == 0) atomicOr(&p.sync[1], (unsigned)STATUS_SCRATCH);
-      return;
-    }
-    for (int e = threadIdx.x; e < NE; e += THREADS) {
-      const int k = e / p.ncols, c = e - k * p.ncols;
-      double2 s = make_double2(0.0, 0.0);
-#pragma unroll
-      for (int w = 0; w < NW; ++w) {
-        s.x += red[w][k][c].x;
-        s.y += red[w][k][c].y;
-      }
-      p.partials[(size_t)blockIdx.x * NE + e] = s;
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) s_ticket = atomicAdd(&p.sync[0], 1u);
-    __syncthreads();
-    if (s_ticket != gridDim.x - 1) return;
-    __threadfence();
-    // Last block: fixed-order sum over blocks.  All threads take part: the
-    // blocks are split into P = THREADS / NE interleaved parts, each summed
-    // with kAcc interleaved accumulators (kAcc loads in flight per thread:
-    // the partials come from L2, and one block reads them all), then the
-    // accumulators and the parts are added in a fixed order, so the result
-    // does not depend on which block finished last.
-    constexpr int kAcc = 8;
-    const int P = max(1, THREADS / NE);
-    const int G = (int)gridDim.x;
-    for (int idx = threadIdx.x; idx < P * NE; idx += THREADS) {
-      const int part = idx / NE, e = idx - part * NE;
-      double2 sa[kAcc];
-#pragma unroll
-      for (int q = 0; q < kAcc; ++q) sa[q] = make_double2(0.0, 0.0);
-      for (int b = part; b < G; b += kAcc * P) {
-#pragma unroll
-        for (int q = 0; q < kAcc; ++q) {
-          const int bq = b + q * P;
-          if (bq < G) {
-            const double2 v = __ldcg(p.partials + (size_t)bq * NE + e);
-            sa[q].x += v.x;
-            sa[q].y += v.y;
-          }
-        }
-      }
-#pragma unroll
-      for (int w = kAcc / 2; w > 0; w >>= 1)
-#pragma unroll
-        for (int q = 0; q < w; ++q) {
-          sa[q].x += sa[q + w].x;
-          sa[q].y += sa[q + w].y;
-        }
-      tmp[part * NE + e] = sa[0];
-    }
-    __syncthreads();
-    for (int ee = threadIdx.x; ee < NE; ee += THREADS) {
-      double2 s = make_double2(0.0, 0.0);
-      for (int q = 0; q < P; ++q) {
-        s.x += tmp[q * NE + ee].x;
-        s.y += tmp[q * NE + ee].y;
-      }
-      const int k = ee / p.ncols, c = ee - k * p.ncols;
-      const int cc = p.c0 + c;
-      if (p.mom_scale) {
-        const double f = p.mom_scale[cc];
-        s.x *= f;
-        s.y *= f;
-      }
-      double2 out = s;
-      if (p.mom == MOM_DOUBLING) {
-        const double2 base = p.mu[(size_t)k * p.ld + cc];
-        out.x = 2.0 * s.x - base.x;
-        out.y = 2.0 * s.y - base.y;
-        if (k == 0 && p.growth_limit > 0.0 && !(s.x <= p.growth_limit * base.x))
-          atomicOr(&p.sync[1], (unsigned)STATUS_GROWTH);
-      }
-      if (p.mom != MOM_NONE) p.mu[(size_t)(p.i0 + k) * p.ld + cc] = out;
-      if (!isfinite(out.x) || !isfinite(out.y)) atomicOr(&p.sync[1], (unsigned)STATUS_NONFINITE);
-    }
-    if (threadIdx.x == 0) p.sync[0] = 0u;
   }
+  return base;
+}
+
+__device__ __forceinline__ float2 ff_merge(float2 a, float2 b) {
+  float s, e;
+  ff::two_sum(a.x, b.x, s, e);
+  return make_float2(s, __fadd_rn(a.y, __fadd_rn(b.y, e)));
+}
+
+// Shared memory of the two reductions below (a kernel that holds both uses
+// one buffer).
+template <int DOUBLES>
+__device__ __forceinline__ double* red_buffer() {
+  __shared__ __align__(16) double red[DOUBLES];
+  return red;
+}
+
+// Block sums of FP64 dot accumulators (all warps of the block reach this
+// point; warps that own no rows pass zeros), fixed order.
+template <int ND, int LPR, int CPL, int NW = kWarps>
+__device__ __forceinline__ void block_dots(const double2 (&d)[ND > 0 ? ND : 1][CPL],
+                                           const KParams& p) {
+  if constexpr (ND > 0) {
+    constexpr int V = ND * CPL * 2;
+    double(*red)[V * LPR] = reinterpret_cast<double(*)[V * LPR]>(red_buffer<NW * V * LPR>());
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double v[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i)
+      v[i] = i & 1 ? d[i / (2 * CPL)][i / 2 % CPL].y : d[i / (2 * CPL)][i / 2 % CPL].x;
+    const int base = lane_fold<V, LPR>(
+        v, lane, [](double a, int off) { return __shfl_xor_sync(0xffffffffu, a, off); },
+        [](double a, double b) { return a + b; });
+    constexpr int kLeft = Fold<V, LPR>::count;
+#pragma unroll
+    for (int i = 0; i < kLeft; ++i)
+      red[warp][(base + i) * LPR + lane % LPR] = v[i];
+    __syncthreads();
+    const int n = 2 * ND * p.ncols;
+    double* out = reinterpret_cast<double*>(p.partials) + (size_t)blockIdx.x * n;
+    for (int e = threadIdx.x; e < n; e += NW * 32) {
+      const int k = e / (2 * p.ncols), col = (e >> 1) % p.ncols;
+      const int at = ((k * CPL + col / LPR) * 2 + (e & 1)) * LPR + col % LPR;
+      double s = 0.0;
+#pragma unroll
+      for (int w = 0; w < NW; ++w) s += red[w][at];
+      out[e] = s;
+    }
+  }
+}
+
+// The same for float-float accumulators (leading S, correction C; NP = 1: real
+// parts only) that hold at most kFlushRows rows per lane: merged by TwoSum
+// over lanes and warps, and joined into FP64 once per entry of the block
+// (two conversions and an addition per lane and value otherwise, 48 clocks of
+// the SM's FP64 pipe per warp and value).
+template <int ND, int LPR, int CPL, int NP, int NW = kWarps>
+__device__ __forceinline__ void block_dots_ff(const float2 (&d)[ND > 0 ? ND : 1][CPL][NP],
+                                              const KParams& p) {
+  if constexpr (ND > 0) {
+    constexpr int V = ND * CPL * NP;
+    float2(*red)[V * LPR] =
+        reinterpret_cast<float2(*)[V * LPR]>(red_buffer<NW * ND * CPL * 2 * LPR>());
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float2 v[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) v[i] = d[i / (NP * CPL)][i / NP % CPL][i % NP];
+    const int base = lane_fold<V, LPR>(
+        v, lane,
+        [](float2 a, int off) {
+          return make_float2(__shfl_xor_sync(0xffffffffu, a.x, off),
+                             __shfl_xor_sync(0xffffffffu, a.y, off));
+        },
+        [](float2 a, float2 b) { return ff_merge(a, b); });
+    constexpr int kLeft = Fold<V, LPR>::count;
+#pragma unroll
+    for (int i = 0; i < kLeft; ++i)
+      red[warp][(base + i) * LPR + lane % LPR] = v[i];
+    __syncthreads();
+    const int n = ND * p.ncols;
+    double2* out = p.partials + (size_t)blockIdx.x * n;
+    for (int e = threadIdx.x; e < n; e += NW * 32) {
+      const int k = e / p.ncols, col = e % p.ncols;
+      double r[2] = {0.0, 0.0};
+#pragma unroll
+      for (int q = 0; q < NP; ++q) {
+        const int at = ((k * CPL + col / LPR) * NP + q) * LPR + col % LPR;
+        float2 s = red[0][at];
+#pragma unroll
+        for (int w = 1; w < NW; ++w) s = ff_merge(s, red[w][at]);
+        r[q] = ff::join(s.x, s.y);
+      }
+      out[e] = make_double2(r[0], r[1]);
+    }
+  }
+}
+
+// Whether any lane of the grid has folded its float-float accumulators into
+// FP64 (a lane does so every kFlushRows row tiles).
+__device__ __forceinline__ bool any_flush(int64_t ntiles, int flush_rows) {
+  return (ntiles + gridDim.x - 1) / gridDim.x >= flush_rows;
 }
 
 // ------------------------------------------------------------------ FP64 path
@@ -321,11 +344,14 @@ __global__ void __launch_bounds__(kThreads) k_step_f64(KParams p) {
     for (int c = 0; c < CPL; ++c) {
       const int cc = lg + c * LPR;
       if (cc >= p.ncols) continue;
-      double2 yv = make_double2(p.alpha * acc[c].x, p.alpha * acc[c].y);
-      if (p.beta != 0.0) {
+      double2 yv = acc[c];
+      if (p.beta_mode != 0) {  // alpha is a power of two: one rounding, as alpha acc, then - z
         const double2 zv = z[base + cc];
-        yv.x = fma(p.beta, zv.x, yv.x);
-        yv.y = fma(p.beta, zv.y, yv.y);
+        yv.x = fma(p.alpha, yv.x, -zv.x);
+        yv.y = fma(p.alpha, yv.y, -zv.y);
+      } else if (p.alpha != 1.0) {
+        yv.x *= p.alpha;
+        yv.y *= p.alpha;
       }
       y[base + cc] = yv;
       if constexpr (DOT == DOT_DOUBLING) {
@@ -342,7 +368,7 @@ __global__ void __launch_bounds__(kThreads) k_step_f64(KParams p) {
       }
     }
   }
-  reduce_finalize<ND, LPR, CPL>(d, p);
+  block_dots<ND, LPR, CPL>(d, p);
 }
 
 // ------------------------------------------------------------ float-float path
@@ -375,7 +401,8 @@ __device__ __forceinline__ void ffmac(float& Ar, float& Cr, float& Ai, float& Ci
   ff::amac(Ai, Ci, h.z, h.w, v.x, v.y);
 }
 
-// y = alpha * (S + C) + beta * z for one real component, normalised.
+// y = alpha * (S + C) - z (beta_mode -1) or without z (0) for one real
+// component, normalised.
 __device__ __forceinline__ float2 ff_epilogue(float S, float C, float alpha, int beta_mode,
                                               float zh, float zl) {
   const float u = __fmul_rn(alpha, S);  // alpha is a power of two: exact
@@ -384,11 +411,9 @@ __device__ __forceinline__ float2 ff_epilogue(float S, float C, float alpha, int
   if (beta_mode == 0) {
     ff::renorm(u, c, h, l);
   } else {
-    const float zs = beta_mode > 0 ? zh : -zh;
-    const float zt = beta_mode > 0 ? zl : -zl;
     float s, e;
-    ff::two_sum(u, zs, s, e);
-    ff::renorm(s, __fadd_rn(e, __fadd_rn(c, zt)), h, l);
+    ff::two_sum(u, -zh, s, e);
+    ff::renorm(s, __fadd_rn(e, __fsub_rn(c, zl)), h, l);
   }
   return make_float2(h, l);
 }
@@ -673,16 +698,27 @@ __global__ void __launch_bounds__(kThreads, (FFTune<CPL, REALH>::min_blocks)) k_
     }
   }
   if constexpr (ND > 0) {
+    if (any_flush(ntiles, kFlushRows)) {
 #pragma unroll
-    for (int k = 0; k < ND; ++k)
+      for (int k = 0; k < ND; ++k)
 #pragma unroll
-      for (int c = 0; c < CPL; ++c) {
-        if constexpr (kSmemAcc) d[k][c] = sacc[threadIdx.x][k * CPL + c];
-        d[k][c].x += ff::join(dS[k][c][0], dC[k][c][0]);
-        d[k][c].y += ff::join(dS[k][c][1], dC[k][c][1]);
-      }
+        for (int c = 0; c < CPL; ++c) {
+          if constexpr (kSmemAcc) d[k][c] = sacc[threadIdx.x][k * CPL + c];
+          d[k][c].x += ff::join(dS[k][c][0], dC[k][c][0]);
+          d[k][c].y += ff::join(dS[k][c][1], dC[k][c][1]);
+        }
+      block_dots<ND, LPR, CPL>(d, p);
+    } else {
+      float2 f[NDA][CPL][2];
+#pragma unroll
+      for (int k = 0; k < ND; ++k)
+#pragma unroll
+        for (int c = 0; c < CPL; ++c)
+#pragma unroll
+          for (int q = 0; q < 2; ++q) f[k][c][q] = make_float2(dS[k][c][q], dC[k][c][q]);
+      block_dots_ff<ND, LPR, CPL, 2>(f, p);
+    }
   }
-  reduce_finalize<ND, LPR, CPL>(d, p);
 }
 
 struct Shape {

@@ -200,16 +200,27 @@ __global__ void __launch_bounds__(kThreads, KPMGB_FFE_MIN_BLOCKS) k_step_ffe(KPa
     }
   }
   if constexpr (ND > 0) {
+    if (any_flush(ntiles, kFlushRows)) {
 #pragma unroll
-    for (int k = 0; k < ND; ++k)
+      for (int k = 0; k < ND; ++k)
 #pragma unroll
-      for (int c = 0; c < CPL; ++c) {
-        if constexpr (kSmemAcc) d[k][c] = sacc[threadIdx.x][k * CPL + c];
-        d[k][c].x += ff::join(dS[k][c][0], dC[k][c][0]);
-        d[k][c].y += ff::join(dS[k][c][1], dC[k][c][1]);
-      }
+        for (int c = 0; c < CPL; ++c) {
+          if constexpr (kSmemAcc) d[k][c] = sacc[threadIdx.x][k * CPL + c];
+          d[k][c].x += ff::join(dS[k][c][0], dC[k][c][0]);
+          d[k][c].y += ff::join(dS[k][c][1], dC[k][c][1]);
+        }
+      block_dots<ND, LPR, CPL>(d, p);
+    } else {
+      float2 f[NDA][CPL][2];
+#pragma unroll
+      for (int k = 0; k < ND; ++k)
+#pragma unroll
+        for (int c = 0; c < CPL; ++c)
+#pragma unroll
+          for (int q = 0; q < 2; ++q) f[k][c][q] = make_float2(dS[k][c][q], dC[k][c][q]);
+      block_dots_ff<ND, LPR, CPL, 2>(f, p);
+    }
   }
-  reduce_finalize<ND, LPR, CPL>(d, p);
 }
 
 namespace {
@@ -401,16 +412,28 @@ __global__ void __launch_bounds__(kThreads, 2) k_step_ffr(KParams p) {
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   if constexpr (ND > 0) {
-    double2 d[NDA][CPL];
+    if (any_flush(ntiles, kFlushRows)) {
+      double2 d[NDA][CPL];
 #pragma unroll
-    for (int k = 0; k < ND; ++k)
+      for (int k = 0; k < ND; ++k)
 #pragma unroll
-      for (int c = 0; c < CPL; ++c) {
-        d[k][c] = sacc[threadIdx.x][k * CPL + c];
-        d[k][c].x += ff::join(dS[k][c][0], dC[k][c][0]);
-        if (!(DOT == DOT_DOUBLING && k == 1)) d[k][c].y += ff::join(dS[k][c][1], dC[k][c][1]);
-      }
-    reduce_finalize<ND, 32, CPL>(d, p);
+        for (int c = 0; c < CPL; ++c) {
+          d[k][c] = sacc[threadIdx.x][k * CPL + c];
+          d[k][c].x += ff::join(dS[k][c][0], dC[k][c][0]);
+          if (!(DOT == DOT_DOUBLING && k == 1)) d[k][c].y += ff::join(dS[k][c][1], dC[k][c][1]);
+        }
+      block_dots<ND, 32, CPL>(d, p);
+    } else {
+      constexpr int NP = DOT == DOT_DOUBLING ? 1 : 2;
+      float2 f[NDA][CPL][NP];
+#pragma unroll
+      for (int k = 0; k < ND; ++k)
+#pragma unroll
+        for (int c = 0; c < CPL; ++c)
+#pragma unroll
+          for (int q = 0; q < NP; ++q) f[k][c][q] = make_float2(dS[k][c][q], dC[k][c][q]);
+      block_dots_ff<ND, 32, CPL, NP>(f, p);
+    }
   }
 }
 
@@ -570,14 +593,24 @@ __global__ void __launch_bounds__(kThreads, 2) k_step_ffc(KParams p) {
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   if constexpr (ND > 0) {
-    double2 d[NDA][1];
+    if (any_flush(ntiles, kFlushRows)) {
+      double2 d[NDA][1];
 #pragma unroll
-    for (int k = 0; k < ND; ++k) {
-      d[k][0] = sacc[threadIdx.x][k];
-      d[k][0].x += ff::join(dS[k][0], dC[k][0]);
-      if (!(DOT == DOT_DOUBLING && k == 1)) d[k][0].y += ff::join(dS[k][1], dC[k][1]);
+      for (int k = 0; k < ND; ++k) {
+        d[k][0] = sacc[threadIdx.x][k];
+        d[k][0].x += ff::join(dS[k][0], dC[k][0]);
+        if (!(DOT == DOT_DOUBLING && k == 1)) d[k][0].y += ff::join(dS[k][1], dC[k][1]);
+      }
+      block_dots<ND, LPR, 1>(d, p);
+    } else {
+      constexpr int NP = DOT == DOT_DOUBLING ? 1 : 2;
+      float2 f[NDA][1][NP];
+#pragma unroll
+      for (int k = 0; k < ND; ++k)
+#pragma unroll
+        for (int q = 0; q < NP; ++q) f[k][0][q] = make_float2(dS[k][q], dC[k][q]);
+      block_dots_ff<ND, LPR, 1, NP>(f, p);
     }
-    reduce_finalize<ND, LPR, 1>(d, p);
   }
 }
 
