@@ -796,10 +796,8 @@ int launch_ensemble_steps(const DeviceCSR& H, const EnsembleArgs& e, EnsParams p
                              cudaMemcpyHostToDevice, s));
   KPMGB_CUDA(cudaMemsetAsync(q.ticket, 0, (size_t)nseg * sizeof(unsigned), s));
   void* fn = pick_ensemble_step(ff, H.is_real != 0, ell, p.NR, H.max_row_nnz);
-  // programmatic dependent launch on created streams: step n+1's CTAs are
-  // scheduled while step n drains and wait (griddepcontrol.wait) for its
-  // completion
-  const bool pdl = s != nullptr && s != cudaStreamLegacy && s != cudaStreamPerThread;
+  // programmatic dependent launch: step n+1's CTAs are scheduled while step n
+  // drains and wait (griddepcontrol.wait) for its completion
   for (int64_t n = 1; n <= p.NC / 2; ++n) {
     q.n = (int)n;
     void* args[] = {&p, &q};
@@ -811,7 +809,7 @@ int launch_ensemble_steps(const DeviceCSR& H, const EnsembleArgs& e, EnsParams p
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = 1;
     KPMGB_CUDA(cudaLaunchKernelExC(&cfg, fn, args));
     KPMGB_LAUNCHED();
   }

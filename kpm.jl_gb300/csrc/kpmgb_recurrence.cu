@@ -135,30 +135,41 @@ int blocks_per_sm(KernelFn fn) {
   return per_sm;
 }
 
+// The kernel of a step for a launch of some columns, with its grid.
+struct StepChoice {
+  KernelFn fn = nullptr;
+  int grid = 0;
+  int threads = kThreads;
+  size_t smem = 0;
+  bool pdl = true;
+};
+
 // Step kernels launch with programmatic stream serialization (see pdl_enter)
-// on created streams; KPMGB_PDL=0 in the environment turns it off.
-int launch_step_kernel(KernelFn fn, int G, cudaStream_t s, const KParams& p,
-                       int threads = kThreads, size_t smem = 0) {
+// on every stream, the default ones included: the next step's blocks are in
+// place when a step ends, 1.5-3 us less per step (square 150x150, NR = 14,
+// float-float 8.3 -> 5.9 us; 512x512, NR = 4, FP64 40.6 -> 37.5 us).
+// KPMGB_PDL=0 in the environment turns it off.
+int launch_step_kernel(const StepChoice& c, cudaStream_t s, const KParams& p) {
   static const bool on = [] {
     const char* e = std::getenv("KPMGB_PDL");
     return !(e && e[0] == '0');
   }();
-  if (!on || s == nullptr || s == cudaStreamLegacy || s == cudaStreamPerThread) {
-    fn<<<G, threads, smem, s>>>(p);
+  if (!on || !c.pdl) {
+    c.fn<<<c.grid, c.threads, c.smem, s>>>(p);
     KPMGB_LAUNCHED();
     return KPMGB_OK;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)G);
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = smem;
+  cfg.gridDim = dim3((unsigned)c.grid);
+  cfg.blockDim = dim3((unsigned)c.threads);
+  cfg.dynamicSmemBytes = c.smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  KPMGB_CUDA(cudaLaunchKernelEx(&cfg, fn, p));
+  KPMGB_CUDA(cudaLaunchKernelEx(&cfg, c.fn, p));
   KPMGB_LAUNCHED();
   return KPMGB_OK;
 }
@@ -238,14 +249,7 @@ bool packed_step_applies(const DeviceCSR& H, int NR) {
 
 namespace {
 
-// The kernel of the step `a` for a launch of ncols columns, with its grid.
-struct StepChoice {
-  KernelFn fn = nullptr;
-  int grid = 0;
-  int threads = kThreads;
-  size_t smem = 0;
-};
-
+// The kernel of the step `a` for a launch of ncols columns.
 int choose_step(const StepArgs& a, int precision, int ncols, StepChoice* out) {
   const DeviceCSR& H = *a.H;
   auto take = [&](KernelFn fn, int lpr) {
@@ -305,7 +309,18 @@ int choose_step(const StepArgs& a, int precision, int ncols, StepChoice* out) {
                                       "columns and rows of at most 16 nonzeros");
   }
   const Shape sh = shape_for(a, ncols);
-  return take(select_kernel(sh, precision, a.dot, real), sh.lpr);
+  KPMGB_TRY(take(select_kernel(sh, precision, a.dot, real), sh.lpr));
+  // The FP64 step of a complex operator is bound by each SM's FP64 pipe.  A
+  // grid that leaves some of the resident slots free, but fewer than it needs,
+  // gets its successor's first blocks all on the SMs with those slots when
+  // they are launched early: such grids launch one after another (Haldane
+  // 101x87, NR = 5: 18.5 us per step against 22.3; 150x80, NR = 11: 35.0
+  // against 43.3), the others early (64x64, NR = 8: 2.7 us less per step).
+  if (precision == KPMGB_PREC_FP64 && !real) {
+    const int slots = blocks_per_sm(out->fn) * num_sms();
+    out->pdl = out->grid == slots || 2 * out->grid <= slots;
+  }
+  return KPMGB_OK;
 }
 
 int num_dots(int dot) { return dot == DOT_NONE ? 0 : (dot == DOT_LR1 ? 1 : 2); }
@@ -468,7 +483,7 @@ int launch_step(const StepArgs& a, int precision, cudaStream_t s) {
     p.beta_mode = a.beta == 0.0 ? 0 : -1;
     StepChoice c;
     KPMGB_TRY(choose_step(a, precision, p.ncols, &c));
-    KPMGB_TRY(launch_step_kernel(c.fn, c.grid, s, p, c.threads, c.smem));
+    KPMGB_TRY(launch_step_kernel(c, s, p));
     if (partials) partials += partials_count(a, c, p.ncols);
   }
   return KPMGB_OK;
