@@ -171,10 +171,20 @@ __device__ __forceinline__ int lane_fold(T (&v)[V], int lane, Shfl shfl, Add add
   return base;
 }
 
-__device__ __forceinline__ float2 ff_merge(float2 a, float2 b) {
-  float s, e;
-  ff::two_sum(a.x, b.x, s, e);
-  return make_float2(s, __fadd_rn(a.y, __fadd_rn(b.y, e)));
+// Unevaluated sums of three floats: block sums lose nothing of the 48 bits
+// that each lane's float-float accumulators carry.
+struct F3 {
+  float s, c, d;
+};
+__device__ __forceinline__ F3 f3_merge(F3 a, F3 b) {
+  float s, e, c, f, g;
+  ff::two_sum(a.s, b.s, s, e);
+  ff::two_sum(a.c, b.c, c, f);
+  ff::two_sum(c, e, c, g);
+  return F3{s, c, __fadd_rn(__fadd_rn(a.d, b.d), __fadd_rn(f, g))};
+}
+__device__ __forceinline__ double f3_join(F3 a) {
+  return (double)a.s + ((double)a.c + (double)a.d);
 }
 
 // Shared memory of the two reductions below (a kernel that holds both uses
@@ -220,28 +230,39 @@ __device__ __forceinline__ void block_dots(const double2 (&d)[ND > 0 ? ND : 1][C
 }
 
 // The same for float-float accumulators (leading S, correction C; NP = 1: real
-// parts only) that hold at most kFlushRows rows per lane: merged by TwoSum
-// over lanes and warps, and joined into FP64 once per entry of the block
+// parts only) that hold at most kFlushRows rows per lane: merged over lanes
+// and warps on the FP32 pipe and joined into FP64 once per entry of the block
 // (two conversions and an addition per lane and value otherwise, 48 clocks of
 // the SM's FP64 pipe per warp and value).
 template <int ND, int LPR, int CPL, int NP, int NW = kWarps>
-__device__ __forceinline__ void block_dots_ff(const float2 (&d)[ND > 0 ? ND : 1][CPL][NP],
+__device__ __forceinline__ void block_dots_ff(const F3 (&d)[ND > 0 ? ND : 1][CPL][NP],
                                               const KParams& p) {
-  if constexpr (ND > 0) {
+  if constexpr (ND > 0 && CPL > 2) {
+    // wide lanes (128 columns): the sums of three floats would take 48 KiB
+    double2 f[ND][CPL];
+#pragma unroll
+    for (int k = 0; k < ND; ++k)
+#pragma unroll
+      for (int c = 0; c < CPL; ++c)
+        f[k][c] = make_double2(f3_join(d[k][c][0]), NP > 1 ? f3_join(d[k][c][NP - 1]) : 0.0);
+    block_dots<ND, LPR, CPL, NW>(f, p);
+  } else if constexpr (ND > 0) {
     constexpr int V = ND * CPL * NP;
-    float2(*red)[V * LPR] =
-        reinterpret_cast<float2(*)[V * LPR]>(red_buffer<NW * ND * CPL * 2 * LPR>());
+    constexpr int kDoubles = NW * ND * CPL * 2 * LPR;  // block_dots' buffer
+    F3(*red)[V * LPR] = reinterpret_cast<F3(*)[V * LPR]>(
+        red_buffer<(NP > 1 ? (kDoubles * 3 + 1) / 2 : kDoubles)>());
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float2 v[V];
+    F3 v[V];
 #pragma unroll
     for (int i = 0; i < V; ++i) v[i] = d[i / (NP * CPL)][i / NP % CPL][i % NP];
     const int base = lane_fold<V, LPR>(
         v, lane,
-        [](float2 a, int off) {
-          return make_float2(__shfl_xor_sync(0xffffffffu, a.x, off),
-                             __shfl_xor_sync(0xffffffffu, a.y, off));
+        [](F3 a, int off) {
+          return F3{__shfl_xor_sync(0xffffffffu, a.s, off),
+                    __shfl_xor_sync(0xffffffffu, a.c, off),
+                    __shfl_xor_sync(0xffffffffu, a.d, off)};
         },
-        [](float2 a, float2 b) { return ff_merge(a, b); });
+        [](F3 a, F3 b) { return f3_merge(a, b); });
     constexpr int kLeft = Fold<V, LPR>::count;
 #pragma unroll
     for (int i = 0; i < kLeft; ++i)
@@ -255,10 +276,10 @@ __device__ __forceinline__ void block_dots_ff(const float2 (&d)[ND > 0 ? ND : 1]
 #pragma unroll
       for (int q = 0; q < NP; ++q) {
         const int at = ((k * CPL + col / LPR) * NP + q) * LPR + col % LPR;
-        float2 s = red[0][at];
+        F3 s = red[0][at];
 #pragma unroll
-        for (int w = 1; w < NW; ++w) s = ff_merge(s, red[w][at]);
-        r[q] = ff::join(s.x, s.y);
+        for (int w = 1; w < NW; ++w) s = f3_merge(s, red[w][at]);
+        r[q] = f3_join(s);
       }
       out[e] = make_double2(r[0], r[1]);
     }
@@ -709,13 +730,13 @@ __global__ void __launch_bounds__(kThreads, (FFTune<CPL, REALH>::min_blocks)) k_
         }
       block_dots<ND, LPR, CPL>(d, p);
     } else {
-      float2 f[NDA][CPL][2];
+      F3 f[NDA][CPL][2];
 #pragma unroll
       for (int k = 0; k < ND; ++k)
 #pragma unroll
         for (int c = 0; c < CPL; ++c)
 #pragma unroll
-          for (int q = 0; q < 2; ++q) f[k][c][q] = make_float2(dS[k][c][q], dC[k][c][q]);
+          for (int q = 0; q < 2; ++q) f[k][c][q] = F3{dS[k][c][q], dC[k][c][q], 0.f};
       block_dots_ff<ND, LPR, CPL, 2>(f, p);
     }
   }

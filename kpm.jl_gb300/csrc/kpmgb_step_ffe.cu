@@ -211,13 +211,13 @@ __global__ void __launch_bounds__(kThreads, KPMGB_FFE_MIN_BLOCKS) k_step_ffe(KPa
         }
       block_dots<ND, LPR, CPL>(d, p);
     } else {
-      float2 f[NDA][CPL][2];
+      F3 f[NDA][CPL][2];
 #pragma unroll
       for (int k = 0; k < ND; ++k)
 #pragma unroll
         for (int c = 0; c < CPL; ++c)
 #pragma unroll
-          for (int q = 0; q < 2; ++q) f[k][c][q] = make_float2(dS[k][c][q], dC[k][c][q]);
+          for (int q = 0; q < 2; ++q) f[k][c][q] = F3{dS[k][c][q], dC[k][c][q], 0.f};
       block_dots_ff<ND, LPR, CPL, 2>(f, p);
     }
   }
@@ -425,13 +425,13 @@ __global__ void __launch_bounds__(kThreads, 2) k_step_ffr(KParams p) {
       block_dots<ND, 32, CPL>(d, p);
     } else {
       constexpr int NP = DOT == DOT_DOUBLING ? 1 : 2;
-      float2 f[NDA][CPL][NP];
+      F3 f[NDA][CPL][NP];
 #pragma unroll
       for (int k = 0; k < ND; ++k)
 #pragma unroll
         for (int c = 0; c < CPL; ++c)
 #pragma unroll
-          for (int q = 0; q < NP; ++q) f[k][c][q] = make_float2(dS[k][c][q], dC[k][c][q]);
+          for (int q = 0; q < NP; ++q) f[k][c][q] = F3{dS[k][c][q], dC[k][c][q], 0.f};
       block_dots_ff<ND, 32, CPL, NP>(f, p);
     }
   }
@@ -604,11 +604,11 @@ __global__ void __launch_bounds__(kThreads, 2) k_step_ffc(KParams p) {
       block_dots<ND, LPR, 1>(d, p);
     } else {
       constexpr int NP = DOT == DOT_DOUBLING ? 1 : 2;
-      float2 f[NDA][1][NP];
+      F3 f[NDA][1][NP];
 #pragma unroll
       for (int k = 0; k < ND; ++k)
 #pragma unroll
-        for (int q = 0; q < NP; ++q) f[k][0][q] = make_float2(dS[k][q], dC[k][q]);
+        for (int q = 0; q < NP; ++q) f[k][0][q] = F3{dS[k][q], dC[k][q], 0.f};
       block_dots_ff<ND, LPR, 1, NP>(f, p);
     }
   }

@@ -50,12 +50,12 @@ __device__ __forceinline__ float2 ld_shared_f2(const float2* p) {
   return v;
 }
 
-// The float-float sum of the two lanes of a pair (leading S, correction C).
-__device__ __forceinline__ float2 pair_sum(f2 S, f2 C) {
-  float s0, s1, c0, c1;
-  upk(S, s0, s1);
-  upk(C, c0, c1);
-  return ff_merge(make_float2(s0, c0), make_float2(s1, c1));
+// The sum of the two lanes of a pair of accumulators.
+__device__ __forceinline__ F3 pair_sum(f2 S, f2 C) {
+  F3 a{0.f, 0.f, 0.f}, b{0.f, 0.f, 0.f};
+  upk(S, a.s, b.s);
+  upk(C, a.c, b.c);
+  return f3_merge(a, b);
 }
 
 template <int W, bool FULL>
@@ -345,9 +345,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_step_ffpk1(KParams p) {
     d[1][0].x += join2(xS, xC);
     block_dots<2, LPR, 1>(d, p);
   } else {
-    float2 f[2][1][1];
-    f[0][0][0] = pair_sum(nS, nC);
-    f[1][0][0] = pair_sum(xS, xC);
+    const F3 f[2][1][1] = {{{pair_sum(nS, nC)}}, {{pair_sum(xS, xC)}}};
     block_dots_ff<2, LPR, 1, 1>(f, p);
   }
 }
