@@ -254,8 +254,8 @@ int kpmgb_chebyshev_action(kpmgb_operator H, int64_t NH, int64_t NR,
  * h_n is applied here.  beta = INFINITY selects the T = 0 step with weight
  * 1/2 at Ef (src/utils/physics.jl:15-39).  quad_N Gauss-Chebyshev nodes,
  * nodes with |x| >= 1 - edge_cutoff dropped, as in the reference.  The
- * Ef-independent node sums run once on the device (two FP64 GEMMs with a
- * fused epilogue), then one reduction per Ef.  Argument errors mirror the
+ * Ef-independent node sums run once on the device (from the moments' diagonal
+ * and antidiagonal sums), then one reduction per Ef.  Argument errors mirror the
  * reference's ArgumentErrors.  Blocking call on the current device. */
 int kpmgb_kubo_bastin(const double* mu2d, int64_t ld, int64_t NC, double a,
                       double b, const double* Ef, int64_t nE, int64_t NH,
