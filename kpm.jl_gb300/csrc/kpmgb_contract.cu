@@ -8,9 +8,11 @@
 // moment_parity mask on (n + m) and the mn_sym row limit applied in the
 // epilogue instead of in a host loop.
 //
-// The double-precision form is a split-K SIMT GEMM: each block owns a 32 x 32
+// The double-precision form runs on the tensor cores with eight digit planes
+// (kpmgb_contract_tc8.cu).  Vectors that those planes do not hold to FP64's
+// accuracy go through the split-K SIMT GEMM below: each block owns a 32 x 32
 // output tile and one slice of K; the slices are summed in a fixed order by a
-// second kernel (deterministic).  The tensor-core form lives in
+// second kernel (deterministic).  The five-digit split form lives in
 // kpmgb_contract_tc.cu.
 #include <cuda_runtime.h>
 
@@ -22,6 +24,8 @@ namespace kpmgb {
 
 int launch_contract_split(const ContractArgs& a, int precision, cudaStream_t s);
 size_t contract_split_scratch_bytes(int64_t K, int nr, int nl);
+size_t contract_planes8_bytes(int64_t K, int nr, int nl);
+int launch_contract_planes8(const ContractArgs& a, int precision, cudaStream_t s);
 
 namespace {
 
@@ -41,7 +45,9 @@ template <bool FF>
 __global__ void __launch_bounds__(256) k_contract_f64(const void* __restrict__ R,
                                                       const void* __restrict__ L, int64_t K,
                                                       int nr, int nl, int64_t kslice,
-                                                      double2* __restrict__ part) {
+                                                      double2* __restrict__ part,
+                                                      const unsigned* __restrict__ need) {
+  if (need && !*need) return;
   __shared__ double2 sR[KC][TM + 1];
   __shared__ double2 sL[KC][TN + 1];
   const int ta = blockIdx.x, tb = blockIdx.y;
@@ -100,7 +106,8 @@ __device__ __forceinline__ bool parity_keep(int parity, int n, int m) {
 __global__ void k_contract_reduce(const double2* __restrict__ part, int nslices, int nr, int nl,
                                   int n0, int m0, int NC, double inv_nr,
                                   const double* __restrict__ dscale, int parity, int nmax_row,
-                                  double2* __restrict__ mu) {
+                                  double2* __restrict__ mu, const unsigned* __restrict__ need) {
+  if (need && !*need) return;
   const int64_t total = (int64_t)nr * nl;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
        e += (int64_t)gridDim.x * blockDim.x) {
@@ -160,30 +167,40 @@ size_t contract_scratch_bytes(int64_t K, int nr, int nl, int precision, int cont
   // slices * nr' * nl' <= (4 * SMs / tiles' + 1) * tiles' * TM * TN.
   const size_t tiles = (size_t)((nr + TM - 1) / TM) * ((nl + TN - 1) / TN);
   const size_t bound = (4 * (size_t)num_sms_c() + tiles) * TM * TN;
-  return std::max(bound, (size_t)slices_for(K, nr, nl) * nr * nl) * sizeof(double2);
+  const size_t simt =
+      std::max(bound, (size_t)slices_for(K, nr, nl) * nr * nl) * sizeof(double2) + kContractGateBytes;
+  return std::max(simt, contract_planes8_bytes(K, nr, nl));
 }
 
 int launch_contract(const ContractArgs& a, int precision, int contraction, cudaStream_t s) {
   if (a.nr <= 0 || a.nl <= 0) return KPMGB_OK;
   if (contraction == KPMGB_CONTRACT_SPLIT) return launch_contract_split(a, precision, s);
   const int S = slices_for(a.K, a.nr, a.nl);
-  const size_t need = (size_t)S * a.nr * a.nl * sizeof(double2);
-  if (need > a.scratch_bytes) return fail(KPMGB_ERR_ALLOC, "contraction scratch too small");
+  const size_t bytes = (size_t)S * a.nr * a.nl * sizeof(double2) + kContractGateBytes;
+  if (bytes > a.scratch_bytes) return fail(KPMGB_ERR_ALLOC, "contraction scratch too small");
   int64_t kslice = (a.K + S - 1) / S;
   kslice = (kslice + KC - 1) / KC * KC;
   dim3 grid((a.nr + TM - 1) / TM, (a.nl + TN - 1) / TN, S);
-  double2* part = static_cast<double2*>(a.scratch);
+  char* const scratch = static_cast<char*>(a.scratch);
+  double2* part = reinterpret_cast<double2*>(scratch + kContractGateBytes);
   cudaEvent_t t0 = timing_mark(s);
+  // The digit planes are the faster form at every size (K = 1024, NC = 8: 0.15
+  // against 1.12 ms per kpm_2d call; K = 65536, NC = 128: 1.9 against 7.9 ms).
+  const unsigned* need = nullptr;  // device word: the FP64 kernels below have to run
+  if (contract_planes8_bytes(a.K, a.nr, a.nl) <= a.scratch_bytes) {
+    need = reinterpret_cast<const unsigned*>(scratch);
+    KPMGB_TRY(launch_contract_planes8(a, precision, s));
+  }
   if (precision == KPMGB_PREC_FF)
-    k_contract_f64<true><<<grid, 256, 0, s>>>(a.R, a.L, a.K, a.nr, a.nl, kslice, part);
+    k_contract_f64<true><<<grid, 256, 0, s>>>(a.R, a.L, a.K, a.nr, a.nl, kslice, part, need);
   else
-    k_contract_f64<false><<<grid, 256, 0, s>>>(a.R, a.L, a.K, a.nr, a.nl, kslice, part);
+    k_contract_f64<false><<<grid, 256, 0, s>>>(a.R, a.L, a.K, a.nr, a.nl, kslice, part, need);
   KPMGB_LAUNCHED();
   timing_add(TIMED_CONTRACT_FP64, t0, timing_mark(s));
   const int64_t total = (int64_t)a.nr * a.nl;
   const int blocks = (int)std::min<int64_t>((total + 255) / 256, 2048);
   k_contract_reduce<<<blocks, 256, 0, s>>>(part, S, a.nr, a.nl, a.n0, a.m0, a.NC, a.inv_nr,
-                                           a.dscale, a.parity, a.nmax_row, a.mu);
+                                           a.dscale, a.parity, a.nmax_row, a.mu, need);
   KPMGB_LAUNCHED();
   return KPMGB_OK;
 }

@@ -21,6 +21,15 @@
 // chunk accumulators are reused.  A K split holds at most 2^24 K' elements,
 // so the int64 stays below 2^62.
 //
+// The double-precision contraction takes the same form with eight digits
+// (Planes8 below): every entry becomes a 63-bit integer of its row's scale, the
+// 36 plane pairs with i + j <= 7 feed eight accumulators, each exact over a
+// chunk of 128 K' elements ((l+1) 2^21 multiples of 2^-8l, l <= 7: at most
+// 2^24), folded into two int64 per output (levels 0-3 in units of 2^-24,
+// levels 4-7 in units of 2^-56).  What it drops is below 2^-64 of the row
+// maxima's product per K' element: against 64-bit sums it is nearer than FP64
+// FMAs, which round every partial sum.
+//
 // MMA shape: the five B planes of a stage lie one after another along N, so
 // A plane i meets B planes 0..4-i in ONE tcgen05.mma of N = 48 (5 - i)
 // whose output columns land on the accumulators of levels i..4 (the level
@@ -34,128 +43,21 @@
 // copies (cp.async.bulk, 40 KiB of A planes and 15 KiB of B planes)
 // completed on an mbarrier.  Warp roles per CTA: 0 producer, 1 MMA issuer
 // (one thread), 2-5 epilogue (one TMEM lane each).  All waits are bounded.
-#include <cuda_bf16.h>
-#include <cuda_runtime.h>
-
-#include <algorithm>
-#include <cmath>
 #include <mutex>
 #include <type_traits>
 
-#include "kpmgb_internal.h"
+#include "kpmgb_tc.cuh"
 
 namespace kpmgb {
 
 namespace {
 
-constexpr int TC_M = 128;      // A rows per tile
-constexpr int TC_N = 48;       // B rows per tile
-constexpr int TC_KT = 32;      // real K' elements per k-tile
-constexpr int TC_SLICES = 5;   // digit planes per operand
-constexpr int TC_ACC = 5;      // TMEM accumulators: one per digit level 0..4
-constexpr int TC_CHUNK = 8;    // k-tiles per exact chunk (256 K' elements)
-constexpr int TC_STAGES = 4;
-constexpr uint32_t A_TILE = TC_M * TC_KT * 2;  // 8 KiB per plane
-constexpr uint32_t B_TILE = TC_N * TC_KT * 2;  // 3 KiB per plane
-constexpr uint32_t A_STAGE = A_TILE * TC_SLICES;
-constexpr uint32_t B_STAGE = B_TILE * TC_SLICES;
-constexpr uint32_t STAGE_BYTES = A_STAGE + B_STAGE;
-constexpr int TMEM_COLS = 512;  // 2 buffers of 256 columns (5 levels x 48 used)
-constexpr int64_t kMaxKtPerSplit = (int64_t)1 << 19;  // 2^24 K' elements: int64 headroom
-constexpr int TMEM_BUF = 256;
-constexpr int kSpin = 1 << 22;
-constexpr int kThreadsTC = 192;  // 6 warps
-
-// --------------------------------------------------------------- PTX helpers
-__device__ __forceinline__ uint32_t saddr(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void bar_init(uint32_t b, uint32_t n) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(b), "r"(n) : "memory");
-}
-__device__ __forceinline__ void bar_expect(uint32_t b, uint32_t tx) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(tx)
-               : "memory");
-}
-__device__ __forceinline__ void bar_arrive(uint32_t b) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(b) : "memory");
-}
-__device__ __forceinline__ bool bar_wait(uint32_t b, uint32_t parity) {
-  for (int i = 0; i < kSpin; ++i) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(b), "r"(parity)
-        : "memory");
-    if (ok) return true;
-  }
-  return false;
-}
-__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes,
-                                          uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-          dst),
-      "l"(src), "r"(bytes), "r"(bar)
-      : "memory");
-}
-// UMMA shared-memory descriptor, no swizzle, K-major: LBO = 128 B between the
-// two K-adjacent 8x16-byte core matrices, SBO = 256 B between 8-row groups.
-__device__ __forceinline__ uint64_t umma_desc(uint32_t addr) {
-  uint64_t d = (uint64_t)((addr & 0x3FFFF) >> 4);
-  d |= (uint64_t)(128 >> 4) << 16;
-  d |= (uint64_t)(256 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  return d;
-}
-// kind::f16 instruction descriptor: D = F32, A = B = BF16, both K-major,
-// M = TC_M, N = n (a multiple of 16 up to 256).
-__host__ __device__ constexpr uint32_t idesc_for(int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) |
-         ((uint32_t)(TC_M >> 4) << 24);
-}
-static_assert(TC_N * TC_SLICES <= 256 && (TC_N * TC_SLICES) % 16 == 0 && TC_N % 16 == 0,
-              "one MMA covers up to five B planes");
-
-__device__ __forceinline__ void umma(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc,
-                                     uint32_t acc) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-      "l"(a), "l"(b), "r"(idesc), "r"(acc)
-      : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-      : "memory");
-}
-// 16 consecutive TMEM columns of this thread's lane (no wait).
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* v) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-        "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-        "=r"(v[14]), "=r"(v[15])
-      : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_wait_ld() {
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
+constexpr int TC_N = Planes5::kN;
+constexpr int TC_KT = Planes5::KT;
+constexpr int TC_SLICES = Planes5::kSlices;
+constexpr uint32_t A_TILE = Planes5::kATile, B_TILE = Planes5::kBTile;
 
 // --------------------------------------------------------------- pre-passes
-// Byte offset of element (r, k) inside a ROWS x TC_KT tile (canonical layout);
-// the five planes of a k-tile form one (5 ROWS) x TC_KT tile, plane i in rows
-// i ROWS .. (i+1) ROWS - 1.
-template <int ROWS>
-__host__ __device__ __forceinline__ uint32_t tile_off(int r, int k) {
-  return (uint32_t)((k >> 4) * (ROWS * 32) + (r >> 3) * 256 + ((k >> 3) & 1) * 128 + (r & 7) * 16 +
-                    (k & 7) * 2);
-}
-
 template <bool FF>
 __device__ __forceinline__ void load_pair(const void* base, int64_t idx, float& rh, float& rl,
                                           float& ih, float& il) {
@@ -466,267 +368,6 @@ __global__ void __launch_bounds__(256) k_slice8(const void* vecs, int64_t K, int
   }
 }
 
-// --------------------------------------------------------------- GEMM
-struct TcArgs {
-  const uint8_t* A;      // planes [mtiles][ktiles][A_STAGE]
-  const uint8_t* B;      // planes [ntiles][ktiles][B_STAGE]
-  int64_t ktiles;
-  int64_t kt_per_split;
-  int nr, ncols;         // real rows of A, real rows of B (2 nl)
-  const int* expA;
-  const int* expB;       // per B row (L vector index = row % nl)
-  int nl;
-  double* part;          // [split][nr][ncols]
-  unsigned* status;
-};
-
-__global__ void __launch_bounds__(kThreadsTC, 1) k_contract_tc(TcArgs p) {
-  extern __shared__ __align__(1024) uint8_t smem[];
-  __shared__ __align__(8) uint64_t bars[4 * TC_STAGES];  // full, empty, tfull, tempty
-  __shared__ uint32_t s_tmem;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int mt = blockIdx.x, nt = blockIdx.y, sp = blockIdx.z;
-  const int64_t kt0 = (int64_t)sp * p.kt_per_split;
-  const int64_t kt1 = min(p.ktiles, kt0 + p.kt_per_split);
-  const int64_t nkt = kt1 > kt0 ? kt1 - kt0 : 0;
-  const int64_t nchunks = (nkt + TC_CHUNK - 1) / TC_CHUNK;
-  const uint32_t full0 = saddr(&bars[0]), empty0 = saddr(&bars[TC_STAGES]);
-  const uint32_t tfull0 = saddr(&bars[2 * TC_STAGES]), tempty0 = saddr(&bars[3 * TC_STAGES]);
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < TC_STAGES; ++s) {
-      bar_init(full0 + 8 * s, 1);
-      bar_init(empty0 + 8 * s, 1);
-      bar_init(tfull0 + 8 * s, 1);
-      bar_init(tempty0 + 8 * s, 4);
-    }
-  }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     saddr(&s_tmem)),
-                 "r"(TMEM_COLS));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-  }
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = s_tmem;
-  const uint32_t sm0 = saddr(smem);
-
-  if (warp == 0) {
-    // ------------------------------------------------------------ producer
-    if (lane == 0) {
-      for (int64_t i = 0; i < nkt; ++i) {
-        const int s = (int)(i % TC_STAGES);
-        const uint32_t ph = (uint32_t)((i / TC_STAGES) & 1);
-        if (!bar_wait(empty0 + 8 * s, ph ^ 1)) {
-          atomicOr(p.status, (unsigned)STATUS_TIMEOUT);
-          break;
-        }
-        const int64_t kt = kt0 + i;
-        bar_expect(full0 + 8 * s, STAGE_BYTES);
-        bulk_copy(sm0 + s * STAGE_BYTES, p.A + (size_t)(mt * p.ktiles + kt) * A_STAGE, A_STAGE,
-                  full0 + 8 * s);
-        bulk_copy(sm0 + s * STAGE_BYTES + A_STAGE, p.B + (size_t)(nt * p.ktiles + kt) * B_STAGE,
-                  B_STAGE, full0 + 8 * s);
-      }
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      int64_t i = 0;
-      bool ok = true;
-      for (int64_t c = 0; c < nchunks && ok; ++c) {
-        const int buf = (int)(c & 1);
-        if (!bar_wait(tempty0 + 8 * buf, (uint32_t)(((c >> 1) & 1) ^ 1))) {
-          ok = false;
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int64_t rem = nkt - c * TC_CHUNK;
-        const int64_t tiles = rem < TC_CHUNK ? rem : TC_CHUNK;
-        for (int64_t t = 0; t < tiles; ++t, ++i) {
-          const int s = (int)(i % TC_STAGES);
-          if (!bar_wait(full0 + 8 * s, (uint32_t)((i / TC_STAGES) & 1))) {
-            ok = false;
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a0 = sm0 + s * STAGE_BYTES, b0 = a0 + A_STAGE;
-#pragma unroll
-          for (int ks = 0; ks < TC_KT / 16; ++ks) {
-            // B planes 0..4 of this K step: rows 0 .. 5 TC_N - 1 of one tile
-            const uint64_t bd = umma_desc(b0 + ks * (TC_SLICES * TC_N * 32));
-#pragma unroll
-            for (int ia = 0; ia < TC_SLICES; ++ia) {
-              // A plane ia x B planes 0 .. 4-ia -> level blocks ia .. 4; the
-              // chunk's first MMA (ia = 0 covers every block) initialises
-              const uint64_t ad =
-                  umma_desc(a0 + ks * (TC_SLICES * TC_M * 32) + ia * (TC_M / 8) * 256);
-              const bool init = t == 0 && ks == 0 && ia == 0;
-              umma(tmem + buf * TMEM_BUF + ia * TC_N, ad, bd, idesc_for(TC_N * (TC_SLICES - ia)),
-                   init ? 0u : 1u);
-            }
-          }
-          umma_commit(empty0 + 8 * s);  // stage free once these MMAs retire
-        }
-        if (ok) umma_commit(tfull0 + 8 * buf);
-      }
-      if (!ok) atomicOr(p.status, (unsigned)STATUS_TIMEOUT);
-    }
-  } else {
-    // ------------------------------------------------------------ epilogue
-    const int q = warp & 3;          // TMEM lane quarter this warp may access
-    const int row = q * 32 + lane;   // tile row = TMEM lane
-    long long acc[TC_N];
-#pragma unroll
-    for (int j = 0; j < TC_N; ++j) acc[j] = 0;
-    bool ok = true;
-    for (int64_t c = 0; c < nchunks; ++c) {
-      const int buf = (int)(c & 1);
-      if (!bar_wait(tfull0 + 8 * buf, (uint32_t)((c >> 1) & 1))) {
-        ok = false;
-        break;
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-      for (int ac = 0; ac < TC_ACC; ++ac) {
-        // in units of 2^-24: level l < 4 is a multiple of 2^-8l below
-        // (l+1) 2^22 of them (exact), level 4 (below 5 2^-10) is rounded to
-        // 2^-24
-        const float unit = ac == 4 ? 16777216.f : (float)(1 << (8 * ac));
-        const int shift = ac == 4 ? 0 : 24 - 8 * ac;
-#pragma unroll
-        for (int h = 0; h < TC_N / 16; ++h) {
-          uint32_t v[16];
-          tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + buf * TMEM_BUF + ac * TC_N + h * 16, v);
-          tmem_wait_ld();
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const long long iv =
-                (long long)__float2int_rn(__fmul_rn(__uint_as_float(v[j]), unit));
-            acc[h * 16 + j] += iv << shift;
-          }
-        }
-      }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) bar_arrive(tempty0 + 8 * buf);
-    }
-    if (!ok) atomicOr(p.status, (unsigned)STATUS_TIMEOUT);
-    const int a = mt * TC_M + row;
-    if (a < p.nr) {
-      // value = acc * 2^-24 * 2^(eA - 7) * 2^(eB - 7)
-      const int ea = p.expA[a];
-#pragma unroll
-      for (int j = 0; j < TC_N; ++j) {
-        const int col = nt * TC_N + j;
-        if (col < p.ncols) {
-          const int eb = p.expB[col % p.nl];
-          const double vv = ldexp((double)acc[j], ea + eb - 38);
-          p.part[((size_t)sp * p.nr + a) * p.ncols + col] = vv;
-        }
-      }
-    }
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (warp == 1) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                 "r"(TMEM_COLS));
-  }
-}
-
-__device__ __forceinline__ bool keep_parity(int parity, int n, int m) {
-  if (parity == KPMGB_PARITY_NONE) return true;
-  const bool odd = ((n + m) & 1) != 0;
-  return parity == KPMGB_PARITY_ODD ? odd : !odd;
-}
-
-__global__ void k_tc_reduce(const double* __restrict__ part, int nsplit, int nr, int nl, int n0,
-                            int m0, int NC, double inv_nr, const double* __restrict__ dscale,
-                            int parity, int nmax_row, double2* __restrict__ mu) {
-  const int64_t total = (int64_t)nr * nl;
-  const int ncols = 2 * nl;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const int a = (int)(e / nl), b = (int)(e % nl);
-    const int n = n0 + a, m = m0 + b;
-    if (n >= nmax_row || !keep_parity(parity, n, m)) continue;
-    double re = 0.0, im = 0.0;
-    for (int s = 0; s < nsplit; ++s) {
-      re += part[((size_t)s * nr + a) * ncols + b];
-      im += part[((size_t)s * nr + a) * ncols + nl + b];
-    }
-    const double f = dscale ? inv_nr * dscale[0] : inv_nr;
-    double2* dst = mu + (size_t)n + (size_t)NC * m;
-    dst->x += re * f;
-    dst->y += im * f;
-  }
-}
-
-int sm_count() {
-  static int n = [] {
-    int dev = 0, v = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    return v > 0 ? v : 1;
-  }();
-  return n;
-}
-
-struct TcPlan {
-  int mtiles, ntiles, nsplit;
-  int64_t ktiles, kt_per_split;
-  size_t a_bytes, b_bytes, exp_bytes, part_bytes;
-};
-
-TcPlan plan_for(int64_t K, int nr, int nl) {
-  TcPlan pl;
-  pl.mtiles = (nr + TC_M - 1) / TC_M;
-  pl.ntiles = (2 * nl + TC_N - 1) / TC_N;
-  pl.ktiles = (2 * K + TC_KT - 1) / TC_KT;
-  const int64_t tiles = (int64_t)pl.mtiles * pl.ntiles;
-  const int64_t S = sm_count();  // one CTA per SM (shared memory)
-  const int64_t kmax = std::max<int64_t>(1, pl.ktiles / (4 * TC_CHUNK));
-  int64_t want = std::max<int64_t>(1, (2 * S + tiles - 1) / tiles);
-  want = std::min<int64_t>(want, kmax);
-  // K splits: the count in [want, 4 want] (at most 8 S + tiles CTAs) whose
-  // grid fills its last wave best, i.e. the least waves per unit of work
-  // ceil(n tiles / S) / n; e.g. 64 tiles on 152 SMs: 19 splits (8 full
-  // waves) instead of 5 (2.1 waves run as 3)
-  int64_t best = want;
-  double best_cost = 1e300;
-  for (int64_t n = want; n <= std::min<int64_t>(4 * want, kmax); ++n) {
-    if (n * tiles > 8 * S + tiles) break;
-    const double cost = (double)((n * tiles + S - 1) / S) / (double)n;
-    if (cost < best_cost * (1.0 - 1e-9)) {
-      best_cost = cost;
-      best = n;
-    }
-  }
-  want = std::max(best, (pl.ktiles + kMaxKtPerSplit - 1) / kMaxKtPerSplit);
-  pl.kt_per_split = (pl.ktiles + want - 1) / want;
-  pl.kt_per_split = (pl.kt_per_split + TC_CHUNK - 1) / TC_CHUNK * TC_CHUNK;
-  pl.kt_per_split = std::min(pl.kt_per_split, kMaxKtPerSplit);
-  pl.nsplit = (int)((pl.ktiles + pl.kt_per_split - 1) / pl.kt_per_split);
-  pl.a_bytes = (size_t)pl.mtiles * pl.ktiles * A_STAGE;
-  pl.b_bytes = (size_t)pl.ntiles * pl.ktiles * B_STAGE;
-  pl.exp_bytes = ((size_t)(nr + nl) * sizeof(int) + 255) & ~size_t(255);
-  pl.part_bytes = (size_t)pl.nsplit * nr * 2 * nl * sizeof(double);
-  return pl;
-}
-
-// Partials of a plan, bounded over its sub-blocks: the split count times the
-// tiles stays within 8*SMs + tiles, or the minimum split count that keeps a
-// split within kMaxKtPerSplit k-tiles times the tiles.
-size_t part_bound_bytes(const TcPlan& pl) {
-  const int64_t tiles = (int64_t)pl.mtiles * pl.ntiles;
-  const int64_t nmin = (pl.ktiles + kMaxKtPerSplit - 1) / kMaxKtPerSplit;
-  return (size_t)std::max<int64_t>(8 * sm_count() + tiles, nmin * tiles) * TC_M * TC_N *
-         sizeof(double);
-}
-
 }  // namespace
 
 int launch_vec_absmax(const void* vecs, int64_t K, int nvec, unsigned* out, cudaStream_t s) {
@@ -746,14 +387,14 @@ int launch_vec_absmax(const void* vecs, int64_t K, int nvec, unsigned* out, cuda
 size_t contract_split_scratch_bytes(int64_t K, int nr, int nl) {
   // the largest plan over sub-blocks nr' <= nr, nl' <= nl is the full block's
   // (plane sizes grow with nr, nl; partials within part_bound_bytes)
-  const TcPlan pl = plan_for(K, nr, nl);
-  const size_t part_bound = part_bound_bytes(pl);
+  const TcPlan pl = plan_for<Planes5>(K, nr, nl);
+  const size_t part_bound = part_bound_bytes<Planes5>(pl);
   return pl.a_bytes + pl.b_bytes + 2 * pl.exp_bytes + std::max(pl.part_bytes, part_bound) + 1024;
 }
 
 int launch_contract_split(const ContractArgs& a, int precision, cudaStream_t s) {
-  const TcPlan pl = plan_for(a.K, a.nr, a.nl);
-  const size_t part_bound = part_bound_bytes(pl);
+  const TcPlan pl = plan_for<Planes5>(a.K, a.nr, a.nl);
+  const size_t part_bound = part_bound_bytes<Planes5>(pl);
   const size_t need = pl.a_bytes + pl.b_bytes + 2 * pl.exp_bytes +
                       std::max(pl.part_bytes, part_bound) + 1024;
   if (need > a.scratch_bytes) return fail(KPMGB_ERR_ALLOC, "split contraction scratch too small");
@@ -828,8 +469,8 @@ int launch_contract_split(const ContractArgs& a, int precision, cudaStream_t s) 
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(k_contract_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(TC_STAGES * STAGE_BYTES));
+    attr_err = cudaFuncSetAttribute(k_contract_tc<Planes5>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)(Planes5::kStages * Planes5::kStage));
   });
   if (attr_err != cudaSuccess)
     return fail(KPMGB_ERR_CUDA, "cannot configure the tensor-core contraction: %s",
@@ -846,15 +487,16 @@ int launch_contract_split(const ContractArgs& a, int precision, cudaStream_t s) 
   t.nl = a.nl;
   t.part = part;
   t.status = a.status;
+  t.skip = nullptr;
   dim3 grid(pl.mtiles, pl.ntiles, pl.nsplit);
   cudaEvent_t t0 = timing_mark(s);
-  k_contract_tc<<<grid, kThreadsTC, TC_STAGES * STAGE_BYTES, s>>>(t);
+  k_contract_tc<Planes5><<<grid, kThreadsTC, Planes5::kStages * Planes5::kStage, s>>>(t);
   KPMGB_LAUNCHED();
   timing_add(TIMED_CONTRACT_SPLIT, t0, timing_mark(s));
   const int64_t total = (int64_t)a.nr * a.nl;
-  const int blocks = (int)std::min<int64_t>((total + 255) / 256, 2048);
+  const int blocks = (int)std::min<int64_t>((total + 31) / 32, 8192);
   k_tc_reduce<<<std::max(blocks, 1), 256, 0, s>>>(part, pl.nsplit, a.nr, a.nl, a.n0, a.m0, a.NC,
-                                                  a.inv_nr, a.dscale, a.parity, a.nmax_row, a.mu);
+                                                  a.inv_nr, a.dscale, a.parity, a.nmax_row, a.mu, nullptr);
   KPMGB_LAUNCHED();
   return KPMGB_OK;
 }

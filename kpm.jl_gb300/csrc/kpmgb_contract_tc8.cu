@@ -1,0 +1,351 @@
+// The double-precision contraction of kpm_2d on the tensor cores: eight digit
+// planes per operand (Planes8, kpmgb_tc.cuh; the scheme of
+// kpmgb_contract_tc.cu).
+//
+// GB300 multiplies FP64 at 0.53 TFMA/s and BF16 at about 1 PFMA/s, so 36 BF16
+// products per FP64 product are still some fifty times the FP64 rate.  Every
+// entry becomes the integer N = round(v 2^(62-e)), |v| < 2^e over its row
+// (exact for entries within 2^-9 of the row maximum, within 2^-63 of it for
+// the rest), cut into eight balanced base-256 digits; the digit products of
+// i + j <= 7 add up exactly and the dropped ones stay below 2^-64 of the
+// product of the row maxima per term.  For vectors whose largest entry is
+// within a factor 32 of their root mean square the sum is nearer to the exact
+// one than FP64 FMAs, which round every partial sum.  Other vectors (probes
+// on single sites, rows that hold infinities or NaN) keep the FP64 kernel:
+// k_vec_gate compares the two figures of every vector on the device and sets
+// a word that each kernel of either form reads first.
+//
+// The planes of a K range are laid out, multiplied and added to the moments
+// before those of the next, so they take at most kPlaneBytes of scratch.
+#include <mutex>
+#include <type_traits>
+
+#include "kpmgb_tc.cuh"
+
+namespace kpmgb {
+
+namespace {
+
+using C8 = Planes8;
+constexpr int S8 = C8::kSlices;
+constexpr size_t kPlaneBytes = size_t(2) << 30;
+// largest entry squared against the mean square: beyond 32^2 the FP64 kernel
+constexpr float kPeak = 1024.f;
+constexpr size_t kGateBytes = kContractGateBytes;
+constexpr int kStatChunk = 8192;  // complex elements per block of the statistics
+
+template <bool FF>
+__device__ __forceinline__ double2 load_f64(const void* base, int64_t idx) {
+  if constexpr (FF) {
+    const float4 v = __ldg(static_cast<const float4*>(base) + idx);
+    return make_double2((double)v.x + (double)v.y, (double)v.z + (double)v.w);
+  } else {
+    return __ldg(static_cast<const double2*>(base) + idx);
+  }
+}
+
+__device__ __forceinline__ unsigned long long abs_bits(double v) {
+  return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+}
+
+// Largest |component| of a chunk (bits of a double) and the chunk's sum of
+// squares in units of that component's power of two squared.
+struct VecStat {
+  unsigned long long peak;
+  float sumsq;
+};
+
+__device__ __forceinline__ int exponent_of(unsigned long long bits) { return (int)(bits >> 52); }
+
+// |v| / 2^(ex - 1023) as a float with 23 bits of v (0 below 2^-40), for v of at
+// most exponent ex: integer operations only, the FP64 pipe stays out of it
+__device__ __forceinline__ float relative(double v, int ex) {
+  const unsigned long long b = abs_bits(v);
+  const int d = exponent_of(b) - ex;
+  return d < -40 || b == 0 ? 0.f : __int_as_float(((127 + d) << 23) | (int)((b >> 29) & 0x7fffff));
+}
+
+// stat[v][chunk]
+template <bool FF>
+__global__ void __launch_bounds__(256) k_vec_stat(const void* vecs, int64_t K, int chunks,
+                                                  VecStat* stat) {
+  __shared__ unsigned long long rp[256];
+  __shared__ float rs[256];
+  const int v = blockIdx.y, tid = threadIdx.x;
+  const int64_t k0 = (int64_t)blockIdx.x * kStatChunk, k1 = min(K, k0 + kStatChunk);
+  unsigned long long m = 0;
+#pragma unroll 4
+  for (int64_t k = k0 + tid; k < k1; k += 256) {
+    const double2 x = load_f64<FF>(vecs, (int64_t)v * K + k);
+    m = max(m, max(abs_bits(x.x), abs_bits(x.y)));
+  }
+  rp[tid] = m;
+  __syncthreads();
+  for (int w = 128; w > 0; w >>= 1) {
+    if (tid < w) rp[tid] = max(rp[tid], rp[tid + w]);
+    __syncthreads();
+  }
+  const int ex = exponent_of(rp[0]);
+  float s = 0.f;
+#pragma unroll 4
+  for (int64_t k = k0 + tid; k < k1; k += 256) {
+    const double2 x = load_f64<FF>(vecs, (int64_t)v * K + k);
+    const float re = relative(x.x, ex), im = relative(x.y, ex);
+    s = fmaf(re, re, fmaf(im, im, s));
+  }
+  rs[tid] = s;
+  __syncthreads();
+  for (int w = 128; w > 0; w >>= 1) {
+    if (tid < w) rs[tid] += rs[tid + w];
+    __syncthreads();
+  }
+  if (tid == 0) stat[(size_t)v * chunks + blockIdx.x] = VecStat{rp[0], rs[0]};
+}
+
+// exps[v]: max |component| < 2^e (0 for a zero vector); *fp64 set when a
+// vector is not finite or too peaked
+__global__ void __launch_bounds__(32) k_vec_gate(const VecStat* stat, int chunks, int64_t K,
+                                                 int* exps, unsigned* fp64) {
+  const int v = blockIdx.x, lane = threadIdx.x;
+  unsigned long long m = 0;
+  for (int c = lane; c < chunks; c += 32) m = max(m, stat[(size_t)v * chunks + c].peak);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, off));
+  const int ex = exponent_of(m);
+  float s = 0.f;
+  for (int c = lane; c < chunks; c += 32) {
+    const VecStat t = stat[(size_t)v * chunks + c];
+    s += ldexpf(t.sumsq, 2 * max(exponent_of(t.peak) - ex, -80));
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+  if (lane == 0) {
+    exps[v] = m == 0 ? 0 : max(ex, 1) - 1022;
+    const float mx = relative(__longlong_as_double((long long)m), ex);
+    if (m != 0 && (ex == 0x7ff || !(mx * mx * 2.f * (float)K <= kPeak * s))) atomicOr(fp64, 1u);
+  }
+}
+
+// round(v 2^(62-e)) for |v| < 2^e
+__device__ __forceinline__ long long to_integer(double v, int e) {
+  const unsigned long long b = abs_bits(v);
+  const int ex = (int)(b >> 52);
+  unsigned long long m = b & 0xfffffffffffffull;
+  if (ex > 0) m |= 0x10000000000000ull;
+  const int sh = 62 - e + (ex > 0 ? ex : 1) - 1075;  // at most 9
+  if (sh >= 0) {
+    m <<= sh;
+  } else {
+    m = sh >= -54 ? (m + (1ull << (-sh - 1))) >> -sh : 0;
+  }
+  return __double_as_longlong(v) < 0 ? -(long long)m : (long long)m;
+}
+
+// Balanced base-256 digits of n, least significant first: digit i in byte i,
+// [-128, 127] below the top one (|top| <= 64).  Adding 128 to every lower byte
+// carries exactly where a digit is negative; taking it off per byte (an
+// exclusive or of the top bit) leaves two's complement digits.
+__device__ __forceinline__ unsigned long long digit_bytes(long long n) {
+  return ((unsigned long long)n + 0x0080808080808080ull) ^ 0x0080808080808080ull;
+}
+
+// The BF16 bits of digit byte d (two's complement) of plane i: d 2^(-8 i).
+template <int I>
+__device__ __forceinline__ uint32_t plane_bits(int d) {
+  // float(d) by the 1.5 2^23 offset, exact; BF16 keeps its 8 leading bits
+  const float f = __int_as_float(0x4B400000 + d) - 12582912.f;
+  constexpr float kScale = I == 0 ? 1.f : I == 1 ? 0x1p-8f : I == 2 ? 0x1p-16f : I == 3 ? 0x1p-24f
+                         : I == 4 ? 0x1p-32f : I == 5 ? 0x1p-40f : I == 6 ? 0x1p-48f : 0x1p-56f;
+  return __float_as_uint(__fmul_rn(f, kScale)) >> 16;
+}
+
+// Digit planes of the K range kb .. ke (complex elements) of nvec vectors in
+// the pre-tiled layout: blocks of 8 vectors x 32 groups of 8 K' elements;
+// warp w reads vector v0 + w, the 16-byte pieces meet in shared memory (rows
+// padded to 9) and leave as whole 128-byte core-matrix rows.  Elements at or
+// past ke are 0.  IS_B: rows v hold (Re, Im), rows nvec + v (-Im, Re).
+template <bool FF, bool IS_B>
+__global__ void __launch_bounds__(256) k_slice_f64(const void* vecs, int64_t K, int64_t kb,
+                                                   int64_t ke, int nvec, const int* exps,
+                                                   int64_t ktiles, uint8_t* planes,
+                                                   const unsigned* skip) {
+  if (*skip) return;
+  constexpr int ROWS = IS_B ? C8::kN : TC_M;
+  constexpr uint32_t TILE = IS_B ? C8::kBTile : C8::kATile;
+  __shared__ __align__(16) uint4 piece[S8][32][9];
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const int v0 = blockIdx.y * 8, v = v0 + w;
+  const int64_t groups = ktiles * (C8::KT / 8);
+  const int64_t g0 = (int64_t)blockIdx.x * 32, g = g0 + l;
+  const bool have = v < nvec && g < groups;
+  unsigned long long dr[4] = {}, di[4] = {};
+  if (have) {
+    const int e = exps[v];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int64_t k = kb + g * 4 + j;
+      if (k < ke) {
+        const double2 x = load_f64<FF>(vecs, (int64_t)v * K + k);
+        dr[j] = digit_bytes(to_integer(x.x, e));
+        di[j] = digit_bytes(to_integer(x.y, e));
+      }
+    }
+  }
+#pragma unroll
+  for (int set = 0; set < (IS_B ? 2 : 1); ++set) {
+    if (set) __syncthreads();  // the pieces of the first set have left
+    if (have) {
+      auto put = [&](auto plane) {
+        constexpr int i = decltype(plane)::value;
+        uint32_t h[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int r = (int)(signed char)(dr[j] >> (8 * (S8 - 1 - i)));
+          const int m = (int)(signed char)(di[j] >> (8 * (S8 - 1 - i)));
+          h[j] = set == 0 ? plane_bits<i>(r) | plane_bits<i>(m) << 16
+                          : plane_bits<i>(-m) | plane_bits<i>(r) << 16;
+        }
+        piece[i][l][w] = make_uint4(h[0], h[1], h[2], h[3]);
+      };
+      put(std::integral_constant<int, 0>{});
+      put(std::integral_constant<int, 1>{});
+      put(std::integral_constant<int, 2>{});
+      put(std::integral_constant<int, 3>{});
+      put(std::integral_constant<int, 4>{});
+      put(std::integral_constant<int, 5>{});
+      put(std::integral_constant<int, 6>{});
+      put(std::integral_constant<int, 7>{});
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < S8 * 32 * 8; q += 256) {
+      const int rr = q & 7, gl = (q >> 3) & 31, i = q >> 8;
+      const int64_t gg = g0 + gl;
+      if (gg >= groups || v0 + rr >= nvec) continue;
+      const int row = (set == 0 ? 0 : nvec) + v0 + rr;
+      const int64_t kt = gg / (C8::KT / 8);
+      const int kin = (int)(gg % (C8::KT / 8)) * 8;
+      uint8_t* tbase = planes + (size_t)(row / ROWS * ktiles + kt) * (S8 * TILE);
+      *reinterpret_cast<uint4*>(tbase + tile_off<S8 * ROWS>(i * ROWS + row % ROWS, kin)) =
+          piece[i][gl][rr];
+    }
+  }
+}
+
+size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
+
+// Complex elements per K range: the planes of nr + 2 nl rows within the size
+// of the vectors themselves, but at least 64 MiB and at most kPlaneBytes, in
+// whole exact chunks.
+int64_t range_for(int64_t K, int nr, int nl) {
+  const size_t most = std::min<size_t>(
+      kPlaneBytes, std::max<size_t>((size_t)64 << 20, (size_t)K * (nr + nl) * 16));
+  const size_t rows = (size_t)((nr + TC_M - 1) / TC_M * TC_M) +
+                      (size_t)((2 * nl + C8::kN - 1) / C8::kN * C8::kN);
+  const int64_t chunk = C8::kChunk * C8::KT / 2;  // complex elements
+  const int64_t fit = (int64_t)(most / (rows * S8 * 2 * 2)) / chunk * chunk;
+  return std::min(K, std::max<int64_t>(fit, 64 * chunk));
+}
+
+struct Layout8 {
+  TcPlan pl;
+  int64_t range;
+  int chunks;  // statistics blocks per vector
+  size_t b, a, expB, expA, stat, gate, part, bytes;
+};
+
+Layout8 layout_for(int64_t K, int nr, int nl) {
+  Layout8 l;
+  l.range = range_for(K, nr, nl);
+  l.pl = plan_for<C8>(l.range, nr, nl);
+  l.chunks = (int)((K + kStatChunk - 1) / kStatChunk);
+  l.gate = 0;
+  l.b = kGateBytes;
+  l.expB = l.b + align256(l.pl.b_bytes);
+  l.a = l.expB + align256((size_t)nl * sizeof(int));
+  l.expA = l.a + align256(l.pl.a_bytes);
+  l.stat = l.expA + align256((size_t)nr * sizeof(int));
+  l.part = l.stat + align256((size_t)(nr + nl) * l.chunks * sizeof(VecStat));
+  l.bytes = l.part + std::max(l.pl.part_bytes, part_bound_bytes<C8>(l.pl));
+  return l;
+}
+
+template <bool FF>
+int launch_planes(const ContractArgs& a, const Layout8& l, uint8_t* base, cudaStream_t s) {
+  const TcPlan& pl = l.pl;
+  uint8_t *B = base + l.b, *A = base + l.a;
+  int* expB = reinterpret_cast<int*>(base + l.expB);
+  int* expA = reinterpret_cast<int*>(base + l.expA);
+  VecStat* stat = reinterpret_cast<VecStat*>(base + l.stat);
+  unsigned* gate = reinterpret_cast<unsigned*>(base + l.gate);
+  double* part = reinterpret_cast<double*>(base + l.part);
+  KPMGB_CUDA(cudaMemsetAsync(gate, 0, sizeof(unsigned), s));
+  auto stats = [&](const void* vecs, int nvec, int* exps) -> int {
+    for (int v0 = 0; v0 < nvec; v0 += 65535) {  // the grid's y limit
+      const int nv = std::min(nvec - v0, 65535);
+      const void* p = static_cast<const char*>(vecs) + (size_t)v0 * a.K * 16;
+      k_vec_stat<FF><<<dim3((unsigned)l.chunks, (unsigned)nv), 256, 0, s>>>(p, a.K, l.chunks, stat);
+      KPMGB_LAUNCHED();
+      k_vec_gate<<<(unsigned)nv, 32, 0, s>>>(stat, l.chunks, a.K, exps + v0, gate);
+      KPMGB_LAUNCHED();
+    }
+    return KPMGB_OK;
+  };
+  KPMGB_TRY(stats(a.L, a.nl, expB));
+  KPMGB_TRY(stats(a.R, a.nr, expA));
+  static std::once_flag once;
+  static cudaError_t attr_err = cudaSuccess;
+  constexpr int kSmem = (int)(C8::kStages * C8::kStage);
+  std::call_once(once, [] {
+    attr_err = cudaFuncSetAttribute(k_contract_tc<C8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    kSmem);
+  });
+  if (attr_err != cudaSuccess)
+    return fail(KPMGB_ERR_CUDA, "cannot configure the tensor-core contraction: %s",
+                cudaGetErrorString(attr_err));
+  const unsigned gx = (unsigned)((pl.ktiles * (C8::KT / 8) + 31) / 32);
+  for (int64_t kb = 0; kb < a.K; kb += l.range) {
+    const int64_t ke = std::min(a.K, kb + l.range);
+    k_slice_f64<FF, true><<<dim3(gx, (unsigned)((a.nl + 7) / 8)), 256, 0, s>>>(
+        a.L, a.K, kb, ke, a.nl, expB, pl.ktiles, B, gate);
+    KPMGB_LAUNCHED();
+    k_slice_f64<FF, false><<<dim3(gx, (unsigned)((a.nr + 7) / 8)), 256, 0, s>>>(
+        a.R, a.K, kb, ke, a.nr, expA, pl.ktiles, A, gate);
+    KPMGB_LAUNCHED();
+    TcArgs t;
+    t.A = A;
+    t.B = B;
+    t.ktiles = pl.ktiles;
+    t.kt_per_split = pl.kt_per_split;
+    t.nr = a.nr;
+    t.ncols = 2 * a.nl;
+    t.expA = expA;
+    t.expB = expB;
+    t.nl = a.nl;
+    t.part = part;
+    t.status = a.status;
+    t.skip = gate;
+    k_contract_tc<C8><<<dim3(pl.mtiles, pl.ntiles, pl.nsplit), kThreadsTC, kSmem, s>>>(t);
+    KPMGB_LAUNCHED();
+    const int64_t total = (int64_t)a.nr * a.nl;
+    k_tc_reduce<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((total + 31) / 32, 8192)), 256,
+                  0, s>>>(part, pl.nsplit, a.nr, a.nl, a.n0, a.m0, a.NC, a.inv_nr, a.dscale,
+                          a.parity, a.nmax_row, a.mu, gate);
+    KPMGB_LAUNCHED();
+  }
+  return KPMGB_OK;
+}
+
+}  // namespace
+
+size_t contract_planes8_bytes(int64_t K, int nr, int nl) { return layout_for(K, nr, nl).bytes; }
+
+// The gate word (nonzero: the FP64 kernel has to run) is the first of scratch.
+int launch_contract_planes8(const ContractArgs& a, int precision, cudaStream_t s) {
+  if (!a.status) return fail(KPMGB_ERR_ARGUMENT, "the contraction needs a status word");
+  const Layout8 l = layout_for(a.K, a.nr, a.nl);
+  uint8_t* base = static_cast<uint8_t*>(a.scratch);
+  return precision == KPMGB_PREC_FF ? launch_planes<true>(a, l, base, s)
+                                    : launch_planes<false>(a, l, base, s);
+}
+
+}  // namespace kpmgb

@@ -315,6 +315,9 @@ int launch_vec_absmax(const void* vecs, int64_t K, int nvec, unsigned* out, cuda
 int launch_contract(const ContractArgs& a, int precision, int contraction,
                     cudaStream_t s);
 size_t contract_scratch_bytes(int64_t K, int nr, int nl, int precision, int contraction);
+// The double-precision contraction's device word at the start of its scratch
+// (nonzero: its vectors need the FP64 kernel), padded to the planes' alignment.
+constexpr size_t kContractGateBytes = 1024;
 int launch_mn_sym(double2* mu, int NC, cudaStream_t s);
 
 // Cluster-resident recurrence (kpmgb_cluster.cu): one thread-block cluster

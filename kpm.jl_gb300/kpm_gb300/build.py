@@ -30,6 +30,7 @@ SOURCES = [
     "kpmgb_cluster.cu",
     "kpmgb_contract.cu",
     "kpmgb_contract_tc.cu",
+    "kpmgb_contract_tc8.cu",
     "kpmgb_noalloc.cu",
     "kpmgb_ensemble.cu",
     "kpmgb_adjoint.cu",
