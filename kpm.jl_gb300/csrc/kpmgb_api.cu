@@ -456,8 +456,8 @@ int run_kpm2d(Operator* H, Operator* Ja, Operator* Jb, int64_t NC, int64_t NR, i
     if (m && n > 0) KPMGB_CUDA(cudaMemsetAsync(m, 0, (size_t)n * sizeof(unsigned), s));
     return KPMGB_OK;
   };
-  auto apply = [&](const DeviceCSR* op, const void* x, const void* z, void* y, double alpha,
-                   double beta, unsigned* vmax = nullptr) {
+  auto step = [&](const DeviceCSR* op, const void* x, const void* z, void* y, double alpha,
+                  double beta, unsigned* vmax = nullptr) {
     StepArgs a;
     a.H = op;
     a.NH = NH;
@@ -469,15 +469,22 @@ int run_kpm2d(Operator* H, Operator* Ja, Operator* Jb, int64_t NC, int64_t NR, i
     a.beta = beta;
     a.colpair = colpair;
     a.vmax = vmax;
-    return launch_step(a, precision, s);
+    return a;
   };
-  // right seed Ja psi_r -> ring slot 3 (src/moment.jl:1021)
-  KPMGB_TRY(apply(&Ja->csr, R(0), nullptr, RING(3), 1.0, 0.0));
-  // left seed psi_l, H psi_l (src/moment.jl:1013-1018)
+  auto apply = [&](const DeviceCSR* op, const void* x, const void* z, void* y, double alpha,
+                   double beta, unsigned* vmax = nullptr) {
+    return launch_step(step(op, x, z, y, alpha, beta, vmax), precision, s);
+  };
   if (colpair) KPMGB_TRY(launch_vec_absmax(L(0), K, 1, maxL, s));
-  if (KLa >= 2) {
-    KPMGB_TRY(zero_max(colpair ? maxL + 1 : nullptr, 1));
-    KPMGB_TRY(apply(&H->csr, L(0), nullptr, L(1), 1.0, 0.0, colpair ? maxL + 1 : nullptr));
+  KPMGB_TRY(zero_max(colpair ? maxL + 1 : nullptr, KLa - 1));
+  {
+    // right seed Ja psi_r -> ring slot 3 (src/moment.jl:1021) and left seed
+    // psi_l, H psi_l (src/moment.jl:1013-1018)
+    const StepArgs seeds[] = {
+        step(&Ja->csr, R(0), nullptr, RING(3), 1.0, 0.0),
+        step(&H->csr, L(0), nullptr, KLa >= 2 ? L(1) : nullptr, 1.0, 0.0,
+             colpair ? maxL + 1 : nullptr)};
+    KPMGB_TRY(launch_steps(seeds, KLa >= 2 ? 2 : 1, precision, s));
   }
 
   // right chain v_n = T_n(H) Ja psi_r (v_0 in ring slot 3, v_n in slot n%3),
@@ -508,7 +515,26 @@ int run_kpm2d(Operator* H, Operator* Ja, Operator* Jb, int64_t NC, int64_t NR, i
     return KPMGB_OK;
   };
   const bool right_resident = KRa >= NC;
-  if (right_resident) {
+  const bool all_resident = right_resident && KLa >= NC;
+  if (all_resident) {
+    // both chains side by side: step n + 2 of the left one, step n + 1 of the
+    // right one and right entry n read nothing that the others write, so one
+    // launch takes all three (a third of the launches: conductivity of a
+    // 128 x 128 lattice, NC = 64, NR = 4, FP64, 191 launches of 4.5 us before)
+    KPMGB_TRY(zero_max(maxR, NC));
+    for (int64_t n = 0; n < NC; ++n) {
+      StepArgs t[3];
+      int nt = 0;
+      t[nt++] = step(&Jb->csr, right_vec(n), nullptr, R(n), 1.0, 0.0, colpair ? maxR + n : nullptr);
+      if (n + 1 < NC)
+        t[nt++] = n == 0 ? step(&H->csr, right_vec(0), nullptr, right_vec(1), 1.0, 0.0)
+                         : step(&H->csr, right_vec(n), right_vec(n - 1), right_vec(n + 1), 2.0, -1.0);
+      if (n + 2 < NC)
+        t[nt++] = step(&H->csr, L(n + 1), L(n), L(n + 2), 2.0, -1.0,
+                       colpair ? maxL + n + 2 : nullptr);
+      KPMGB_TRY(launch_steps(t, nt, precision, s));
+    }
+  } else if (right_resident) {
     chain_n = -1;
     KPMGB_TRY(fill_right(0, NC - 1));
   }
@@ -517,8 +543,8 @@ int run_kpm2d(Operator* H, Operator* Ja, Operator* Jb, int64_t NC, int64_t NR, i
     const int64_t m1 = rep * KL;
     const int64_t m2 = std::min<int64_t>(m1 + KL, NC);  // exclusive
     const int64_t rep_size = m2 - m1;
-    KPMGB_TRY(zero_max(colpair ? maxL + 2 : nullptr, rep_size - 2));
-    for (int64_t i = 2; i < rep_size; ++i)
+    if (rep > 0) KPMGB_TRY(zero_max(colpair ? maxL + 2 : nullptr, rep_size - 2));
+    for (int64_t i = all_resident ? rep_size : 2; i < rep_size; ++i)
       KPMGB_TRY(apply(&H->csr, L(i - 1), L(i - 2), L(i), 2.0, -1.0, colpair ? maxL + i : nullptr));
     const int64_t nmax = opt.mn_sym ? m2 : NC;  // exclusive
     for (int64_t n1 = 0; n1 < nmax; n1 += KR) {

@@ -222,6 +222,9 @@ enum VecLayout : int { VEC_STD = 0, VEC_PAIRED = 1, VEC_COLPAIR = 2 };
 
 // precision: KPMGB_PREC_FP64 or KPMGB_PREC_FF.  Returns KPMGB_OK or an error.
 int launch_step(const StepArgs& a, int precision, cudaStream_t s);
+// The same for n independent steps without dots (equal NH and NR; no step
+// reads what another writes): one launch for as many of them as share a kernel.
+int launch_steps(const StepArgs* steps, int n, int precision, cudaStream_t s);
 // Whether float-float doubling steps of NR columns on H can run on packed
 // FP32 pairs over the paired vector layout (StepArgs::paired).
 bool packed_step_applies(const DeviceCSR& H, int NR);

@@ -141,7 +141,7 @@ struct StepChoice {
   int grid = 0;
   int threads = kThreads;
   size_t smem = 0;
-  bool pdl = true;
+  int slots = 0;  // resident blocks where early launches depend on them, else 0
 };
 
 // Step kernels launch with programmatic stream serialization (see pdl_enter)
@@ -149,18 +149,20 @@ struct StepChoice {
 // place when a step ends, 1.5-3 us less per step (square 150x150, NR = 14,
 // float-float 8.3 -> 5.9 us; 512x512, NR = 4, FP64 40.6 -> 37.5 us).
 // KPMGB_PDL=0 in the environment turns it off.
-int launch_step_kernel(const StepChoice& c, cudaStream_t s, const KParams& p) {
+int launch_step_kernel(const StepChoice& c, int n, cudaStream_t s, const KBatch& p) {
   static const bool on = [] {
     const char* e = std::getenv("KPMGB_PDL");
     return !(e && e[0] == '0');
   }();
-  if (!on || !c.pdl) {
-    c.fn<<<c.grid, c.threads, c.smem, s>>>(p);
+  const int blocks = c.grid * n;
+  const bool early = c.slots == 0 || blocks >= c.slots || 2 * blocks <= c.slots;
+  if (!on || !early) {
+    c.fn<<<dim3((unsigned)c.grid, (unsigned)n), c.threads, c.smem, s>>>(p);
     KPMGB_LAUNCHED();
     return KPMGB_OK;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)c.grid);
+  cfg.gridDim = dim3((unsigned)c.grid, (unsigned)n);
   cfg.blockDim = dim3((unsigned)c.threads);
   cfg.dynamicSmemBytes = c.smem;
   cfg.stream = s;
@@ -316,10 +318,7 @@ int choose_step(const StepArgs& a, int precision, int ncols, StepChoice* out) {
   // they are launched early: such grids launch one after another (Haldane
   // 101x87, NR = 5: 18.5 us per step against 22.3; 150x80, NR = 11: 35.0
   // against 43.3), the others early (64x64, NR = 8: 2.7 us less per step).
-  if (precision == KPMGB_PREC_FP64 && !real) {
-    const int slots = blocks_per_sm(out->fn) * num_sms();
-    out->pdl = out->grid == slots || 2 * out->grid <= slots;
-  }
+  if (precision == KPMGB_PREC_FP64 && !real) out->slots = blocks_per_sm(out->fn) * num_sms();
   return KPMGB_OK;
 }
 
@@ -445,48 +444,68 @@ int64_t later_steps(int64_t NC, bool lr) { return lr ? NC - 2 : NC / 2 - 1; }
 
 }  // namespace
 
-int launch_step(const StepArgs& a, int precision, cudaStream_t s) {
-  const DeviceCSR& H = *a.H;
-  const double al = std::fabs(a.alpha);
-  int e = 0;
-  const double m = std::frexp(al, &e);
-  if (!(m == 0.5) || !(a.beta == 0.0 || a.beta == -1.0))
-    return fail(KPMGB_ERR_ARGUMENT,
-                "the recurrence step supports alpha = +-2^k and beta in {-1, 0}");
-  if (precision == KPMGB_PREC_FF && !H.val_ff)
-    return fail(KPMGB_ERR_ARGUMENT, "operator has no float-float values");
+int launch_steps(const StepArgs* steps, int n, int precision, cudaStream_t s) {
+  for (int i = 0; i < n; ++i) {
+    const StepArgs& a = steps[i];
+    int e = 0;
+    const double m = std::frexp(std::fabs(a.alpha), &e);
+    if (!(m == 0.5) || !(a.beta == 0.0 || a.beta == -1.0))
+      return fail(KPMGB_ERR_ARGUMENT,
+                  "the recurrence step supports alpha = +-2^k and beta in {-1, 0}");
+    if (precision == KPMGB_PREC_FF && !a.H->val_ff)
+      return fail(KPMGB_ERR_ARGUMENT, "operator has no float-float values");
+    if (a.dot != DOT_NONE && !a.partials)
+      return fail(KPMGB_ERR_CUDA, "internal: a step with dots needs its partial sums");
+  }
   const int W = cols_per_launch();
-  double2* partials = static_cast<double2*>(a.partials);
-  if (a.dot != DOT_NONE && !partials)
-    return fail(KPMGB_ERR_CUDA, "internal: a step with dots needs its partial sums");
-  for (int c0 = 0; c0 < a.NR; c0 += W) {
-    KParams p;
-    p.rowptr = H.rowptr;
-    p.col = H.col;
-    p.val = precision == KPMGB_PREC_FF ? H.val_ff
-                                       : (H.is_real ? (const void*)H.val_real : (const void*)H.val);
-    p.NH = a.NH;
-    p.ld = a.NR;
-    p.c0 = c0;
-    p.ncols = std::min(W, a.NR - c0);
-    p.x = a.x;
-    p.z = a.z;
-    p.y = a.y;
-    p.bra = a.bra;
-    p.alpha = a.alpha;
-    p.partials = partials;
-    p.vmax = a.vmax;
-    p.ell_col = H.ell_col;
-    p.ell_val = H.ell_val;
-    p.ell_w = H.ell_w;
-    p.alpha_f = (float)a.alpha;
-    p.beta_mode = a.beta == 0.0 ? 0 : -1;
-    StepChoice c;
-    KPMGB_TRY(choose_step(a, precision, p.ncols, &c));
-    KPMGB_TRY(launch_step_kernel(c, s, p));
-    if (partials) partials += partials_count(a, c, p.ncols);
+  const int NR = steps[0].NR;
+  double2* partials = static_cast<double2*>(steps[0].partials);  // steps with dots launch alone
+  for (int c0 = 0; c0 < NR; c0 += W) {
+    const int ncols = std::min(W, NR - c0);
+    StepChoice c;  // of the steps filled in so far
+    KBatch batch;
+    int held = 0;
+    for (int i = 0; i < n; ++i) {
+      const StepArgs& a = steps[i];
+      const DeviceCSR& H = *a.H;
+      StepChoice ci;
+      KPMGB_TRY(choose_step(a, precision, ncols, &ci));
+      if (held > 0 && (ci.fn != c.fn || ci.grid != c.grid || held == kMaxBatch)) {
+        KPMGB_TRY(launch_step_kernel(c, held, s, batch));
+        held = 0;
+      }
+      c = ci;
+      KParams& p = batch.p[held++];
+      p.rowptr = H.rowptr;
+      p.col = H.col;
+      p.val = precision == KPMGB_PREC_FF
+                  ? H.val_ff
+                  : (H.is_real ? (const void*)H.val_real : (const void*)H.val);
+      p.NH = a.NH;
+      p.ld = a.NR;
+      p.c0 = c0;
+      p.ncols = ncols;
+      p.x = a.x;
+      p.z = a.z;
+      p.y = a.y;
+      p.bra = a.bra;
+      p.alpha = a.alpha;
+      p.partials = partials;
+      p.vmax = a.vmax;
+      p.ell_col = H.ell_col;
+      p.ell_val = H.ell_val;
+      p.ell_w = H.ell_w;
+      p.alpha_f = (float)a.alpha;
+      p.beta_mode = a.beta == 0.0 ? 0 : -1;
+    }
+    KPMGB_TRY(launch_step_kernel(c, held, s, batch));
+    if (partials) partials += partials_count(steps[0], c, ncols);
   }
   return KPMGB_OK;
+}
+
+int launch_step(const StepArgs& a, int precision, cudaStream_t s) {
+  return launch_steps(&a, 1, precision, s);
 }
 
 int recurrence_scratch_bytes(const StepArgs& a0, int precision, int64_t NC, bool lr,

@@ -118,6 +118,14 @@ struct KParams {
   unsigned* vmax;
 };
 
+// One launch applies up to kMaxBatch independent steps without dots (the
+// chains and the current applications of kpm_2d): step blockIdx.y of the
+// batch.  Steps with dots launch alone.
+constexpr int kMaxBatch = 3;
+struct KBatch {
+  KParams p[kMaxBatch];
+};
+
 template <int DOT>
 struct NDots {
   static constexpr int value = DOT == DOT_NONE ? 0 : (DOT == DOT_LR1 ? 1 : 2);
@@ -323,7 +331,8 @@ __device__ __forceinline__ void cdot(double2& acc, double2 a, double2 b) {
 }
 
 template <int LPR, int CPL, bool REALH, int DOT>
-__global__ void __launch_bounds__(kThreads) k_step_f64(KParams p) {
+__global__ void __launch_bounds__(kThreads) k_step_f64(const __grid_constant__ KBatch batch) {
+  const KParams& p = batch.p[DOT == DOT_NONE ? blockIdx.y : 0];
   pdl_enter();
   constexpr int ND = NDots<DOT>::value;
   constexpr int GROUPS = kThreads / LPR;
@@ -539,7 +548,9 @@ __device__ __forceinline__ void ff_chunk_n(int cnt, const KParams& p,
 }
 
 template <int LPR, int CPL, bool REALH, int DOT, int CH>
-__global__ void __launch_bounds__(kThreads, (FFTune<CPL, REALH>::min_blocks)) k_step_ff(KParams p) {
+__global__ void __launch_bounds__(kThreads, (FFTune<CPL, REALH>::min_blocks)) k_step_ff(
+    const __grid_constant__ KBatch batch) {
+  const KParams& p = batch.p[DOT == DOT_NONE ? blockIdx.y : 0];
   pdl_enter();
   constexpr int ND = NDots<DOT>::value;
   constexpr int NDA = ND > 0 ? ND : 1;
@@ -746,7 +757,7 @@ struct Shape {
   int lpr, cpl;
 };
 
-using KernelFn = void (*)(KParams);
+using KernelFn = void (*)(KBatch);
 
 template <int LPR, int CPL, bool REALH, int DOT, int PREC>
 KernelFn kernel_for_prec() {

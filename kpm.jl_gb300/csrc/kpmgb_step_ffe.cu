@@ -63,7 +63,9 @@ __global__ void k_build_ell(const int* __restrict__ rowptr, const int* __restric
 #endif
 
 template <int LPR, int CPL, bool REALH, int DOT, bool FULL>
-__global__ void __launch_bounds__(kThreads, KPMGB_FFE_MIN_BLOCKS) k_step_ffe(KParams p) {
+__global__ void __launch_bounds__(kThreads, KPMGB_FFE_MIN_BLOCKS) k_step_ffe(
+    const __grid_constant__ KBatch batch) {
+  const KParams& p = batch.p[DOT == DOT_NONE ? blockIdx.y : 0];
   pdl_enter();
   constexpr int CH = kEllChunk;
   constexpr int ND = NDots<DOT>::value;
@@ -267,7 +269,9 @@ KernelFn ffe_shape(int ncols, int dot) {
 // Hermitian H only (src/moment.jl:420-492), and then <x|y> =
 // <psi|T_{n-1}(H) T_n(H)|psi> is real: its imaginary part is stored as 0.
 template <int W, int DOT, bool FULL>
-__global__ void __launch_bounds__(kThreads, 2) k_step_ffr(KParams p) {
+__global__ void __launch_bounds__(kThreads, 2) k_step_ffr(
+    const __grid_constant__ KBatch batch) {
+  const KParams& p = batch.p[DOT == DOT_NONE ? blockIdx.y : 0];
   pdl_enter();
   constexpr int GROUPS = kThreads / 32;  // rows per block tile
   constexpr int CPL = 2;
@@ -476,7 +480,9 @@ KernelFn select_kernel_ffr(int ncols, int dot, bool real, int max_row_nnz, int e
 // WL: slots that may hold nonzeros (the operator's longest row), the rest of
 // the W-slot row is padding that every row shares and that is skipped.
 template <int LPR, int W, int DOT, bool FULL, int WL = W>
-__global__ void __launch_bounds__(kThreads, 2) k_step_ffc(KParams p) {
+__global__ void __launch_bounds__(kThreads, 2) k_step_ffc(
+    const __grid_constant__ KBatch batch) {
+  const KParams& p = batch.p[DOT == DOT_NONE ? blockIdx.y : 0];
   pdl_enter();
   constexpr int RPW = 32 / LPR;                 // rows per warp
   constexpr int GROUPS = kThreads / LPR;        // rows per block tile

@@ -59,7 +59,9 @@ __device__ __forceinline__ F3 pair_sum(f2 S, f2 C) {
 }
 
 template <int W, bool FULL>
-__global__ void __launch_bounds__(kThreads, 2) k_step_ffpk(KParams p) {
+__global__ void __launch_bounds__(kThreads, 2) k_step_ffpk(
+    const __grid_constant__ KBatch batch) {
+  const KParams& p = batch.p[0];
   pdl_enter();
   constexpr int GROUPS = kThreads / 32;  // rows per block tile
   constexpr int CPL = 2;
@@ -225,7 +227,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_step_ffpk(KParams p) {
 // columns, LPR lanes per row (RPW = 32 / LPR rows per warp), with half the
 // loads per lane of k_step_ffpk and so three blocks per SM.
 template <int LPR, int W>
-__global__ void __launch_bounds__(kThreads, 3) k_step_ffpk1(KParams p) {
+__global__ void __launch_bounds__(kThreads, 3) k_step_ffpk1(
+    const __grid_constant__ KBatch batch) {
+  const KParams& p = batch.p[0];
   pdl_enter();
   constexpr int RPW = 32 / LPR;           // rows per warp
   constexpr int GROUPS = kThreads / LPR;  // rows per block tile
@@ -365,7 +369,9 @@ __global__ void __launch_bounds__(kThreads, 3) k_step_ffpk1(KParams p) {
 // rows take two chunks merged by TwoSum (the gathers of one row and two
 // columns would not fit the registers of two blocks per SM).
 template <int LPH, int W, int WL>
-__global__ void __launch_bounds__(kThreads, 2) k_step_ffcp(KParams p) {
+__global__ void __launch_bounds__(kThreads, 2) k_step_ffcp(
+    const __grid_constant__ KBatch batch) {
+  const KParams& p = batch.p[blockIdx.y];
   pdl_enter();
   constexpr int RPW = 32 / LPH;            // rows per warp
   constexpr int GROUPS = kThreads / LPH;   // rows per block tile
