@@ -99,10 +99,10 @@ typedef struct kpmgb_kpm1d_options {
                               columns).  Other values fail with
                               KPMGB_ERR_ARGUMENT.
                               Automatic selection (0) is the cluster kernel
-                              (10) for small operators (float-float:
-                              NH <= 16384, NH * NR <= 131072; FP64:
-                              NH <= 16384, NH * NR <= 524288, or NH <= 32768
-                              with NR <= 4), else per-step launches of the
+                              (10) for small operators (those whose step it is
+                              measured to take faster than a launch does: up
+                              to about 16000 rows at a few columns, 4000 at
+                              32), else per-step launches of the
                               row-streaming kernels (11) where they apply,
                               else of the padded-row kernel for real
                               operators with 33..64 columns, else of the

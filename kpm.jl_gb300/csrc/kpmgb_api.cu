@@ -184,13 +184,8 @@ int run_kpm1d(Operator* op, int64_t NC, int64_t NR, int64_t NH, const void* psi_
   const bool ff = precision == KPMGB_PREC_FF;
   // kernel_variant 10: one thread-block cluster per probe column, the
   // recurrence resident in distributed shared memory.  Automatic selection
-  // takes it for small operators, where it measured faster on GB300 than
-  // per-step launches replayed from a CUDA graph (2D Anderson, NC=1024):
-  // FP64 for NH <= 16384 at NR <= 32 (1.3-1.8x at NH = 16384; 2D Anderson
-  // L=64, NR=12: 3.6 ms against 6.9 ms) and at NH = 32768 with NR = 4;
-  // float-float for NH * NR <= 131072 (NH = 16384: 1.3x at NR = 4, 0.9x at
-  // NR = 16; NH = 32768: slower at every NR).
-  // KPMGB_CLUSTER_AUTO=0 turns the automatic choice off.
+  // takes it where it is expected to beat a launch per step
+  // (cluster_is_faster).  KPMGB_CLUSTER_AUTO=0 turns the automatic choice off.
   static const bool cluster_auto_on = [] {
     const char* e = std::getenv("KPMGB_CLUSTER_AUTO");
     return !(e && std::atoi(e) == 0);
@@ -200,10 +195,7 @@ int run_kpm1d(Operator* op, int64_t NC, int64_t NR, int64_t NH, const void* psi_
       variant != 10 && variant != 11)
     return fail(KPMGB_ERR_ARGUMENT, "unknown kernel_variant %d", variant);
   const bool auto_cluster =
-      variant == 0 && cluster_auto_on &&
-      (precision == KPMGB_PREC_FF
-           ? NH <= 16384 && NH * NR <= 131072
-           : (NH <= 16384 && NH * NR <= 524288) || (NH <= 32768 && NR <= 4));
+      variant == 0 && cluster_auto_on && cluster_is_faster(op->csr, NH, (int)NR, precision);
   // Float-float doubling calls with 9..64 columns on real operators of at
   // most 8 nonzeros per row keep their vectors in the paired element layout
   // and run every step on packed FP32 pairs (k_step_ffpk / k_step_ffpk1;
@@ -222,11 +214,14 @@ int run_kpm1d(Operator* op, int64_t NC, int64_t NR, int64_t NH, const void* psi_
     KPMGB_TRY(launch_scale_product(sc, lr ? sc + NR : sc, sc + 2 * NR, (int)NR, s));
     mom_scale = sc + 2 * NR;
   }
+  MomentArgs m;
+  m.mu = mu;
+  m.scale = mom_scale;
+  m.growth_limit = !lr && o && o->stability_check ? 2.25 : 0.0;
+  m.status = ws.sync.as<unsigned>() + 1;
   if (variant == 10 || auto_cluster) {
-    const int rc = launch_kpm1d_cluster(op->csr, NH, (int)NR, NC, lr, precision, sl[0],
-                                        lr ? ws.bra.ptr : nullptr, mu, mom_scale,
-                                        (!lr && o && o->stability_check) ? 2.25 : 0.0,
-                                        ws.sync.as<unsigned>() + 1, s);
+    const int rc = launch_kpm1d_cluster(op->csr, NH, (int)NR, NC, lr, precision, sl,
+                                        lr ? ws.bra.ptr : nullptr, ws.partials, m, s);
     if (variant == 10 || rc != KPMGB_ERR_ARGUMENT) return rc;
     clear_error();  // no resident cluster of that shape: per-step launches
   }
@@ -290,11 +285,6 @@ int run_kpm1d(Operator* op, int64_t NC, int64_t NR, int64_t NH, const void* psi_
   KPMGB_TRY(recurrence_scratch_bytes(a, precision, NC, lr, &held));
   KPMGB_TRY(ws.partials.ensure(std::max(ws.partials.bytes, held)));
   a.partials = ws.partials.ptr;
-  MomentArgs m;
-  m.mu = mu;
-  m.scale = mom_scale;
-  m.growth_limit = !lr && o && o->stability_check ? 2.25 : 0.0;
-  m.status = ws.sync.as<unsigned>() + 1;
   auto recurrence = [&]() -> int {
     return launch_recurrence(a, precision, NC, lr, sl, held, m, s);
   };

@@ -2,25 +2,33 @@
 //
 // For operators small enough that one probe column's two recurrence slots fit
 // in the shared memory of a thread-block cluster (NH up to ~100k rows with 16
-// CTAs), the whole recurrence of a column runs inside one cluster: CTA q of
-// the cluster owns rows [q R, (q+1) R) of both slots in its own shared memory,
+// CTAs), the recurrence of a column runs inside one cluster: CTA q of the
+// cluster owns rows [q R, (q+1) R) of both slots in its own shared memory,
 // gathers neighbour rows owned by other CTAs through distributed shared memory
-// (mapa + ld.shared::cluster), and the steps are separated by the hardware
-// cluster barrier.  After the initial load nothing touches global memory but
-// the operator's index and value arrays (L2-resident) and the moments, and a
-// whole kpm_1d call is one launch of NR clusters.
+// (ld.shared::cluster), and the steps are separated by the hardware cluster
+// barrier.  After the initial load nothing touches global memory but the
+// operator's index and value arrays where they do not fit in shared memory,
+// and each warp's sums of its rows' dots, which k_finish_moments turns into
+// moments afterwards.
 //
-// Moments: every CTA reduces its rows' dot terms in a fixed order (shuffle
-// trees) and stores the partial into rank 0's shared memory (double-buffered
-// by step parity); after the step's barrier rank 0 sums the partials in rank
-// order and writes the moments (doubling or bra/ket conventions of the step
-// kernels), so results are deterministic.  A final barrier keeps every CTA's
-// shared memory alive until no other CTA can still access it.  Every thread of every CTA executes the same sequence
-// of cluster barriers (CTAs without rows still take part); there is no
-// spin-wait.
+// A step is a chain of latencies: gather, row sum, barrier.  What is not on
+// that chain is kept off it: y is stored, the barrier's arrival is signalled,
+// and only then are the dots of the step taken, summed over the warp and
+// stored, while the other CTAs arrive.  FP64 runs at one warp instruction per
+// 64 clocks and SM quarter, so FP64 rows are split over two lanes, one for the
+// real and one for the imaginary part, and the warp sum halves its values per
+// level (lane_fold).  The operator's column indices are kept as shared-memory
+// addresses within the cluster.
+//
+// The moments are those of the step kernels in a fixed order, whatever the
+// schedule.  Every thread of every CTA executes the same sequence of cluster
+// barriers (CTAs without rows still take part); there is no spin-wait.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
+#include <map>
+#include <mutex>
 #include <type_traits>
 
 #include "kpmgb_step.cuh"
@@ -34,10 +42,14 @@ using step::ffmac;
 using step::ffnorm2;
 using step::ff_epilogue;
 
-constexpr int kCT = 256;          // threads per CTA
-constexpr int kWarpsCT = kCT / 32;
+constexpr int kMaxThreads = 512;
 constexpr int kMaxCluster = 16;   // non-portable cluster size limit
 constexpr int kChunk = 8;         // nonzeros per anchored chunk (float-float)
+// shared memory kept free beside the slots (bounds the rows per CTA)
+constexpr size_t kReserved = 1280;
+// sums of the dots that one launch may store; longer recurrences take several
+// launches that pass the two slots through global memory
+constexpr size_t kSumBytes = size_t(64) << 20;
 
 struct ClusterParams {
   const int* rowptr;
@@ -45,14 +57,14 @@ struct ClusterParams {
   const void* val;
   int64_t NH;
   int NR;
-  int64_t NC;
   int lr;
-  const void* psi;           // row-major NH x NR block (loaded, scaled)
+  int64_t n0, n1;            // steps n0 .. n1 - 1 (1 is the first)
+  int last;                  // no launch follows
+  void* slot[2];             // row-major NH x NR blocks: v_{n0-1} and (n0 > 1)
+                             // v_{n0-2} in, at parity n & 1
   const void* bra;           // row-major NH x NR bra block (lr) or null
-  double2* mu;               // [NC][NR]
-  const double* mom_scale;   // per column (float-float) or null
-  double growth_limit;
-  unsigned* status;
+  double2* first;            // [warps][2][NR] sums of step 1
+  double2* later;            // [step][warps][dots][NR] sums of steps max(n0, 2) ..
   int rows;                  // rows per CTA (the last CTAs may own fewer)
   int cs;                    // CTAs per cluster
   int cap;                   // nonzeros a CTA's shared copy of its rows holds
@@ -79,9 +91,11 @@ __device__ __forceinline__ unsigned cluster_id() {
   asm volatile("mov.u32 %0, %%clusterid.x;" : "=r"(r));
   return r;
 }
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n"
-               "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
 // shared::cluster address of the same offset in CTA `rank`'s shared memory
 __device__ __forceinline__ uint32_t map_rank(uint32_t local, unsigned rank) {
@@ -102,113 +116,110 @@ __device__ __forceinline__ void ld_dsmem(uint32_t a, double2& v) {
                : "memory");
 }
 
-__device__ __forceinline__ void st_dsmem(uint32_t a, double2 v) {
-  asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v.x), "d"(v.y)
-               : "memory");
+__device__ __forceinline__ void ld_dsmem(uint32_t a, double& v) {
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
 }
 
-__device__ __forceinline__ void f64mac(double2& a, double h, double2 v) {
-  a.x = fma(h, v.x, a.x);
-  a.y = fma(h, v.y, a.y);
-}
-__device__ __forceinline__ void f64mac(double2& a, double2 h, double2 v) {
-  a.x = fma(h.x, v.x, a.x);
-  a.x = fma(-h.y, v.y, a.x);
-  a.y = fma(h.x, v.y, a.y);
-  a.y = fma(h.y, v.x, a.y);
-}
-__device__ __forceinline__ void f64dot(double2& acc, double2 a, double2 b) {  // += conj(a) b
-  acc.x = fma(a.x, b.x, fma(a.y, b.y, acc.x));
-  acc.y = fma(a.x, b.y, fma(-a.y, b.x, acc.y));
-}
-
-// CACHE: the CTA copies its rows of the operator (row pointers, columns,
-// values) into shared memory once, so a step reads no global memory but the
-// bra of the l/r path.
+// CACHE: the CTA copies its rows of the operator (row pointers, neighbour
+// addresses, values) into shared memory once, so a step reads no global memory
+// but the bra of the l/r path.
 template <bool FF, bool REALH, bool CACHE>
-__global__ void __launch_bounds__(kCT, 1) k_kpm1d_cluster(ClusterParams p) {
+__global__ void __launch_bounds__(kMaxThreads, 1) k_kpm1d_cluster(
+    const __grid_constant__ ClusterParams p) {
   using V = typename CVal<FF>::T;
   using HT = typename std::conditional<FF, typename FFVal<REALH>::T,
                                        typename std::conditional<REALH, double, double2>::type>::type;
+  constexpr uint32_t kElem = sizeof(V);
+  // lanes per row: FP64 splits a row into its real and imaginary part
+  constexpr int LR = FF ? 1 : 2;
   extern __shared__ __align__(16) unsigned char smem[];
-  V* slot = reinterpret_cast<V*>(smem);                          // [2][rows]
-  // partials of every CTA of the cluster, which each CTA stores into rank 0's
-  // copy (the other ranks' copies stay unused): [2 parity][kMaxCluster][2 dots]
-  double2* part = reinterpret_cast<double2*>(slot + 2 * p.rows);
-  double2* red = part + 2 * kMaxCluster * 2;                      // [2][kWarpsCT]
-  HT* s_val = reinterpret_cast<HT*>(red + 2 * kWarpsCT);          // [cap]  (CACHE)
-  int* s_col = reinterpret_cast<int*>(s_val + (CACHE ? p.cap : 0));  // [cap]
-  int* s_rowptr = s_col + (CACHE ? p.cap : 0);                       // [rows + 1]
+  V* slot = reinterpret_cast<V*>(smem);                               // [2][rows]
+  HT* s_val = reinterpret_cast<HT*>(slot + 2 * p.rows);                // [cap]  (CACHE)
+  uint32_t* s_adr = reinterpret_cast<uint32_t*>(s_val + (CACHE ? p.cap : 0));  // [cap]
+  int* s_rowptr = reinterpret_cast<int*>(s_adr + (CACHE ? p.cap : 0));         // [rows + 1]
   const unsigned rank = cluster_rank();
   const int c = (int)cluster_id();  // probe column of this cluster
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const int warp = tid >> 5, lane = tid & 31, nwarps = nt >> 5;
   const int64_t r0 = (int64_t)rank * p.rows;
   const int64_t left = p.NH - r0;
   const int own = left <= 0 ? 0 : (left < p.rows ? (int)left : p.rows);
   const uint32_t slot_base = (uint32_t)__cvta_generic_to_shared(slot);
-  const uint32_t part_base = (uint32_t)__cvta_generic_to_shared(part);
   const HT* __restrict__ val = static_cast<const HT*>(p.val);
-  const V* __restrict__ psi = static_cast<const V*>(p.psi);
   const V* __restrict__ bra = static_cast<const V*>(p.bra);
+  // slot-0 address of row j within the cluster (row j lives in CTA j / rows)
+  auto address = [&](int j) -> uint32_t {
+    const unsigned q = (unsigned)(j / p.rows);
+    return map_rank(slot_base + (uint32_t)(j - (int)q * p.rows) * kElem, q);
+  };
 
-  // v_0: this CTA's rows of probe column c (and its rows of the operator)
-  for (int i = tid; i < own; i += kCT) slot[i] = __ldg(psi + (r0 + i) * p.NR + c);
+  // v_{n0-1} and, past the first step, v_{n0-2}
+  for (int i = tid; i < own; i += nt) {
+    const int64_t g = (r0 + i) * p.NR + c;
+    const int x = (int)((p.n0 - 1) & 1);
+    slot[x * p.rows + i] = static_cast<const V*>(p.slot[x])[g];
+    if (p.n0 > 1) slot[(x ^ 1) * p.rows + i] = static_cast<const V*>(p.slot[x ^ 1])[g];
+  }
   if constexpr (CACHE) {
     if (own > 0) {
       const int kb = __ldg(p.rowptr + r0);
       const int nk = __ldg(p.rowptr + r0 + own) - kb;  // <= cap (host bound)
-      for (int i = tid; i <= own; i += kCT) s_rowptr[i] = __ldg(p.rowptr + r0 + i) - kb;
-      for (int k = tid; k < nk && k < p.cap; k += kCT) {
-        s_col[k] = __ldg(p.col + kb + k);
+      for (int i = tid; i <= own; i += nt) s_rowptr[i] = __ldg(p.rowptr + r0 + i) - kb;
+      for (int k = tid; k < nk && k < p.cap; k += nt) {
+        s_adr[k] = address(__ldg(p.col + kb + k));
         s_val[k] = __ldg(val + kb + k);
       }
     }
   }
-  cluster_sync();
+  cluster_arrive();
+  cluster_wait();
 
-  const int64_t N = p.lr ? p.NC - 1 : p.NC / 2;
-  for (int64_t n = 1; n <= N; ++n) {
-    const int xs = (int)((n - 1) & 1), ys = (int)(n & 1);
+  const int work = own * LR;
+  for (int64_t n = p.n0; n < p.n1; ++n) {
+    const int xs = (int)((n - 1) & 1), ys = xs ^ 1;
     const bool first = n == 1;
-    const int dot = p.lr ? (first ? DOT_LR2 : DOT_LR1) : DOT_DOUBLING;
-    double2 dd[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
-    // float-float: the dot terms of the thread's rows stay float-float
-    // (leading S, correction Cc; [dot][re/im]) through the warp's sum, so the
-    // step does no FP64 work but one join per warp
-    float fS[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, fC[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-    const uint32_t xbase = slot_base + (uint32_t)(xs * p.rows) * (uint32_t)sizeof(V);
-    for (int i = tid; i < own; i += kCT) {
-      const int64_t r = r0 + i;
+    const uint32_t xoff = (uint32_t)(xs * p.rows) * kElem;
+    // ---- y = H x, or 2 H x - z over z
+    for (int e = tid; e < work; e += nt) {
+      const int i = e / LR;
       // CACHE: row-local indices into the shared copy; else CSR positions
-      const int k0 = CACHE ? s_rowptr[i] : __ldg(p.rowptr + r);
-      const int k1 = CACHE ? s_rowptr[i + 1] : __ldg(p.rowptr + r + 1);
-      auto col_at = [&](int k) { return CACHE ? s_col[k] : __ldg(p.col + k); };
+      const int k0 = CACHE ? s_rowptr[i] : __ldg(p.rowptr + r0 + i);
+      const int k1 = CACHE ? s_rowptr[i + 1] : __ldg(p.rowptr + r0 + i + 1);
+      auto adr_at = [&](int k) { return (CACHE ? s_adr[k] : address(__ldg(p.col + k))) + xoff; };
       auto val_at = [&](int k) { return CACHE ? s_val[k] : __ldg(val + k); };
-      // neighbour row j lives in CTA j / rows at local index j % rows
-      auto gather = [&](int j, V& out) {
-        const unsigned q = (unsigned)(j / p.rows);
-        if (q < (unsigned)p.cs) {
-          const uint32_t loc = xbase + (uint32_t)(j - (int)q * p.rows) * (uint32_t)sizeof(V);
-          ld_dsmem(map_rank(loc, q), out);
-        } else {
-          atomicOr(p.status, (unsigned)STATUS_SCRATCH);
-          out = V{};
-        }
-      };
-      V y;
       if constexpr (!FF) {
-        double2 acc = make_double2(0.0, 0.0);
-        for (int k = k0; k < k1; ++k) {
-          double2 xv;
-          gather(col_at(k), xv);
-          f64mac(acc, val_at(k), xv);
+        const int part = e & 1;
+        double acc = 0.0;
+        for (int k = k0; k < k1; k += 4) {
+          // four gathers in flight
+          HT h[4];
+          double a[4], b[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            if (k + u >= k1) break;
+            h[u] = val_at(k + u);
+            if constexpr (REALH) {
+              ld_dsmem(adr_at(k + u) + 8 * part, a[u]);
+            } else {
+              double2 v;
+              ld_dsmem(adr_at(k + u), v);
+              a[u] = part ? v.y : v.x;
+              b[u] = part ? v.x : -v.y;
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            if (k + u >= k1) break;
+            if constexpr (REALH) {
+              acc = fma(h[u], a[u], acc);
+            } else {
+              acc = fma(h[u].x, a[u], acc);
+              acc = fma(h[u].y, b[u], acc);
+            }
+          }
         }
-        if (first) {
-          y = acc;
-        } else {
-          const double2 z = slot[ys * p.rows + i];
-          y = make_double2(2.0 * acc.x - z.x, 2.0 * acc.y - z.y);
-        }
+        double* const yp = reinterpret_cast<double*>(slot + ys * p.rows) + e;
+        *yp = first ? acc : fma(2.0, acc, -*yp);
       } else {
         float Sr = 0.f, Cr = 0.f, Si = 0.f, Ci = 0.f;
         for (int kc = k0; kc < k1; kc += kChunk) {
@@ -221,7 +232,7 @@ __global__ void __launch_bounds__(kCT, 1) k_kpm1d_cluster(ClusterParams p) {
           for (int u = 0; u < kChunk; ++u) {
             if (u < cnt) {
               hv[u] = val_at(kc + u);
-              gather(col_at(kc + u), xv[u]);
+              ld_dsmem(adr_at(kc + u), xv[u]);
             } else {
               step::hzero(hv[u]);
               xv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -261,133 +272,94 @@ __global__ void __launch_bounds__(kCT, 1) k_kpm1d_cluster(ClusterParams p) {
         if (!first) z = slot[ys * p.rows + i];
         const float2 yr = ff_epilogue(Sr, Cr, alpha, beta_mode, z.x, z.y);
         const float2 yi = ff_epilogue(Si, Ci, alpha, beta_mode, z.z, z.w);
-        y = make_float4(yr.x, yr.y, yi.x, yi.y);
+        // y overwrites z (this row only; other CTAs read the x slot this step)
+        slot[ys * p.rows + i] = make_float4(yr.x, yr.y, yi.x, yi.y);
       }
-      // dot terms of this row
-      const V xr = slot[xs * p.rows + i];
-      if constexpr (!FF) {
-        if (dot == DOT_DOUBLING) {
-          f64dot(dd[0], xr, xr);
-          f64dot(dd[1], xr, y);
-        } else {
-          const double2 b = __ldg(bra + r * p.NR + c);
-          if (dot == DOT_LR2) {
-            f64dot(dd[0], b, xr);
-            f64dot(dd[1], b, y);
-          } else {
-            f64dot(dd[0], b, y);
-          }
-        }
-      } else {
-        if (dot == DOT_DOUBLING) {
-          ffnorm2(fS[0], fC[0], xr);
-          ffdot(fS[1], fC[1], xr, y);
-        } else {
-          const float4 b = __ldg(bra + r * p.NR + c);
-          if (dot == DOT_LR2) {
-            ffdot(fS[0], fC[0], b, xr);
-            ffdot(fS[1], fC[1], b, y);
-          } else {
-            ffdot(fS[0], fC[0], b, y);
-          }
-        }
-      }
-      // y overwrites z (this row only; other CTAs read the x slot this step)
-      slot[ys * p.rows + i] = y;
     }
-    // fixed-order block reduction of the dot terms: a shuffle tree in every
-    // warp (float-float: merged by TwoSum, then joined once), then warp 0
-    // adds the warp sums in warp order
-    if constexpr (FF) {
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-        for (int k = 0; k < 2; ++k)
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            const float s2 = __shfl_down_sync(0xffffffffu, fS[k][q], off);
-            const float c2 = __shfl_down_sync(0xffffffffu, fC[k][q], off);
-            float sum, err;
-            ff::two_sum(fS[k][q], s2, sum, err);
-            fS[k][q] = sum;
-            fC[k][q] = __fadd_rn(fC[k][q], __fadd_rn(c2, err));
+    __syncwarp();
+    cluster_arrive();  // y of step n
+    // ---- the dots of the thread's own rows, while the others arrive:
+    // <x|x>, <x|y> (doubling), <b|x>, <b|y> or <b|y> alone (bra/ket)
+    const bool two = !p.lr || first;
+    double2 d[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+    if constexpr (!FF) {
+      double v[4] = {0.0, 0.0, 0.0, 0.0};
+      const double* xp = reinterpret_cast<const double*>(slot + xs * p.rows);
+      const double* yp = reinterpret_cast<const double*>(slot + ys * p.rows);
+      for (int e = tid; e < work; e += nt) {
+        const double x = xp[e], y = yp[e], yo = yp[e ^ 1];
+        if (!p.lr) {
+          v[0] = fma(x, x, v[0]);
+          v[2] = fma(x, y, v[2]);
+          v[3] = fma(e & 1 ? -x : x, yo, v[3]);
+        } else {
+          const double b =
+              __ldg(reinterpret_cast<const double*>(bra + (r0 + (e >> 1)) * p.NR + c) + (e & 1));
+          if (first) {
+            v[0] = fma(b, x, v[0]);
+            v[1] = fma(e & 1 ? -b : b, xp[e ^ 1], v[1]);
           }
-#pragma unroll
-      for (int k = 0; k < 2; ++k)
-        dd[k] = make_double2(ff::join(fS[k][0], fC[k][0]), ff::join(fS[k][1], fC[k][1]));
+          v[2] = fma(b, y, v[2]);
+          v[3] = fma(e & 1 ? -b : b, yo, v[3]);
+        }
+      }
+      // four values over 32 lanes: after two levels each lane holds one
+      step::lane_fold<4, 1>(
+          v, lane, [](double a, int off) { return __shfl_xor_sync(0xffffffffu, a, off); },
+          [](double a, double b) { return a + b; });
+      d[0] = make_double2(__shfl_sync(0xffffffffu, v[0], 0), __shfl_sync(0xffffffffu, v[0], 8));
+      d[1] = make_double2(__shfl_sync(0xffffffffu, v[0], 16), __shfl_sync(0xffffffffu, v[0], 24));
     } else {
-#pragma unroll
-      for (int k = 0; k < 2; ++k)
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-          dd[k].x += __shfl_down_sync(0xffffffffu, dd[k].x, off);
-          dd[k].y += __shfl_down_sync(0xffffffffu, dd[k].y, off);
-        }
-    }
-    const int warp = tid >> 5, lane = tid & 31;
-    if (lane == 0) {
-      red[warp] = dd[0];
-      red[kWarpsCT + warp] = dd[1];
-    }
-    __syncthreads();
-    if (warp == 0) {
-      double2 v[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
-      if (lane < kWarpsCT) {
-        v[0] = red[lane];
-        v[1] = red[kWarpsCT + lane];
-      }
-#pragma unroll
-      for (int k = 0; k < 2; ++k)
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-          v[k].x += __shfl_down_sync(0xffffffffu, v[k].x, off);
-          v[k].y += __shfl_down_sync(0xffffffffu, v[k].y, off);
-        }
-      // push this CTA's partials (the tree's totals are in lane 0) into rank
-      // 0's shared memory
-      if (lane == 0) {
-        const uint32_t dst = map_rank(
-            part_base + (uint32_t)((ys * kMaxCluster + (int)rank) * 2) * (uint32_t)sizeof(double2),
-            0u);
-        st_dsmem(dst, v[0]);
-        st_dsmem(dst + (uint32_t)sizeof(double2), v[1]);
-      }
-    }
-    cluster_sync();  // y and the partials of step n are visible cluster-wide
-    if (rank == 0 && tid < 2) {
-      const int k = tid;
-      const int nd = dot == DOT_LR1 ? 1 : 2;
-      if (k < nd) {
-        double2 s = make_double2(0.0, 0.0);
-        for (int q = 0; q < p.cs; ++q) {
-          const double2 v = part[(ys * kMaxCluster + q) * 2 + k];
-          s.x += v.x;
-          s.y += v.y;
-        }
-        if (p.mom_scale) {
-          s.x *= p.mom_scale[c];
-          s.y *= p.mom_scale[c];
-        }
-        double2 out = s;
-        int64_t idx;
-        if (p.lr) {
-          idx = first ? k : n;
-        } else if (first) {
-          idx = k;
+      float S[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, C[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+      for (int i = tid; i < own; i += nt) {
+        const float4 x = slot[xs * p.rows + i], y = slot[ys * p.rows + i];
+        if (!p.lr) {
+          ffnorm2(S[0], C[0], x);
+          ffdot(S[1], C[1], x, y);
         } else {
-          const double2 b0 = p.mu[(size_t)k * p.NR + c];
-          out.x = 2.0 * s.x - b0.x;
-          out.y = 2.0 * s.y - b0.y;
-          if (k == 0 && p.growth_limit > 0.0 && !(s.x <= p.growth_limit * b0.x))
-            atomicOr(p.status, (unsigned)STATUS_GROWTH);
-          idx = 2 * n - 2 + k;
+          const float4 b = __ldg(bra + (r0 + i) * p.NR + c);
+          if (first) ffdot(S[0], C[0], b, x);
+          ffdot(S[1], C[1], b, y);
         }
-        p.mu[(size_t)idx * p.NR + c] = out;
-        if (!isfinite(out.x) || !isfinite(out.y)) atomicOr(p.status, (unsigned)STATUS_NONFINITE);
       }
+      step::F3 v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] = step::F3{S[q >> 1][q & 1], C[q >> 1][q & 1], 0.f};
+      step::lane_fold<4, 1>(
+          v, lane,
+          [](step::F3 a, int off) {
+            return step::F3{__shfl_xor_sync(0xffffffffu, a.s, off),
+                            __shfl_xor_sync(0xffffffffu, a.c, off),
+                            __shfl_xor_sync(0xffffffffu, a.d, off)};
+          },
+          [](step::F3 a, step::F3 b) { return step::f3_merge(a, b); });
+      const double w = step::f3_join(v[0]);
+      d[0] = make_double2(__shfl_sync(0xffffffffu, w, 0), __shfl_sync(0xffffffffu, w, 8));
+      d[1] = make_double2(__shfl_sync(0xffffffffu, w, 16), __shfl_sync(0xffffffffu, w, 24));
+    }
+    if (lane < 2) {
+      const int64_t g = (int64_t)rank * nwarps + warp, G = (int64_t)p.cs * nwarps;
+      if (first) {
+        p.first[(g * 2 + lane) * p.NR + c] = d[lane];
+      } else if (two) {
+        const int64_t q = n - (p.n0 > 2 ? p.n0 : 2);
+        p.later[((q * G + g) * 2 + lane) * p.NR + c] = d[lane];
+      } else if (lane == 1) {
+        const int64_t q = n - (p.n0 > 2 ? p.n0 : 2);
+        p.later[(q * G + g) * p.NR + c] = d[1];
+      }
+    }
+    __syncwarp();
+    cluster_wait();  // y of step n is visible cluster-wide, x no longer read
+  }
+  // the two slots for the next launch
+  if (!p.last) {
+    for (int i = tid; i < own; i += nt) {
+      const int64_t g = (r0 + i) * p.NR + c;
+      static_cast<V*>(p.slot[0])[g] = slot[i];
+      static_cast<V*>(p.slot[1])[g] = slot[p.rows + i];
     }
   }
-  cluster_sync();  // no CTA exits while another may still store into it
 }
 
 template <bool FF, bool REALH>
@@ -398,36 +370,146 @@ const void* cluster_fn(bool cache) {
 
 }  // namespace
 
+namespace {
+
+// Clusters of 1..16 CTAs that the device holds side by side with one CTA per
+// SM (clusters lie within one of its processing clusters, so 16 CTAs fit far
+// fewer times than SMs / 16).
+const int* clusters_side_by_side() {
+  static std::mutex mtx;
+  static std::map<int, std::array<int, kMaxCluster + 1>> table;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lk(mtx);
+  auto it = table.find(dev);
+  if (it != table.end()) return it->second.data();
+  std::array<int, kMaxCluster + 1> side{};
+  const void* fn = cluster_fn<false, true>(true);
+  constexpr int kOnePerSm = 120 * 1024;  // more than half of an SM's shared memory
+  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kOnePerSm);
+  cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  for (int cs = 1; cs <= kMaxCluster; ++cs) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)cs);
+    cfg.blockDim = dim3(64);
+    cfg.dynamicSmemBytes = kOnePerSm;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cs;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess) side[cs] = n;
+  }
+  cudaGetLastError();
+  return table.emplace(dev, side).first->second.data();
+}
+
+struct ClusterShape {
+  int cs = 0;        // CTAs per cluster; 0: no cluster holds the rows
+  int64_t load = 0;  // rows of all columns on the busiest SM
+};
+
+int64_t max_rows_per_cta() {
+  int dev = 0, optin = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  return ((int64_t)optin - (int64_t)kReserved) / 32;  // two slots of 16 bytes
+}
+
+// The cluster size that leaves the busiest SM the fewest rows, counting the
+// columns that have to share SMs; rows per CTA stay at 32 or more.
+ClusterShape cluster_shape(int64_t NH, int NR) {
+  const int* side = clusters_side_by_side();
+  const int64_t max_rows = max_rows_per_cta();
+  ClusterShape s;
+  for (int k = 1; k <= kMaxCluster; ++k) {
+    const int64_t r = (NH + k - 1) / k;
+    if (r > max_rows || (k > 1 && r < 32) || side[k] < 1) continue;
+    const int64_t load = ((NR + side[k] - 1) / side[k]) * r;
+    if (s.cs == 0 || load < s.load) {
+      s.load = load;
+      s.cs = k;
+    }
+  }
+  return s;
+}
+
+// Shared memory of one CTA of `rows` rows with its rows of the operator; false
+// when that is more than a CTA can have.
+bool cached_bytes(const DeviceCSR& H, bool ff, int64_t rows, size_t* bytes, int64_t* cap) {
+  int dev = 0, optin = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  const bool real = H.is_real != 0;
+  const size_t hbytes = ff ? (real ? sizeof(float2) : sizeof(float4))
+                           : (real ? sizeof(double) : sizeof(double2));
+  *cap = rows * (int64_t)std::max(H.max_row_nnz, 1);
+  *bytes = 32 * (size_t)rows + (size_t)*cap * (hbytes + sizeof(int)) +
+           (size_t)(rows + 1) * sizeof(int);
+  return *cap < (1ll << 30) && *bytes + kReserved <= (size_t)optin;
+}
+
+}  // namespace
+
+// Whether one cluster launch is expected to beat a launch per step: both times
+// per step (us) from measurements on GB300 (2D lattices, 5 entries per real
+// row; Haldane, 10 per complex row), linear in the rows that the busiest SM
+// holds and in all rows x columns.  Measured, cluster / launches: FP64 real
+// NH = 1024, NR = 8 1.8 / 4.2; 4096, 12 3.8 / 7.2; 9216, 4 5.0 / 4.1; 16384, 4
+// 6.6 / 5.3; 16384, 12 10.2 / 15.8; float-float 4096, 12 2.2 / 3.6; 16384, 8
+// 4.1 / 6.0; 32761, 1 4.8 / 3.7; FP64 complex 2048, 8 4.7 / 6.6; 8192, 4 11.2 /
+// 6.6; float-float complex 8192, 4 3.8 / 4.3.  Rows whose operator does not fit
+// beside them, or more than 2048 on an SM, take launches (65536, 12 FP64 50 /
+// 34).
+bool cluster_is_faster(const DeviceCSR& H, int64_t NH, int NR, int precision) {
+  const bool ff = precision == KPMGB_PREC_FF, real = H.is_real != 0;
+  const ClusterShape shape = cluster_shape(NH, NR);
+  size_t bytes = 0;
+  int64_t cap = 0;
+  if (shape.cs < 1 || shape.load > 2048 ||
+      !cached_bytes(H, ff, (NH + shape.cs - 1) / shape.cs, &bytes, &cap))
+    return false;
+  const double row = (double)H.nnz / (double)NH / (real ? 5.0 : 10.0);
+  const double load = row * (double)shape.load, work = row * (double)NH * NR;
+  double cluster, launches;
+  if (!ff) {
+    cluster = 2.2 + (real ? 0.0044 : 0.0165) * load;
+    launches = real ? std::max(4.1, 2.2 + 5.8e-5 * work) : std::max(6.4, 1.0 + 1.25e-4 * work);
+  } else {
+    cluster = real ? 1.6 + 0.0017 * load : 2.0 + 0.0038 * load;
+    if (NR <= 8)
+      launches = real ? 3.5 + 1.9e-5 * work : 4.0 + 2.9e-5 * work;
+    else
+      launches = real ? 2.6 + 1.1e-5 * work : 2.8 + 2.4e-5 * work;
+  }
+  return cluster < launches;
+}
+
 int launch_kpm1d_cluster(const DeviceCSR& H, int64_t NH, int NR, int64_t NC, bool lr,
-                         int precision, const void* psi, const void* bra, double2* mu,
-                         const double* mom_scale, double growth_limit, unsigned* status,
-                         cudaStream_t s) {
+                         int precision, void* const (&slots)[2], const void* bra, DevBuf& sums,
+                         const MomentArgs& m0, cudaStream_t s) {
   if (NR < 1) return fail(KPMGB_ERR_ARGUMENT, "Invalid NR=%d", NR);
   const bool ff = precision == KPMGB_PREC_FF;
   const bool real = H.is_real != 0;
-  int dev = 0, smem_optin = 0;
-  KPMGB_CUDA(cudaGetDevice(&dev));
-  KPMGB_CUDA(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  const size_t fixed = (2 * kMaxCluster * 2 + 2 * kWarpsCT) * sizeof(double2);
-  const size_t elem = 16;  // float4 or double2
-  const int64_t max_rows = ((int64_t)smem_optin - (int64_t)fixed) / (2 * (int64_t)elem);
-  // cluster size: rows per CTA near 512 for parallelism, and within capacity
-  int cs = 1;
-  while (cs < kMaxCluster && ((NH + cs - 1) / cs > 512 || (NH + cs - 1) / cs > max_rows)) cs *= 2;
-  const int64_t rows = (NH + cs - 1) / cs;
-  if (rows > max_rows)
+  const int64_t max_rows = max_rows_per_cta();
+  if ((NH + kMaxCluster - 1) / kMaxCluster > max_rows)
     return fail(KPMGB_ERR_ARGUMENT,
                 "the cluster-resident kernel holds at most %lld rows per probe column "
                 "(%d CTAs of %lld rows)",
                 (long long)(kMaxCluster * max_rows), kMaxCluster, (long long)max_rows);
-  size_t smem = fixed + 2 * (size_t)rows * elem;
+  const int cs = cluster_shape(NH, NR).cs;
+  if (cs < 1) return fail(KPMGB_ERR_ARGUMENT, "the device holds no thread-block clusters");
+  const int64_t rows = (NH + cs - 1) / cs;
   // the CTA's rows of the operator in shared memory when they fit
-  const size_t hbytes = ff ? (real ? sizeof(float2) : sizeof(float4))
-                           : (real ? sizeof(double) : sizeof(double2));
-  const int64_t cap = rows * (int64_t)std::max(H.max_row_nnz, 1);
-  const size_t cache_bytes = (size_t)cap * (hbytes + sizeof(int)) + (size_t)(rows + 1) * sizeof(int);
-  const bool cache = cap < (1ll << 30) && smem + cache_bytes <= (size_t)smem_optin;
-  if (cache) smem += cache_bytes;
+  size_t smem = 0;
+  int64_t cap = 0;
+  const bool cache = cached_bytes(H, ff, rows, &smem, &cap);
+  if (!cache) smem = 32 * (size_t)rows;
+  const int64_t lanes = rows * (ff ? 1 : 2);
+  const int threads = (int)std::min<int64_t>(kMaxThreads, std::max<int64_t>(64, (lanes + 31) / 32 * 32));
   const void* fn = ff ? (real ? cluster_fn<true, true>(cache) : cluster_fn<true, false>(cache))
                       : (real ? cluster_fn<false, true>(cache) : cluster_fn<false, false>(cache));
   // setup failures (no cluster support, attribute limits) are "does not
@@ -443,7 +525,7 @@ int launch_kpm1d_cluster(const DeviceCSR& H, int64_t NH, int NR, int64_t NC, boo
     KPMGB_TRY(setup(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(NR * cs));
-  cfg.blockDim = dim3(kCT);
+  cfg.blockDim = dim3((unsigned)threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
@@ -458,26 +540,50 @@ int launch_kpm1d_cluster(const DeviceCSR& H, int64_t NH, int NR, int64_t NC, boo
   if (nclusters < 1)
     return fail(KPMGB_ERR_ARGUMENT, "a cluster of %d CTAs with %zu bytes of shared memory each "
                                     "cannot be resident on this device", cs, smem);
+  const int64_t N = lr ? NC - 1 : NC / 2;  // steps
+  const int G = cs * (threads / 32);
+  const int nd = lr ? 1 : 2;
+  const size_t first_bytes = (size_t)G * 2 * NR * sizeof(double2);
+  const size_t step_bytes = (size_t)G * nd * NR * sizeof(double2);
+  const int64_t hold = std::max<int64_t>(
+      1, std::min<int64_t>(N - 1, (int64_t)(kSumBytes / step_bytes)));
+  KPMGB_TRY(sums.ensure(std::max(sums.bytes, first_bytes + (size_t)hold * step_bytes)));
   ClusterParams p;
   p.rowptr = H.rowptr;
   p.col = H.col;
   p.val = ff ? H.val_ff : (real ? (const void*)H.val_real : (const void*)H.val);
   p.NH = NH;
   p.NR = NR;
-  p.NC = NC;
   p.lr = lr ? 1 : 0;
-  p.psi = psi;
+  p.slot[0] = slots[0];
+  p.slot[1] = slots[1];
   p.bra = bra;
-  p.mu = mu;
-  p.mom_scale = mom_scale;
-  p.growth_limit = growth_limit;
-  p.status = status;
+  p.first = sums.as<double2>();
+  p.later = reinterpret_cast<double2*>(sums.as<char>() + first_bytes);
   p.rows = (int)rows;
   p.cs = cs;
   p.cap = cache ? (int)cap : 0;
-  void* args[] = {&p};
-  KPMGB_CUDA(cudaLaunchKernelExC(&cfg, fn, args));
-  KPMGB_LAUNCHED();
+  MomentArgs m = m0;
+  for (int64_t n = 1; n <= N;) {
+    const int64_t later = std::max<int64_t>(n, 2);
+    p.n0 = n;
+    p.n1 = std::min<int64_t>(N + 1, later + hold);
+    p.last = p.n1 > N;
+    void* args[] = {&p};
+    KPMGB_CUDA(cudaLaunchKernelExC(&cfg, fn, args));
+    KPMGB_LAUNCHED();
+    if (n == 1) {
+      m.mom = MOM_STORE;
+      m.i0 = 0;
+      m.growth_limit = 0.0;
+      KPMGB_TRY(launch_finish_sums(p.first, G, 2, NR, 1, m, s));
+    }
+    m.mom = lr ? MOM_STORE : MOM_DOUBLING;
+    m.i0 = lr ? later : 2 * later - 2;
+    m.growth_limit = m0.growth_limit;
+    if (p.n1 > later) KPMGB_TRY(launch_finish_sums(p.later, G, nd, NR, p.n1 - later, m, s));
+    n = p.n1;
+  }
   return KPMGB_OK;
 }
 

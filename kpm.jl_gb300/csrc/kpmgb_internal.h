@@ -325,11 +325,17 @@ int launch_mn_sym(double2* mu, int NC, cudaStream_t s);
 
 // Cluster-resident recurrence (kpmgb_cluster.cu): one thread-block cluster
 // per probe column holds the column's recurrence in distributed shared memory;
-// psi / bra are the loaded row-major NH x NR blocks; moments [NC][NR].
+// slots[0] / bra are the loaded row-major NH x NR blocks (both slots are
+// overwritten), `sums` the scratch of the dots' sums, m the moments [NC][NR].
 int launch_kpm1d_cluster(const DeviceCSR& H, int64_t NH, int NR, int64_t NC, bool lr,
-                         int precision, const void* psi, const void* bra, double2* mu,
-                         const double* mom_scale, double growth_limit, unsigned* status,
-                         cudaStream_t s);
+                         int precision, void* const (&slots)[2], const void* bra, DevBuf& sums,
+                         const MomentArgs& m, cudaStream_t s);
+// Whether that is expected to take less time than a launch per step.
+bool cluster_is_faster(const DeviceCSR& H, int64_t NH, int NR, int precision);
+// Moments of nsteps steps from their sums, [step][G][nd][NR], as
+// launch_recurrence makes them from its block sums.
+int launch_finish_sums(const double2* sums, int G, int nd, int NR, int64_t nsteps,
+                       const MomentArgs& m, cudaStream_t s);
 
 // Launch shape of the ensemble kernels (chosen by their autotuner): threads
 // per CTA, CSR rows or padded float-float rows, and the schedule -- rows == 0:

@@ -89,38 +89,44 @@ k_kubo_harmonics(const double2* __restrict__ mu, int NC, const double* __restric
 }
 
 // phi[j] = w / s_j^3 Re S_j.  32 nodes per block, the harmonics in 16
-// interleaved parts, then the parts in order.  A thread turns (cos, sin) of its
-// harmonic on by 16 theta_j (four products and sums, an error of about one
-// rounding per turn, 64 turns at NC = 512), which takes as many FP64 operations
-// as the four sums and no memory: 64 us of the FP64 pipe at Q = 4096.  (Exact
-// angles from a table came out 1e-14 apart from the reference's formula, whose
-// theta_j, s_j all follow from the rounded x_j.)
+// interleaved parts, then the parts in order.  Harmonic part + 16 t of a node is
+// the product of its turns by part and by 16 t, both from sincos: the second
+// in shared memory, 64 of them at a time for the block's 16 parts.  So every
+// harmonic carries two roundings (turning it on and on by 16 theta_j came out
+// 1e-14 apart from the direct sums), for 4 FP64 operations beside the 4 of the
+// sums: 64 us of the FP64 pipe at NC = 512, Q = 4096, and half as much for the
+// turns.
 __global__ void __launch_bounds__(kNodeThreads)
 k_kubo_nodes(const double2* __restrict__ coef, int NK, int64_t Q, const double* __restrict__ x,
              const double* __restrict__ sn, double w, double* __restrict__ phi) {
   constexpr int kParts = kNodeThreads / kNodesPerBlock;
+  constexpr int kTurns = 64;
+  __shared__ double2 turn[kTurns][kNodesPerBlock];
   __shared__ double red[kParts][kNodesPerBlock];
   const int part = threadIdx.x / kNodesPerBlock, l = threadIdx.x % kNodesPerBlock;
   const int64_t j = blockIdx.x * (int64_t)kNodesPerBlock + l;
-  double a = 0.0;
-  if (j < Q) {
-    const double th = acos(x[j]);
-    double cs, ss, c, s;  // the turn, and the harmonic
-    sincos((double)kParts * th, &ss, &cs);
-    sincos((double)part * th, &s, &c);
-    double ca = 0.0, ce = 0.0, sg = 0.0, sd = 0.0;
-    for (int k = part; k < NK; k += kParts) {
-      const double2 u = __ldg(coef + k), v = __ldg(coef + NK + k);
+  const double th = j < Q ? acos(x[j]) : 0.0;
+  double c0, s0;
+  sincos((double)part * th, &s0, &c0);
+  double ca = 0.0, ce = 0.0, sg = 0.0, sd = 0.0;
+  for (int k0 = 0; k0 < NK; k0 += kParts * kTurns) {
+    __syncthreads();
+    for (int t = part; t < kTurns && k0 + kParts * t < NK; t += kParts) {
+      double st, ct;
+      sincos((double)(k0 + kParts * t) * th, &st, &ct);
+      turn[t][l] = make_double2(ct, st);
+    }
+    __syncthreads();
+    for (int t = 0, k = k0 + part; t < kTurns && k < NK; ++t, k += kParts) {
+      const double2 u = __ldg(coef + k), v = __ldg(coef + NK + k), r = turn[t][l];
+      const double c = fma(c0, r.x, -s0 * r.y), s = fma(s0, r.x, c0 * r.y);
       ca = fma(u.x, c, ca);
       ce = fma(u.y, c, ce);
       sg = fma(v.x, s, sg);
       sd = fma(v.y, s, sd);
-      const double t = fma(c, cs, -s * ss);
-      s = fma(s, cs, c * ss);
-      c = t;
     }
-    a = x[j] * (ca - sd) + sn[j] * (ce + sg);
   }
+  double a = j < Q ? x[j] * (ca - sd) + sn[j] * (ce + sg) : 0.0;
   red[part][l] = a;
   __syncthreads();
   if (part == 0 && j < Q) {

@@ -37,12 +37,15 @@ namespace {
 using namespace step;
 
 // --------------------------------------------------------------- dispatch
-Shape pick_shape(int ncols) {
+// 9..12 columns: FP64 takes four lanes of three columns, which leaves none of
+// its scarce FP64 lanes idle (NH = 262144, 12 columns 106 us per step against
+// the 144 of 16 lanes); float-float takes 16 lanes (more rows in flight).
+Shape pick_shape(int ncols, int precision) {
   if (ncols <= 1) return {1, 1};
   if (ncols <= 2) return {2, 1};
   if (ncols <= 4) return {4, 1};
   if (ncols <= 8) return {8, 1};
-  if (ncols <= 12) return {4, 3};
+  if (ncols <= 12 && precision == KPMGB_PREC_FP64) return {4, 3};
   if (ncols <= 16) return {16, 1};
   if (ncols <= 32) return {32, 1};
   if (ncols <= 64) return {32, 2};
@@ -51,10 +54,10 @@ Shape pick_shape(int ncols) {
 
 // Register-gather shapes that cover ncols columns with at most 4x idle lanes,
 // the automatic one first (candidates of the autotuner).
-std::vector<Shape> candidate_shapes(int ncols) {
+std::vector<Shape> candidate_shapes(int ncols, int precision) {
   static const Shape all[] = {{1, 1}, {2, 1}, {4, 1}, {8, 1}, {4, 3},
                               {16, 1}, {32, 1}, {32, 2}, {32, 4}};
-  std::vector<Shape> out{pick_shape(ncols)};
+  std::vector<Shape> out{pick_shape(ncols, precision)};
   for (const Shape& s : all) {
     const int cover = s.lpr * s.cpl;
     if (cover >= ncols && cover <= 4 * std::max(ncols, 8) &&
@@ -64,12 +67,12 @@ std::vector<Shape> candidate_shapes(int ncols) {
   return out;
 }
 
-Shape shape_for(const StepArgs& a, int ncols) {
+Shape shape_for(const StepArgs& a, int ncols, int precision) {
   if (a.shape > 0) {
     const Shape s{a.shape / 10, a.shape % 10};
     if (s.lpr * s.cpl >= ncols) return s;
   }
-  return pick_shape(ncols);
+  return pick_shape(ncols, precision);
 }
 
 KernelFn select_kernel(Shape s, int precision, int dot, bool real) {
@@ -310,7 +313,7 @@ int choose_step(const StepArgs& a, int precision, int ncols, StepChoice* out) {
       return fail(KPMGB_ERR_ARGUMENT, "the padded-row kernel serves float-float steps with 5..64 "
                                       "columns and rows of at most 16 nonzeros");
   }
-  const Shape sh = shape_for(a, ncols);
+  const Shape sh = shape_for(a, ncols, precision);
   KPMGB_TRY(take(select_kernel(sh, precision, a.dot, real), sh.lpr));
   // The FP64 step of a complex operator is bound by each SM's FP64 pipe.  A
   // grid that leaves some of the resident slots free, but fewer than it needs,
@@ -508,6 +511,22 @@ int launch_step(const StepArgs& a, int precision, cudaStream_t s) {
   return launch_steps(&a, 1, precision, s);
 }
 
+int launch_finish_sums(const double2* sums, int G, int nd, int NR, int64_t nsteps,
+                       const MomentArgs& m, cudaStream_t s) {
+  FinishParams f;
+  f.partials = sums;
+  f.stride = (int64_t)G * nd * NR;
+  f.G = G;
+  f.nd = nd;
+  f.ncols = NR;
+  f.c0 = 0;
+  f.ld = NR;
+  f.m = m;
+  k_finish_moments<<<dim3((unsigned)nsteps, (unsigned)((nd * NR + 31) / 32)), 256, 0, s>>>(f);
+  KPMGB_LAUNCHED();
+  return KPMGB_OK;
+}
+
 int recurrence_scratch_bytes(const StepArgs& a0, int precision, int64_t NC, bool lr,
                              size_t* bytes, size_t* least) {
   // 32 MiB of block sums stay in L2 and cover 25 steps of the widest grids
@@ -581,7 +600,7 @@ int tune_step(const StepArgs& a0, int precision, DevBuf& partials, cudaStream_t 
     int variant, shape;
   };
   std::vector<Cand> cands;
-  for (const Shape& c : candidate_shapes(a0.NR)) cands.push_back({1, c.lpr * 10 + c.cpl});
+  for (const Shape& c : candidate_shapes(a0.NR, precision)) cands.push_back({1, c.lpr * 10 + c.cpl});
   if (precision == KPMGB_PREC_FF && a0.H->ell_w > 0 &&
       select_kernel_ffe(a0.NR, a0.dot, a0.H->is_real != 0))
     cands.push_back({9, 0});

@@ -56,3 +56,32 @@ def test_bra_ket(L, NR, NC, prec):
     # recurrence is relative to the unit norms
     ref = ko.kpm_1d_lr(H, NC, pl, pr)
     assert np.abs(got - ref).max() < TOL[prec]
+
+
+@pytest.mark.parametrize("prec", ["fp64", "ff"])
+@pytest.mark.parametrize("lr", [False, True])
+@pytest.mark.parametrize("L,NR,NC", [
+    (6, 3, 40),      # one CTA
+    (9, 1, 5),       # two CTAs, the second of fewer rows
+    (33, 5, 1001),   # sixteen CTAs, odd rows
+    (64, 17, 35),    # clusters that share SMs
+    (40, 28, 3000),  # two launches: the slots pass through global memory
+])
+def test_cluster(L, NR, NC, lr, prec):
+    rng = np.random.default_rng(L + NR)
+    if lr:
+        H, _, _, _ = models.haldane(L, max(3, L // 3))
+        H = (H / 4.5).tocsc()
+    else:
+        H = (models.square_anderson(L, W=2.0, rng=rng) / 5.1).tocsc()
+        NC += NC % 2
+    NH = H.shape[0]
+    pr = ko.random_phase_vectors(rng, NH, NR)
+    if lr:
+        pl = ko.random_phase_vectors(rng, NH, NR)
+        got = kg.kpm_1d(H, NC, NR, psi_in_l=pl, psi_in_r=pr, avg_output=False, precision=prec,
+                        kernel="cluster")
+        assert np.abs(got - ko.kpm_1d_lr(H, NC, pl, pr)).max() < TOL[prec]
+    else:
+        got = kg.kpm_1d(H, NC, NR, psi_in=pr, avg_output=False, precision=prec, kernel="cluster")
+        assert relerr(got, ko.kpm_1d_doubling(H, NC, pr)) < TOL[prec]
