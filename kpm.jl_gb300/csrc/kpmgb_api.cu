@@ -195,8 +195,8 @@ int run_kpm1d(Operator* op, int64_t NC, int64_t NR, int64_t NH, const void* psi_
       variant != 10 && variant != 11)
     return fail(KPMGB_ERR_ARGUMENT, "unknown kernel_variant %d", variant);
   const bool auto_cluster =
-      variant == 0 && cluster_auto_on && cluster_is_faster(op->csr, NH, (int)NR, precision);
-  // Float-float doubling calls with 9..64 columns on real operators of at
+      variant == 0 && cluster_auto_on && cluster_is_faster(op->csr, NH, (int)NR, precision, lr);
+  // Float-float doubling calls with 2..64 columns on real operators of at
   // most 8 nonzeros per row keep their vectors in the paired element layout
   // and run every step on packed FP32 pairs (k_step_ffpk / k_step_ffpk1;
   // KPMGB_PAIRED=0 keeps the standard layout and k_step_ffr).
@@ -204,7 +204,8 @@ int run_kpm1d(Operator* op, int64_t NC, int64_t NR, int64_t NH, const void* psi_
     const char* e = std::getenv("KPMGB_PAIRED");
     return !(e && std::atoi(e) == 0);
   }();
-  const bool paired = paired_on && ff && !lr && !auto_cluster && (variant == 0 || variant == 11) &&
+  const bool paired = paired_on && ff && !lr && !auto_cluster &&
+                      (variant == 0 || (variant == 11 && NR >= 9)) &&
                       packed_step_applies(op->csr, (int)NR);
   KPMGB_TRY(launch_load_block(psi_r, sl[0], NH, (int)NR, precision, sc, false, s,
                               paired ? VEC_PAIRED : VEC_STD));

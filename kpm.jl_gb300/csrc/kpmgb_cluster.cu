@@ -459,12 +459,13 @@ bool cached_bytes(const DeviceCSR& H, bool ff, int64_t rows, size_t* bytes, int6
 // row; Haldane, 10 per complex row), linear in the rows that the busiest SM
 // holds and in all rows x columns.  Measured, cluster / launches: FP64 real
 // NH = 1024, NR = 8 1.8 / 4.2; 4096, 12 3.8 / 7.2; 9216, 4 5.0 / 4.1; 16384, 4
-// 6.6 / 5.3; 16384, 12 10.2 / 15.8; float-float 4096, 12 2.2 / 3.6; 16384, 8
-// 4.1 / 6.0; 32761, 1 4.8 / 3.7; FP64 complex 2048, 8 4.7 / 6.6; 8192, 4 11.2 /
-// 6.6; float-float complex 8192, 4 3.8 / 4.3.  Rows whose operator does not fit
+// 6.6 / 5.3; 16384, 12 10.2 / 15.8; float-float 4096, 12 2.2 / 3.5; 16384, 8
+// 4.1 / 4.4; 32761, 1 4.8 / 3.7; FP64 complex 2048, 8 4.7 / 6.6; 8192, 4 11.2 /
+// 6.6; float-float complex 8192, 4 3.8 / 4.3 (float-float real, 16384, 4
+// 3.0 / 4.0 and 32761, 4 4.8 / 4.5 with the packed step).  Rows whose operator does not fit
 // beside them, or more than 2048 on an SM, take launches (65536, 12 FP64 50 /
 // 34).
-bool cluster_is_faster(const DeviceCSR& H, int64_t NH, int NR, int precision) {
+bool cluster_is_faster(const DeviceCSR& H, int64_t NH, int NR, int precision, bool lr) {
   const bool ff = precision == KPMGB_PREC_FF, real = H.is_real != 0;
   const ClusterShape shape = cluster_shape(NH, NR);
   size_t bytes = 0;
@@ -480,10 +481,10 @@ bool cluster_is_faster(const DeviceCSR& H, int64_t NH, int NR, int precision) {
     launches = real ? std::max(4.1, 2.2 + 5.8e-5 * work) : std::max(6.4, 1.0 + 1.25e-4 * work);
   } else {
     cluster = real ? 1.6 + 0.0017 * load : 2.0 + 0.0038 * load;
-    if (NR <= 8)
-      launches = real ? 3.5 + 1.9e-5 * work : 4.0 + 2.9e-5 * work;
+    if (real)
+      launches = !lr && packed_step_applies(H, NR) ? 2.7 + 1.15e-5 * work : 3.5 + 1.9e-5 * work;
     else
-      launches = real ? 2.6 + 1.1e-5 * work : 2.8 + 2.4e-5 * work;
+      launches = NR <= 8 ? 4.0 + 2.9e-5 * work : 2.8 + 2.4e-5 * work;
   }
   return cluster < launches;
 }

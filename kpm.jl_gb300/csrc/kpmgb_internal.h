@@ -331,7 +331,7 @@ int launch_kpm1d_cluster(const DeviceCSR& H, int64_t NH, int NR, int64_t NC, boo
                          int precision, void* const (&slots)[2], const void* bra, DevBuf& sums,
                          const MomentArgs& m, cudaStream_t s);
 // Whether that is expected to take less time than a launch per step.
-bool cluster_is_faster(const DeviceCSR& H, int64_t NH, int NR, int precision);
+bool cluster_is_faster(const DeviceCSR& H, int64_t NH, int NR, int precision, bool lr);
 // Moments of nsteps steps from their sums, [step][G][nd][NR], as
 // launch_recurrence makes them from its block sums.
 int launch_finish_sums(const double2* sums, int G, int nd, int NR, int64_t nsteps,

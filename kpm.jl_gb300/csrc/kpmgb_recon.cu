@@ -88,12 +88,20 @@ k_kubo_harmonics(const double2* __restrict__ mu, int NC, const double* __restric
   }
 }
 
+// (cos, sin)(k th) of the exact product: its rounding is k th 2^-53, which a
+// thousand harmonics would add up to 1e-13 of the conductivity.
+__device__ __forceinline__ double2 turn_by(int k, double th) {
+  const double a = (double)k * th, lo = fma((double)k, th, -a);
+  double s, c;
+  sincos(a, &s, &c);
+  return make_double2(fma(-lo, s, c), fma(lo, c, s));
+}
+
 // phi[j] = w / s_j^3 Re S_j.  32 nodes per block, the harmonics in 16
 // interleaved parts, then the parts in order.  Harmonic part + 16 t of a node is
 // the product of its turns by part and by 16 t, both from sincos: the second
 // in shared memory, 64 of them at a time for the block's 16 parts.  So every
-// harmonic carries two roundings (turning it on and on by 16 theta_j came out
-// 1e-14 apart from the direct sums), for 4 FP64 operations beside the 4 of the
+// harmonic carries two roundings, for 4 FP64 operations beside the 4 of the
 // sums: 64 us of the FP64 pipe at NC = 512, Q = 4096, and half as much for the
 // turns.
 __global__ void __launch_bounds__(kNodeThreads)
@@ -106,20 +114,16 @@ k_kubo_nodes(const double2* __restrict__ coef, int NK, int64_t Q, const double* 
   const int part = threadIdx.x / kNodesPerBlock, l = threadIdx.x % kNodesPerBlock;
   const int64_t j = blockIdx.x * (int64_t)kNodesPerBlock + l;
   const double th = j < Q ? acos(x[j]) : 0.0;
-  double c0, s0;
-  sincos((double)part * th, &s0, &c0);
+  const double2 t0 = turn_by(part, th);
   double ca = 0.0, ce = 0.0, sg = 0.0, sd = 0.0;
   for (int k0 = 0; k0 < NK; k0 += kParts * kTurns) {
     __syncthreads();
-    for (int t = part; t < kTurns && k0 + kParts * t < NK; t += kParts) {
-      double st, ct;
-      sincos((double)(k0 + kParts * t) * th, &st, &ct);
-      turn[t][l] = make_double2(ct, st);
-    }
+    for (int t = part; t < kTurns && k0 + kParts * t < NK; t += kParts)
+      turn[t][l] = turn_by(k0 + kParts * t, th);
     __syncthreads();
     for (int t = 0, k = k0 + part; t < kTurns && k < NK; ++t, k += kParts) {
       const double2 u = __ldg(coef + k), v = __ldg(coef + NK + k), r = turn[t][l];
-      const double c = fma(c0, r.x, -s0 * r.y), s = fma(s0, r.x, c0 * r.y);
+      const double c = fma(t0.x, r.x, -t0.y * r.y), s = fma(t0.y, r.x, t0.x * r.y);
       ca = fma(u.x, c, ca);
       ce = fma(u.y, c, ce);
       sg = fma(v.x, s, sg);

@@ -1,6 +1,6 @@
 // Row-streaming float-float step on packed FP32 pairs (k_step_ffpk): real
 // operators, 33..64 columns (two per lane), doubling dots; k_step_ffpk1 below
-// serves 9..32 columns (one per lane).
+// serves 2..32 columns (one per lane).
 //
 // Blackwell executes `fma/add/sub/mul.rn.f32x2` on a 64-bit register pair:
 // one instruction for two correctly rounded FP32 operations.  For real H the
@@ -223,9 +223,12 @@ __global__ void __launch_bounds__(kThreads, 2) k_step_ffpk(
 }
 
 // ---------------------------------------------------------------------------
-// One column per lane (k_step_ffpk1): the packed row-streaming step for 9..32
+// One column per lane (k_step_ffpk1): the packed row-streaming step for 2..32
 // columns, LPR lanes per row (RPW = 32 / LPR rows per warp), with half the
-// loads per lane of k_step_ffpk and so three blocks per SM.
+// loads per lane of k_step_ffpk and so three blocks per SM.  Bound by the
+// gathers from L2; below 9 columns the CSR kernel, whose rows wait for their
+// row pointers and column indices in turn, took 14.4 us per step at
+// NH = 65536, NR = 8.
 template <int LPR, int W>
 __global__ void __launch_bounds__(kThreads, 3) k_step_ffpk1(
     const __grid_constant__ KBatch batch) {
@@ -576,6 +579,9 @@ KernelFn ffpk1_w(int max_row_nnz) {
 
 KernelFn select_kernel_ffpk(int ncols, bool real, int max_row_nnz, int ell_w) {
   if (!real || ell_w != 8 || max_row_nnz > 8) return nullptr;
+  if (ncols == 2) return ffpk1_w<2>(max_row_nnz);
+  if (ncols == 3 || ncols == 4) return ffpk1_w<4>(max_row_nnz);
+  if (ncols >= 5 && ncols <= 8) return ffpk1_w<8>(max_row_nnz);
   if (ncols >= 9 && ncols <= 16) return ffpk1_w<16>(max_row_nnz);
   if (ncols >= 17 && ncols <= 32) return ffpk1_w<32>(max_row_nnz);
   if (ncols < 33 || ncols > 64) return nullptr;
@@ -589,7 +595,9 @@ KernelFn select_kernel_ffpk(int ncols, bool real, int max_row_nnz, int ell_w) {
   }
 }
 
-int ffpk_lanes(int ncols) { return ncols <= 16 ? 16 : 32; }
+int ffpk_lanes(int ncols) {
+  return ncols <= 2 ? 2 : ncols <= 4 ? 4 : ncols <= 8 ? 8 : ncols <= 16 ? 16 : 32;
+}
 
 PackedStep select_packed_step(int ncols, bool real, int max_row_nnz, int ell_w) {
   PackedStep ps;

@@ -30,6 +30,7 @@ def _lib(built_lib):
     (40, 3, 4),        # one later step
     (330, 9, 34),      # more than 64 row tiles per block
     (130, 33, 20),     # 66 entries: a ragged third chunk
+    (191, 2, 64), (191, 3, 64), (191, 5, 64), (191, 8, 64),  # narrow packed rows
 ])
 def test_doubling(L, NR, NC, prec):
     rng = np.random.default_rng(L)
