@@ -20,9 +20,10 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
-#include "kpmgb_internal.h"
+#include "kpmgb_step.cuh"
 
 namespace kpmgb {
 namespace {
@@ -32,7 +33,7 @@ constexpr int kAdjThreads = 256;
 struct AdjParams {
   const int* rowptr;
   const int* col;
-  const double2* val;     // complex values (FP64)
+  const void* val;        // double (real operators) or double2
   int64_t NH;
   int NR;
   const double2* lam1;    // lambda_k+1
@@ -48,64 +49,137 @@ struct AdjParams {
   double2* grad;          // per stored entry (CSR order), accumulated
 };
 
-// One lane group of LPR lanes per row; lane owns column lg (NR <= LPR).
+// Sums v[0..8) over the lanes lg = 0 .. LPR-1 of a group, the lanes of a pair
+// each taking half of the values as long as there are several: 8 FP64 additions
+// for four entries' products over 16 lanes instead of 32.  Value base + i,
+// i < count, of the group is then v[i].
 template <int LPR>
-__global__ void __launch_bounds__(kAdjThreads) k_adjoint_step(AdjParams p) {
+__device__ __forceinline__ int group_fold(double (&v)[8], int lg, unsigned mask, int& count) {
+  int base = 0, cnt = 8;
+#pragma unroll
+  for (int off = LPR / 2; off > 0; off >>= 1) {
+    if (cnt > 1) {
+      const int h = cnt / 2;
+      const bool up = (lg & off) != 0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (i < h) {
+          const double keep = up ? v[i + h] : v[i];
+          const double send = up ? v[i] : v[i + h];
+          v[i] = keep + __shfl_xor_sync(mask, send, off, LPR);
+        }
+      base += up ? h : 0;
+      cnt = h;
+    } else {
+      v[0] += __shfl_xor_sync(mask, v[0], off, LPR);
+    }
+  }
+  count = cnt;
+  return base;
+}
+
+// One lane group of LPR lanes per row; lane owns column lg (NR <= LPR).  Bound
+// by the FP64 pipe (two FMAs per clock and SM): per entry 2 (real H) or 4 FMAs
+// of the SpMM, 4 of the SDDMM product and 2 of its sum over the columns, four
+// entries at a time; the butterfly of every entry by itself and complex values
+// for a real H took 16 (graphene 128x128, NR = 16: 88 us per step).
+template <int LPR, bool REALH>
+__global__ void __launch_bounds__(kAdjThreads) k_adjoint_step(
+    const __grid_constant__ AdjParams p) {
+  step::pdl_enter();
+  using HV = typename std::conditional<REALH, double, double2>::type;
   constexpr int GROUPS = kAdjThreads / LPR;
+  constexpr int CH = 4;  // entries per fold
   const int g = threadIdx.x / LPR, lg = threadIdx.x % LPR;
   const unsigned mask = LPR == 32 ? 0xffffffffu
                                   : (((1u << LPR) - 1u) << ((threadIdx.x & 31) / LPR * LPR));
+  const HV* __restrict__ val = static_cast<const HV*>(p.val);
+  const bool act = lg < p.NR;
+  const bool spmm = p.lam_out != nullptr && p.lam1 != nullptr;
+  const bool sddmm = p.sddmm_coef != 0.0;
+  const double2 zero = make_double2(0.0, 0.0);
   for (int64_t r = (int64_t)blockIdx.x * GROUPS + g; r < p.NH; r += (int64_t)gridDim.x * GROUPS) {
-    const bool act = lg < p.NR;
     const int64_t own = r * p.NR + lg;
-    const double2 l_own = act && p.lam1 ? p.lam1[own] : make_double2(0.0, 0.0);
-    double2 acc = make_double2(0.0, 0.0);
+    const double2 l_own = act && p.lam1 ? p.lam1[own] : zero;
+    double2 acc = zero;
     const int k0 = p.rowptr[r], k1 = p.rowptr[r + 1];
-    for (int k = k0; k < k1; ++k) {
-      const int j = p.col[k];
-      const double2 h = p.val[k];
-      double2 lj = make_double2(0.0, 0.0), vj = make_double2(0.0, 0.0);
-      if (act) {
-        if (p.lam1) lj = p.lam1[(int64_t)j * p.NR + lg];
-        vj = p.vk[(int64_t)j * p.NR + lg];
-      }
-      acc.x = fma(h.x, lj.x, acc.x);
-      acc.x = fma(-h.y, lj.y, acc.x);
-      acc.y = fma(h.x, lj.y, acc.y);
-      acc.y = fma(h.y, lj.x, acc.y);
-      if (p.sddmm_coef != 0.0) {
-        // conj(lambda_k+1[i]) v_k[j], summed over the probe columns
-        double sr = l_own.x * vj.x + l_own.y * vj.y;
-        double si = l_own.x * vj.y - l_own.y * vj.x;
+    for (int kc = k0; kc < k1; kc += CH) {
+      double2 lj[CH], vj[CH];
+      HV h[CH];
 #pragma unroll
-        for (int off = LPR / 2; off > 0; off >>= 1) {
-          sr += __shfl_xor_sync(mask, sr, off, LPR);
-          si += __shfl_xor_sync(mask, si, off, LPR);
+      for (int u = 0; u < CH; ++u) {
+        lj[u] = vj[u] = zero;
+        h[u] = HV{};
+        if (kc + u < k1) {
+          const int64_t j = (int64_t)__ldg(p.col + kc + u) * p.NR + lg;
+          h[u] = __ldg(val + kc + u);
+          if (act && spmm) lj[u] = __ldg(p.lam1 + j);
+          if (act && sddmm) vj[u] = __ldg(p.vk + j);
         }
-        if (lg == 0) {
-          p.grad[k].x += p.sddmm_coef * sr;
-          p.grad[k].y += p.sddmm_coef * si;
+      }
+      if (spmm) {
+#pragma unroll
+        for (int u = 0; u < CH; ++u) {
+          if (kc + u >= k1) break;
+          if constexpr (REALH) {
+            acc.x = fma(h[u], lj[u].x, acc.x);
+            acc.y = fma(h[u], lj[u].y, acc.y);
+          } else {
+            acc.x = fma(h[u].x, lj[u].x, acc.x);
+            acc.x = fma(-h[u].y, lj[u].y, acc.x);
+            acc.y = fma(h[u].x, lj[u].y, acc.y);
+            acc.y = fma(h[u].y, lj[u].x, acc.y);
+          }
+        }
+      }
+      if (sddmm) {
+        // conj(lambda_k+1[i]) v_k[j], summed over the probe columns
+        double v[2 * CH];
+#pragma unroll
+        for (int u = 0; u < CH; ++u) {
+          v[2 * u] = v[2 * u + 1] = 0.0;
+          if (kc + u < k1) {
+            v[2 * u] = fma(l_own.x, vj[u].x, l_own.y * vj[u].y);
+            v[2 * u + 1] = fma(l_own.x, vj[u].y, -l_own.y * vj[u].x);
+          }
+        }
+        int count;
+        const int base = group_fold<LPR>(v, lg, mask, count);
+        // the first lane that holds a value adds it
+        constexpr int kSame = LPR > 8 ? LPR / 8 : 1;  // lanes that end with the same value
+        if (lg % kSame == 0) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            if (i < count && kc + ((base + i) >> 1) < k1) {
+              double* const out = reinterpret_cast<double*>(p.grad + kc) + base + i;
+              *out = fma(p.sddmm_coef, v[i], *out);
+            }
         }
       }
     }
     if (act && p.lam_out) {
-      double2 w = make_double2(p.c_k * p.vk[own].x, p.c_k * p.vk[own].y);
+      const double2 v = p.vk[own];
+      double2 w = make_double2(p.c_k * v.x, p.c_k * v.y);
       if (p.aseed) {
-        w.x += p.aseed[own].x;
-        w.y += p.aseed[own].y;
+        const double2 t = p.aseed[own];
+        w.x += t.x;
+        w.y += t.y;
       }
       if (p.vkp1) {
-        w.x = fma(p.c_p, p.vkp1[own].x, w.x);
-        w.y = fma(p.c_p, p.vkp1[own].y, w.y);
+        const double2 t = p.vkp1[own];
+        w.x = fma(p.c_p, t.x, w.x);
+        w.y = fma(p.c_p, t.y, w.y);
       }
       if (p.vkm1) {
-        w.x = fma(p.c_m, p.vkm1[own].x, w.x);
-        w.y = fma(p.c_m, p.vkm1[own].y, w.y);
+        const double2 t = p.vkm1[own];
+        w.x = fma(p.c_m, t.x, w.x);
+        w.y = fma(p.c_m, t.y, w.y);
       }
       double2 lo = make_double2(fma(p.spmm_coef, acc.x, w.x), fma(p.spmm_coef, acc.y, w.y));
       if (p.lam2) {
-        lo.x -= p.lam2[own].x;
-        lo.y -= p.lam2[own].y;
+        const double2 t = p.lam2[own];
+        lo.x -= t.x;
+        lo.y -= t.y;
       }
       p.lam_out[own] = lo;
     }
@@ -119,25 +193,41 @@ __global__ void k_scatter_grad(const double2* G, const int* perm, int64_t nnz, d
     out[perm[q]] = make_double2(G[q].x, -G[q].y);
 }
 
-void* adj_kernel(int NR) {
-  if (NR <= 1) return (void*)k_adjoint_step<1>;
-  if (NR <= 2) return (void*)k_adjoint_step<2>;
-  if (NR <= 4) return (void*)k_adjoint_step<4>;
-  if (NR <= 8) return (void*)k_adjoint_step<8>;
-  if (NR <= 16) return (void*)k_adjoint_step<16>;
-  return (void*)k_adjoint_step<32>;
+const void* adj_values(const DeviceCSR& H) {
+  return H.is_real ? (const void*)H.val_real : (const void*)H.val;
 }
 
-int launch_adj(const AdjParams& p, cudaStream_t s) {
-  void* fn = adj_kernel(p.NR);
+template <bool REALH>
+void* adj_kernel(int lpr) {
+  switch (lpr) {
+    case 1: return (void*)k_adjoint_step<1, REALH>;
+    case 2: return (void*)k_adjoint_step<2, REALH>;
+    case 4: return (void*)k_adjoint_step<4, REALH>;
+    case 8: return (void*)k_adjoint_step<8, REALH>;
+    case 16: return (void*)k_adjoint_step<16, REALH>;
+    default: return (void*)k_adjoint_step<32, REALH>;
+  }
+}
+
+int launch_adj(const AdjParams& p, bool real, cudaStream_t s) {
   int lpr = 32;
   for (int c : {1, 2, 4, 8, 16, 32})
     if (p.NR <= c) { lpr = c; break; }
+  void* fn = real ? adj_kernel<true>(lpr) : adj_kernel<false>(lpr);
   const int64_t groups = kAdjThreads / lpr;
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((p.NH + groups - 1) / groups, 8192));
   AdjParams q = p;
   void* args[] = {&q};
-  KPMGB_CUDA(cudaLaunchKernel(fn, dim3(grid), dim3(kAdjThreads), args, 0, s));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)std::max<int64_t>(
+      1, std::min<int64_t>((p.NH + groups - 1) / groups, 8192)));
+  cfg.blockDim = dim3(kAdjThreads);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  KPMGB_CUDA(cudaLaunchKernelExC(&cfg, fn, args));
   KPMGB_LAUNCHED();
   return KPMGB_OK;
 }
@@ -228,7 +318,7 @@ int run_kpm1d_grad(const DeviceCSR& H, const int* d_perm, int64_t NC, int NR, in
     AdjParams p{};
     p.rowptr = H.rowptr;
     p.col = H.col;
-    p.val = H.val;
+    p.val = adj_values(H);
     p.NH = NH;
     p.NR = NR;
     p.grad = d_grad_csr;
@@ -257,7 +347,7 @@ int run_kpm1d_grad(const DeviceCSR& H, const int* d_perm, int64_t NC, int NR, in
       p.c_m = k >= 2 ? 2.0 * Gw(2 * k - 1) * inv : 0.0;
       // SDDMM term 2 conj(lambda_{k+1}[i]) v_k[j] (k >= 1)
       p.sddmm_coef = k + 1 <= N ? 2.0 : 0.0;
-      KPMGB_TRY(launch_adj(p, s));
+      KPMGB_TRY(launch_adj(p, H.is_real != 0, s));
     }
   }
   // ---- closing terms: conj(lambda_1[i]) v_0[j] and c1 conj(psi[i]) psi[j]
@@ -266,12 +356,12 @@ int run_kpm1d_grad(const DeviceCSR& H, const int* d_perm, int64_t NC, int NR, in
     p.lam1 = lam(1);
     p.vk = seg(0);  // v_0 after the last (segment 0) recompute
     p.sddmm_coef = 1.0;
-    KPMGB_TRY(launch_adj(p, s));
+    KPMGB_TRY(launch_adj(p, H.is_real != 0, s));
     AdjParams q = base_params();
     q.lam1 = seg(0);
     q.vk = seg(0);
     q.sddmm_coef = c1 * inv;
-    KPMGB_TRY(launch_adj(q, s));
+    KPMGB_TRY(launch_adj(q, H.is_real != 0, s));
   }
   const int blocks = (int)std::min<int64_t>((H.nnz + 255) / 256, 4096);
   if (!last) return KPMGB_OK;
@@ -421,7 +511,7 @@ AdjParams adj_params(const DeviceCSR& H, int64_t NH, int NR, double2* grad) {
   AdjParams p{};
   p.rowptr = H.rowptr;
   p.col = H.col;
-  p.val = H.val;
+  p.val = adj_values(H);
   p.NH = NH;
   p.NR = NR;
   p.grad = grad;
@@ -443,7 +533,7 @@ int chain_adjoint(const DeviceCSR& H, int64_t NH, int NR, int64_t N, VF v, WF w,
     p.vk = v(k);
     p.aseed = w(k);
     p.sddmm_coef = k + 1 <= N - 1 ? 2.0 : 0.0;  // 2 conj(lambda_{k+1}[i]) v_k[j]
-    KPMGB_TRY(launch_adj(p, s));
+    KPMGB_TRY(launch_adj(p, H.is_real != 0, s));
   }
   // closing terms: conj(lambda_1[i]) v_0[j] and u_0
   AdjParams p = adj_params(H, NH, NR, gH);
@@ -454,7 +544,7 @@ int chain_adjoint(const DeviceCSR& H, int64_t NH, int NR, int64_t N, VF v, WF w,
   p.aseed = w(0);
   p.spmm_coef = 1.0;
   p.sddmm_coef = N >= 2 ? 1.0 : 0.0;
-  return launch_adj(p, s);
+  return launch_adj(p, H.is_real != 0, s);
 }
 
 }  // namespace
@@ -509,7 +599,7 @@ int run_kpm2d_grad(const DeviceCSR& H, const DeviceCSR& Ja, const DeviceCSR& Jb,
     p.lam1 = u0;
     p.vk = psir;
     p.sddmm_coef = 1.0;
-    KPMGB_TRY(launch_adj(p, s));
+    KPMGB_TRY(launch_adj(p, Ja.is_real != 0, s));
   }
   // Jb: sum_n conj(Lambda_n[i]) S_n[j] on Jb's pattern
   return launch_sddmm_sum(Jb, NH, NR, (int)NC, LAM(0), S(0), K, gJb, s);
