@@ -813,20 +813,18 @@ KernelFn select_kernel_ffr(int ncols, int dot, bool real, int max_row_nnz, int e
 // nullptr otherwise.  ffc_lanes: lanes per row (16 or 32).
 KernelFn select_kernel_ffc(int ncols, int dot, bool real, int ell_w, int max_row_nnz);
 int ffc_lanes(int ncols);
-// Row-streaming float-float kernel on packed FP32 pairs (kpmgb_step_ffpk.cu):
+// Row-streaming float-float kernels on packed FP32 pairs (kpmgb_step_ffpk.cu):
 // real operators, 2..64 columns, doubling dots, rows of 5..8 nonzeros,
-// vectors in the paired element layout (re.hi, im.hi, re.lo, im.lo);
-// nullptr otherwise.  Rows per block tile: 8.
-KernelFn select_kernel_ffpk(int ncols, bool real, int max_row_nnz, int ell_w);
-// The packed step to launch for such a call (fn = nullptr when none applies):
-// threads per block, dynamic shared memory, rows per block tile.
+// vectors in the paired element layout (re.hi, im.hi, re.lo, im.lo).  The
+// kernel to launch for such a call of NH rows (fn = nullptr when none
+// applies): threads per block, dynamic shared memory, rows per block tile.
 struct PackedStep {
   KernelFn fn = nullptr;
   int threads = 0;
   size_t smem = 0;
   int rows_per_block = 0;
 };
-PackedStep select_packed_step(int ncols, bool real, int max_row_nnz, int ell_w);
+PackedStep select_packed_step(int ncols, bool real, int max_row_nnz, int ell_w, int64_t NH);
 // Complex operators on column pairs (kpmgb_step_ffpk.cu): steps without dots
 // of exactly 16 or 32 columns over padded rows of stride 8 or 12, vectors in
 // the column-pair layout; nullptr otherwise.  Lanes per row: ncols / 2.

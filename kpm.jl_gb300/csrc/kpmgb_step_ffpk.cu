@@ -225,30 +225,36 @@ __global__ void __launch_bounds__(kThreads, 2) k_step_ffpk(
 // ---------------------------------------------------------------------------
 // One column per lane (k_step_ffpk1): the packed row-streaming step for 2..32
 // columns, LPR lanes per row (RPW = 32 / LPR rows per warp), with half the
-// loads per lane of k_step_ffpk and so three blocks per SM.  Bound by the
-// gathers from L2; below 9 columns the CSR kernel, whose rows wait for their
-// row pointers and column indices in turn, took 14.4 us per step at
-// NH = 65536, NR = 8.
-template <int LPR, int W>
-__global__ void __launch_bounds__(kThreads, 3) k_step_ffpk1(
+// loads per lane of k_step_ffpk and so three blocks per SM.  Half of the issue
+// slots and the latency of the gathers bound it (57% issued with 22 warps per
+// SM at NH = 262144, NR = 8), so the loop keeps to 32-bit indices, the staging
+// addresses advance by constants and lanes past the last column repeat it
+// instead of holding zeros: 26.1 -> 23.0 us per step (65536, 8 8.6 -> 7.6; 3D
+// L = 128, NR = 16 414 -> 386).  Four blocks per SM (64 registers, rows of 5)
+// pay where the slots come from HBM: 1048576, 8 95 -> 92 us, 262144, 32 90 -> 85,
+// but 65536, 8 7.5 -> 8.1.  Below 9
+// columns the CSR kernel, whose rows wait for their row pointers and column
+// indices in turn, took 14.4 us at NH = 65536, NR = 8.
+template <int LPR, int W, int BLOCKS>
+__global__ void __launch_bounds__(kThreads, BLOCKS) k_step_ffpk1(
     const __grid_constant__ KBatch batch) {
   const KParams& p = batch.p[0];
   pdl_enter();
   constexpr int RPW = 32 / LPR;           // rows per warp
   constexpr int GROUPS = kThreads / LPR;  // rows per block tile
   constexpr int kStride = 8;              // padded row stride (ints / float2 values)
-  const int g = threadIdx.x / LPR, lg = threadIdx.x % LPR;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int sub = lane / LPR;             // row of this lane within the warp
+  const int lg = lane % LPR, sub = lane / LPR;  // column, and row within the warp
   const bool live = lg < p.ncols;
-  const ulonglong2* __restrict__ x = static_cast<const ulonglong2*>(p.x);
-  const ulonglong2* z = static_cast<const ulonglong2*>(p.z);
-  ulonglong2* y = static_cast<ulonglong2*>(p.y);
-  const int* __restrict__ ecol = p.ell_col;
-  const float2* __restrict__ eval = static_cast<const float2*>(p.ell_val);
+  const unsigned NH = (unsigned)p.NH;  // below 2^31
+  const unsigned row_bytes = p.ld * 16;
+  // this lane's column (lanes past the last one repeat it and store nothing)
+  const int64_t col_bytes = (p.c0 + (live ? lg : p.ncols - 1)) * 16;
+  const char* const xl = static_cast<const char*>(p.x) + col_bytes;
+  const char* const zl = static_cast<const char*>(p.z) + col_bytes;
+  char* const yl = static_cast<char*>(p.y) + col_bytes;
   const f2 alpha2 = pk(p.alpha_f, p.alpha_f);
   const int beta_mode = p.beta_mode;
-  const int ld = p.ld;
   const f2 zero2 = pk(0.f, 0.f);
   __shared__ double2 sacc[kThreads][2];
   // per warp, two buffers of RPW padded rows: 8 column indices, 8 values
@@ -256,40 +262,57 @@ __global__ void __launch_bounds__(kThreads, 3) k_step_ffpk1(
   f2 nS = zero2, nC = zero2, xS = zero2, xC = zero2;
   sacc[threadIdx.x][0] = sacc[threadIdx.x][1] = make_double2(0.0, 0.0);
   int rows_since_flush = 0;
-  const int64_t ntiles = (p.NH + GROUPS - 1) / GROUPS;
-  // the warp's lanes copy the RPW rows of tile t (6 pieces of 16 bytes each)
-  auto stage = [&](int64_t t, int b) {
-    for (int q = lane; q < RPW * 6; q += 32) {
-      const int rr = q / 6, piece = q % 6;
-      const int64_t r = t * GROUPS + warp * RPW + rr;
-      if (t < ntiles && r < p.NH) {
-        const char* src = piece < 2
-                              ? reinterpret_cast<const char*>(ecol + r * kStride) + piece * 16
-                              : reinterpret_cast<const char*>(eval + r * kStride) + (piece - 2) * 16;
-        const unsigned dst = (unsigned)__cvta_generic_to_shared(&sidx[warp][b][rr][piece * 4]);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-      }
+  const unsigned ntiles = (NH + GROUPS - 1) / GROUPS;
+  // the warp's lanes copy the RPW rows of a tile: 6 pieces of 16 bytes each, at
+  // most kPer of them per lane, whose places in the tile stay the same
+  constexpr int kPer = (RPW * 6 + 31) / 32;
+  const char* src[kPer];
+  int step_bytes[kPer];
+  unsigned first_row[kPer], dst[kPer];
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
+    const int q = lane + 32 * i;
+    const int rr = q / 6, piece = q % 6;
+    const bool idx = piece < 2;
+    first_row[i] = warp * RPW + rr;
+    const int64_t r = (int64_t)blockIdx.x * GROUPS + warp * RPW + rr;
+    src[i] = idx ? reinterpret_cast<const char*>(p.ell_col) + r * (kStride * 4) + piece * 16
+                 : static_cast<const char*>(p.ell_val) + r * (kStride * 8) + (piece - 2) * 16;
+    step_bytes[i] = (int)gridDim.x * GROUPS * kStride * (idx ? 4 : 8);
+    dst[i] = (unsigned)__cvta_generic_to_shared(&sidx[warp][0][rr < RPW ? rr : 0][piece * 4]);
+  }
+  auto stage = [&](unsigned t, int b) {  // called for the tiles of this block in order
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      if (lane + 32 * i < RPW * 6 && t * GROUPS + first_row[i] < NH)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                         dst[i] + b * (unsigned)sizeof(sidx[0][0])),
+                     "l"(src[i])
+                     : "memory");
+      src[i] += step_bytes[i];
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   int buf = 0;
   stage(blockIdx.x, 0);
-  for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    stage(t + gridDim.x, buf ^ 1);
+  for (unsigned t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    if (t + gridDim.x < ntiles) stage(t + gridDim.x, buf ^ 1);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncwarp();
-    const int64_t r = t * GROUPS + g;
-    const bool ok = r < p.NH && live;
+    const unsigned row = t * GROUPS + warp * RPW + sub;
+    const bool ok = row < NH && live;
     const int* jrow = &sidx[warp][buf][sub][0];
     const float4* hrow = reinterpret_cast<const float4*>(&sidx[warp][buf][sub][kStride]);
-    const int64_t e = r * ld + p.c0 + lg;
+    const uint64_t e = (uint64_t)row * row_bytes;
     const ulonglong2 zero = make_ulonglong2(0ull, 0ull);
     ulonglong2 zv = zero, xo = zero, xv[W];
-    if (ok) {
-      if (beta_mode != 0) zv = __ldcs(z + e);
-      xo = __ldg(x + e);
+    if (row < NH) {
+      if (beta_mode != 0) zv = __ldcs(reinterpret_cast<const ulonglong2*>(zl + e));
+      xo = __ldg(reinterpret_cast<const ulonglong2*>(xl + e));
 #pragma unroll
-      for (int u = 0; u < W; ++u) xv[u] = __ldg(x + (int64_t)jrow[u] * ld + p.c0 + lg);
+      for (int u = 0; u < W; ++u)
+        xv[u] = __ldg(reinterpret_cast<const ulonglong2*>(xl + (uint64_t)(unsigned)jrow[u] * row_bytes));
     } else {
 #pragma unroll
       for (int u = 0; u < W; ++u) xv[u] = zero;
@@ -322,19 +345,19 @@ __global__ void __launch_bounds__(kThreads, 3) k_step_ffpk1(
       const f2 S = sub2(A, sig2);
       const f2 u2 = mul2(alpha2, S);
       const f2 c2 = mul2(alpha2, C);
-      f2 yh, yl;
+      f2 yh, yl2;
       if (beta_mode == 0) {
-        two_sum2(u2, c2, yh, yl);
+        two_sum2(u2, c2, yh, yl2);
       } else {
         const f2 s2 = sub2(u2, zv.x);
         const f2 bb = sub2(s2, u2);
         const f2 e2 = sub2(sub2(u2, sub2(s2, bb)), add2(zv.x, bb));
-        two_sum2(s2, add2(e2, sub2(c2, zv.y)), yh, yl);
+        two_sum2(s2, add2(e2, sub2(c2, zv.y)), yh, yl2);
       }
-      __stcs(y + e, make_ulonglong2(yh, yl));
+      __stcs(reinterpret_cast<ulonglong2*>(yl + e), make_ulonglong2(yh, yl2));
       const f2 nxh = sub2(zero2, xo.x);
       dacc2(nS, nC, xo.x, nxh, xo.y, xo.x, xo.y);
-      dacc2(xS, xC, xo.x, nxh, xo.y, yh, yl);
+      dacc2(xS, xC, xo.x, nxh, xo.y, yh, yl2);
     }
     if (++rows_since_flush == kFlushRows) {
       rows_since_flush = 0;
@@ -566,24 +589,23 @@ KernelFn select_kernel_ffcp(int ncols, bool real, int ell_w, int max_row_nnz) {
 
 namespace {
 template <int LPR>
-KernelFn ffpk1_w(int max_row_nnz) {
+KernelFn ffpk1_w(int max_row_nnz, bool from_hbm) {
   switch (max_row_nnz) {
-    case 5: return k_step_ffpk1<LPR, 5>;
-    case 6: return k_step_ffpk1<LPR, 6>;
-    case 7: return k_step_ffpk1<LPR, 7>;
-    case 8: return k_step_ffpk1<LPR, 8>;
+    case 5: return from_hbm ? k_step_ffpk1<LPR, 5, 4> : k_step_ffpk1<LPR, 5, 3>;
+    case 6: return k_step_ffpk1<LPR, 6, 3>;
+    case 7: return k_step_ffpk1<LPR, 7, 3>;
+    case 8: return k_step_ffpk1<LPR, 8, 3>;
     default: return nullptr;
   }
 }
-}  // namespace
 
-KernelFn select_kernel_ffpk(int ncols, bool real, int max_row_nnz, int ell_w) {
+KernelFn select_kernel_ffpk(int ncols, bool real, int max_row_nnz, int ell_w, bool from_hbm) {
   if (!real || ell_w != 8 || max_row_nnz > 8) return nullptr;
-  if (ncols == 2) return ffpk1_w<2>(max_row_nnz);
-  if (ncols == 3 || ncols == 4) return ffpk1_w<4>(max_row_nnz);
-  if (ncols >= 5 && ncols <= 8) return ffpk1_w<8>(max_row_nnz);
-  if (ncols >= 9 && ncols <= 16) return ffpk1_w<16>(max_row_nnz);
-  if (ncols >= 17 && ncols <= 32) return ffpk1_w<32>(max_row_nnz);
+  if (ncols == 2) return ffpk1_w<2>(max_row_nnz, from_hbm);
+  if (ncols == 3 || ncols == 4) return ffpk1_w<4>(max_row_nnz, from_hbm);
+  if (ncols >= 5 && ncols <= 8) return ffpk1_w<8>(max_row_nnz, from_hbm);
+  if (ncols >= 9 && ncols <= 16) return ffpk1_w<16>(max_row_nnz, from_hbm);
+  if (ncols >= 17 && ncols <= 32) return ffpk1_w<32>(max_row_nnz, from_hbm);
   if (ncols < 33 || ncols > 64) return nullptr;
   const bool full = ncols == 64;
   switch (max_row_nnz) {
@@ -594,14 +616,17 @@ KernelFn select_kernel_ffpk(int ncols, bool real, int max_row_nnz, int ell_w) {
     default: return nullptr;
   }
 }
+}  // namespace
 
 int ffpk_lanes(int ncols) {
   return ncols <= 2 ? 2 : ncols <= 4 ? 4 : ncols <= 8 ? 8 : ncols <= 16 ? 16 : 32;
 }
 
-PackedStep select_packed_step(int ncols, bool real, int max_row_nnz, int ell_w) {
+PackedStep select_packed_step(int ncols, bool real, int max_row_nnz, int ell_w, int64_t NH) {
+  // both slots within about 100 MB stay in L2 from step to step
+  const bool from_hbm = NH * ncols * 32 > (int64_t)100 << 20;
   PackedStep ps;
-  ps.fn = select_kernel_ffpk(ncols, real, max_row_nnz, ell_w);
+  ps.fn = select_kernel_ffpk(ncols, real, max_row_nnz, ell_w, from_hbm);
   ps.threads = kThreads;
   ps.rows_per_block = ncols > 32 ? kThreads / 32 : kThreads / ffpk_lanes(ncols);
   ps.smem = 0;
