@@ -402,47 +402,63 @@ __global__ void __launch_bounds__(kThreads, 2) k_step_ffcp(
   constexpr int RPW = 32 / LPH;            // rows per warp
   constexpr int GROUPS = kThreads / LPH;   // rows per block tile
   constexpr int kPieces = W / 4 + W;       // 16-byte pieces of one padded row
-  const int g = threadIdx.x / LPH, lg = threadIdx.x % LPH;
+  const int lg = threadIdx.x % LPH;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane / LPH;              // row of this lane within the warp
   const ulonglong2* __restrict__ x = static_cast<const ulonglong2*>(p.x);
   const ulonglong2* z = static_cast<const ulonglong2*>(p.z);
   ulonglong2* y = static_cast<ulonglong2*>(p.y);
-  const int* __restrict__ ecol = p.ell_col;
-  const float4* __restrict__ eval = static_cast<const float4*>(p.ell_val);
   const f2 alpha2 = pk(p.alpha_f, p.alpha_f);
   const int beta_mode = p.beta_mode;
   const f2 zero2 = pk(0.f, 0.f);
   // per warp, two buffers of RPW padded rows: W indices then W values each
   __shared__ __align__(16) float4 sidx[kThreads / 32][2][RPW][kPieces];
-  const int64_t ntiles = (p.NH + GROUPS - 1) / GROUPS;
-  auto stage = [&](int64_t t, int b) {
-    for (int q = lane; q < RPW * kPieces; q += 32) {
-      const int rr = q / kPieces, piece = q % kPieces;
-      const int64_t r = t * GROUPS + warp * RPW + rr;
-      if (t < ntiles && r < p.NH) {
-        const char* src = piece < W / 4
-                              ? reinterpret_cast<const char*>(ecol + r * W) + piece * 16
-                              : reinterpret_cast<const char*>(eval + r * W + (piece - W / 4));
-        const unsigned dst = (unsigned)__cvta_generic_to_shared(&sidx[warp][b][rr][piece]);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-      }
+  const unsigned NH = (unsigned)p.NH;  // below 2^31
+  const unsigned ntiles = (NH + GROUPS - 1) / GROUPS;
+  // the warp's lanes copy the RPW rows of a tile, at most kPer pieces of 16
+  // bytes per lane, whose places in the tile stay the same
+  constexpr int kPer = (RPW * kPieces + 31) / 32;
+  const char* src[kPer];
+  int step_bytes[kPer];
+  unsigned first_row[kPer], dst[kPer];
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
+    const int q = lane + 32 * i;
+    const int rr = q / kPieces, piece = q % kPieces;
+    const bool idx = piece < W / 4;
+    first_row[i] = warp * RPW + rr;
+    const int64_t r = (int64_t)blockIdx.x * GROUPS + warp * RPW + rr;
+    src[i] = idx ? reinterpret_cast<const char*>(p.ell_col) + r * (W * 4) + piece * 16
+                 : static_cast<const char*>(p.ell_val) + r * (W * 16) + (piece - W / 4) * 16;
+    step_bytes[i] = (int)gridDim.x * GROUPS * W * (idx ? 4 : 16);
+    dst[i] = (unsigned)__cvta_generic_to_shared(&sidx[warp][0][rr < RPW ? rr : 0][piece]);
+  }
+  auto stage = [&](unsigned t, int b) {  // called for the tiles of this block in order
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      if (lane + 32 * i < RPW * kPieces && t * GROUPS + first_row[i] < NH)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                         dst[i] + b * (unsigned)sizeof(sidx[0][0])),
+                     "l"(src[i])
+                     : "memory");
+      src[i] += step_bytes[i];
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   int buf = 0;
   float ymax = 0.f;  // largest |high part| of this thread's outputs (p.vmax)
   stage(blockIdx.x, 0);
-  for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    stage(t + gridDim.x, buf ^ 1);
+  for (unsigned t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    if (t + gridDim.x < ntiles) stage(t + gridDim.x, buf ^ 1);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncwarp();
-    const int64_t r = t * GROUPS + g;
-    const bool row_ok = r < p.NH;
+    const unsigned r = t * GROUPS + warp * RPW + sub;
+    const bool row_ok = r < NH;
     const int* jrow = reinterpret_cast<const int*>(&sidx[warp][buf][sub][0]);
     const float4* hrow = &sidx[warp][buf][sub][W / 4];
     // blocks of 32 bytes: [2 q] = {re.hi pair, re.lo pair}, [2 q + 1] = {im.hi, im.lo}
-    const int64_t base = (r * LPH + lg) * 2;
+    const int64_t base = ((int64_t)r * LPH + lg) * 2;
     const ulonglong2 zero = make_ulonglong2(0ull, 0ull);
     ulonglong2 z0 = zero, z1 = zero;
     if (row_ok && beta_mode != 0) {
