@@ -153,6 +153,12 @@ int check_precision(int precision) {
   return KPMGB_OK;
 }
 
+// Column-pair vectors for complex operators (KPMGB_COLPAIR=0: never).
+const bool colpair_on = [] {
+  const char* e = std::getenv("KPMGB_COLPAIR");
+  return !(e && std::atoi(e) == 0);
+}();
+
 // -------------------------------------------------------------- kpm_1d
 int run_kpm1d(Operator* op, int64_t NC, int64_t NR, int64_t NH, const void* psi_l,
               const void* psi_r, double2* mu, const kpmgb_kpm1d_options* o, cudaStream_t s,
@@ -172,7 +178,7 @@ int run_kpm1d(Operator* op, int64_t NC, int64_t NR, int64_t NH, const void* psi_
   }
   if (!psi_r || !mu) return fail(KPMGB_ERR_ARGUMENT, "null buffer");
   Workspace& ws = op->ws;
-  const size_t slot = (size_t)NH * NR * 16;
+  const size_t slot = (size_t)NH * (NR + (NR & 1)) * 16;  // whole column pairs
   KPMGB_TRY(ws.slots.ensure(2 * slot));
   if (lr) KPMGB_TRY(ws.bra.ensure(slot));
   // scales: column factors of the ket and the bra, and their products
@@ -207,9 +213,16 @@ int run_kpm1d(Operator* op, int64_t NC, int64_t NR, int64_t NH, const void* psi_
   const bool paired = paired_on && ff && !lr && !auto_cluster &&
                       (variant == 0 || (variant == 11 && NR >= 9)) &&
                       packed_step_applies(op->csr, (int)NR);
-  KPMGB_TRY(launch_load_block(psi_r, sl[0], NH, (int)NR, precision, sc, false, s,
-                              paired ? VEC_PAIRED : VEC_STD));
-  if (lr) KPMGB_TRY(launch_load_block(psi_l, ws.bra.ptr, NH, (int)NR, precision, sc + NR, false, s));
+  // Float-float calls with 2..32 columns on complex operators of at most 12
+  // nonzeros per row keep them in the column-pair layout (k_step_ffcp;
+  // KPMGB_COLPAIR=0 keeps the standard layout and k_step_ffc).
+  const bool colpair = colpair_on && ff && !auto_cluster && variant == 0 &&
+                       colpair_step_applies(op->csr, (int)NR, lr ? DOT_LR1 : DOT_DOUBLING);
+  const int layout = paired ? VEC_PAIRED : colpair ? VEC_COLPAIR : VEC_STD;
+  KPMGB_TRY(launch_load_block(psi_r, sl[0], NH, (int)NR, precision, sc, false, s, layout));
+  if (lr)
+    KPMGB_TRY(launch_load_block(psi_l, ws.bra.ptr, NH, (int)NR, precision, sc + NR, false, s,
+                                layout));
   const double* mom_scale = nullptr;
   if (ff) {
     KPMGB_TRY(launch_scale_product(sc, lr ? sc + NR : sc, sc + 2 * NR, (int)NR, s));
@@ -282,6 +295,7 @@ int run_kpm1d(Operator* op, int64_t NC, int64_t NR, int64_t NH, const void* psi_
   a.variant = chosen_variant;
   a.shape = chosen_shape;
   a.paired = paired;
+  a.colpair = colpair;
   size_t held = 0;
   KPMGB_TRY(recurrence_scratch_bytes(a, precision, NC, lr, &held));
   KPMGB_TRY(ws.partials.ensure(std::max(ws.partials.bytes, held)));
@@ -418,14 +432,10 @@ int run_kpm2d(Operator* H, Operator* Ja, Operator* Jb, int64_t NC, int64_t NR, i
   // (k_step_ffcp); the contraction sums over memory order, the same
   // permutation of K on both sides.  KPMGB_COLPAIR=0 keeps the standard
   // layout.
-  static const bool colpair_on = [] {
-    const char* e = std::getenv("KPMGB_COLPAIR");
-    return !(e && std::atoi(e) == 0);
-  }();
   const bool colpair = colpair_on && ff && opt.contraction == KPMGB_CONTRACT_SPLIT &&
-                       colpair_step_applies(H->csr, (int)NR) &&
-                       colpair_step_applies(Ja->csr, (int)NR) &&
-                       colpair_step_applies(Jb->csr, (int)NR);
+                       colpair_step_applies(H->csr, (int)NR, DOT_NONE) &&
+                       colpair_step_applies(Ja->csr, (int)NR, DOT_NONE) &&
+                       colpair_step_applies(Jb->csr, (int)NR, DOT_NONE);
   const int layout = colpair ? VEC_COLPAIR : VEC_STD;
   // ff: one power-of-two factor per probe block (the contraction sums over
   // columns, so all columns of a block share it)

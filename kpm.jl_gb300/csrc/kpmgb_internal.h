@@ -215,9 +215,9 @@ struct StepArgs {
 
 // Float-float vector layouts of the row-major probe blocks: the standard one
 // (re.hi, re.lo, im.hi, im.lo) per element; the paired one (re.hi, im.hi,
-// re.lo, im.lo) per element; the column-pair one, per row and p < NR/2 a
-// 32-byte block (re.hi, re.hi', re.lo, re.lo', im.hi, im.hi', im.lo, im.lo')
-// of columns p and p + NR/2.
+// re.lo, im.lo) per element; the column-pair one, per row and p < h = ceil(NR/2)
+// a 32-byte block (re.hi, re.hi', re.lo, re.lo', im.hi, im.hi', im.lo, im.lo')
+// of columns p and p + h.
 enum VecLayout : int { VEC_STD = 0, VEC_PAIRED = 1, VEC_COLPAIR = 2 };
 
 // precision: KPMGB_PREC_FP64 or KPMGB_PREC_FF.  Returns KPMGB_OK or an error.
@@ -228,9 +228,9 @@ int launch_steps(const StepArgs* steps, int n, int precision, cudaStream_t s);
 // Whether float-float doubling steps of NR columns on H can run on packed
 // FP32 pairs over the paired vector layout (StepArgs::paired).
 bool packed_step_applies(const DeviceCSR& H, int NR);
-// Whether float-float steps without dots of NR columns on H can run on
+// Whether float-float steps of NR columns on H with these dots can run on
 // column pairs over the column-pair vector layout (StepArgs::colpair).
-bool colpair_step_applies(const DeviceCSR& H, int NR);
+bool colpair_step_applies(const DeviceCSR& H, int NR, int dot);
 // Autotuning: times every (variant, shape) candidate of the step `a` (which
 // must not write its own inputs: y aliasing neither x nor z) with CUDA events
 // on `s`, after one warm launch each, and returns the fastest in

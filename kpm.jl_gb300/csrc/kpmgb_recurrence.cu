@@ -242,9 +242,9 @@ int grid_packed(const PackedStep& ps, int64_t NH) {
 
 }  // namespace
 
-bool colpair_step_applies(const DeviceCSR& H, int NR) {
+bool colpair_step_applies(const DeviceCSR& H, int NR, int dot) {
   return NR <= cols_per_launch() &&
-         select_kernel_ffcp(NR, H.is_real != 0, H.ell_w, H.max_row_nnz) != nullptr;
+         select_kernel_ffcp(NR, dot, H.is_real != 0, H.ell_w, H.max_row_nnz) != nullptr;
 }
 
 bool packed_step_applies(const DeviceCSR& H, int NR) {
@@ -273,11 +273,11 @@ int choose_step(const StepArgs& a, int precision, int ncols, StepChoice* out) {
   if (a.colpair) {
     // the call keeps its vectors in the column-pair layout: only the
     // column-pair kernel reads them
-    KernelFn fq = precision == KPMGB_PREC_FF && a.dot == DOT_NONE
-                      ? select_kernel_ffcp(ncols, real, H.ell_w, H.max_row_nnz)
+    KernelFn fq = precision == KPMGB_PREC_FF
+                      ? select_kernel_ffcp(ncols, a.dot, real, H.ell_w, H.max_row_nnz)
                       : nullptr;
     if (!fq) return fail(KPMGB_ERR_CUDA, "internal: column-pair layout without its kernel");
-    return take(fq, ncols / 2);
+    return take(fq, ffcp_lanes(ncols));
   }
   if (a.paired) {
     // the call keeps its vectors in the paired layout: only the packed
@@ -706,14 +706,15 @@ __global__ void __launch_bounds__(256) k_transpose_in(const double2* __restrict_
   for (int k = ty; k < 32; k += 8) {
     const int64_t r = r0 + k;
     const int c = c0 + tx;
-    if (c < NR && r < NH) {
+    // column pairs: the missing second column of an odd NR is stored as 0
+    if (c < NR + (FF && layout == VEC_COLPAIR ? NR & 1 : 0) && r < NH) {
       const double2 v = tile[tx][k];
       if constexpr (FF) {
-        const double f = 1.0 / col_scale[c];
+        const double f = c < NR ? 1.0 / col_scale[c] : 0.0;
         const float2 re = ff::split_double(v.x * f);
         const float2 im = ff::split_double(v.y * f);
         if (layout == VEC_COLPAIR) {
-          const int half = NR / 2, q = c % half, side = c / half;
+          const int half = (NR + 1) / 2, q = c % half, side = c / half;
           float* f = static_cast<float*>(out) + (r * half + q) * 8 + side;
           f[0] = re.x;
           f[2] = re.y;
@@ -754,8 +755,8 @@ __global__ void k_copy2(const double2* src, double2* dst, int64_t n) {
 
 int launch_load_block(const void* psi, void* slot, int64_t NH, int NR, int precision,
                       double* col_scale, bool uniform, cudaStream_t s, int layout) {
-  if (layout == VEC_COLPAIR && (NR % 2 != 0 || precision != KPMGB_PREC_FF))
-    return fail(KPMGB_ERR_CUDA, "internal: column-pair layout needs float-float and even NR");
+  if (layout == VEC_COLPAIR && precision != KPMGB_PREC_FF)
+    return fail(KPMGB_ERR_CUDA, "internal: column-pair layout needs float-float");
   const bool ff = precision == KPMGB_PREC_FF;
   if (ff) {
     k_colnorm2<<<NR, 256, 0, s>>>(static_cast<const double2*>(psi), NH, col_scale);
@@ -765,7 +766,8 @@ int launch_load_block(const void* psi, void* slot, int64_t NH, int NR, int preci
       KPMGB_LAUNCHED();
     }
   }
-  dim3 grid((unsigned)((NH + 31) / 32), (unsigned)((NR + 31) / 32));
+  const int cols = layout == VEC_COLPAIR ? NR + (NR & 1) : NR;
+  dim3 grid((unsigned)((NH + 31) / 32), (unsigned)((cols + 31) / 32));
   if (ff)
     k_transpose_in<true><<<grid, 256, 0, s>>>(static_cast<const double2*>(psi), slot, NH, NR,
                                               col_scale, layout);

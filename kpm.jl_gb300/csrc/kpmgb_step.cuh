@@ -204,10 +204,11 @@ __device__ __forceinline__ double* red_buffer() {
 }
 
 // Block sums of FP64 dot accumulators (all warps of the block reach this
-// point; warps that own no rows pass zeros), fixed order.
+// point; warps that own no rows pass zeros), fixed order.  Lane l of a row owns
+// the columns l, l + stride, ...
 template <int ND, int LPR, int CPL, int NW = kWarps>
 __device__ __forceinline__ void block_dots(const double2 (&d)[ND > 0 ? ND : 1][CPL],
-                                           const KParams& p) {
+                                           const KParams& p, int stride = LPR) {
   if constexpr (ND > 0) {
     constexpr int V = ND * CPL * 2;
     double(*red)[V * LPR] = reinterpret_cast<double(*)[V * LPR]>(red_buffer<NW * V * LPR>());
@@ -228,7 +229,7 @@ __device__ __forceinline__ void block_dots(const double2 (&d)[ND > 0 ? ND : 1][C
     double* out = reinterpret_cast<double*>(p.partials) + (size_t)blockIdx.x * n;
     for (int e = threadIdx.x; e < n; e += NW * 32) {
       const int k = e / (2 * p.ncols), col = (e >> 1) % p.ncols;
-      const int at = ((k * CPL + col / LPR) * 2 + (e & 1)) * LPR + col % LPR;
+      const int at = ((k * CPL + col / stride) * 2 + (e & 1)) * LPR + col % stride;
       double s = 0.0;
 #pragma unroll
       for (int w = 0; w < NW; ++w) s += red[w][at];
@@ -244,7 +245,7 @@ __device__ __forceinline__ void block_dots(const double2 (&d)[ND > 0 ? ND : 1][C
 // the SM's FP64 pipe per warp and value).
 template <int ND, int LPR, int CPL, int NP, int NW = kWarps>
 __device__ __forceinline__ void block_dots_ff(const F3 (&d)[ND > 0 ? ND : 1][CPL][NP],
-                                              const KParams& p) {
+                                              const KParams& p, int stride = LPR) {
   if constexpr (ND > 0 && CPL > 2) {
     // wide lanes (128 columns): the sums of three floats would take 48 KiB
     double2 f[ND][CPL];
@@ -253,7 +254,7 @@ __device__ __forceinline__ void block_dots_ff(const F3 (&d)[ND > 0 ? ND : 1][CPL
 #pragma unroll
       for (int c = 0; c < CPL; ++c)
         f[k][c] = make_double2(f3_join(d[k][c][0]), NP > 1 ? f3_join(d[k][c][NP - 1]) : 0.0);
-    block_dots<ND, LPR, CPL, NW>(f, p);
+    block_dots<ND, LPR, CPL, NW>(f, p, stride);
   } else if constexpr (ND > 0) {
     constexpr int V = ND * CPL * NP;
     constexpr int kDoubles = NW * ND * CPL * 2 * LPR;  // block_dots' buffer
@@ -283,7 +284,7 @@ __device__ __forceinline__ void block_dots_ff(const F3 (&d)[ND > 0 ? ND : 1][CPL
       double r[2] = {0.0, 0.0};
 #pragma unroll
       for (int q = 0; q < NP; ++q) {
-        const int at = ((k * CPL + col / LPR) * NP + q) * LPR + col % LPR;
+        const int at = ((k * CPL + col / stride) * NP + q) * LPR + col % stride;
         F3 s = red[0][at];
 #pragma unroll
         for (int w = 1; w < NW; ++w) s = f3_merge(s, red[w][at]);
@@ -825,10 +826,12 @@ struct PackedStep {
   int rows_per_block = 0;
 };
 PackedStep select_packed_step(int ncols, bool real, int max_row_nnz, int ell_w, int64_t NH);
-// Complex operators on column pairs (kpmgb_step_ffpk.cu): steps without dots
-// of exactly 16 or 32 columns over padded rows of stride 8 or 12, vectors in
-// the column-pair layout; nullptr otherwise.  Lanes per row: ncols / 2.
-KernelFn select_kernel_ffcp(int ncols, bool real, int ell_w, int max_row_nnz);
+// Complex operators on column pairs (kpmgb_step_ffcp.cu) over padded rows of
+// stride 8 or 12, vectors in the column-pair layout: steps without dots of
+// exactly 16 or 32 columns, steps with dots of 2..32; nullptr otherwise.
+// ffcp_lanes: lanes per row.
+KernelFn select_kernel_ffcp(int ncols, int dot, bool real, int ell_w, int max_row_nnz);
+int ffcp_lanes(int ncols);
 
 }  // namespace step
 }  // namespace kpmgb

@@ -41,6 +41,7 @@ SOURCES = [
     "kpmgb_alloc.cu",
     "kpmgb_hostio.cu",
     "kpmgb_step_ffpk.cu",
+    "kpmgb_step_ffcp.cu",
 ]
 
 
