@@ -200,11 +200,12 @@ int kpmgb_kpm2d_device(kpmgb_operator H, kpmgb_operator Ja, kpmgb_operator Jb,
  * columns run in batches of 32.  opts->kernel_variant: 0 automatic (= 9 where
  * it applies, else 1); 1 one launch per recurrence step over all members,
  * CTAs of at most 512 rows of one member, CSR rows; 9 the same over padded
- * float-float rows (float-float, at most 8 nonzeros per row); 6 one
- * persistent launch in which each CTA runs whole members; 4 autotune (the
- * schedules, CTA sizes and row formats timed once per ensemble shape and
- * device, the choice kept in the persistent tuning cache); other values fail
- * with KPMGB_ERR_ARGUMENT.  Blocking call. */
+ * float-float rows (float-float, at most 8 nonzeros per row; real members with
+ * 5..8 in the longest row, batches of at least 2 columns: the packed step on
+ * blocks of 128 or 256 rows); 6 one persistent launch in which each CTA runs
+ * whole members; 4 autotune (the schedules, CTA sizes and row formats timed
+ * once per ensemble shape and device, the choice kept in the persistent tuning
+ * cache); other values fail with KPMGB_ERR_ARGUMENT.  Blocking call. */
 int kpmgb_kpm1d_ensemble(kpmgb_operator H, int32_t nseg, const int64_t* seg,
                          int64_t NC, int64_t NR, const double* psi,
                          double* mu_all, const kpmgb_kpm1d_options* opts);

@@ -159,6 +159,12 @@ const bool colpair_on = [] {
   return !(e && std::atoi(e) == 0);
 }();
 
+// Paired vectors for real operators (KPMGB_PAIRED=0: never).
+const bool paired_on = [] {
+  const char* e = std::getenv("KPMGB_PAIRED");
+  return !(e && std::atoi(e) == 0);
+}();
+
 // -------------------------------------------------------------- kpm_1d
 int run_kpm1d(Operator* op, int64_t NC, int64_t NR, int64_t NH, const void* psi_l,
               const void* psi_r, double2* mu, const kpmgb_kpm1d_options* o, cudaStream_t s,
@@ -206,10 +212,6 @@ int run_kpm1d(Operator* op, int64_t NC, int64_t NR, int64_t NH, const void* psi_
   // most 8 nonzeros per row keep their vectors in the paired element layout
   // and run every step on packed FP32 pairs (k_step_ffpk / k_step_ffpk1;
   // KPMGB_PAIRED=0 keeps the standard layout and k_step_ffr).
-  static const bool paired_on = [] {
-    const char* e = std::getenv("KPMGB_PAIRED");
-    return !(e && std::atoi(e) == 0);
-  }();
   const bool paired = paired_on && ff && !lr && !auto_cluster &&
                       (variant == 0 || (variant == 11 && NR >= 9)) &&
                       packed_step_applies(op->csr, (int)NR);
@@ -856,7 +858,14 @@ int kpmgb_kpm2d(kpmgb_operator H, kpmgb_operator Ja, kpmgb_operator Jb, int64_t 
 // Rows per CTA of the per-step ensemble schedule: the default and the
 // autotuner's candidates (the smallest sizes the scratch).
 constexpr int kEnsRows = 512;
-constexpr int kEnsRowsCand[] = {256, 512, 1024, 2048};
+// Rows per block of the packed schedule: a few tiles (eight columns: 64 rows
+// per tile; 32 columns: 16), fewer where 256 leave SMs without a block.
+// Per step, 128 / 256 / 512 / 1024 rows: 1.08M x 8, 126 / 118 / 117 / 119 us;
+// 277k x 8, 34.8 / 32.5 / 36.6 / 40.6 us; 514k x 32, 185 / 196 / 204 / 203 us;
+// 27k x 16, 11.3 / 13.4 / 15.5 / 15.5 us; 11k x 4, 3.9 / 5.2 / 7.6 / 11.3 us.
+constexpr int kEnsPackedRowsMin = 128;
+int ens_packed_rows(int64_t rows, int64_t cols) { return cols > 8 || rows <= 1 << 16 ? 128 : 256; }
+constexpr int kEnsRowsCand[] = {256, 512, 1024, 2048};  // packed: half of each
 constexpr int kEnsRowsMin = 256;
 
 // The ensemble call on host buffers (psi copied in, moments copied out,
@@ -912,7 +921,10 @@ static int run_ensemble(kpmgb_operator h, int32_t nseg, const int64_t* seg, int6
   // partial dots, in the partials buffer
   const size_t meta = ((size_t)(nseg + 1) * sizeof(int64_t) + (size_t)nseg * sizeof(int) + 15) &
                       ~(size_t)15;
-  const size_t step_scratch = ensemble_step_scratch_bytes(seg, nseg, (int)nb_max, kEnsRowsMin);
+  const bool packed_ok = ff && paired_on && packed_members_apply(op->csr, (int)nb_max);
+  const size_t step_scratch = std::max(
+      ensemble_step_scratch_bytes(seg, nseg, (int)nb_max, kEnsRowsMin),
+      packed_ok ? ensemble_packed_scratch_bytes(seg, nseg, (int)nb_max, kEnsPackedRowsMin) : 0);
   KPMGB_TRY(ws.partials.ensure(std::max(meta + step_scratch, ws.partials.bytes)));
   KPMGB_TRY(ensure_sync(op, s));
   char* mp = ws.partials.as<char>();
@@ -932,7 +944,7 @@ static int run_ensemble(kpmgb_operator h, int32_t nseg, const int64_t* seg, int6
   char* slots = ws.slots.as<char>();
   double* sc = ws.scales.as<double>();
   // load column batch c0 into slot 0 (probes scaled for the float-float path)
-  auto load = [&](int64_t c0, int nb, const double** scale) -> int {
+  auto load = [&](int64_t c0, int nb, bool packed, const double** scale) -> int {
     const size_t bb = (size_t)NH * nb * 16;
     KPMGB_CUDA(cudaMemsetAsync(ea.next, 0, sizeof(unsigned), s));
     const double* src = psi + 2 * c0 * NH;
@@ -940,7 +952,8 @@ static int run_ensemble(kpmgb_operator h, int32_t nseg, const int64_t* seg, int6
       KPMGB_TRY(copy_to_device(ws.psi_in.ptr, src, bb, s));
       src = ws.psi_in.as<double>();
     }
-    KPMGB_TRY(launch_load_block(src, slots, NH, nb, precision, sc, false, s));
+    KPMGB_TRY(launch_load_block(src, slots, NH, nb, precision, sc, false, s,
+                                packed ? VEC_PAIRED : VEC_STD));
     *scale = nullptr;
     if (ff) {
       KPMGB_TRY(launch_scale_product(sc, sc, sc + 2 * nb, nb, s));
@@ -948,10 +961,12 @@ static int run_ensemble(kpmgb_operator h, int32_t nseg, const int64_t* seg, int6
     }
     return KPMGB_OK;
   };
-  // Schedule and launch shape.  Automatic: one launch per step over CTAs of
-  // at most 512 rows of a member, padded rows where the float-float members
-  // allow them (256 2D Anderson realisations L = 24..96, NR = 8, NC = 512 on
-  // GB300: see the tuning record).  kernel_variant 4 times the candidates on
+  // Schedule and launch shape.  Automatic: one launch per step over blocks of
+  // rows of a member, of padded float-float rows where the members allow them
+  // (kernel_variant 9 asks for these): the packed step for real members with
+  // 5..8 nonzeros in the longest row, else the step with one column per lane (256 2D Anderson realisations L =
+  // 24..96, NR = 8, NC = 256: 15.0 ms packed, 19.1 ms; 16 of L = 10..40,
+  // NR = 4: 0.50 against 1.56 ms).  kernel_variant 4 times the candidates on
   // a short recurrence of the first column batch and keeps the fastest per
   // (device, ensemble shape) in the persistent autotuning cache.
   EnsembleShape shape;
@@ -959,6 +974,8 @@ static int run_ensemble(kpmgb_operator h, int32_t nseg, const int64_t* seg, int6
     shape = EnsembleShape{1024, false, 0};
   } else if (variant == 1) {
     shape = EnsembleShape{256, false, kEnsRows};
+  } else if ((variant == 0 || variant == 9) && packed_ok) {
+    shape = EnsembleShape{256, true, ens_packed_rows(NH, nb_max), true};
   } else if (variant == 9 || variant == 0) {
     shape = EnsembleShape{256, ell_ok, kEnsRows};
   } else {
@@ -973,9 +990,10 @@ static int run_ensemble(kpmgb_operator h, int32_t nseg, const int64_t* seg, int6
     const int nf = tune_cache_get(key, &cached)
                        ? std::sscanf(cached.c_str(), "%d,%d,%d", &th, &pad, &rows)
                        : 0;
-    if (nf == 3 && th >= 32 && th <= 1024 && th % 32 == 0 && (pad == 0 || (pad == 1 && ell_ok)) &&
-        (rows == 0 || rows >= kEnsRowsMin)) {
-      shape = EnsembleShape{th, pad != 0, rows};
+    if (nf == 3 && th >= 32 && th <= 1024 && th % 32 == 0 &&
+        (pad == 0 || (pad == 1 && ell_ok) || (pad == 2 && packed_ok && rows > 0)) &&
+        (rows == 0 || rows >= (pad == 2 ? kEnsPackedRowsMin : kEnsRowsMin))) {
+      shape = EnsembleShape{th, pad != 0, rows, pad == 2};
     } else {
       std::vector<EnsembleShape> cands;
       for (int t : {256, 512, 1024}) {
@@ -985,6 +1003,7 @@ static int run_ensemble(kpmgb_operator h, int32_t nseg, const int64_t* seg, int6
       for (int r : kEnsRowsCand) {
         cands.push_back({256, false, r});
         if (ell_ok) cands.push_back({256, true, r});
+        if (packed_ok) cands.push_back({256, true, r / 2, true});
       }
       const int64_t NCt = std::min<int64_t>(NC, 64);
       cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -994,7 +1013,7 @@ static int run_ensemble(kpmgb_operator h, int32_t nseg, const int64_t* seg, int6
       int rc = KPMGB_OK;
       for (const EnsembleShape& c : cands) {
         const double* scale = nullptr;
-        if ((rc = load(0, nb0, &scale)) != KPMGB_OK) break;
+        if ((rc = load(0, nb0, c.packed, &scale)) != KPMGB_OK) break;
         cudaEventRecord(e0, s);
         rc = launch_ensemble(op->csr, ea, nb0, NCt, slots, slots + (size_t)NH * nb0 * 16,
                              ws.mu.as<double2>(), scale, precision, s, c);
@@ -1015,7 +1034,8 @@ static int run_ensemble(kpmgb_operator h, int32_t nseg, const int64_t* seg, int6
       cudaEventDestroy(e0);
       cudaEventDestroy(e1);
       KPMGB_TRY(rc);
-      tune_cache_put(key, std::to_string(shape.threads) + "," + (shape.padded ? "1" : "0") + "," +
+      tune_cache_put(key, std::to_string(shape.threads) + "," +
+                              (shape.packed ? "2" : shape.padded ? "1" : "0") + "," +
                               std::to_string(shape.rows));
     }
   }
@@ -1023,9 +1043,13 @@ static int run_ensemble(kpmgb_operator h, int32_t nseg, const int64_t* seg, int6
     const int nb = (int)std::min<int64_t>(kBatch, NR - c0);
     const size_t bb = (size_t)NH * nb * 16;
     const double* scale = nullptr;
-    KPMGB_TRY(load(c0, nb, &scale));
+    // a last batch of one column has no packed step
+    const EnsembleShape sh = shape.packed && !packed_members_apply(op->csr, nb)
+                                 ? EnsembleShape{256, ell_ok, kEnsRows}
+                                 : shape;
+    KPMGB_TRY(load(c0, nb, sh.packed, &scale));
     KPMGB_TRY(launch_ensemble(op->csr, ea, nb, NC, slots, slots + bb, ws.mu.as<double2>(), scale,
-                              precision, s, shape));
+                              precision, s, sh));
     // [nseg][NC][nb] -> columns c0 .. c0+nb of the caller's [nseg][NC][NR]
     KPMGB_CUDA(cudaMemcpy2DAsync(mu_all + 2 * c0, (size_t)NR * 16, ws.mu.ptr, (size_t)nb * 16,
                                  (size_t)nb * 16, (size_t)nseg * NC,

@@ -11,7 +11,9 @@
 // * per step (NC/2 launches): every launch applies one step to all members,
 //   each CTA to at most `rows` rows of one member, so a large member spreads
 //   over many SMs; the last CTA of a member to finish adds the member's
-//   per-CTA partial dots in CTA order (ticket counter per member).
+//   per-CTA partial dots in CTA order (ticket counter per member).  Real
+//   float-float members run it on the packed step kernel, whose block sums are
+//   added per member after several steps.
 //
 // Both reduce in a fixed order, so the moments of a member do not depend on
 // the schedule of the CTAs.  Arithmetic is FP64 or float-float (the same
@@ -816,6 +818,43 @@ int launch_ensemble_steps(const DeviceCSR& H, const EnsembleArgs& e, EnsParams p
   return KPMGB_OK;
 }
 
+// Sums of the packed schedule that are kept between finishing launches.
+constexpr size_t kHeldBytes = size_t(32) << 20;
+
+int launch_ensemble_packed(const DeviceCSR& H, const EnsembleArgs& e, const EnsParams& p,
+                           cudaStream_t s, const EnsembleShape& shape) {
+  const int nseg = e.nseg;
+  const int64_t nb = step_blocks(e.seg_host, nseg, shape.rows);
+  if (nb > (int64_t)INT32_MAX / 2) return fail(KPMGB_ERR_ARGUMENT, "too many ensemble blocks");
+  if (ensemble_packed_scratch_bytes(e.seg_host, nseg, p.NR, shape.rows) > e.scratch_bytes)
+    return fail(KPMGB_ERR_CUDA, "internal scratch buffer too small for the ensemble kernel");
+  std::vector<int2> blk((size_t)nb);
+  std::vector<int> first((size_t)nseg + 1);
+  int64_t k = 0;
+  for (int m = 0; m < nseg; ++m) {
+    first[m] = (int)k;
+    for (int64_t r = e.seg_host[m]; r < e.seg_host[m + 1]; r += shape.rows, ++k)
+      blk[k] = make_int2((int)r, (int)std::min<int64_t>(r + shape.rows, e.seg_host[m + 1]));
+  }
+  first[nseg] = (int)k;
+  char* sp = static_cast<char*>(e.scratch);
+  MemberArgs a;
+  a.blk = reinterpret_cast<const int2*>(sp);
+  sp += align16((size_t)nb * sizeof(int2));
+  a.first = reinterpret_cast<const int*>(sp);
+  sp += align16(((size_t)nseg + 1) * sizeof(int));
+  a.nblk = (int)nb;
+  a.nseg = nseg;
+  a.partials = sp;
+  a.held = std::max(kHeldBytes, (size_t)nb * 2 * p.NR * sizeof(double2));
+  KPMGB_CUDA(cudaMemcpyAsync((void*)a.blk, blk.data(), blk.size() * sizeof(int2),
+                             cudaMemcpyHostToDevice, s));
+  KPMGB_CUDA(cudaMemcpyAsync((void*)a.first, first.data(), first.size() * sizeof(int),
+                             cudaMemcpyHostToDevice, s));
+  return launch_member_recurrence(H, H.n, p.NR, p.NC, p.slot0, p.slot1, a, p.mu, p.scale, p.status,
+                                  s);
+}
+
 }  // namespace
 
 size_t ensemble_step_scratch_bytes(const int64_t* seg, int nseg, int NR, int rows) {
@@ -824,6 +863,13 @@ size_t ensemble_step_scratch_bytes(const int64_t* seg, int nseg, int NR, int row
   return align16(nb * sizeof(int2)) + align16(nb * sizeof(int)) +
          align16(((size_t)nseg + 1) * sizeof(int)) + align16((size_t)nseg * sizeof(unsigned)) +
          nb * 2 * (size_t)NR * sizeof(double2);
+}
+
+size_t ensemble_packed_scratch_bytes(const int64_t* seg, int nseg, int NR, int rows) {
+  if (rows < 1) return 0;
+  const size_t nb = (size_t)step_blocks(seg, nseg, rows);
+  return align16(nb * sizeof(int2)) + align16(((size_t)nseg + 1) * sizeof(int)) +
+         std::max(kHeldBytes, nb * 2 * (size_t)NR * sizeof(double2));
 }
 
 int launch_ensemble(const DeviceCSR& H, const EnsembleArgs& e, int NR, int64_t NC, void* slot0,
@@ -850,6 +896,7 @@ int launch_ensemble(const DeviceCSR& H, const EnsembleArgs& e, int NR, int64_t N
   p.scale = scale;
   p.next = e.next;
   p.status = e.status;
+  if (shape.packed) return launch_ensemble_packed(H, e, p, s, shape);
   const bool ell = shape.padded && ff && H.ell_w > 0 && H.max_row_nnz <= 8;
   if (shape.padded && !ell)
     return fail(KPMGB_ERR_ARGUMENT, "the padded-row ensemble kernel serves float-float members "

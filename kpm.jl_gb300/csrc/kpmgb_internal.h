@@ -337,16 +337,34 @@ bool cluster_is_faster(const DeviceCSR& H, int64_t NH, int NR, int precision, bo
 int launch_finish_sums(const double2* sums, int G, int nd, int NR, int64_t nsteps,
                        const MomentArgs& m, cudaStream_t s);
 
+// The doubling recurrence of an ensemble's members on the packed step: blocks
+// of rows of one member (blk, nblk of them; member m has the blocks first[m] ..
+// first[m + 1] - 1), sums of `held` bytes at partials, moments [nseg][NC][NR].
+struct MemberArgs {
+  const int2* blk = nullptr;    // device
+  const int* first = nullptr;   // device
+  int nblk = 0, nseg = 0;
+  void* partials = nullptr;
+  size_t held = 0;
+};
+bool packed_members_apply(const DeviceCSR& H, int NR);
+int launch_member_recurrence(const DeviceCSR& H, int64_t NH, int NR, int64_t NC, void* slot0,
+                             void* slot1, const MemberArgs& a, double2* mu, const double* scale,
+                             unsigned* status, cudaStream_t s);
+
 // Launch shape of the ensemble kernels (chosen by their autotuner): threads
 // per CTA, CSR rows or padded float-float rows, and the schedule -- rows == 0:
 // one persistent launch, each CTA runs whole members; rows > 0: one launch
 // per recurrence step over the stacked operator, each CTA takes at most
 // `rows` rows of one member and the last CTA of a member to finish sums the
 // member's partial dots.
+// packed: one launch per step of the packed step kernel over blocks of `rows`
+// rows of one member (vectors in the paired layout).
 struct EnsembleShape {
   int threads = 1024;
   bool padded = false;
   int rows = 0;
+  bool packed = false;
 };
 
 // Tables of an ensemble call (kpmgb_ensemble.cu): the segment table on the
@@ -369,6 +387,7 @@ struct EnsembleArgs {
 int copy_to_device(void* dst, const void* src, size_t bytes, cudaStream_t s);
 
 size_t ensemble_step_scratch_bytes(const int64_t* seg, int nseg, int NR, int rows);
+size_t ensemble_packed_scratch_bytes(const int64_t* seg, int nseg, int NR, int rows);
 int launch_ensemble(const DeviceCSR& H, const EnsembleArgs& e, int NR, int64_t NC, void* slot0,
                     void* slot1, double2* mu, const double* scale, int precision, cudaStream_t s,
                     const EnsembleShape& shape);

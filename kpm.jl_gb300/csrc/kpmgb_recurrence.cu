@@ -494,6 +494,7 @@ int launch_steps(const StepArgs* steps, int n, int precision, cudaStream_t s) {
       p.bra = a.bra;
       p.alpha = a.alpha;
       p.partials = partials;
+      p.blk = nullptr;
       p.vmax = a.vmax;
       p.ell_col = H.ell_col;
       p.ell_val = H.ell_val;
@@ -585,6 +586,132 @@ int launch_recurrence(StepArgs a, int precision, int64_t NC, bool lr, void* cons
       b.partials = base;
       KPMGB_TRY(launch_finish_moments(b, precision, (int)n, m, s));
       m.i0 += n * (lr ? 1 : 2);
+      n = 0;
+    }
+  }
+  return KPMGB_OK;
+}
+
+namespace {
+
+// Moments of nsteps steps of every member from the sums of its blocks: one
+// block per step and member, its blocks in P interleaved parts.
+struct FinishMembers {
+  const double2* partials;
+  int64_t stride;  // double2 elements from step to step
+  const int* first;
+  int NR;
+  int64_t NC;
+  double2* mu;
+  const double* scale;
+  unsigned* status;
+  int doubling;
+  int64_t i0;
+};
+
+__global__ void __launch_bounds__(128) k_finish_members(FinishMembers f) {
+  __shared__ double2 part[128];
+  const int ne = 2 * f.NR;  // at most 64
+  const int P = 128 / ne;
+  const int q = threadIdx.x / ne, e = threadIdx.x % ne;
+  const int b0 = f.first[blockIdx.y], b1 = f.first[blockIdx.y + 1];
+  double2 a = make_double2(0.0, 0.0);
+  if (q < P) {
+    const double2* src = f.partials + (int64_t)blockIdx.x * f.stride + e;
+    for (int b = b0 + q; b < b1; b += P) {
+      const double2 v = src[(int64_t)b * ne];
+      a.x += v.x;
+      a.y += v.y;
+    }
+    part[threadIdx.x] = a;
+  }
+  __syncthreads();
+  if (q != 0) return;
+  for (int k = 1; k < P; ++k) {
+    a.x += part[k * ne + e].x;
+    a.y += part[k * ne + e].y;
+  }
+  const int k = e / f.NR, c = e % f.NR;
+  if (f.scale) {
+    a.x *= f.scale[c];
+    a.y *= f.scale[c];
+  }
+  double2* mu = f.mu + (size_t)blockIdx.y * f.NC * f.NR;
+  if (f.doubling) {
+    const double2 base = mu[k * f.NR + c];
+    a.x = 2.0 * a.x - base.x;
+    a.y = 2.0 * a.y - base.y;
+  }
+  mu[(f.i0 + (int64_t)blockIdx.x * 2 + k) * f.NR + c] = a;
+  if (!isfinite(a.x) || !isfinite(a.y)) atomicOr(f.status, (unsigned)STATUS_NONFINITE);
+}
+
+}  // namespace
+
+bool packed_members_apply(const DeviceCSR& H, int NR) {
+  return select_packed_members(NR, H.is_real != 0, H.max_row_nnz, H.ell_w, H.n) != nullptr;
+}
+
+int launch_member_recurrence(const DeviceCSR& H, int64_t NH, int NR, int64_t NC, void* slot0,
+                             void* slot1, const MemberArgs& a, double2* mu, const double* scale,
+                             unsigned* status, cudaStream_t s) {
+  StepChoice c;
+  c.fn = select_packed_members(NR, H.is_real != 0, H.max_row_nnz, H.ell_w, NH);
+  if (!c.fn) return fail(KPMGB_ERR_CUDA, "internal: no packed step for these members");
+  c.grid = a.nblk;
+  void* const slot[2] = {slot0, slot1};
+  KBatch batch;
+  KParams& p = batch.p[0];
+  p.rowptr = H.rowptr;
+  p.col = H.col;
+  p.val = H.val_ff;
+  p.NH = NH;
+  p.ld = NR;
+  p.c0 = 0;
+  p.ncols = NR;
+  p.bra = nullptr;
+  p.blk = a.blk;
+  p.vmax = nullptr;
+  p.ell_col = H.ell_col;
+  p.ell_val = H.ell_val;
+  p.ell_w = H.ell_w;
+  FinishMembers f;
+  f.partials = static_cast<const double2*>(a.partials);
+  f.stride = (int64_t)a.nblk * 2 * NR;
+  f.first = a.first;
+  f.NR = NR;
+  f.NC = NC;
+  f.mu = mu;
+  f.scale = scale;
+  f.status = status;
+  const int64_t steps = NC / 2;
+  const int64_t hold =
+      std::max<int64_t>(1, (int64_t)(a.held / ((size_t)f.stride * sizeof(double2))));
+  int64_t n = 0;
+  f.i0 = 0;
+  for (int64_t i = 0; i < steps; ++i) {
+    // y = H x, then 2 H x - y in place; the first step's moments come before
+    // those of the doubling identities that use them
+    const bool first = i == 0;
+    p.x = slot[i & 1];
+    p.y = slot[(i & 1) ^ 1];
+    p.z = first ? nullptr : p.y;
+    p.alpha = first ? 1.0 : 2.0;
+    p.alpha_f = first ? 1.f : 2.f;
+    p.beta_mode = first ? 0 : -1;
+    p.partials = static_cast<double2*>(a.partials) + n * f.stride;
+    KPMGB_TRY(launch_step_kernel(c, 1, s, batch));
+    if (++n == hold || first || i + 1 == steps) {
+      f.doubling = first ? 0 : 1;
+      for (int m0 = 0; m0 < a.nseg; m0 += 65535) {  // the grid's y limit
+        FinishMembers g = f;
+        g.first += m0;
+        g.mu += (size_t)m0 * NC * NR;
+        k_finish_members<<<dim3((unsigned)n, (unsigned)std::min(a.nseg - m0, 65535)), 128, 0,
+                           s>>>(g);
+        KPMGB_LAUNCHED();
+      }
+      f.i0 += 2 * n;
       n = 0;
     }
   }

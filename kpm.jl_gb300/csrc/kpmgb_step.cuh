@@ -105,6 +105,7 @@ struct KParams {
   const void* bra;
   double alpha;          // +-2^k
   double2* partials;     // [block][dots][ncols] sums of this launch (null: none)
+  const int2* blk;       // rows [x, y) of each block (member steps), else null
   // fixed-width padded rows (k_step_ffe): NH x ell_w columns / values
   const int* ell_col;
   const void* ell_val;
@@ -826,6 +827,8 @@ struct PackedStep {
   int rows_per_block = 0;
 };
 PackedStep select_packed_step(int ncols, bool real, int max_row_nnz, int ell_w, int64_t NH);
+// The same over blocks of given rows (KParams::blk), 2..32 columns.
+KernelFn select_packed_members(int ncols, bool real, int max_row_nnz, int ell_w, int64_t NH);
 // Complex operators on column pairs (kpmgb_step_ffcp.cu) over padded rows of
 // stride 8 or 12, vectors in the column-pair layout: steps without dots of
 // exactly 16 or 32 columns, steps with dots of 2..32; nullptr otherwise.

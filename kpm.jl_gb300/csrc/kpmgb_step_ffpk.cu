@@ -235,7 +235,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_step_ffpk(
 // but 65536, 8 7.5 -> 8.1.  Below 9
 // columns the CSR kernel, whose rows wait for their row pointers and column
 // indices in turn, took 14.4 us at NH = 65536, NR = 8.
-template <int LPR, int W, int BLOCKS>
+//
+// MEMBERS: each block takes the consecutive rows p.blk[block] (the rows of one
+// member of an ensemble) instead of every gridDim-th tile.
+template <int LPR, int W, int BLOCKS, bool MEMBERS>
 __global__ void __launch_bounds__(kThreads, BLOCKS) k_step_ffpk1(
     const __grid_constant__ KBatch batch) {
   const KParams& p = batch.p[0];
@@ -246,7 +249,10 @@ __global__ void __launch_bounds__(kThreads, BLOCKS) k_step_ffpk1(
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int lg = lane % LPR, sub = lane / LPR;  // column, and row within the warp
   const bool live = lg < p.ncols;
-  const unsigned NH = (unsigned)p.NH;  // below 2^31
+  // tiles t0, t0 + dt, .. of rows origin + t GROUPS .. up to NH (below 2^31)
+  const int2 rows = MEMBERS ? __ldg(p.blk + blockIdx.x) : make_int2(0, (int)p.NH);
+  const unsigned origin = (unsigned)rows.x, NH = (unsigned)rows.y;
+  const unsigned t0 = MEMBERS ? 0 : blockIdx.x, dt = MEMBERS ? 1 : gridDim.x;
   const unsigned row_bytes = p.ld * 16;
   // this lane's column (lanes past the last one repeat it and store nothing)
   const int64_t col_bytes = (p.c0 + (live ? lg : p.ncols - 1)) * 16;
@@ -262,7 +268,7 @@ __global__ void __launch_bounds__(kThreads, BLOCKS) k_step_ffpk1(
   f2 nS = zero2, nC = zero2, xS = zero2, xC = zero2;
   sacc[threadIdx.x][0] = sacc[threadIdx.x][1] = make_double2(0.0, 0.0);
   int rows_since_flush = 0;
-  const unsigned ntiles = (NH + GROUPS - 1) / GROUPS;
+  const unsigned ntiles = (NH - origin + GROUPS - 1) / GROUPS;
   // the warp's lanes copy the RPW rows of a tile: 6 pieces of 16 bytes each, at
   // most kPer of them per lane, whose places in the tile stay the same
   constexpr int kPer = (RPW * 6 + 31) / 32;
@@ -274,11 +280,11 @@ __global__ void __launch_bounds__(kThreads, BLOCKS) k_step_ffpk1(
     const int q = lane + 32 * i;
     const int rr = q / 6, piece = q % 6;
     const bool idx = piece < 2;
-    first_row[i] = warp * RPW + rr;
-    const int64_t r = (int64_t)blockIdx.x * GROUPS + warp * RPW + rr;
+    first_row[i] = origin + warp * RPW + rr;
+    const int64_t r = origin + (int64_t)t0 * GROUPS + warp * RPW + rr;
     src[i] = idx ? reinterpret_cast<const char*>(p.ell_col) + r * (kStride * 4) + piece * 16
                  : static_cast<const char*>(p.ell_val) + r * (kStride * 8) + (piece - 2) * 16;
-    step_bytes[i] = (int)gridDim.x * GROUPS * kStride * (idx ? 4 : 8);
+    step_bytes[i] = (int)dt * GROUPS * kStride * (idx ? 4 : 8);
     dst[i] = (unsigned)__cvta_generic_to_shared(&sidx[warp][0][rr < RPW ? rr : 0][piece * 4]);
   }
   auto stage = [&](unsigned t, int b) {  // called for the tiles of this block in order
@@ -294,13 +300,13 @@ __global__ void __launch_bounds__(kThreads, BLOCKS) k_step_ffpk1(
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   int buf = 0;
-  stage(blockIdx.x, 0);
-  for (unsigned t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    if (t + gridDim.x < ntiles) stage(t + gridDim.x, buf ^ 1);
+  stage(t0, 0);
+  for (unsigned t = t0; t < ntiles; t += dt) {
+    if (t + dt < ntiles) stage(t + dt, buf ^ 1);
     else asm volatile("cp.async.commit_group;" ::: "memory");
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncwarp();
-    const unsigned row = t * GROUPS + warp * RPW + sub;
+    const unsigned row = origin + t * GROUPS + warp * RPW + sub;
     const bool ok = row < NH && live;
     const int* jrow = &sidx[warp][buf][sub][0];
     const float4* hrow = reinterpret_cast<const float4*>(&sidx[warp][buf][sub][kStride]);
@@ -367,7 +373,7 @@ __global__ void __launch_bounds__(kThreads, BLOCKS) k_step_ffpk1(
     }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-  if (any_flush(ntiles, kFlushRows)) {
+  if (MEMBERS ? ntiles >= kFlushRows : any_flush(ntiles, kFlushRows)) {
     double2 d[2][1];
     d[0][0] = sacc[threadIdx.x][0];
     d[0][0].x += join2(nS, nC);
@@ -381,16 +387,19 @@ __global__ void __launch_bounds__(kThreads, BLOCKS) k_step_ffpk1(
 }
 
 namespace {
-template <int LPR>
+template <int LPR, bool MEMBERS = false>
 KernelFn ffpk1_w(int max_row_nnz, bool from_hbm) {
   switch (max_row_nnz) {
-    case 5: return from_hbm ? k_step_ffpk1<LPR, 5, 4> : k_step_ffpk1<LPR, 5, 3>;
-    case 6: return k_step_ffpk1<LPR, 6, 3>;
-    case 7: return k_step_ffpk1<LPR, 7, 3>;
-    case 8: return k_step_ffpk1<LPR, 8, 3>;
+    case 5: return from_hbm ? k_step_ffpk1<LPR, 5, 4, MEMBERS> : k_step_ffpk1<LPR, 5, 3, MEMBERS>;
+    case 6: return k_step_ffpk1<LPR, 6, 3, MEMBERS>;
+    case 7: return k_step_ffpk1<LPR, 7, 3, MEMBERS>;
+    case 8: return k_step_ffpk1<LPR, 8, 3, MEMBERS>;
     default: return nullptr;
   }
 }
+
+// both slots within about 100 MB stay in L2 from step to step
+bool slots_from_hbm(int64_t NH, int ncols) { return NH * ncols * 32 > (int64_t)100 << 20; }
 
 KernelFn select_kernel_ffpk(int ncols, bool real, int max_row_nnz, int ell_w, bool from_hbm) {
   if (!real || ell_w != 8 || max_row_nnz > 8) return nullptr;
@@ -415,11 +424,21 @@ int ffpk_lanes(int ncols) {
   return ncols <= 2 ? 2 : ncols <= 4 ? 4 : ncols <= 8 ? 8 : ncols <= 16 ? 16 : 32;
 }
 
+KernelFn select_packed_members(int ncols, bool real, int max_row_nnz, int ell_w, int64_t NH) {
+  if (!real || ell_w != 8 || max_row_nnz > 8 || ncols < 2 || ncols > 32) return nullptr;
+  const bool from_hbm = slots_from_hbm(NH, ncols);
+  switch (ffpk_lanes(ncols)) {
+    case 2: return ffpk1_w<2, true>(max_row_nnz, from_hbm);
+    case 4: return ffpk1_w<4, true>(max_row_nnz, from_hbm);
+    case 8: return ffpk1_w<8, true>(max_row_nnz, from_hbm);
+    case 16: return ffpk1_w<16, true>(max_row_nnz, from_hbm);
+    default: return ffpk1_w<32, true>(max_row_nnz, from_hbm);
+  }
+}
+
 PackedStep select_packed_step(int ncols, bool real, int max_row_nnz, int ell_w, int64_t NH) {
-  // both slots within about 100 MB stay in L2 from step to step
-  const bool from_hbm = NH * ncols * 32 > (int64_t)100 << 20;
   PackedStep ps;
-  ps.fn = select_kernel_ffpk(ncols, real, max_row_nnz, ell_w, from_hbm);
+  ps.fn = select_kernel_ffpk(ncols, real, max_row_nnz, ell_w, slots_from_hbm(NH, ncols));
   ps.threads = kThreads;
   ps.rows_per_block = ncols > 32 ? kThreads / 32 : kThreads / ffpk_lanes(ncols);
   ps.smem = 0;
