@@ -243,7 +243,10 @@ int64_t range_for(int64_t K, int nr, int nl) {
                       (size_t)((2 * nl + C8::kN - 1) / C8::kN * C8::kN);
   const int64_t chunk = C8::kChunk * C8::KT / 2;  // complex elements
   const int64_t fit = (int64_t)(most / (rows * S8 * 2 * 2)) / chunk * chunk;
-  return std::min(K, std::max<int64_t>(fit, 64 * chunk));
+  const int64_t range = std::max<int64_t>(fit, 64 * chunk);
+  // equal ranges: the tiles of a short last one would leave SMs idle
+  const int64_t n = (K + range - 1) / range;
+  return std::min(K, ((K + n - 1) / n + chunk - 1) / chunk * chunk);
 }
 
 struct Layout8 {
