@@ -145,6 +145,7 @@ struct StepChoice {
   int threads = kThreads;
   size_t smem = 0;
   int slots = 0;  // resident blocks where early launches depend on them, else 0
+  int split = 1;  // parts of the columns (steps that launch alone)
 };
 
 // Step kernels launch with programmatic stream serialization (see pdl_enter)
@@ -157,15 +158,16 @@ int launch_step_kernel(const StepChoice& c, int n, cudaStream_t s, const KBatch&
     const char* e = std::getenv("KPMGB_PDL");
     return !(e && e[0] == '0');
   }();
+  const dim3 grid((unsigned)c.grid, (unsigned)(n * c.split));
   const int blocks = c.grid * n;
   const bool early = c.slots == 0 || blocks >= c.slots || 2 * blocks <= c.slots;
   if (!on || !early) {
-    c.fn<<<dim3((unsigned)c.grid, (unsigned)n), c.threads, c.smem, s>>>(p);
+    c.fn<<<grid, c.threads, c.smem, s>>>(p);
     KPMGB_LAUNCHED();
     return KPMGB_OK;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)c.grid, (unsigned)n);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3((unsigned)c.threads);
   cfg.dynamicSmemBytes = c.smem;
   cfg.stream = s;
@@ -237,7 +239,8 @@ int grid_packed(const PackedStep& ps, int64_t NH) {
     }
   }
   const int64_t tiles = (NH + ps.rows_per_block - 1) / ps.rows_per_block;
-  return (int)std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)per_sm * num_sms()));
+  return (int)std::max<int64_t>(
+      1, std::min<int64_t>(tiles, (int64_t)per_sm * num_sms() / ps.split));
 }
 
 }  // namespace
@@ -286,7 +289,7 @@ int choose_step(const StepArgs& a, int precision, int ncols, StepChoice* out) {
                               ? select_packed_step(ncols, real, H.max_row_nnz, H.ell_w, a.NH)
                               : PackedStep{};
     if (!ps.fn) return fail(KPMGB_ERR_CUDA, "internal: paired layout without the packed kernel");
-    *out = StepChoice{ps.fn, grid_packed(ps, a.NH), ps.threads, ps.smem};
+    *out = StepChoice{ps.fn, grid_packed(ps, a.NH), ps.threads, ps.smem, 0, ps.split};
     return KPMGB_OK;
   }
   if (a.variant == 11 && precision != KPMGB_PREC_FF)
@@ -649,14 +652,16 @@ __global__ void __launch_bounds__(128) k_finish_members(FinishMembers f) {
 }  // namespace
 
 bool packed_members_apply(const DeviceCSR& H, int NR) {
-  return select_packed_members(NR, H.is_real != 0, H.max_row_nnz, H.ell_w, H.n) != nullptr;
+  return select_packed_members(NR, H.is_real != 0, H.max_row_nnz, H.ell_w, H.n).fn != nullptr;
 }
 
 int launch_member_recurrence(const DeviceCSR& H, int64_t NH, int NR, int64_t NC, void* slot0,
                              void* slot1, const MemberArgs& a, double2* mu, const double* scale,
                              unsigned* status, cudaStream_t s) {
   StepChoice c;
-  c.fn = select_packed_members(NR, H.is_real != 0, H.max_row_nnz, H.ell_w, NH);
+  const PackedStep ps = select_packed_members(NR, H.is_real != 0, H.max_row_nnz, H.ell_w, NH);
+  c.fn = ps.fn;
+  c.split = ps.split;
   if (!c.fn) return fail(KPMGB_ERR_CUDA, "internal: no packed step for these members");
   c.grid = a.nblk;
   void* const slot[2] = {slot0, slot1};

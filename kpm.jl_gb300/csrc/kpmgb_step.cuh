@@ -206,10 +206,12 @@ __device__ __forceinline__ double* red_buffer() {
 
 // Block sums of FP64 dot accumulators (all warps of the block reach this
 // point; warps that own no rows pass zeros), fixed order.  Lane l of a row owns
-// the columns l, l + stride, ...
+// the columns l, l + stride, ...  The block has the columns off .. off + count - 1
+// of the launch (count < 0: all).
 template <int ND, int LPR, int CPL, int NW = kWarps>
 __device__ __forceinline__ void block_dots(const double2 (&d)[ND > 0 ? ND : 1][CPL],
-                                           const KParams& p, int stride = LPR) {
+                                           const KParams& p, int stride = LPR, int off = 0,
+                                           int count = -1) {
   if constexpr (ND > 0) {
     constexpr int V = ND * CPL * 2;
     double(*red)[V * LPR] = reinterpret_cast<double(*)[V * LPR]>(red_buffer<NW * V * LPR>());
@@ -226,15 +228,16 @@ __device__ __forceinline__ void block_dots(const double2 (&d)[ND > 0 ? ND : 1][C
     for (int i = 0; i < kLeft; ++i)
       red[warp][(base + i) * LPR + lane % LPR] = v[i];
     __syncthreads();
-    const int n = 2 * ND * p.ncols;
-    double* out = reinterpret_cast<double*>(p.partials) + (size_t)blockIdx.x * n;
-    for (int e = threadIdx.x; e < n; e += NW * 32) {
-      const int k = e / (2 * p.ncols), col = (e >> 1) % p.ncols;
+    const int nc = count < 0 ? p.ncols : count;
+    double* out =
+        reinterpret_cast<double*>(p.partials + (size_t)blockIdx.x * ND * p.ncols + off);
+    for (int e = threadIdx.x; e < 2 * ND * nc; e += NW * 32) {
+      const int k = e / (2 * nc), col = (e >> 1) % nc;
       const int at = ((k * CPL + col / stride) * 2 + (e & 1)) * LPR + col % stride;
       double s = 0.0;
 #pragma unroll
       for (int w = 0; w < NW; ++w) s += red[w][at];
-      out[e] = s;
+      out[2 * (k * p.ncols + col) + (e & 1)] = s;
     }
   }
 }
@@ -246,7 +249,8 @@ __device__ __forceinline__ void block_dots(const double2 (&d)[ND > 0 ? ND : 1][C
 // the SM's FP64 pipe per warp and value).
 template <int ND, int LPR, int CPL, int NP, int NW = kWarps>
 __device__ __forceinline__ void block_dots_ff(const F3 (&d)[ND > 0 ? ND : 1][CPL][NP],
-                                              const KParams& p, int stride = LPR) {
+                                              const KParams& p, int stride = LPR, int off = 0,
+                                              int count = -1) {
   if constexpr (ND > 0 && CPL > 2) {
     // wide lanes (128 columns): the sums of three floats would take 48 KiB
     double2 f[ND][CPL];
@@ -255,7 +259,7 @@ __device__ __forceinline__ void block_dots_ff(const F3 (&d)[ND > 0 ? ND : 1][CPL
 #pragma unroll
       for (int c = 0; c < CPL; ++c)
         f[k][c] = make_double2(f3_join(d[k][c][0]), NP > 1 ? f3_join(d[k][c][NP - 1]) : 0.0);
-    block_dots<ND, LPR, CPL, NW>(f, p, stride);
+    block_dots<ND, LPR, CPL, NW>(f, p, stride, off, count);
   } else if constexpr (ND > 0) {
     constexpr int V = ND * CPL * NP;
     constexpr int kDoubles = NW * ND * CPL * 2 * LPR;  // block_dots' buffer
@@ -278,10 +282,10 @@ __device__ __forceinline__ void block_dots_ff(const F3 (&d)[ND > 0 ? ND : 1][CPL
     for (int i = 0; i < kLeft; ++i)
       red[warp][(base + i) * LPR + lane % LPR] = v[i];
     __syncthreads();
-    const int n = ND * p.ncols;
-    double2* out = p.partials + (size_t)blockIdx.x * n;
-    for (int e = threadIdx.x; e < n; e += NW * 32) {
-      const int k = e / p.ncols, col = e % p.ncols;
+    const int nc = count < 0 ? p.ncols : count;
+    double2* out = p.partials + (size_t)blockIdx.x * ND * p.ncols + off;
+    for (int e = threadIdx.x; e < ND * nc; e += NW * 32) {
+      const int k = e / nc, col = e % nc;
       double r[2] = {0.0, 0.0};
 #pragma unroll
       for (int q = 0; q < NP; ++q) {
@@ -291,7 +295,7 @@ __device__ __forceinline__ void block_dots_ff(const F3 (&d)[ND > 0 ? ND : 1][CPL
         for (int w = 1; w < NW; ++w) s = f3_merge(s, red[w][at]);
         r[q] = f3_join(s);
       }
-      out[e] = make_double2(r[0], r[1]);
+      out[k * p.ncols + col] = make_double2(r[0], r[1]);
     }
   }
 }
@@ -816,19 +820,21 @@ KernelFn select_kernel_ffr(int ncols, int dot, bool real, int max_row_nnz, int e
 KernelFn select_kernel_ffc(int ncols, int dot, bool real, int ell_w, int max_row_nnz);
 int ffc_lanes(int ncols);
 // Row-streaming float-float kernels on packed FP32 pairs (kpmgb_step_ffpk.cu):
-// real operators, 2..64 columns, doubling dots, rows of 5..8 nonzeros,
+// real operators, 2..128 columns, doubling dots, rows of 5..8 nonzeros,
 // vectors in the paired element layout (re.hi, im.hi, re.lo, im.lo).  The
 // kernel to launch for such a call of NH rows (fn = nullptr when none
-// applies): threads per block, dynamic shared memory, rows per block tile.
+// applies): threads per block, dynamic shared memory, rows per block tile and
+// the parts of the columns (gridDim.y).
 struct PackedStep {
   KernelFn fn = nullptr;
   int threads = 0;
   size_t smem = 0;
   int rows_per_block = 0;
+  int split = 1;
 };
 PackedStep select_packed_step(int ncols, bool real, int max_row_nnz, int ell_w, int64_t NH);
 // The same over blocks of given rows (KParams::blk), 2..32 columns.
-KernelFn select_packed_members(int ncols, bool real, int max_row_nnz, int ell_w, int64_t NH);
+PackedStep select_packed_members(int ncols, bool real, int max_row_nnz, int ell_w, int64_t NH);
 // Complex operators on column pairs (kpmgb_step_ffcp.cu) over padded rows of
 // stride 8 or 12, vectors in the column-pair layout: steps without dots of
 // exactly 16 or 32 columns, steps with dots of 2..32; nullptr otherwise.

@@ -1,6 +1,6 @@
 // Row-streaming float-float step on packed FP32 pairs (k_step_ffpk): real
-// operators, 33..64 columns (two per lane), doubling dots; k_step_ffpk1 below
-// serves 2..32 columns (one per lane).
+// operators with rows of 6..8, 49..64 columns (two per lane), doubling dots;
+// k_step_ffpk1 below serves the others of 2..128 columns (one per lane).
 //
 // Blackwell executes `fma/add/sub/mul.rn.f32x2` on a 64-bit register pair:
 // one instruction for two correctly rounded FP32 operations.  For real H the
@@ -223,9 +223,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_step_ffpk(
 }
 
 // ---------------------------------------------------------------------------
-// One column per lane (k_step_ffpk1): the packed row-streaming step for 2..32
-// columns, LPR lanes per row (RPW = 32 / LPR rows per warp), with half the
-// loads per lane of k_step_ffpk and so three blocks per SM.  Half of the issue
+// One column per lane (k_step_ffpk1): the packed row-streaming step for 2..128
+// columns in parts of LPR, LPR lanes per row (RPW = 32 / LPR rows per warp; all
+// parts of the columns in one launch), with half the loads per lane of k_step_ffpk and so three blocks per SM.  Half of the issue
 // slots and the latency of the gathers bound it (57% issued with 22 warps per
 // SM at NH = 262144, NR = 8), so the loop keeps to 32-bit indices, the staging
 // addresses advance by constants and lanes past the last column repeat it
@@ -248,14 +248,16 @@ __global__ void __launch_bounds__(kThreads, BLOCKS) k_step_ffpk1(
   constexpr int kStride = 8;              // padded row stride (ints / float2 values)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int lg = lane % LPR, sub = lane / LPR;  // column, and row within the warp
-  const bool live = lg < p.ncols;
+  // the columns of blockIdx.y: LPR each, the rest in the last
+  const int off = blockIdx.y * LPR, ncols = min(LPR, p.ncols - off);
+  const bool live = lg < ncols;
   // tiles t0, t0 + dt, .. of rows origin + t GROUPS .. up to NH (below 2^31)
   const int2 rows = MEMBERS ? __ldg(p.blk + blockIdx.x) : make_int2(0, (int)p.NH);
   const unsigned origin = (unsigned)rows.x, NH = (unsigned)rows.y;
   const unsigned t0 = MEMBERS ? 0 : blockIdx.x, dt = MEMBERS ? 1 : gridDim.x;
   const unsigned row_bytes = p.ld * 16;
   // this lane's column (lanes past the last one repeat it and store nothing)
-  const int64_t col_bytes = (p.c0 + (live ? lg : p.ncols - 1)) * 16;
+  const int64_t col_bytes = (p.c0 + off + (live ? lg : ncols - 1)) * 16;
   const char* const xl = static_cast<const char*>(p.x) + col_bytes;
   const char* const zl = static_cast<const char*>(p.z) + col_bytes;
   char* const yl = static_cast<char*>(p.y) + col_bytes;
@@ -379,10 +381,10 @@ __global__ void __launch_bounds__(kThreads, BLOCKS) k_step_ffpk1(
     d[0][0].x += join2(nS, nC);
     d[1][0] = sacc[threadIdx.x][1];
     d[1][0].x += join2(xS, xC);
-    block_dots<2, LPR, 1>(d, p);
+    block_dots<2, LPR, 1>(d, p, LPR, off, ncols);
   } else {
     const F3 f[2][1][1] = {{{pair_sum(nS, nC)}}, {{pair_sum(xS, xC)}}};
-    block_dots_ff<2, LPR, 1, 1>(f, p);
+    block_dots_ff<2, LPR, 1, 1>(f, p, LPR, off, ncols);
   }
 }
 
@@ -401,47 +403,72 @@ KernelFn ffpk1_w(int max_row_nnz, bool from_hbm) {
 // both slots within about 100 MB stay in L2 from step to step
 bool slots_from_hbm(int64_t NH, int ncols) { return NH * ncols * 32 > (int64_t)100 << 20; }
 
-KernelFn select_kernel_ffpk(int ncols, bool real, int max_row_nnz, int ell_w, bool from_hbm) {
-  if (!real || ell_w != 8 || max_row_nnz > 8) return nullptr;
-  if (ncols == 2) return ffpk1_w<2>(max_row_nnz, from_hbm);
-  if (ncols == 3 || ncols == 4) return ffpk1_w<4>(max_row_nnz, from_hbm);
-  if (ncols >= 5 && ncols <= 8) return ffpk1_w<8>(max_row_nnz, from_hbm);
-  if (ncols >= 9 && ncols <= 16) return ffpk1_w<16>(max_row_nnz, from_hbm);
-  if (ncols >= 17 && ncols <= 32) return ffpk1_w<32>(max_row_nnz, from_hbm);
-  if (ncols < 33 || ncols > 64) return nullptr;
-  const bool full = ncols == 64;
-  switch (max_row_nnz) {
-    case 5: return full ? k_step_ffpk<5, true> : k_step_ffpk<5, false>;
-    case 6: return full ? k_step_ffpk<6, true> : k_step_ffpk<6, false>;
-    case 7: return full ? k_step_ffpk<7, true> : k_step_ffpk<7, false>;
-    case 8: return full ? k_step_ffpk<8, true> : k_step_ffpk<8, false>;
-    default: return nullptr;
+template <bool MEMBERS>
+KernelFn ffpk1_lanes(int lanes, int max_row_nnz, bool from_hbm) {
+  switch (lanes) {
+    case 2: return ffpk1_w<2, MEMBERS>(max_row_nnz, from_hbm);
+    case 4: return ffpk1_w<4, MEMBERS>(max_row_nnz, from_hbm);
+    case 8: return ffpk1_w<8, MEMBERS>(max_row_nnz, from_hbm);
+    case 16: return ffpk1_w<16, MEMBERS>(max_row_nnz, from_hbm);
+    default: return ffpk1_w<32, MEMBERS>(max_row_nnz, from_hbm);
   }
+}
+
+int ffpk1_cols(int ncols, int lanes) { return (ncols + lanes - 1) / lanes * lanes; }
+
+// Lanes per row of k_step_ffpk1 (the columns run in parts of that many, one
+// per gridDim.y): 32, or 16 or 8 where that saves over an eighth of the lanes.
+// Idle lanes cost as much as live ones, narrow parts little: 2D L = 1024, 40
+// columns 8 x 5 lanes 509 us per step, 32 x 2 670; 24 columns 8 x 3 306, 32 363;
+// 48 columns 16 x 3 586, 32 x 2 677; but 50 columns 8 x 7 746, 32 x 2 701.  Parts
+// of 4 read half lines of 64 bytes and gain nothing (12 columns 229, 16 lanes 217).
+int ffpk1_lanes_for(int ncols) {
+  if (ncols <= 8) return ncols <= 2 ? 2 : ncols <= 4 ? 4 : 8;
+  int best = 32;
+  for (int lanes : {16, 8})
+    if (ffpk1_cols(ncols, lanes) * 8 < ffpk1_cols(ncols, best) * 7) best = lanes;
+  return best;
+}
+
+template <int W>
+KernelFn ffpk_w(bool full) {
+  return full ? k_step_ffpk<W, true> : k_step_ffpk<W, false>;
 }
 }  // namespace
 
-int ffpk_lanes(int ncols) {
-  return ncols <= 2 ? 2 : ncols <= 4 ? 4 : ncols <= 8 ? 8 : ncols <= 16 ? 16 : 32;
-}
-
-KernelFn select_packed_members(int ncols, bool real, int max_row_nnz, int ell_w, int64_t NH) {
-  if (!real || ell_w != 8 || max_row_nnz > 8 || ncols < 2 || ncols > 32) return nullptr;
-  const bool from_hbm = slots_from_hbm(NH, ncols);
-  switch (ffpk_lanes(ncols)) {
-    case 2: return ffpk1_w<2, true>(max_row_nnz, from_hbm);
-    case 4: return ffpk1_w<4, true>(max_row_nnz, from_hbm);
-    case 8: return ffpk1_w<8, true>(max_row_nnz, from_hbm);
-    case 16: return ffpk1_w<16, true>(max_row_nnz, from_hbm);
-    default: return ffpk1_w<32, true>(max_row_nnz, from_hbm);
-  }
+PackedStep select_packed_members(int ncols, bool real, int max_row_nnz, int ell_w, int64_t NH) {
+  PackedStep ps;
+  if (!real || ell_w != 8 || max_row_nnz > 8 || ncols < 2 || ncols > 32) return ps;
+  const int lanes = ffpk1_lanes_for(ncols);
+  ps.fn = ffpk1_lanes<true>(lanes, max_row_nnz, slots_from_hbm(NH, ncols));
+  ps.threads = kThreads;
+  ps.rows_per_block = kThreads / lanes;
+  ps.split = (ncols + lanes - 1) / lanes;
+  return ps;
 }
 
 PackedStep select_packed_step(int ncols, bool real, int max_row_nnz, int ell_w, int64_t NH) {
   PackedStep ps;
-  ps.fn = select_kernel_ffpk(ncols, real, max_row_nnz, ell_w, slots_from_hbm(NH, ncols));
+  if (!real || ell_w != 8 || max_row_nnz > 8 || ncols < 2 || ncols > kMaxCols) return ps;
+  const int lanes = ffpk1_lanes_for(ncols);
   ps.threads = kThreads;
-  ps.rows_per_block = ncols > 32 ? kThreads / 32 : kThreads / ffpk_lanes(ncols);
-  ps.smem = 0;
+  // 49..64 columns with rows of 6..8: two columns per lane (3D L = 100, 64
+  // columns 732 us per step, k_step_ffpk1 829); rows of 5: one per lane (2D
+  // L = 1024 708 against 702 us, L = 150 17.7 against 15.3)
+  if (ncols > 48 && ncols <= 64 && max_row_nnz > 5) {
+    const bool full = ncols == 64;
+    switch (max_row_nnz) {
+      case 6: ps.fn = ffpk_w<6>(full); break;
+      case 7: ps.fn = ffpk_w<7>(full); break;
+      case 8: ps.fn = ffpk_w<8>(full); break;
+      default: break;
+    }
+    ps.rows_per_block = kThreads / 32;
+    return ps;
+  }
+  ps.fn = ffpk1_lanes<false>(lanes, max_row_nnz, slots_from_hbm(NH, ncols));
+  ps.rows_per_block = kThreads / lanes;
+  ps.split = (ncols + lanes - 1) / lanes;
   return ps;
 }
 

@@ -1,0 +1,36 @@
+"""Columns that run in several parts of one launch: parts of every width,
+ragged last parts, and both sides of each rule that picks the width."""
+import numpy as np
+import pytest
+
+from conftest import relerr
+import kpm_gb300 as kg
+from kpm_gb300 import models
+from oracle import kpm_oracle as ko
+
+pytestmark = pytest.mark.gpu
+
+TOL = {"fp64": 1e-12, "ff": 1e-9}
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _lib(built_lib):
+    return built_lib
+
+
+@pytest.mark.parametrize("prec", ["ff", "fp64"])
+@pytest.mark.parametrize("NR", [9, 11, 12, 13, 17, 20, 24, 25, 29, 33, 40, 41, 48, 49, 56, 57, 63,
+                                64, 65, 72, 80, 97, 127, 128])
+@pytest.mark.parametrize("lattice", ["square", "cubic", "haldane"])
+def test_doubling(lattice, NR, prec):
+    rng = np.random.default_rng(NR)
+    H = {"square": lambda: models.square_anderson(150, W=2.0, rng=rng) / 5.1,
+         "cubic": lambda: models.cubic_anderson(29, W=2.0, rng=rng) / 7.1,
+         "haldane": lambda: models.haldane(110, 100)[0] / 4.5}[lattice]().tocsc()
+    psi = ko.random_phase_vectors(rng, H.shape[0], NR)
+    got = kg.kpm_1d(H, 12, NR, psi_in=psi, avg_output=False, precision=prec)
+    assert relerr(got, ko.kpm_1d_doubling(H, 12, psi)) < TOL[prec]
+    if lattice == "haldane":
+        bra = ko.random_phase_vectors(rng, H.shape[0], NR)
+        got = kg.kpm_1d(H, 9, NR, psi_in_l=bra, psi_in_r=psi, avg_output=False, precision=prec)
+        assert np.abs(got - ko.kpm_1d_lr(H, 9, bra, psi)).max() < TOL[prec]
