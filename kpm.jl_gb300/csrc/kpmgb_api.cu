@@ -215,7 +215,7 @@ int run_kpm1d(Operator* op, int64_t NC, int64_t NR, int64_t NH, const void* psi_
   const bool paired = paired_on && ff && !lr && !auto_cluster &&
                       (variant == 0 || (variant == 11 && NR >= 9 && NR <= 64)) &&
                       packed_step_applies(op->csr, (int)NR);
-  // Float-float calls with 2..32 columns on complex operators of at most 12
+  // Float-float calls with 2..128 columns on complex operators of at most 12
   // nonzeros per row keep them in the column-pair layout (k_step_ffcp;
   // KPMGB_COLPAIR=0 keeps the standard layout and k_step_ffc).
   const bool colpair = colpair_on && ff && !auto_cluster && variant == 0 &&

@@ -40,6 +40,14 @@ using namespace step;
 // 9..12 columns: FP64 takes four lanes of three columns, which leaves none of
 // its scarce FP64 lanes idle (NH = 262144, 12 columns 106 us per step against
 // the 144 of 16 lanes); float-float takes 16 lanes (more rows in flight).
+// Lanes per row times columns per lane; a shape narrower than the launch runs
+// the columns in parts.  Idle lanes cost as much as live ones (FP64: the pipe
+// serves whole warps; float-float: the issue slots), so parts of 16 or 8 serve
+// where they save over a sixteenth of the lanes.  FP64, per step: Haldane
+// 256x256, 20 columns 8 x 3 268 us, 32 lanes 347; 40 columns 8 x 5 440, 32 x 2
+// 681; 72 columns 8 x 9 786, 32 x 4 1373; square 512x512, 48 columns 16 x 3
+// 409, 8 x 6 413, 32 x 2 553; 150x150, 20 columns 24.1, 32 lanes 28.1.
+// Float-float bra moments, square 512x512, 72 columns 531 us, 32 x 4 lanes 705.
 Shape pick_shape(int ncols, int precision) {
   if (ncols <= 1) return {1, 1};
   if (ncols <= 2) return {2, 1};
@@ -47,9 +55,19 @@ Shape pick_shape(int ncols, int precision) {
   if (ncols <= 8) return {8, 1};
   if (ncols <= 12 && precision == KPMGB_PREC_FP64) return {4, 3};
   if (ncols <= 16) return {16, 1};
-  if (ncols <= 32) return {32, 1};
-  if (ncols <= 64) return {32, 2};
-  return {32, 4};
+  Shape best = ncols <= 32 ? Shape{32, 1} : ncols <= 64 ? Shape{32, 2} : Shape{32, 4};
+  int width = best.lpr * best.cpl;
+  // float-float shapes of one and two columns per lane anchor other chunks of a
+  // row; up to 64 columns keep theirs
+  if (precision == KPMGB_PREC_FF && ncols <= 64) return best;
+  for (int lanes : {32, 16, 8}) {
+    const int held = (ncols + lanes - 1) / lanes * lanes;
+    if (held * 16 < width * 15) {
+      best = {lanes, 1};
+      width = held;
+    }
+  }
+  return best;
 }
 
 // Register-gather shapes that cover ncols columns with at most 4x idle lanes,
@@ -68,6 +86,8 @@ std::vector<Shape> candidate_shapes(int ncols, int precision) {
 }
 
 Shape shape_for(const StepArgs& a, int ncols, int precision) {
+  static const int forced = std::getenv("KPMGB_SHAPE") ? std::atoi(std::getenv("KPMGB_SHAPE")) : 0;
+  if (forced && a.shape == 0) return Shape{forced / 10, forced % 10};
   if (a.shape > 0) {
     const Shape s{a.shape / 10, a.shape % 10};
     if (s.lpr * s.cpl >= ncols) return s;
@@ -159,7 +179,7 @@ int launch_step_kernel(const StepChoice& c, int n, cudaStream_t s, const KBatch&
     return !(e && e[0] == '0');
   }();
   const dim3 grid((unsigned)c.grid, (unsigned)(n * c.split));
-  const int blocks = c.grid * n;
+  const int blocks = c.grid * n * c.split;
   const bool early = c.slots == 0 || blocks >= c.slots || 2 * blocks <= c.slots;
   if (!on || !early) {
     c.fn<<<grid, c.threads, c.smem, s>>>(p);
@@ -209,11 +229,12 @@ const bool kStreamingComplex = [] {
   return !(e && std::atoi(e) == 0);
 }();
 
-int grid_for(KernelFn fn, int64_t NH, int lpr) {
+int grid_for(KernelFn fn, int64_t NH, int lpr, int split = 1) {
   const int per_sm = blocks_per_sm(fn);
   const int64_t groups = kThreads / lpr;
   const int64_t tiles = (NH + groups - 1) / groups;
-  return (int)std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)per_sm * num_sms()));
+  return (int)std::max<int64_t>(
+      1, std::min<int64_t>(tiles, (int64_t)per_sm * num_sms() / split));
 }
 
 // Grid of a packed step: resident blocks per SM (with its threads and
@@ -247,7 +268,7 @@ int grid_packed(const PackedStep& ps, int64_t NH) {
 
 bool colpair_step_applies(const DeviceCSR& H, int NR, int dot) {
   return NR <= cols_per_launch() &&
-         select_kernel_ffcp(NR, dot, H.is_real != 0, H.ell_w, H.max_row_nnz) != nullptr;
+         select_colpair_step(NR, dot, H.is_real != 0, H.ell_w, H.max_row_nnz, H.n).fn != nullptr;
 }
 
 bool packed_step_applies(const DeviceCSR& H, int NR) {
@@ -265,22 +286,22 @@ int choose_step(const StepArgs& a, int precision, int ncols, StepChoice* out) {
     return KPMGB_OK;
   };
   const bool real = H.is_real != 0;
-  // Automatic selection for real operators with 33..64 columns per launch:
-  // the row-streaming kernel when rows hold at most 8 nonzeros (measured on
-  // GB300, 3D Anderson L=128, NR=64: 61.6% of the HBM roofline), else the
-  // padded-row kernel (43.5%; the CSR register-gather kernel 35.3%).
-  // Elsewhere the CSR kernel measured faster: complex Haldane 256x256,
-  // NR=16, kpm_2d 183 ms against 189 ms (exact-length last chunk); the
-  // L2-resident 2D Anderson L=64, NR=12, 7.4 ms against 8.3 ms per call
-  // (4 lanes x 3 columns against 16 x 1).
+  // Calls in the standard layout.  Automatic selection for real operators with
+  // 33..64 columns per launch (bra-ket moments): the row-streaming kernel when
+  // rows hold at most 8 nonzeros, else the padded-row kernel; elsewhere the CSR
+  // kernel (L2-resident 2D Anderson L = 64, 12 columns, 7.4 ms per call against
+  // the padded rows' 8.3).
   if (a.colpair) {
     // the call keeps its vectors in the column-pair layout: only the
     // column-pair kernel reads them
-    KernelFn fq = precision == KPMGB_PREC_FF
-                      ? select_kernel_ffcp(ncols, a.dot, real, H.ell_w, H.max_row_nnz)
-                      : nullptr;
-    if (!fq) return fail(KPMGB_ERR_CUDA, "internal: column-pair layout without its kernel");
-    return take(fq, ffcp_lanes(ncols));
+    const PackedStep ps = precision == KPMGB_PREC_FF
+                              ? select_colpair_step(ncols, a.dot, real, H.ell_w, H.max_row_nnz,
+                                                    a.NH)
+                              : PackedStep{};
+    if (!ps.fn) return fail(KPMGB_ERR_CUDA, "internal: column-pair layout without its kernel");
+    *out = StepChoice{ps.fn, grid_for(ps.fn, a.NH, kThreads / ps.rows_per_block, ps.split),
+                      ps.threads, ps.smem, 0, ps.split};
+    return KPMGB_OK;
   }
   if (a.paired) {
     // the call keeps its vectors in the paired layout: only the packed
@@ -317,7 +338,10 @@ int choose_step(const StepArgs& a, int precision, int ncols, StepChoice* out) {
                                       "columns and rows of at most 16 nonzeros");
   }
   const Shape sh = shape_for(a, ncols, precision);
-  KPMGB_TRY(take(select_kernel(sh, precision, a.dot, real), sh.lpr));
+  const int width = sh.lpr * sh.cpl;
+  out->fn = select_kernel(sh, precision, a.dot, real);
+  out->split = (ncols + width - 1) / width;
+  out->grid = grid_for(out->fn, a.NH, sh.lpr, out->split);
   // The FP64 step of a complex operator is bound by each SM's FP64 pipe.  A
   // grid that leaves some of the resident slots free, but fewer than it needs,
   // gets its successor's first blocks all on the SMs with those slots when
@@ -491,6 +515,7 @@ int launch_steps(const StepArgs* steps, int n, int precision, cudaStream_t s) {
       p.ld = a.NR;
       p.c0 = c0;
       p.ncols = ncols;
+      p.parts = c.split;
       p.x = a.x;
       p.z = a.z;
       p.y = a.y;

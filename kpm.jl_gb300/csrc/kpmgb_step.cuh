@@ -99,6 +99,7 @@ struct KParams {
   int ld;      // row stride of the blocks (total NR)
   int c0;      // first column handled by this launch
   int ncols;   // columns handled by this launch
+  int parts;   // parts of the columns (CSR kernels, consecutive blockIdx.y)
   const void* x;
   const void* z;
   void* y;
@@ -118,6 +119,17 @@ struct KParams {
   // split contraction's exponent (the column-pair kernel only)
   unsigned* vmax;
 };
+
+// The columns of a block whose lanes hold W: the part blockIdx.y % parts of the
+// launch's, from `off` on.
+struct PartCols {
+  int off, c0, n;
+};
+template <int W>
+__device__ __forceinline__ PartCols part_columns(const KParams& p) {
+  const int off = (int)(blockIdx.y % (unsigned)p.parts) * W;
+  return {off, p.c0 + off, min(W, p.ncols - off)};
+}
 
 // One launch applies up to kMaxBatch independent steps without dots (the
 // chains and the current applications of kpm_2d): step blockIdx.y of the
@@ -206,12 +218,12 @@ __device__ __forceinline__ double* red_buffer() {
 
 // Block sums of FP64 dot accumulators (all warps of the block reach this
 // point; warps that own no rows pass zeros), fixed order.  Lane l of a row owns
-// the columns l, l + stride, ...  The block has the columns off .. off + count - 1
-// of the launch (count < 0: all).
+// the columns off + l, off + l + stride, ... of the launch; the first `lanes`
+// lanes of a row have columns.
 template <int ND, int LPR, int CPL, int NW = kWarps>
 __device__ __forceinline__ void block_dots(const double2 (&d)[ND > 0 ? ND : 1][CPL],
                                            const KParams& p, int stride = LPR, int off = 0,
-                                           int count = -1) {
+                                           int lanes = LPR) {
   if constexpr (ND > 0) {
     constexpr int V = ND * CPL * 2;
     double(*red)[V * LPR] = reinterpret_cast<double(*)[V * LPR]>(red_buffer<NW * V * LPR>());
@@ -228,16 +240,15 @@ __device__ __forceinline__ void block_dots(const double2 (&d)[ND > 0 ? ND : 1][C
     for (int i = 0; i < kLeft; ++i)
       red[warp][(base + i) * LPR + lane % LPR] = v[i];
     __syncthreads();
-    const int nc = count < 0 ? p.ncols : count;
-    double* out =
-        reinterpret_cast<double*>(p.partials + (size_t)blockIdx.x * ND * p.ncols + off);
-    for (int e = threadIdx.x; e < 2 * ND * nc; e += NW * 32) {
-      const int k = e / (2 * nc), col = (e >> 1) % nc;
-      const int at = ((k * CPL + col / stride) * 2 + (e & 1)) * LPR + col % stride;
+    double* out = reinterpret_cast<double*>(p.partials + (size_t)blockIdx.x * ND * p.ncols);
+    for (int e = threadIdx.x; e < 2 * ND * CPL * lanes; e += NW * 32) {
+      const int l = (e >> 1) % lanes, kc = (e >> 1) / lanes;
+      const int col = off + kc % CPL * stride + l;
+      if (col >= p.ncols) continue;
       double s = 0.0;
 #pragma unroll
-      for (int w = 0; w < NW; ++w) s += red[w][at];
-      out[2 * (k * p.ncols + col) + (e & 1)] = s;
+      for (int w = 0; w < NW; ++w) s += red[w][(2 * kc + (e & 1)) * LPR + l];
+      out[2 * (kc / CPL * p.ncols + col) + (e & 1)] = s;
     }
   }
 }
@@ -250,7 +261,7 @@ __device__ __forceinline__ void block_dots(const double2 (&d)[ND > 0 ? ND : 1][C
 template <int ND, int LPR, int CPL, int NP, int NW = kWarps>
 __device__ __forceinline__ void block_dots_ff(const F3 (&d)[ND > 0 ? ND : 1][CPL][NP],
                                               const KParams& p, int stride = LPR, int off = 0,
-                                              int count = -1) {
+                                              int lanes = LPR) {
   if constexpr (ND > 0 && CPL > 2) {
     // wide lanes (128 columns): the sums of three floats would take 48 KiB
     double2 f[ND][CPL];
@@ -259,7 +270,7 @@ __device__ __forceinline__ void block_dots_ff(const F3 (&d)[ND > 0 ? ND : 1][CPL
 #pragma unroll
       for (int c = 0; c < CPL; ++c)
         f[k][c] = make_double2(f3_join(d[k][c][0]), NP > 1 ? f3_join(d[k][c][NP - 1]) : 0.0);
-    block_dots<ND, LPR, CPL, NW>(f, p, stride, off, count);
+    block_dots<ND, LPR, CPL, NW>(f, p, stride, off, lanes);
   } else if constexpr (ND > 0) {
     constexpr int V = ND * CPL * NP;
     constexpr int kDoubles = NW * ND * CPL * 2 * LPR;  // block_dots' buffer
@@ -282,20 +293,21 @@ __device__ __forceinline__ void block_dots_ff(const F3 (&d)[ND > 0 ? ND : 1][CPL
     for (int i = 0; i < kLeft; ++i)
       red[warp][(base + i) * LPR + lane % LPR] = v[i];
     __syncthreads();
-    const int nc = count < 0 ? p.ncols : count;
-    double2* out = p.partials + (size_t)blockIdx.x * ND * p.ncols + off;
-    for (int e = threadIdx.x; e < ND * nc; e += NW * 32) {
-      const int k = e / nc, col = e % nc;
+    double2* out = p.partials + (size_t)blockIdx.x * ND * p.ncols;
+    for (int e = threadIdx.x; e < ND * CPL * lanes; e += NW * 32) {
+      const int l = e % lanes, kc = e / lanes;
+      const int col = off + kc % CPL * stride + l;
+      if (col >= p.ncols) continue;
       double r[2] = {0.0, 0.0};
 #pragma unroll
       for (int q = 0; q < NP; ++q) {
-        const int at = ((k * CPL + col / stride) * NP + q) * LPR + col % stride;
+        const int at = (kc * NP + q) * LPR + l;
         F3 s = red[0][at];
 #pragma unroll
         for (int w = 1; w < NW; ++w) s = f3_merge(s, red[w][at]);
         r[q] = f3_join(s);
       }
-      out[k * p.ncols + col] = make_double2(r[0], r[1]);
+      out[kc / CPL * p.ncols + col] = make_double2(r[0], r[1]);
     }
   }
 }
@@ -336,10 +348,14 @@ __device__ __forceinline__ void cdot(double2& acc, double2 a, double2 b) {
   acc.y = fma(-a.y, b.x, acc.y);
 }
 
+// Resident blocks: 42 or 85 registers suffice, and more blocks than this start
+// out unevenly over the SMs when a launch has few tiles (150x150, 10 columns
+// 16.2 us per step at 3 blocks of {4, 3}, 20.6 at 4).
 template <int LPR, int CPL, bool REALH, int DOT>
-__global__ void __launch_bounds__(kThreads) k_step_f64(const __grid_constant__ KBatch batch) {
-  const KParams& p = batch.p[DOT == DOT_NONE ? blockIdx.y : 0];
+__global__ void __launch_bounds__(kThreads, CPL == 1 ? 6 : CPL < 4 ? 3 : 2) k_step_f64(const __grid_constant__ KBatch batch) {
+  const KParams& p = batch.p[DOT == DOT_NONE ? blockIdx.y / (unsigned)batch.p[0].parts : 0];
   pdl_enter();
+  const PartCols cols = part_columns<LPR * CPL>(p);
   constexpr int ND = NDots<DOT>::value;
   constexpr int GROUPS = kThreads / LPR;
   using HV = typename F64Val<REALH>::T;
@@ -368,18 +384,18 @@ __global__ void __launch_bounds__(kThreads) k_step_f64(const __grid_constant__ K
     for (int k = k0; k < k1; ++k) {
       const int j = __ldg(p.col + k);
       const HV h = __ldg(val + k);
-      const double2* xr = x + (int64_t)j * p.ld + p.c0;
+      const double2* xr = x + (int64_t)j * p.ld + cols.c0;
 #pragma unroll
       for (int c = 0; c < CPL; ++c) {
         const int cc = lg + c * LPR;
-        if (cc < p.ncols) cmac(acc[c], h, __ldg(xr + cc));
+        if (cc < cols.n) cmac(acc[c], h, __ldg(xr + cc));
       }
     }
-    const int64_t base = r * p.ld + p.c0;
+    const int64_t base = r * p.ld + cols.c0;
 #pragma unroll
     for (int c = 0; c < CPL; ++c) {
       const int cc = lg + c * LPR;
-      if (cc >= p.ncols) continue;
+      if (cc >= cols.n) continue;
       double2 yv = acc[c];
       if (p.beta_mode != 0) {  // alpha is a power of two: one rounding, as alpha acc, then - z
         const double2 zv = z[base + cc];
@@ -404,7 +420,7 @@ __global__ void __launch_bounds__(kThreads) k_step_f64(const __grid_constant__ K
       }
     }
   }
-  block_dots<ND, LPR, CPL>(d, p);
+  block_dots<ND, LPR, CPL>(d, p, LPR, cols.off);
 }
 
 // ------------------------------------------------------------ float-float path
@@ -492,6 +508,7 @@ __device__ __forceinline__ void ff_chunk(const KParams& p,
                                          float (&Sr)[CPL], float (&Cr)[CPL], float (&Si)[CPL],
                                          float (&Ci)[CPL]) {
   using HV = typename FFVal<REALH>::T;
+  const PartCols cols = part_columns<LPR * CPL>(p);
   int jj[N];
   HV hv[N];
   float R = 0.f;
@@ -507,7 +524,7 @@ __device__ __forceinline__ void ff_chunk(const KParams& p,
     const int cc = lg + c * LPR;
 #pragma unroll
     for (int u = 0; u < N; ++u)
-      xv[c][u] = cc < p.ncols ? __ldg(x + (int64_t)jj[u] * p.ld + p.c0 + cc)
+      xv[c][u] = cc < cols.n ? __ldg(x + (int64_t)jj[u] * p.ld + cols.c0 + cc)
                               : make_float4(0.f, 0.f, 0.f, 0.f);
   }
 #pragma unroll
@@ -556,8 +573,9 @@ __device__ __forceinline__ void ff_chunk_n(int cnt, const KParams& p,
 template <int LPR, int CPL, bool REALH, int DOT, int CH>
 __global__ void __launch_bounds__(kThreads, (FFTune<CPL, REALH>::min_blocks)) k_step_ff(
     const __grid_constant__ KBatch batch) {
-  const KParams& p = batch.p[DOT == DOT_NONE ? blockIdx.y : 0];
+  const KParams& p = batch.p[DOT == DOT_NONE ? blockIdx.y / (unsigned)batch.p[0].parts : 0];
   pdl_enter();
+  const PartCols cols = part_columns<LPR * CPL>(p);
   constexpr int ND = NDots<DOT>::value;
   constexpr int NDA = ND > 0 ? ND : 1;
   constexpr int GROUPS = kThreads / LPR;
@@ -654,8 +672,8 @@ __global__ void __launch_bounds__(kThreads, (FFTune<CPL, REALH>::min_blocks)) k_
           const int cc = lg + c * LPR;
 #pragma unroll
           for (int u = 0; u < CH; ++u) {
-            if (u < cnt && cc < p.ncols)
-              xv[c][u] = __ldg(x + (int64_t)jj[u] * p.ld + p.c0 + cc);
+            if (u < cnt && cc < cols.n)
+              xv[c][u] = __ldg(x + (int64_t)jj[u] * p.ld + cols.c0 + cc);
             else
               xv[c][u] = make_float4(0.f, 0.f, 0.f, 0.f);
           }
@@ -691,11 +709,11 @@ __global__ void __launch_bounds__(kThreads, (FFTune<CPL, REALH>::min_blocks)) k_
         }
       }
     }
-    const int64_t base = r * p.ld + p.c0;
+    const int64_t base = r * p.ld + cols.c0;
 #pragma unroll
     for (int c = 0; c < CPL; ++c) {
       const int cc = lg + c * LPR;
-      if (cc >= p.ncols) continue;
+      if (cc >= cols.n) continue;
       float4 zv = make_float4(0.f, 0.f, 0.f, 0.f);
       if (beta_mode != 0) zv = kStreamHints ? __ldcs(z + base + cc) : z[base + cc];
       const float2 yr = ff_epilogue(Sr[c], Cr[c], alpha, beta_mode, zv.x, zv.y);
@@ -745,7 +763,7 @@ __global__ void __launch_bounds__(kThreads, (FFTune<CPL, REALH>::min_blocks)) k_
           d[k][c].x += ff::join(dS[k][c][0], dC[k][c][0]);
           d[k][c].y += ff::join(dS[k][c][1], dC[k][c][1]);
         }
-      block_dots<ND, LPR, CPL>(d, p);
+      block_dots<ND, LPR, CPL>(d, p, LPR, cols.off);
     } else {
       F3 f[NDA][CPL][2];
 #pragma unroll
@@ -754,7 +772,7 @@ __global__ void __launch_bounds__(kThreads, (FFTune<CPL, REALH>::min_blocks)) k_
         for (int c = 0; c < CPL; ++c)
 #pragma unroll
           for (int q = 0; q < 2; ++q) f[k][c][q] = F3{dS[k][c][q], dC[k][c][q], 0.f};
-      block_dots_ff<ND, LPR, CPL, 2>(f, p);
+      block_dots_ff<ND, LPR, CPL, 2>(f, p, LPR, cols.off);
     }
   }
 }
@@ -837,10 +855,9 @@ PackedStep select_packed_step(int ncols, bool real, int max_row_nnz, int ell_w, 
 PackedStep select_packed_members(int ncols, bool real, int max_row_nnz, int ell_w, int64_t NH);
 // Complex operators on column pairs (kpmgb_step_ffcp.cu) over padded rows of
 // stride 8 or 12, vectors in the column-pair layout: steps without dots of
-// exactly 16 or 32 columns, steps with dots of 2..32; nullptr otherwise.
-// ffcp_lanes: lanes per row.
-KernelFn select_kernel_ffcp(int ncols, int dot, bool real, int ell_w, int max_row_nnz);
-int ffcp_lanes(int ncols);
+// exactly 16 or 32 columns, steps with dots of 2..128.
+PackedStep select_colpair_step(int ncols, int dot, bool real, int ell_w, int max_row_nnz,
+                               int64_t NH);
 
 }  // namespace step
 }  // namespace kpmgb

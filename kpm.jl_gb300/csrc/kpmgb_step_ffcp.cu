@@ -1,5 +1,6 @@
-// Complex operators on column pairs (k_step_ffcp), 2..32 columns: kpm_2d's
-// steps without dots (chains and current applications) and kpm_1d's with them.
+// Complex operators on column pairs (k_step_ffcp): kpm_2d's steps without dots
+// (chains and current applications, 16 or 32 columns) and kpm_1d's with them
+// (2..128 columns, in parts of 4, 8 or 16 pairs, all parts in one launch).
 // A lane owns columns q and q + h of a row, h = ceil(NR / 2), and the call
 // stores its vectors in the column-pair layout: per row and q one 32-byte block
 // (re.hi, re.hi', re.lo, re.lo', im.hi, im.hi', im.lo, im.lo') for the two
@@ -47,14 +48,18 @@ __global__ void __launch_bounds__(kThreads, 2) k_step_ffcp(
   constexpr int kPieces = W / 4 + W;       // 16-byte pieces of one padded row
   const int lane_q = threadIdx.x % LPH;
   const int half = FULL ? LPH : (p.ncols + 1) / 2;  // pairs per row
-  // lanes past the last pair repeat it and store nothing
-  const bool live = FULL || lane_q < half;
-  const int lg = live ? lane_q : half - 1;
+  // the pairs of this part of the columns (steps with dots: blockIdx.y, LPH pairs
+  // each, the rest in the last); lanes past the last pair repeat it and store
+  // nothing
+  const int off = DOT == DOT_NONE ? 0 : blockIdx.y * LPH;
+  const int pairs = FULL ? LPH : min(LPH, half - off);
+  const bool live = FULL || lane_q < pairs;
+  const int lg = live ? lane_q : pairs - 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane / LPH;              // row of this lane within the warp
-  const ulonglong2* __restrict__ x = static_cast<const ulonglong2*>(p.x);
-  const ulonglong2* z = static_cast<const ulonglong2*>(p.z);
-  ulonglong2* y = static_cast<ulonglong2*>(p.y);
+  const ulonglong2* __restrict__ x = static_cast<const ulonglong2*>(p.x) + 2 * off;
+  const ulonglong2* z = static_cast<const ulonglong2*>(p.z) + 2 * off;
+  ulonglong2* y = static_cast<ulonglong2*>(p.y) + 2 * off;
   const f2 alpha2 = pk(p.alpha_f, p.alpha_f);
   const int beta_mode = p.beta_mode;
   const f2 zero2 = pk(0.f, 0.f);
@@ -97,7 +102,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_step_ffcp(
   constexpr int ND = NDots<DOT>::value;
   constexpr int NP = DOT == DOT_DOUBLING ? 1 : 2;
   constexpr int NV = ND * NP > 0 ? ND * NP : 1;
-  const ulonglong2* __restrict__ bra = static_cast<const ulonglong2*>(p.bra);
+  const ulonglong2* __restrict__ bra = static_cast<const ulonglong2*>(p.bra) + 2 * off;
   __shared__ double sacc[ND > 0 ? 2 * NV : 1][ND > 0 ? kThreads : 1];
   f2 dS[NV], dC[NV];
 #pragma unroll
@@ -283,7 +288,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_step_ffcp(
                       side_join(dS[n * NP + q], dC[n * NP + q], c);
           d[n][c] = make_double2(part[0], part[1]);
         }
-      block_dots<ND, LPH, 2>(d, p, half);
+      block_dots<ND, LPH, 2>(d, p, half, off, pairs);
     } else {
       F3 f[ND][2][NP];
 #pragma unroll
@@ -292,7 +297,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_step_ffcp(
         for (int c = 0; c < 2; ++c)
 #pragma unroll
           for (int q = 0; q < NP; ++q) f[n][c][q] = side_f3(dS[n * NP + q], dC[n * NP + q], c);
-      block_dots_ff<ND, LPH, 2, NP>(f, p, half);
+      block_dots_ff<ND, LPH, 2, NP>(f, p, half, off, pairs);
     }
     return;
   }
@@ -323,33 +328,53 @@ KernelFn ffcp_w(int ell_w, int max_row_nnz) {
   }
 }
 template <int DOT>
-KernelFn ffcp_lanes_of(int half, int ell_w, int max_row_nnz) {
-  if (half <= 2) return ffcp_w<2, DOT, false>(ell_w, max_row_nnz);
-  if (half <= 4) return ffcp_w<4, DOT, false>(ell_w, max_row_nnz);
-  if (half <= 8) return ffcp_w<8, DOT, false>(ell_w, max_row_nnz);
-  return ffcp_w<16, DOT, false>(ell_w, max_row_nnz);
+KernelFn ffcp_lanes_of(int lanes, int ell_w, int max_row_nnz) {
+  switch (lanes) {
+    case 2: return ffcp_w<2, DOT, false>(ell_w, max_row_nnz);
+    case 4: return ffcp_w<4, DOT, false>(ell_w, max_row_nnz);
+    case 8: return ffcp_w<8, DOT, false>(ell_w, max_row_nnz);
+    default: return ffcp_w<16, DOT, false>(ell_w, max_row_nnz);
+  }
+}
+
+// Lanes per row: 16, or 8 or (long vectors) 4 where that saves over an eighth of
+// the lanes.  Doubling step, Haldane 256x256: 24 columns 4 x 3 lanes 70 us, 16
+// lanes 82; 40 columns 4 x 5 112 (CSR kernel 264); 72 columns 4 x 9 208 (440);
+// 128 columns 310 (495).  100x100, 18 columns: 4 x 3 15.1 us, 16 lanes 14.0.
+int ffcp_lanes(int half, int64_t NH) {
+  if (half <= 8) return half <= 2 ? 2 : half <= 4 ? 4 : 8;
+  auto held = [&](int lanes) { return (half + lanes - 1) / lanes * lanes; };
+  int best = 16;
+  for (int lanes : {8, 4})
+    if (held(lanes) * 8 < held(best) * 7 && (lanes > 4 || NH > 1 << 16 || half > 16)) best = lanes;
+  return best;
 }
 }  // namespace
 
-int ffcp_lanes(int ncols) {
-  const int half = (ncols + 1) / 2;
-  return half <= 2 ? 2 : half <= 4 ? 4 : half <= 8 ? 8 : 16;
-}
-
-KernelFn select_kernel_ffcp(int ncols, int dot, bool real, int ell_w, int max_row_nnz) {
-  if (real || max_row_nnz < 1 || max_row_nnz > ell_w) return nullptr;
+PackedStep select_colpair_step(int ncols, int dot, bool real, int ell_w, int max_row_nnz,
+                               int64_t NH) {
+  PackedStep ps;
+  if (real || max_row_nnz < 1 || max_row_nnz > ell_w || ncols < 2 || ncols > kMaxCols) return ps;
+  const int half = (ncols + 1) / 2, lanes = ffcp_lanes(half, NH);
+  ps.threads = kThreads;
+  ps.rows_per_block = kThreads / lanes;
   if (dot == DOT_NONE) {
-    if (ncols == 16) return ffcp_w<8, DOT_NONE, true>(ell_w, max_row_nnz);
-    if (ncols == 32) return ffcp_w<16, DOT_NONE, true>(ell_w, max_row_nnz);
-    return nullptr;
+    if (ncols == 16) ps.fn = ffcp_w<8, DOT_NONE, true>(ell_w, max_row_nnz);
+    if (ncols == 32) ps.fn = ffcp_w<16, DOT_NONE, true>(ell_w, max_row_nnz);
+    return ps;
   }
-  if (ncols < 2 || ncols > 32) return nullptr;
-  const int half = (ncols + 1) / 2;
+  ps.split = (half + lanes - 1) / lanes;
   switch (dot) {
-    case DOT_DOUBLING: return ffcp_lanes_of<DOT_DOUBLING>(half, ell_w, max_row_nnz);
-    case DOT_LR2: return ffcp_lanes_of<DOT_LR2>(half, ell_w, max_row_nnz);
-    default: return ffcp_lanes_of<DOT_LR1>(half, ell_w, max_row_nnz);
+    case DOT_DOUBLING:
+      ps.fn = ffcp_lanes_of<DOT_DOUBLING>(lanes, ell_w, max_row_nnz);
+      break;
+    case DOT_LR2:
+      ps.fn = ffcp_lanes_of<DOT_LR2>(lanes, ell_w, max_row_nnz);
+      break;
+    default:
+      ps.fn = ffcp_lanes_of<DOT_LR1>(lanes, ell_w, max_row_nnz);
   }
+  return ps;
 }
 
 }  // namespace step

@@ -381,10 +381,10 @@ __global__ void __launch_bounds__(kThreads, BLOCKS) k_step_ffpk1(
     d[0][0].x += join2(nS, nC);
     d[1][0] = sacc[threadIdx.x][1];
     d[1][0].x += join2(xS, xC);
-    block_dots<2, LPR, 1>(d, p, LPR, off, ncols);
+    block_dots<2, LPR, 1>(d, p, LPR, off);
   } else {
     const F3 f[2][1][1] = {{{pair_sum(nS, nC)}}, {{pair_sum(xS, xC)}}};
-    block_dots_ff<2, LPR, 1, 1>(f, p, LPR, off, ncols);
+    block_dots_ff<2, LPR, 1, 1>(f, p, LPR, off);
   }
 }
 

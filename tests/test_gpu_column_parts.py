@@ -30,7 +30,18 @@ def test_doubling(lattice, NR, prec):
     psi = ko.random_phase_vectors(rng, H.shape[0], NR)
     got = kg.kpm_1d(H, 12, NR, psi_in=psi, avg_output=False, precision=prec)
     assert relerr(got, ko.kpm_1d_doubling(H, 12, psi)) < TOL[prec]
-    if lattice == "haldane":
-        bra = ko.random_phase_vectors(rng, H.shape[0], NR)
-        got = kg.kpm_1d(H, 9, NR, psi_in_l=bra, psi_in_r=psi, avg_output=False, precision=prec)
-        assert np.abs(got - ko.kpm_1d_lr(H, 9, bra, psi)).max() < TOL[prec]
+    bra = ko.random_phase_vectors(rng, H.shape[0], NR)
+    got = kg.kpm_1d(H, 9, NR, psi_in_l=bra, psi_in_r=psi, avg_output=False, precision=prec)
+    assert np.abs(got - ko.kpm_1d_lr(H, 9, bra, psi)).max() < TOL[prec]
+
+
+@pytest.mark.parametrize("prec", ["ff", "fp64"])
+@pytest.mark.parametrize("NR", [17, 33, 65, 100, 129])
+def test_two_dimensional(NR, prec):
+    """Batched steps without dots in parts."""
+    rng = np.random.default_rng(NR)
+    H, Jx, Jy, _ = models.haldane(14, 10)
+    H = (H / 4.5).tocsc()
+    psi = ko.random_phase_vectors(rng, H.shape[0], NR)
+    got = kg.kpm_2d(H, Jx, Jy, 16, NR, H.shape[0], psi_in=psi, precision=prec)
+    assert relerr(got, ko.kpm_2d(H, Jx, Jy, 16, psi, psi, 16, 16)) < TOL[prec]
