@@ -429,7 +429,7 @@ int run_kpm2d(Operator* H, Operator* Ja, Operator* Jb, int64_t NC, int64_t NR, i
   auto RING = [&](int64_t i) { return (void*)(ws.ring.as<char>() + i * block); };
   double* sc = ws.scales.as<double>();
   // Float-float calls with the split contraction on complex H, Ja, Jb of at
-  // most 12 nonzeros per row and 16 or 32 probe columns keep their vectors in
+  // most 12 nonzeros per row and an even number (6 or more) of probe columns keep their vectors in
   // the column-pair layout and run every step on column pairs
   // (k_step_ffcp); the contraction sums over memory order, the same
   // permutation of K on both sides.  KPMGB_COLPAIR=0 keeps the standard

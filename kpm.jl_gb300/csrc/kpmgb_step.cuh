@@ -854,8 +854,8 @@ PackedStep select_packed_step(int ncols, bool real, int max_row_nnz, int ell_w, 
 // The same over blocks of given rows (KParams::blk), 2..32 columns.
 PackedStep select_packed_members(int ncols, bool real, int max_row_nnz, int ell_w, int64_t NH);
 // Complex operators on column pairs (kpmgb_step_ffcp.cu) over padded rows of
-// stride 8 or 12, vectors in the column-pair layout: steps without dots of
-// exactly 16 or 32 columns, steps with dots of 2..128.
+// stride 8 or 12, vectors in the column-pair layout: 2..128 columns, an even
+// number from 6 on in steps without dots.
 PackedStep select_colpair_step(int ncols, int dot, bool real, int ell_w, int max_row_nnz,
                                int64_t NH);
 

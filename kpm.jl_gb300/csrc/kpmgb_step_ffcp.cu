@@ -1,6 +1,6 @@
 // Complex operators on column pairs (k_step_ffcp): kpm_2d's steps without dots
-// (chains and current applications, 16 or 32 columns) and kpm_1d's with them
-// (2..128 columns, in parts of 4, 8 or 16 pairs, all parts in one launch).
+// (chains and current applications, an even number of columns) and kpm_1d's with
+// them (2..128 columns, in parts of 4, 8 or 16 pairs, all parts in one launch).
 // A lane owns columns q and q + h of a row, h = ceil(NR / 2), and the call
 // stores its vectors in the column-pair layout: per row and q one 32-byte block
 // (re.hi, re.hi', re.lo, re.lo', im.hi, im.hi', im.lo, im.lo') for the two
@@ -41,17 +41,16 @@ __device__ __forceinline__ double side_join(f2 S, f2 C, int side) {
 template <int LPH, int W, int WL, int DOT, bool FULL>
 __global__ void __launch_bounds__(kThreads, 2) k_step_ffcp(
     const __grid_constant__ KBatch batch) {
-  const KParams& p = batch.p[DOT == DOT_NONE ? blockIdx.y : 0];
+  const KParams& p = batch.p[DOT == DOT_NONE ? blockIdx.y / (unsigned)batch.p[0].parts : 0];
   pdl_enter();
   constexpr int RPW = 32 / LPH;            // rows per warp
   constexpr int GROUPS = kThreads / LPH;   // rows per block tile
   constexpr int kPieces = W / 4 + W;       // 16-byte pieces of one padded row
   const int lane_q = threadIdx.x % LPH;
   const int half = FULL ? LPH : (p.ncols + 1) / 2;  // pairs per row
-  // the pairs of this part of the columns (steps with dots: blockIdx.y, LPH pairs
-  // each, the rest in the last); lanes past the last pair repeat it and store
-  // nothing
-  const int off = DOT == DOT_NONE ? 0 : blockIdx.y * LPH;
+  // the pairs of this part of the columns (LPH each, the rest in the last); lanes
+  // past the last pair repeat it and store nothing
+  const int off = FULL ? 0 : (int)(blockIdx.y % (unsigned)p.parts) * LPH;
   const int pairs = FULL ? LPH : min(LPH, half - off);
   const bool live = FULL || lane_q < pairs;
   const int lg = live ? lane_q : pairs - 1;
@@ -358,13 +357,18 @@ PackedStep select_colpair_step(int ncols, int dot, bool real, int ell_w, int max
   const int half = (ncols + 1) / 2, lanes = ffcp_lanes(half, NH);
   ps.threads = kThreads;
   ps.rows_per_block = kThreads / lanes;
-  if (dot == DOT_NONE) {
-    if (ncols == 16) ps.fn = ffcp_w<8, DOT_NONE, true>(ell_w, max_row_nnz);
-    if (ncols == 32) ps.fn = ffcp_w<16, DOT_NONE, true>(ell_w, max_row_nnz);
-    return ps;
-  }
   ps.split = (half + lanes - 1) / lanes;
   switch (dot) {
+    case DOT_NONE:
+      // the contraction walks memory order, whole pairs only; below 6 columns a
+      // step has too few lanes in flight (kpm_2d of a Haldane 64x64, 128 moments,
+      // NR = 4 1.15 ms, CSR steps 0.96; NR = 6 1.36 and 1.39; 200x150, 64
+      // moments, NR = 6 2.86 and 3.72, NR = 24 8.6 and 12.2)
+      if (ncols % 2 || ncols < 6) return PackedStep{};
+      if (ncols == 16) ps.fn = ffcp_w<8, DOT_NONE, true>(ell_w, max_row_nnz);
+      else if (ncols == 32) ps.fn = ffcp_w<16, DOT_NONE, true>(ell_w, max_row_nnz);
+      else ps.fn = ffcp_lanes_of<DOT_NONE>(lanes, ell_w, max_row_nnz);
+      break;
     case DOT_DOUBLING:
       ps.fn = ffcp_lanes_of<DOT_DOUBLING>(lanes, ell_w, max_row_nnz);
       break;

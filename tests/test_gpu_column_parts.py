@@ -45,3 +45,19 @@ def test_two_dimensional(NR, prec):
     psi = ko.random_phase_vectors(rng, H.shape[0], NR)
     got = kg.kpm_2d(H, Jx, Jy, 16, NR, H.shape[0], psi_in=psi, precision=prec)
     assert relerr(got, ko.kpm_2d(H, Jx, Jy, 16, psi, psi, 16, 16)) < TOL[prec]
+
+
+@pytest.mark.parametrize("cells", [(9, 7), (15, 13)])   # K = 126 NR and 390 NR
+@pytest.mark.parametrize("NR", [2, 4, 6, 8, 10, 14, 18, 20, 24, 30, 34, 40, 66])
+def test_two_dimensional_column_pairs(NR, cells):
+    """Column pairs without dots: every lane count and parts, with and without
+    blocks of the left chain."""
+    rng = np.random.default_rng(NR)
+    H, Jx, Jy, _ = models.haldane(*cells)
+    H = (H / 4.5).tocsc()
+    psi = ko.random_phase_vectors(rng, H.shape[0], NR)
+    ref = ko.kpm_2d(H, Jx, Jy, 20, psi, psi, 20, 20)
+    for kw in (dict(), dict(arr_size=7, right_block=4)):
+        got = kg.kpm_2d(H, Jx, Jy, 20, NR, H.shape[0], psi_in=psi, precision="ff",
+                        contraction="split", **kw)
+        assert relerr(got, ref) < TOL["ff"]
