@@ -208,13 +208,13 @@ int run_kpm1d(Operator* op, int64_t NC, int64_t NR, int64_t NH, const void* psi_
     return fail(KPMGB_ERR_ARGUMENT, "unknown kernel_variant %d", variant);
   const bool auto_cluster =
       variant == 0 && cluster_auto_on && cluster_is_faster(op->csr, NH, (int)NR, precision, lr);
-  // Float-float doubling calls with 2..128 columns on real operators of 5..8
+  // Float-float calls with 2..128 columns on real operators of 5..8
   // nonzeros in the longest row keep their vectors in the paired element layout
   // and run every step on packed FP32 pairs (k_step_ffpk / k_step_ffpk1;
   // KPMGB_PAIRED=0 keeps the standard layout and k_step_ffr).
-  const bool paired = paired_on && ff && !lr && !auto_cluster &&
-                      (variant == 0 || (variant == 11 && NR >= 9 && NR <= 64)) &&
-                      packed_step_applies(op->csr, (int)NR);
+  const bool paired = paired_on && ff && !auto_cluster &&
+                      (variant == 0 || (variant == 11 && !lr && NR >= 9 && NR <= 64)) &&
+                      packed_step_applies(op->csr, (int)NR, lr ? DOT_LR1 : DOT_DOUBLING);
   // Float-float calls with 2..128 columns on complex operators of at most 12
   // nonzeros per row keep them in the column-pair layout (k_step_ffcp;
   // KPMGB_COLPAIR=0 keeps the standard layout and k_step_ffc).

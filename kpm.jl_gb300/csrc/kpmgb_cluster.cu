@@ -482,7 +482,9 @@ bool cluster_is_faster(const DeviceCSR& H, int64_t NH, int NR, int precision, bo
   } else {
     cluster = real ? 1.6 + 0.0017 * load : 2.0 + 0.0038 * load;
     if (real)
-      launches = !lr && packed_step_applies(H, NR) ? 2.7 + 1.15e-5 * work : 3.5 + 1.9e-5 * work;
+      launches = packed_step_applies(H, NR, lr ? DOT_LR1 : DOT_DOUBLING)
+                     ? 2.7 + 1.15e-5 * work
+                     : 3.5 + 1.9e-5 * work;
     else
       launches = NR <= 8 ? 4.0 + 2.9e-5 * work : 2.8 + 2.4e-5 * work;
   }

@@ -227,7 +227,7 @@ int launch_step(const StepArgs& a, int precision, cudaStream_t s);
 int launch_steps(const StepArgs* steps, int n, int precision, cudaStream_t s);
 // Whether float-float doubling steps of NR columns on H can run on packed
 // FP32 pairs over the paired vector layout (StepArgs::paired).
-bool packed_step_applies(const DeviceCSR& H, int NR);
+bool packed_step_applies(const DeviceCSR& H, int NR, int dot);
 // Whether float-float steps of NR columns on H with these dots can run on
 // column pairs over the column-pair vector layout (StepArgs::colpair).
 bool colpair_step_applies(const DeviceCSR& H, int NR, int dot);

@@ -271,9 +271,9 @@ bool colpair_step_applies(const DeviceCSR& H, int NR, int dot) {
          select_colpair_step(NR, dot, H.is_real != 0, H.ell_w, H.max_row_nnz, H.n).fn != nullptr;
 }
 
-bool packed_step_applies(const DeviceCSR& H, int NR) {
+bool packed_step_applies(const DeviceCSR& H, int NR, int dot) {
   return NR <= cols_per_launch() &&
-         select_packed_step(NR, H.is_real != 0, H.max_row_nnz, H.ell_w, H.n).fn != nullptr;
+         select_packed_step(NR, dot, H.is_real != 0, H.max_row_nnz, H.ell_w, H.n).fn != nullptr;
 }
 
 namespace {
@@ -306,8 +306,8 @@ int choose_step(const StepArgs& a, int precision, int ncols, StepChoice* out) {
   if (a.paired) {
     // the call keeps its vectors in the paired layout: only the packed
     // kernel reads them
-    const PackedStep ps = precision == KPMGB_PREC_FF && a.dot == DOT_DOUBLING
-                              ? select_packed_step(ncols, real, H.max_row_nnz, H.ell_w, a.NH)
+    const PackedStep ps = precision == KPMGB_PREC_FF
+                              ? select_packed_step(ncols, a.dot, real, H.max_row_nnz, H.ell_w, a.NH)
                               : PackedStep{};
     if (!ps.fn) return fail(KPMGB_ERR_CUDA, "internal: paired layout without the packed kernel");
     *out = StepChoice{ps.fn, grid_packed(ps, a.NH), ps.threads, ps.smem, 0, ps.split};

@@ -838,7 +838,7 @@ KernelFn select_kernel_ffr(int ncols, int dot, bool real, int max_row_nnz, int e
 KernelFn select_kernel_ffc(int ncols, int dot, bool real, int ell_w, int max_row_nnz);
 int ffc_lanes(int ncols);
 // Row-streaming float-float kernels on packed FP32 pairs (kpmgb_step_ffpk.cu):
-// real operators, 2..128 columns, doubling dots, rows of 5..8 nonzeros,
+// real operators, 2..128 columns, steps with dots, rows of 5..8 nonzeros,
 // vectors in the paired element layout (re.hi, im.hi, re.lo, im.lo).  The
 // kernel to launch for such a call of NH rows (fn = nullptr when none
 // applies): threads per block, dynamic shared memory, rows per block tile and
@@ -850,7 +850,8 @@ struct PackedStep {
   int rows_per_block = 0;
   int split = 1;
 };
-PackedStep select_packed_step(int ncols, bool real, int max_row_nnz, int ell_w, int64_t NH);
+PackedStep select_packed_step(int ncols, int dot, bool real, int max_row_nnz, int ell_w,
+                              int64_t NH);
 // The same over blocks of given rows (KParams::blk), 2..32 columns.
 PackedStep select_packed_members(int ncols, bool real, int max_row_nnz, int ell_w, int64_t NH);
 // Complex operators on column pairs (kpmgb_step_ffcp.cu) over padded rows of

@@ -58,6 +58,25 @@ __device__ __forceinline__ F3 pair_sum(f2 S, f2 C) {
   return f3_merge(a, b);
 }
 
+// The first lane less the second.
+__device__ __forceinline__ F3 pair_diff(f2 S, f2 C) {
+  F3 a{0.f, 0.f, 0.f}, b{0.f, 0.f, 0.f};
+  upk(S, a.s, b.s);
+  upk(C, a.c, b.c);
+  return f3_merge(a, F3{-b.s, -b.c, 0.f});
+}
+__device__ __forceinline__ double diff2(f2 S, f2 C) {
+  float s0, s1, c0, c1;
+  upk(S, s0, s1);
+  upk(C, c0, c1);
+  return ((double)s0 + (double)c0) - ((double)s1 + (double)c1);
+}
+__device__ __forceinline__ f2 swap2(f2 v) {
+  float a, b;
+  upk(v, a, b);
+  return pk(b, a);
+}
+
 template <int W, bool FULL>
 __global__ void __launch_bounds__(kThreads, 2) k_step_ffpk(
     const __grid_constant__ KBatch batch) {
@@ -238,7 +257,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_step_ffpk(
 //
 // MEMBERS: each block takes the consecutive rows p.blk[block] (the rows of one
 // member of an ensemble) instead of every gridDim-th tile.
-template <int LPR, int W, int BLOCKS, bool MEMBERS>
+template <int LPR, int W, int BLOCKS, int DOT, bool MEMBERS>
 __global__ void __launch_bounds__(kThreads, BLOCKS) k_step_ffpk1(
     const __grid_constant__ KBatch batch) {
   const KParams& p = batch.p[0];
@@ -261,14 +280,34 @@ __global__ void __launch_bounds__(kThreads, BLOCKS) k_step_ffpk1(
   const char* const xl = static_cast<const char*>(p.x) + col_bytes;
   const char* const zl = static_cast<const char*>(p.z) + col_bytes;
   char* const yl = static_cast<char*>(p.y) + col_bytes;
+  const char* const bl = DOT == DOT_DOUBLING ? nullptr : static_cast<const char*>(p.bra) + col_bytes;
   const f2 alpha2 = pk(p.alpha_f, p.alpha_f);
   const int beta_mode = p.beta_mode;
   const f2 zero2 = pk(0.f, 0.f);
-  __shared__ double2 sacc[kThreads][2];
+  constexpr int ND = NDots<DOT>::value;
+  constexpr int NV = DOT == DOT_DOUBLING ? 2 : 2 * ND;
+  __shared__ double2 sacc[kThreads][ND];
   // per warp, two buffers of RPW padded rows: 8 column indices, 8 values
   __shared__ __align__(16) int sidx[kThreads / 32][2][RPW][3 * kStride];
-  f2 nS = zero2, nC = zero2, xS = zero2, xC = zero2;
-  sacc[threadIdx.x][0] = sacc[threadIdx.x][1] = make_double2(0.0, 0.0);
+  // DOUBLING: <x|x>, Re<x|y>; LR: of <b|x> (LR2) and <b|y> the products
+  // {re re, im im} and {re im, im re}
+  f2 dS[NV], dC[NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) dS[v] = dC[v] = zero2;
+#pragma unroll
+  for (int n = 0; n < ND; ++n) sacc[threadIdx.x][n] = make_double2(0.0, 0.0);
+  auto fold = [&](double2 (&d)[ND][1]) {
+#pragma unroll
+    for (int n = 0; n < ND; ++n) {
+      d[n][0] = sacc[threadIdx.x][n];
+      if constexpr (DOT == DOT_DOUBLING) {
+        d[n][0].x += join2(dS[n], dC[n]);
+      } else {
+        d[n][0].x += join2(dS[2 * n], dC[2 * n]);
+        d[n][0].y += diff2(dS[2 * n + 1], dC[2 * n + 1]);
+      }
+    }
+  };
   int rows_since_flush = 0;
   const unsigned ntiles = (NH - origin + GROUPS - 1) / GROUPS;
   // the warp's lanes copy the RPW rows of a tile: 6 pieces of 16 bytes each, at
@@ -314,10 +353,11 @@ __global__ void __launch_bounds__(kThreads, BLOCKS) k_step_ffpk1(
     const float4* hrow = reinterpret_cast<const float4*>(&sidx[warp][buf][sub][kStride]);
     const uint64_t e = (uint64_t)row * row_bytes;
     const ulonglong2 zero = make_ulonglong2(0ull, 0ull);
-    ulonglong2 zv = zero, xo = zero, xv[W];
+    ulonglong2 zv = zero, xo = zero, bv = zero, xv[W];
     if (row < NH) {
       if (beta_mode != 0) zv = __ldcs(reinterpret_cast<const ulonglong2*>(zl + e));
-      xo = __ldg(reinterpret_cast<const ulonglong2*>(xl + e));
+      if constexpr (DOT != DOT_LR1) xo = __ldg(reinterpret_cast<const ulonglong2*>(xl + e));
+      if constexpr (DOT != DOT_DOUBLING) bv = __ldg(reinterpret_cast<const ulonglong2*>(bl + e));
 #pragma unroll
       for (int u = 0; u < W; ++u)
         xv[u] = __ldg(reinterpret_cast<const ulonglong2*>(xl + (uint64_t)(unsigned)jrow[u] * row_bytes));
@@ -363,39 +403,58 @@ __global__ void __launch_bounds__(kThreads, BLOCKS) k_step_ffpk1(
         two_sum2(s2, add2(e2, sub2(c2, zv.y)), yh, yl2);
       }
       __stcs(reinterpret_cast<ulonglong2*>(yl + e), make_ulonglong2(yh, yl2));
-      const f2 nxh = sub2(zero2, xo.x);
-      dacc2(nS, nC, xo.x, nxh, xo.y, xo.x, xo.y);
-      dacc2(xS, xC, xo.x, nxh, xo.y, yh, yl2);
+      if constexpr (DOT == DOT_DOUBLING) {
+        const f2 nxh = sub2(zero2, xo.x);
+        dacc2(dS[0], dC[0], xo.x, nxh, xo.y, xo.x, xo.y);
+        dacc2(dS[1], dC[1], xo.x, nxh, xo.y, yh, yl2);
+      } else {
+        const f2 nbh = sub2(zero2, bv.x);
+        auto dot = [&](int v, f2 h, f2 l) {
+          dacc2(dS[v], dC[v], bv.x, nbh, bv.y, h, l);
+          dacc2(dS[v + 1], dC[v + 1], bv.x, nbh, bv.y, swap2(h), swap2(l));
+        };
+        if constexpr (DOT == DOT_LR2) dot(0, xo.x, xo.y);
+        dot(NV - 2, yh, yl2);
+      }
     }
     if (++rows_since_flush == kFlushRows) {
       rows_since_flush = 0;
-      sacc[threadIdx.x][0].x += join2(nS, nC);
-      sacc[threadIdx.x][1].x += join2(xS, xC);
-      nS = nC = xS = xC = zero2;
+      double2 d[ND][1];
+      fold(d);
+#pragma unroll
+      for (int n = 0; n < ND; ++n) sacc[threadIdx.x][n] = d[n][0];
+#pragma unroll
+      for (int v = 0; v < NV; ++v) dS[v] = dC[v] = zero2;
     }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   if (MEMBERS ? ntiles >= kFlushRows : any_flush(ntiles, kFlushRows)) {
-    double2 d[2][1];
-    d[0][0] = sacc[threadIdx.x][0];
-    d[0][0].x += join2(nS, nC);
-    d[1][0] = sacc[threadIdx.x][1];
-    d[1][0].x += join2(xS, xC);
-    block_dots<2, LPR, 1>(d, p, LPR, off);
-  } else {
-    const F3 f[2][1][1] = {{{pair_sum(nS, nC)}}, {{pair_sum(xS, xC)}}};
+    double2 d[ND][1];
+    fold(d);
+    block_dots<ND, LPR, 1>(d, p, LPR, off);
+  } else if constexpr (DOT == DOT_DOUBLING) {
+    const F3 f[2][1][1] = {{{pair_sum(dS[0], dC[0])}}, {{pair_sum(dS[1], dC[1])}}};
     block_dots_ff<2, LPR, 1, 1>(f, p, LPR, off);
+  } else {
+    F3 f[ND][1][2];
+#pragma unroll
+    for (int n = 0; n < ND; ++n) {
+      f[n][0][0] = pair_sum(dS[2 * n], dC[2 * n]);
+      f[n][0][1] = pair_diff(dS[2 * n + 1], dC[2 * n + 1]);
+    }
+    block_dots_ff<ND, LPR, 1, 2>(f, p, LPR, off);
   }
 }
 
 namespace {
-template <int LPR, bool MEMBERS = false>
+template <int LPR, int DOT, bool MEMBERS>
 KernelFn ffpk1_w(int max_row_nnz, bool from_hbm) {
   switch (max_row_nnz) {
-    case 5: return from_hbm ? k_step_ffpk1<LPR, 5, 4, MEMBERS> : k_step_ffpk1<LPR, 5, 3, MEMBERS>;
-    case 6: return k_step_ffpk1<LPR, 6, 3, MEMBERS>;
-    case 7: return k_step_ffpk1<LPR, 7, 3, MEMBERS>;
-    case 8: return k_step_ffpk1<LPR, 8, 3, MEMBERS>;
+    case 5:
+      return from_hbm ? k_step_ffpk1<LPR, 5, 4, DOT, MEMBERS> : k_step_ffpk1<LPR, 5, 3, DOT, MEMBERS>;
+    case 6: return k_step_ffpk1<LPR, 6, 3, DOT, MEMBERS>;
+    case 7: return k_step_ffpk1<LPR, 7, 3, DOT, MEMBERS>;
+    case 8: return k_step_ffpk1<LPR, 8, 3, DOT, MEMBERS>;
     default: return nullptr;
   }
 }
@@ -403,14 +462,14 @@ KernelFn ffpk1_w(int max_row_nnz, bool from_hbm) {
 // both slots within about 100 MB stay in L2 from step to step
 bool slots_from_hbm(int64_t NH, int ncols) { return NH * ncols * 32 > (int64_t)100 << 20; }
 
-template <bool MEMBERS>
+template <int DOT, bool MEMBERS>
 KernelFn ffpk1_lanes(int lanes, int max_row_nnz, bool from_hbm) {
   switch (lanes) {
-    case 2: return ffpk1_w<2, MEMBERS>(max_row_nnz, from_hbm);
-    case 4: return ffpk1_w<4, MEMBERS>(max_row_nnz, from_hbm);
-    case 8: return ffpk1_w<8, MEMBERS>(max_row_nnz, from_hbm);
-    case 16: return ffpk1_w<16, MEMBERS>(max_row_nnz, from_hbm);
-    default: return ffpk1_w<32, MEMBERS>(max_row_nnz, from_hbm);
+    case 2: return ffpk1_w<2, DOT, MEMBERS>(max_row_nnz, from_hbm);
+    case 4: return ffpk1_w<4, DOT, MEMBERS>(max_row_nnz, from_hbm);
+    case 8: return ffpk1_w<8, DOT, MEMBERS>(max_row_nnz, from_hbm);
+    case 16: return ffpk1_w<16, DOT, MEMBERS>(max_row_nnz, from_hbm);
+    default: return ffpk1_w<32, DOT, MEMBERS>(max_row_nnz, from_hbm);
   }
 }
 
@@ -440,22 +499,23 @@ PackedStep select_packed_members(int ncols, bool real, int max_row_nnz, int ell_
   PackedStep ps;
   if (!real || ell_w != 8 || max_row_nnz > 8 || ncols < 2 || ncols > 32) return ps;
   const int lanes = ffpk1_lanes_for(ncols);
-  ps.fn = ffpk1_lanes<true>(lanes, max_row_nnz, slots_from_hbm(NH, ncols));
+  ps.fn = ffpk1_lanes<DOT_DOUBLING, true>(lanes, max_row_nnz, slots_from_hbm(NH, ncols));
   ps.threads = kThreads;
   ps.rows_per_block = kThreads / lanes;
   ps.split = (ncols + lanes - 1) / lanes;
   return ps;
 }
 
-PackedStep select_packed_step(int ncols, bool real, int max_row_nnz, int ell_w, int64_t NH) {
+PackedStep select_packed_step(int ncols, int dot, bool real, int max_row_nnz, int ell_w,
+                              int64_t NH) {
   PackedStep ps;
-  if (!real || ell_w != 8 || max_row_nnz > 8 || ncols < 2 || ncols > kMaxCols) return ps;
+  if (dot == DOT_NONE || !real || ell_w != 8 || max_row_nnz > 8 || ncols < 2 || ncols > kMaxCols) return ps;
   const int lanes = ffpk1_lanes_for(ncols);
   ps.threads = kThreads;
   // 49..64 columns with rows of 6..8: two columns per lane (3D L = 100, 64
   // columns 732 us per step, k_step_ffpk1 829); rows of 5: one per lane (2D
   // L = 1024 708 against 702 us, L = 150 17.7 against 15.3)
-  if (ncols > 48 && ncols <= 64 && max_row_nnz > 5) {
+  if (dot == DOT_DOUBLING && ncols > 48 && ncols <= 64 && max_row_nnz > 5) {
     const bool full = ncols == 64;
     switch (max_row_nnz) {
       case 6: ps.fn = ffpk_w<6>(full); break;
@@ -466,7 +526,10 @@ PackedStep select_packed_step(int ncols, bool real, int max_row_nnz, int ell_w, 
     ps.rows_per_block = kThreads / 32;
     return ps;
   }
-  ps.fn = ffpk1_lanes<false>(lanes, max_row_nnz, slots_from_hbm(NH, ncols));
+  const bool hbm = slots_from_hbm(NH, ncols);
+  ps.fn = dot == DOT_DOUBLING ? ffpk1_lanes<DOT_DOUBLING, false>(lanes, max_row_nnz, hbm)
+          : dot == DOT_LR2    ? ffpk1_lanes<DOT_LR2, false>(lanes, max_row_nnz, hbm)
+                              : ffpk1_lanes<DOT_LR1, false>(lanes, max_row_nnz, hbm);
   ps.rows_per_block = kThreads / lanes;
   ps.split = (ncols + lanes - 1) / lanes;
   return ps;

@@ -2,6 +2,7 @@
 ragged last parts, and both sides of each rule that picks the width."""
 import numpy as np
 import pytest
+import scipy.sparse as sp
 
 from conftest import relerr
 import kpm_gb300 as kg
@@ -33,6 +34,26 @@ def test_doubling(lattice, NR, prec):
     bra = ko.random_phase_vectors(rng, H.shape[0], NR)
     got = kg.kpm_1d(H, 9, NR, psi_in_l=bra, psi_in_r=psi, avg_output=False, precision=prec)
     assert np.abs(got - ko.kpm_1d_lr(H, 9, bra, psi)).max() < TOL[prec]
+
+
+@pytest.mark.parametrize("W", [5, 6, 7, 8])
+@pytest.mark.parametrize("n,NR", [(25001, 2), (25001, 3), (25001, 5), (300001, 8)])
+def test_bra_ket_real_bands(W, n, NR):
+    """Bra-ket moments of real bands on packed pairs: ragged rows of up to W
+    entries, narrow columns, and lanes that fold their sums."""
+    rng = np.random.default_rng(W + NR)
+    H = sp.diags(rng.uniform(-1, 1, n)).tocsr()
+    for d in (1, 3, 4, 7)[:W // 2]:
+        v = rng.uniform(0.2, 1, n - d) * (rng.random(n - d) < 0.9)
+        H = H + sp.diags(v, d) + sp.diags(v, -d)
+    if W % 2 == 0:
+        H = H - sp.diags(H.diagonal())
+        H.eliminate_zeros()
+    H = (H / (1.02 * abs(H).sum(axis=1).max())).astype(complex).tocsc()
+    assert np.diff(H.indptr).max() == W
+    ket, bra = (ko.random_phase_vectors(rng, n, NR) for _ in range(2))
+    got = kg.kpm_1d(H, 9, NR, psi_in_l=bra, psi_in_r=ket, avg_output=False, precision="ff")
+    assert np.abs(got - ko.kpm_1d_lr(H, 9, bra, ket)).max() < TOL["ff"]
 
 
 @pytest.mark.parametrize("prec", ["ff", "fp64"])
