@@ -523,7 +523,13 @@ int run_kpm2d(Operator* H, Operator* Ja, Operator* Jb, int64_t NC, int64_t NR, i
     // both chains side by side: step n + 2 of the left one, step n + 1 of the
     // right one and right entry n read nothing that the others write, so one
     // launch takes all three (a third of the launches: conductivity of a
-    // 128 x 128 lattice, NC = 64, NR = 4, FP64, 191 launches of 4.5 us before)
+    // 128 x 128 lattice, NC = 64, NR = 4, FP64, 191 launches of 4.5 us before).
+    // Where their seven blocks do not stay in L2 together the left chain runs
+    // first, by itself: it then finds its own three there.
+    const bool together = 7 * (int64_t)block <= (int64_t)100 << 20;
+    if (!together)
+      for (int64_t n = 2; n < NC; ++n)
+        KPMGB_TRY(apply(&H->csr, L(n - 1), L(n - 2), L(n), 2.0, -1.0, colpair ? maxL + n : nullptr));
     KPMGB_TRY(zero_max(maxR, NC));
     for (int64_t n = 0; n < NC; ++n) {
       StepArgs t[3];
@@ -532,7 +538,7 @@ int run_kpm2d(Operator* H, Operator* Ja, Operator* Jb, int64_t NC, int64_t NR, i
       if (n + 1 < NC)
         t[nt++] = n == 0 ? step(&H->csr, right_vec(0), nullptr, right_vec(1), 1.0, 0.0)
                          : step(&H->csr, right_vec(n), right_vec(n - 1), right_vec(n + 1), 2.0, -1.0);
-      if (n + 2 < NC)
+      if (together && n + 2 < NC)
         t[nt++] = step(&H->csr, L(n + 1), L(n), L(n + 2), 2.0, -1.0,
                        colpair ? maxL + n + 2 : nullptr);
       KPMGB_TRY(launch_steps(t, nt, precision, s));

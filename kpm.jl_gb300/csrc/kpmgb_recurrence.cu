@@ -39,7 +39,9 @@ using namespace step;
 // --------------------------------------------------------------- dispatch
 // 9..12 columns: FP64 takes four lanes of three columns, which leaves none of
 // its scarce FP64 lanes idle (NH = 262144, 12 columns 106 us per step against
-// the 144 of 16 lanes); float-float takes 16 lanes (more rows in flight).
+// the 144 of 16 lanes), float-float too in steps without dots (kpm_2d of a
+// square 360x360, 64 moments, 12 columns 9.4 ms, 16 lanes 12.9); with dots it
+// takes 16 lanes (more rows in flight).
 // Lanes per row times columns per lane; a shape narrower than the launch runs
 // the columns in parts.  Idle lanes cost as much as live ones (FP64: the pipe
 // serves whole warps; float-float: the issue slots), so parts of 16 or 8 serve
@@ -48,12 +50,14 @@ using namespace step;
 // 681; 72 columns 8 x 9 786, 32 x 4 1373; square 512x512, 48 columns 16 x 3
 // 409, 8 x 6 413, 32 x 2 553; 150x150, 20 columns 24.1, 32 lanes 28.1.
 // Float-float bra moments, square 512x512, 72 columns 531 us, 32 x 4 lanes 705.
-Shape pick_shape(int ncols, int precision) {
+// Below 8192 rows, where parts leave few rows in flight, they have to save more
+// (3D L = 14, bra moments, 56 columns 8 x 7 19.4 us, 32 x 2 16.3).
+Shape pick_shape(int ncols, int precision, int dot, int64_t NH) {
   if (ncols <= 1) return {1, 1};
   if (ncols <= 2) return {2, 1};
   if (ncols <= 4) return {4, 1};
   if (ncols <= 8) return {8, 1};
-  if (ncols <= 12 && precision == KPMGB_PREC_FP64) return {4, 3};
+  if (ncols <= 12 && (precision == KPMGB_PREC_FP64 || dot == DOT_NONE)) return {4, 3};
   if (ncols <= 16) return {16, 1};
   Shape best = ncols <= 32 ? Shape{32, 1} : ncols <= 64 ? Shape{32, 2} : Shape{32, 4};
   int width = best.lpr * best.cpl;
@@ -62,7 +66,7 @@ Shape pick_shape(int ncols, int precision) {
   if (precision == KPMGB_PREC_FF && ncols <= 64) return best;
   for (int lanes : {32, 16, 8}) {
     const int held = (ncols + lanes - 1) / lanes * lanes;
-    if (held * 16 < width * 15) {
+    if (held * 16 < width * (NH < 8192 ? 13 : 15)) {
       best = {lanes, 1};
       width = held;
     }
@@ -72,10 +76,10 @@ Shape pick_shape(int ncols, int precision) {
 
 // Register-gather shapes that cover ncols columns with at most 4x idle lanes,
 // the automatic one first (candidates of the autotuner).
-std::vector<Shape> candidate_shapes(int ncols, int precision) {
+std::vector<Shape> candidate_shapes(int ncols, int precision, int dot, int64_t NH) {
   static const Shape all[] = {{1, 1}, {2, 1}, {4, 1}, {8, 1}, {4, 3},
                               {16, 1}, {32, 1}, {32, 2}, {32, 4}};
-  std::vector<Shape> out{pick_shape(ncols, precision)};
+  std::vector<Shape> out{pick_shape(ncols, precision, dot, NH)};
   for (const Shape& s : all) {
     const int cover = s.lpr * s.cpl;
     if (cover >= ncols && cover <= 4 * std::max(ncols, 8) &&
@@ -86,13 +90,11 @@ std::vector<Shape> candidate_shapes(int ncols, int precision) {
 }
 
 Shape shape_for(const StepArgs& a, int ncols, int precision) {
-  static const int forced = std::getenv("KPMGB_SHAPE") ? std::atoi(std::getenv("KPMGB_SHAPE")) : 0;
-  if (forced && a.shape == 0) return Shape{forced / 10, forced % 10};
   if (a.shape > 0) {
     const Shape s{a.shape / 10, a.shape % 10};
     if (s.lpr * s.cpl >= ncols) return s;
   }
-  return pick_shape(ncols, precision);
+  return pick_shape(ncols, precision, a.dot, a.NH);
 }
 
 KernelFn select_kernel(Shape s, int precision, int dot, bool real) {
@@ -165,7 +167,8 @@ struct StepChoice {
   int threads = kThreads;
   size_t smem = 0;
   int slots = 0;  // resident blocks where early launches depend on them, else 0
-  int split = 1;  // parts of the columns (steps that launch alone)
+  int split = 1;  // parts of the columns
+  int batch = kMaxBatch;  // steps without dots per launch
 };
 
 // Step kernels launch with programmatic stream serialization (see pdl_enter)
@@ -341,6 +344,7 @@ int choose_step(const StepArgs& a, int precision, int ncols, StepChoice* out) {
   const int width = sh.lpr * sh.cpl;
   out->fn = select_kernel(sh, precision, a.dot, real);
   out->split = (ncols + width - 1) / width;
+  if (precision == KPMGB_PREC_FF && sh.cpl > 2) out->batch = 1;
   out->grid = grid_for(out->fn, a.NH, sh.lpr, out->split);
   // The FP64 step of a complex operator is bound by each SM's FP64 pipe.  A
   // grid that leaves some of the resident slots free, but fewer than it needs,
@@ -500,7 +504,7 @@ int launch_steps(const StepArgs* steps, int n, int precision, cudaStream_t s) {
       const DeviceCSR& H = *a.H;
       StepChoice ci;
       KPMGB_TRY(choose_step(a, precision, ncols, &ci));
-      if (held > 0 && (ci.fn != c.fn || ci.grid != c.grid || held == kMaxBatch)) {
+      if (held > 0 && (ci.fn != c.fn || ci.grid != c.grid || held >= c.batch)) {
         KPMGB_TRY(launch_step_kernel(c, held, s, batch));
         held = 0;
       }
@@ -757,7 +761,7 @@ int tune_step(const StepArgs& a0, int precision, DevBuf& partials, cudaStream_t 
     int variant, shape;
   };
   std::vector<Cand> cands;
-  for (const Shape& c : candidate_shapes(a0.NR, precision)) cands.push_back({1, c.lpr * 10 + c.cpl});
+  for (const Shape& c : candidate_shapes(a0.NR, precision, a0.dot, a0.NH)) cands.push_back({1, c.lpr * 10 + c.cpl});
   if (precision == KPMGB_PREC_FF && a0.H->ell_w > 0 &&
       select_kernel_ffe(a0.NR, a0.dot, a0.H->is_real != 0))
     cands.push_back({9, 0});

@@ -127,6 +127,7 @@ struct PartCols {
 };
 template <int W>
 __device__ __forceinline__ PartCols part_columns(const KParams& p) {
+  if constexpr (W == 12) return {0, p.c0, p.ncols};  // {4, 3}: never in parts
   const int off = (int)(blockIdx.y % (unsigned)p.parts) * W;
   return {off, p.c0 + off, min(W, p.ncols - off)};
 }
@@ -571,9 +572,14 @@ __device__ __forceinline__ void ff_chunk_n(int cnt, const KParams& p,
 }
 
 template <int LPR, int CPL, bool REALH, int DOT, int CH>
-__global__ void __launch_bounds__(kThreads, (FFTune<CPL, REALH>::min_blocks)) k_step_ff(
+__global__ void __launch_bounds__(kThreads, (FFTune<CPL, REALH>::min_blocks +
+                                            (DOT == DOT_NONE && CPL == 1 && !REALH))) k_step_ff(
     const __grid_constant__ KBatch batch) {
-  const KParams& p = batch.p[DOT == DOT_NONE ? blockIdx.y / (unsigned)batch.p[0].parts : 0];
+  // three and four columns per lane launch alone: parameters of a step known
+  // at run time only cost them registers (square 360x360, 12 columns, kpm_2d
+  // 9.6 ms against 10.5)
+  const KParams& p =
+      batch.p[DOT == DOT_NONE && CPL < 3 ? blockIdx.y / (unsigned)batch.p[0].parts : 0];
   pdl_enter();
   const PartCols cols = part_columns<LPR * CPL>(p);
   constexpr int ND = NDots<DOT>::value;

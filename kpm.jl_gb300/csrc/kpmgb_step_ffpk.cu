@@ -1,6 +1,8 @@
 // Row-streaming float-float step on packed FP32 pairs (k_step_ffpk): real
 // operators with rows of 6..8, 49..64 columns (two per lane), doubling dots;
-// k_step_ffpk1 below serves the others of 2..128 columns (one per lane).
+// k_step_ffpk1 below serves the others of 2..128 columns (one per lane) and the
+// bra-ket dots (2D 512x512, 16 columns 131 us per step with the CSR kernel, 60
+// here; 40 columns 212 with k_step_ffr, 138).
 //
 // Blackwell executes `fma/add/sub/mul.rn.f32x2` on a 64-bit register pair:
 // one instruction for two correctly rounded FP32 operations.  For real H the
@@ -510,6 +512,9 @@ PackedStep select_packed_step(int ncols, int dot, bool real, int max_row_nnz, in
                               int64_t NH) {
   PackedStep ps;
   if (dot == DOT_NONE || !real || ell_w != 8 || max_row_nnz > 8 || ncols < 2 || ncols > kMaxCols) return ps;
+  // bra-ket steps of 57..64 columns with rows of 6..8: k_step_ffr (3D L = 100, 64
+  // columns 930 us per step, k_step_ffpk1 967; 56 columns 1013 and 937)
+  if (dot != DOT_DOUBLING && ncols > 56 && ncols <= 64 && max_row_nnz > 5) return ps;
   const int lanes = ffpk1_lanes_for(ncols);
   ps.threads = kThreads;
   // 49..64 columns with rows of 6..8: two columns per lane (3D L = 100, 64
