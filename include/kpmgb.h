@@ -57,7 +57,7 @@ extern "C" {
 #define KPMGB_PREC_FF 1
 
 /* kpm_2d contraction arithmetic (mu = R L^H over K = NH*NR). */
-#define KPMGB_CONTRACT_FP64 0  /* double-precision SIMT GEMM              */
+#define KPMGB_CONTRACT_FP64 0  /* double precision (digit planes, FP64)   */
 #define KPMGB_CONTRACT_SPLIT 1 /* BF16 slices on tcgen05, FP32 accumulate */
 
 /* moment_parity of kpm_2d (src/moment.jl:913-915, :1067-1069). */
@@ -363,7 +363,7 @@ int kpmgb_kpm1d_noalloc(int64_t NH, const int32_t* rowptr, const int32_t* col,
  * of that kernel and returns their summed device time and count.  Off by
  * default (nothing is recorded). */
 #define KPMGB_TIMED_CONTRACT_SPLIT 0 /* tcgen05 split contraction kernel    */
-#define KPMGB_TIMED_CONTRACT_FP64 1  /* FP64 SIMT contraction kernel        */
+#define KPMGB_TIMED_CONTRACT_FP64 1  /* FP64 contraction kernels            */
 int kpmgb_timing_enable(int32_t on);
 int kpmgb_timing_read(int32_t kernel, double* total_ms, int64_t* launches);
 
