@@ -231,11 +231,11 @@ def measured_bf16():
 
 
 # FP64 operations of the plain recurrence per row x column x step for a real
-# operator: 2 FMAs per nonzero (re, im), the update alpha*acc + beta*z (2 MUL +
-# 2 FMA) and the doubling dots <x|x> (2 FMA) and <x|y> (4 FMA); an FMA counts 2.
+# operator: 2 FMAs per nonzero (re, im), the update alpha*acc - z (2 FMA)
+# and the doubling dots <x|x> (2 FMA) and <x|y> (4 FMA); an FMA counts 2.
 def fp64_flop_per_row_col(nnz_per_row, real=True):
     per_nz = 4 if real else 8
-    return per_nz * nnz_per_row + 6 + 12
+    return per_nz * nnz_per_row + 4 + 12
 
 
 def cond_summary(args):
@@ -880,7 +880,7 @@ def main():
                      "peak_source": "measured in this run (kpmgb_measure_fp64_peak: independent "
                                     "FP64 FMA chains on every SM)",
                      "flop_per_launch": fl,
-                     "flop_model": "per row x column x step: 4 per nonzero (real H) + 6 "
+                     "flop_model": "per row x column x step: 4 per nonzero (real H) + 4 "
                                    "(update) + 12 (doubling dots)",
                      "hbm": {"achieved": plain_hbm, "peak": peak, "unit": "GB/s",
                              "frac": plain_hbm / peak}}}
