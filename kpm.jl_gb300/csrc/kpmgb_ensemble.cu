@@ -799,7 +799,19 @@ int launch_ensemble_steps(const DeviceCSR& H, const EnsembleArgs& e, EnsParams p
   KPMGB_CUDA(cudaMemsetAsync(q.ticket, 0, (size_t)nseg * sizeof(unsigned), s));
   void* fn = pick_ensemble_step(ff, H.is_real != 0, ell, p.NR, H.max_row_nnz);
   // programmatic dependent launch: step n+1's CTAs are scheduled while step n
-  // drains and wait (griddepcontrol.wait) for its completion
+  // drains and wait (griddepcontrol.wait) for its completion.  An FP64 grid that
+  // leaves resident slots free, but fewer than it needs, would crowd its
+  // successor onto the SMs that have them (120 members L = 24..70, 1 column, 48
+  // steps: 1.44 ms early, 1.34 one after another): not early then
+  bool early = true;
+  if (!ff) {
+    int dev = 0, sms = 0, per_sm = 0;
+    KPMGB_CUDA(cudaGetDevice(&dev));
+    KPMGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    KPMGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, shape.threads, 0));
+    const int64_t slots = (int64_t)per_sm * sms;
+    early = nb >= slots || 2 * nb <= slots;
+  }
   for (int64_t n = 1; n <= p.NC / 2; ++n) {
     q.n = (int)n;
     void* args[] = {&p, &q};
@@ -811,7 +823,7 @@ int launch_ensemble_steps(const DeviceCSR& H, const EnsembleArgs& e, EnsParams p
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = early ? 1 : 0;
     KPMGB_CUDA(cudaLaunchKernelExC(&cfg, fn, args));
     KPMGB_LAUNCHED();
   }
