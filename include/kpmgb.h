@@ -149,6 +149,9 @@ int kpmgb_operator_info(kpmgb_operator op, int64_t* n, int64_t* nnz,
 /* Equal-vector moments with the doubling identities: the entry point behind
  * kpm_1d!(H, NC, NR, NH, mu_all, psi_in) (src/moment.jl:420-492).  NC must be
  * even.  psi: host NH x NR column-major; mu_all: host NR x NC column-major.
+ * Odd moments of a Hermitian H are real; float-float calls with
+ * kernel_variant 0 compute their imaginary part where H is not Hermitian,
+ * those with variant 11 (or 4, where it picks that) and ensembles store 0.
  * Blocking call. */
 int kpmgb_kpm1d(kpmgb_operator H, int64_t NC, int64_t NR, int64_t NH,
                 const double* psi, double* mu_all,

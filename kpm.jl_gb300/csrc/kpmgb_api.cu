@@ -109,6 +109,37 @@ __global__ void k_split_values(const double2* __restrict__ v, int64_t nnz, int i
   }
 }
 
+// *differs set where H is not its own adjoint: the entries of (i, j) add up to
+// a value further than 2^-48 of it from the conjugate of those of (j, i).
+// One thread per row; rows sorted by column, at most 16 long.
+__global__ void __launch_bounds__(256) k_check_hermitian(const int* __restrict__ rowptr,
+                                                         const int* __restrict__ col,
+                                                         const double2* __restrict__ val, int n,
+                                                         unsigned* differs) {
+  const int64_t i = blockIdx.x * 256ll + threadIdx.x;
+  if (i >= n) return;
+  const int k1 = rowptr[i + 1];
+  for (int k = rowptr[i]; k < k1;) {
+    const int j = col[k];
+    double2 a = make_double2(0.0, 0.0), b = a;
+    for (; k < k1 && col[k] == j; ++k) {
+      a.x += val[k].x;
+      a.y += val[k].y;
+    }
+    for (int q = rowptr[j]; q < rowptr[j + 1]; ++q)
+      if (col[q] == (int)i) {
+        b.x += val[q].x;
+        b.y -= val[q].y;
+      }
+    const double size = fmax(fmax(fabs(a.x), fabs(a.y)), fmax(fabs(b.x), fabs(b.y)));
+    // not <= : a NaN differs
+    if (!(fmax(fabs(a.x - b.x), fabs(a.y - b.y)) <= 0x1p-48 * size)) {
+      *differs = 1u;
+      return;
+    }
+  }
+}
+
 __global__ void k_mul_scalar(const double* a, const double* b, double* out) { out[0] = a[0] * b[0]; }
 
 struct Guard {
@@ -211,14 +242,17 @@ int run_kpm1d(Operator* op, int64_t NC, int64_t NR, int64_t NH, const void* psi_
   // Float-float calls with 2..128 columns on real operators of 5..8
   // nonzeros in the longest row keep their vectors in the paired element layout
   // and run every step on packed FP32 pairs (k_step_ffpk / k_step_ffpk1;
-  // KPMGB_PAIRED=0 keeps the standard layout and k_step_ffr).
-  const bool paired = paired_on && ff && !auto_cluster &&
+  // KPMGB_PAIRED=0 keeps the standard layout and k_step_ffr).  The doubling
+  // steps of both layouts leave out Im<x|y>, which is 0 for a Hermitian H;
+  // other operators keep to the kernels that compute it.
+  const bool real_dots = lr || op->csr.hermitian || variant == 11;
+  const bool paired = paired_on && ff && !auto_cluster && real_dots &&
                       (variant == 0 || (variant == 11 && !lr && NR >= 9 && NR <= 64)) &&
                       packed_step_applies(op->csr, (int)NR, lr ? DOT_LR1 : DOT_DOUBLING);
   // Float-float calls with 2..128 columns on complex operators of at most 12
   // nonzeros per row keep them in the column-pair layout (k_step_ffcp;
   // KPMGB_COLPAIR=0 keeps the standard layout and k_step_ffc).
-  const bool colpair = colpair_on && ff && !auto_cluster && variant == 0 &&
+  const bool colpair = colpair_on && ff && !auto_cluster && variant == 0 && real_dots &&
                        colpair_step_applies(op->csr, (int)NR, lr ? DOT_LR1 : DOT_DOUBLING);
   const int layout = paired ? VEC_PAIRED : colpair ? VEC_COLPAIR : VEC_STD;
   KPMGB_TRY(launch_load_block(psi_r, sl[0], NH, (int)NR, precision, sc, false, s, layout));
@@ -686,6 +720,7 @@ int kpmgb_operator_create(int64_t n, int64_t nnz, const int64_t* colptr, const i
   c.max_row_nnz = hc.max_row_nnz;
   c.rmax = hc.rmax;
   const int is_real = hc.is_real;
+  unsigned differs = 0;
   const size_t nz = (size_t)std::max<int64_t>(nnz, 1);
   // one device block: the converted arrays (laid out as the host buffer, so
   // one copy uploads them), then the arrays built on the device
@@ -694,7 +729,9 @@ int kpmgb_operator_create(int64_t n, int64_t nnz, const int64_t* colptr, const i
   const size_t off_ff = off_real + (is_real ? csr_align256(nz * sizeof(double)) : 0);
   const size_t off_ecol = off_ff + csr_align256(nz * (is_real ? sizeof(float2) : sizeof(float4)));
   const size_t off_eval = off_ecol + csr_align256((size_t)n * W * sizeof(int));
-  const size_t total = off_eval + (size_t)n * W * (is_real ? sizeof(float2) : sizeof(float4));
+  const size_t off_flag =
+      csr_align256(off_eval + (size_t)n * W * (is_real ? sizeof(float2) : sizeof(float4)));
+  const size_t total = off_flag + sizeof(unsigned);
 #define CREATE_CUDA(call)                                                                   \
   do {                                                                                      \
     cudaError_t e_ = (call);                                                                \
@@ -726,10 +763,19 @@ int kpmgb_operator_create(int64_t n, int64_t nnz, const int64_t* colptr, const i
         CREATE_CUDA(cudaGetLastError());
       g_launches.fetch_add(1);
       c.ell_w = W;
+      unsigned* flag = reinterpret_cast<unsigned*>(base + off_flag);
+      CREATE_CUDA(cudaMemsetAsync(flag, 0, sizeof(unsigned), op->stream));
+      k_check_hermitian<<<(unsigned)((n + 255) / 256), 256, 0, op->stream>>>(c.rowptr, c.col, c.val,
+                                                                             (int)n, flag);
+      g_launches.fetch_add(1);
+      CREATE_CUDA(cudaGetLastError());
+      CREATE_CUDA(cudaMemcpyAsync(&differs, flag, sizeof(unsigned), cudaMemcpyDeviceToHost,
+                                  op->stream));
     }
   }
   // the host buffer is released on return: the copy must have completed
   CREATE_CUDA(cudaStreamSynchronize(op->stream));
+  c.hermitian = differs == 0;
 #undef CREATE_CUDA
   *out = reinterpret_cast<kpmgb_operator>(op);
   return KPMGB_OK;

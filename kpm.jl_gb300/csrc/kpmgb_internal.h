@@ -107,6 +107,9 @@ struct DeviceCSR {
   void* val_ff = nullptr;
   int is_real = 0;
   int max_row_nnz = 0;
+  // H = H^dagger to the 48 bits that float-float values hold (checked for rows
+  // of at most 16, the float-float kernels that rely on it)
+  int hermitian = 0;
   double rmax = 0.0;  // max over rows of sum_k (|Re H_rk| + |Im H_rk|)
   // float-float values in fixed-width padded rows (n x ell_w, ell_w = 0 when
   // rows are longer than 16): padding slots hold 0 and repeat a column of

@@ -318,7 +318,11 @@ int choose_step(const StepArgs& a, int precision, int ncols, StepChoice* out) {
   }
   if (a.variant == 11 && precision != KPMGB_PREC_FF)
     return fail(KPMGB_ERR_ARGUMENT, "the row-streaming kernel is float-float only");
-  if (precision == KPMGB_PREC_FF && (a.variant == 11 || a.variant == 0)) {
+  // the row-streaming kernels leave out Im<x|y> of the doubling dots (0 for a
+  // Hermitian H)
+  const bool streaming =
+      a.variant == 11 || (a.variant == 0 && (H.hermitian || a.dot != DOT_DOUBLING));
+  if (precision == KPMGB_PREC_FF && streaming) {
     if (KernelFn fr = select_kernel_ffr(ncols, a.dot, real, H.max_row_nnz, H.ell_w))
       return take(fr, 32);
     KernelFn fc = H.ell_w > 0 && (kStreamingComplex || a.variant == 11)
