@@ -8,12 +8,19 @@
 // (exact for entries within 2^-9 of the row maximum, within 2^-63 of it for
 // the rest), cut into eight balanced base-256 digits; the digit products of
 // i + j <= 7 add up exactly and the dropped ones stay below 2^-64 of the
-// product of the row maxima per term.  For vectors whose largest entry is
-// within a factor 32 of their root mean square the sum is nearer to the exact
-// one than FP64 FMAs, which round every partial sum.  Other vectors (probes
-// on single sites, rows that hold infinities or NaN) keep the FP64 kernel:
-// k_vec_gate compares the two figures of every vector on the device and sets
-// a word that each kernel of either form reads first.
+// product of the row maxima per term.  Entries below 2^-9 of their row's
+// maximum keep fewer bits than FP64, so the planes serve vectors in which such
+// entries cannot decide a sum; the others keep the FP64 kernel.  A vector
+// passes when its largest entry is within a factor 32 of its root mean square
+// and when, of its real parts and of its imaginary parts, 9 in 16 or more lie
+// within 2^-7 of that entry (or all are 0): any two such vectors share an
+// eighth of their sites with products of 2^-14 of the maxima's or more, whose
+// FP64 sum is rounded by more than the planes drop.  Random-phase probes and
+// what the recurrence makes of them pass (of a Gaussian vector nearly nine in
+// ten parts are that large); probes on single sites, wave packets, vectors
+// whose imaginary part is small throughout, infinities and NaN do not.
+// k_vec_gate decides on the device and sets a word that each kernel of either
+// form reads first.
 //
 // The planes of a K range are laid out, multiplied and added to the moments
 // before those of the next, so they take at most kPlaneBytes of scratch.
@@ -48,12 +55,17 @@ __device__ __forceinline__ unsigned long long abs_bits(double v) {
   return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
 }
 
-// Largest |component| of a chunk (bits of a double) and the chunk's sum of
-// squares in units of that component's power of two squared.
+// Largest |component| of a chunk (bits of a double), the chunk's sum of squares
+// in units of that component's power of two squared, and how many real parts
+// (low half of `large`) and imaginary parts reach 2^-5 of that power; kAnyRe,
+// kAnyIm: some are not 0.
 struct VecStat {
   unsigned long long peak;
   float sumsq;
+  unsigned large;
 };
+constexpr unsigned kAnyRe = 1u << 15, kAnyIm = 1u << 31;
+static_assert(kStatChunk < kAnyRe, "counts and flags share a half word");
 
 __device__ __forceinline__ int exponent_of(unsigned long long bits) { return (int)(bits >> 52); }
 
@@ -71,6 +83,7 @@ __global__ void __launch_bounds__(256) k_vec_stat(const void* vecs, int64_t K, i
                                                   VecStat* stat) {
   __shared__ unsigned long long rp[256];
   __shared__ float rs[256];
+  __shared__ unsigned rl[256];
   const int v = blockIdx.y, tid = threadIdx.x;
   const int64_t k0 = (int64_t)blockIdx.x * kStatChunk, k1 = min(K, k0 + kStatChunk);
   unsigned long long m = 0;
@@ -87,23 +100,33 @@ __global__ void __launch_bounds__(256) k_vec_stat(const void* vecs, int64_t K, i
   }
   const int ex = exponent_of(rp[0]);
   float s = 0.f;
+  unsigned large = 0;
+  bool re_any = false, im_any = false;
 #pragma unroll 4
   for (int64_t k = k0 + tid; k < k1; k += 256) {
     const double2 x = load_f64<FF>(vecs, (int64_t)v * K + k);
     const float re = relative(x.x, ex), im = relative(x.y, ex);
     s = fmaf(re, re, fmaf(im, im, s));
+    large += (re >= 0.03125f ? 1u : 0u) + (im >= 0.03125f ? 1u << 16 : 0u);
+    re_any |= abs_bits(x.x) != 0;
+    im_any |= abs_bits(x.y) != 0;
   }
   rs[tid] = s;
-  __syncthreads();
+  rl[tid] = large;
+  const unsigned any =
+      (__syncthreads_or(re_any) ? kAnyRe : 0u) | (__syncthreads_or(im_any) ? kAnyIm : 0u);
   for (int w = 128; w > 0; w >>= 1) {
-    if (tid < w) rs[tid] += rs[tid + w];
+    if (tid < w) {
+      rs[tid] += rs[tid + w];
+      rl[tid] += rl[tid + w];
+    }
     __syncthreads();
   }
-  if (tid == 0) stat[(size_t)v * chunks + blockIdx.x] = VecStat{rp[0], rs[0]};
+  if (tid == 0) stat[(size_t)v * chunks + blockIdx.x] = VecStat{rp[0], rs[0], rl[0] | any};
 }
 
 // exps[v]: max |component| < 2^e (0 for a zero vector); *fp64 set when a
-// vector is not finite or too peaked
+// vector is not finite, too peaked or too unevenly spread
 __global__ void __launch_bounds__(32) k_vec_gate(const VecStat* stat, int chunks, int64_t K,
                                                  int* exps, unsigned* fp64) {
   const int v = blockIdx.x, lane = threadIdx.x;
@@ -113,16 +136,32 @@ __global__ void __launch_bounds__(32) k_vec_gate(const VecStat* stat, int chunks
   for (int off = 16; off > 0; off >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, off));
   const int ex = exponent_of(m);
   float s = 0.f;
+  // parts of 2^-6 of the vector's power or more: those of the chunks whose own
+  // power is at most one less (chunks of 8192 Gaussian entries all are)
+  long long re = 0, im = 0;
+  unsigned any = 0;
   for (int c = lane; c < chunks; c += 32) {
     const VecStat t = stat[(size_t)v * chunks + c];
     s += ldexpf(t.sumsq, 2 * max(exponent_of(t.peak) - ex, -80));
+    any |= t.large & (kAnyRe | kAnyIm);
+    if (exponent_of(t.peak) >= ex - 1) {
+      re += t.large & (kAnyRe - 1);
+      im += (t.large >> 16) & (kAnyRe - 1);
+    }
   }
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+  for (int off = 16; off > 0; off >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, off);
+    re += __shfl_xor_sync(0xffffffffu, re, off);
+    im += __shfl_xor_sync(0xffffffffu, im, off);
+    any |= __shfl_xor_sync(0xffffffffu, any, off);
+  }
   if (lane == 0) {
     exps[v] = m == 0 ? 0 : max(ex, 1) - 1022;
     const float mx = relative(__longlong_as_double((long long)m), ex);
-    if (m != 0 && (ex == 0x7ff || !(mx * mx * 2.f * (float)K <= kPeak * s))) atomicOr(fp64, 1u);
+    const bool peaked = !(mx * mx * 2.f * (float)K <= kPeak * s);
+    const bool uneven = ((any & kAnyRe) && 16 * re < 9 * K) || ((any & kAnyIm) && 16 * im < 9 * K);
+    if (m != 0 && (ex == 0x7ff || peaked || uneven)) atomicOr(fp64, 1u);
   }
 }
 
