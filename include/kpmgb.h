@@ -116,7 +116,10 @@ typedef struct kpmgb_kpm1d_options {
 typedef struct kpmgb_kpm2d_options {
   int64_t arr_size;        /* K_left; 0 = automatic (src/moment.jl:759-810)   */
   int64_t right_block;     /* K_right; 0 = automatic                          */
-  int64_t workspace_bytes; /* device budget; < 0 = half of free memory        */
+  int64_t workspace_bytes; /* device budget of the blocks and, for the double-
+                              precision contraction, its scratch beyond a few
+                              MB; < 0 = half of free memory; bounds nothing
+                              when both block sizes are explicit             */
   int32_t moment_parity;   /* KPMGB_PARITY_*                                  */
   int32_t mn_sym;          /* 1: symmetrise as src/moment.jl:1078-1086        */
   int32_t precision;       /* recurrence arithmetic, KPMGB_PREC_*             */

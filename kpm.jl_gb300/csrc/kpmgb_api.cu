@@ -22,6 +22,7 @@
 #include <string>
 #include <vector>
 
+#include "kpmgb_contract_plan.h"
 #include "kpmgb_csr_host.h"
 #include "kpmgb_ffmath.cuh"
 #include "kpmgb_internal.h"
@@ -409,9 +410,6 @@ int run_kpm2d(Operator* H, Operator* Ja, Operator* Jb, int64_t NC, int64_t NR, i
   const size_t block = (size_t)NH * NR * 16;
   const int64_t K = NH * NR;
 
-  // Block sizes: explicit values are honoured (results are blocking
-  // invariant); otherwise keep both chains resident when the budget allows
-  // (src/moment.jl:759-810 for the reference's rule).
   size_t budget;
   if (opt.workspace_bytes >= 0) {
     budget = (size_t)opt.workspace_bytes;
@@ -423,29 +421,13 @@ int run_kpm2d(Operator* H, Operator* Ja, Operator* Jb, int64_t NC, int64_t NR, i
     const size_t held = ws.left.bytes + ws.right.bytes + ws.ring.bytes + ws.gemm.bytes;
     budget = (fr + held) / 2;
   }
-  int64_t KR = opt.right_block > 0 ? opt.right_block : 0;
-  int64_t KL = opt.arr_size > 0 ? opt.arr_size : 0;
-  if (KL == 0 || KR == 0) {
-    const int64_t kr_auto = KR ? KR : NC;
-    const size_t full = (size_t)(NC + kr_auto + 4) * block +
-                        contract_scratch_bytes(K, (int)std::min<int64_t>(kr_auto, NC), (int)NC,
-                                               precision, opt.contraction);
-    if (full <= budget) {
-      if (!KR) KR = NC;
-      if (!KL) KL = NC;
-    } else {
-      if (!KR) KR = std::min<int64_t>(NC, 16);
-      if (!KL) {
-        const int64_t base = (KR + 7) * (int64_t)block;
-        const int64_t per_left = (int64_t)block + KR * 16;
-        const int64_t kl = ((int64_t)budget - base) / per_left;
-        if (kl < 2)
-          return fail(KPMGB_ERR_ARGUMENT,
-                      "workspace_bytes=%zu cannot fit the minimum kpm_2d workspace", budget);
-        KL = std::min<int64_t>(kl, NC);
-      }
-    }
-  }
+  const bool split = opt.contraction == KPMGB_CONTRACT_SPLIT;
+  Kpm2dBlocks plan =
+      kpm2d_blocks(K, NC, opt.arr_size, opt.right_block, budget, split, contract_sms());
+  const int64_t KL = plan.KL, KR = plan.KR;
+  if (KL == 0)
+    return fail(KPMGB_ERR_ARGUMENT, "workspace_bytes=%zu cannot fit the minimum kpm_2d workspace",
+                budget);
   const int64_t KLa = std::min<int64_t>(KL, NC), KRa = std::min<int64_t>(KR, NC);
   KPMGB_TRY(ws.left.ensure(KLa * block));
   KPMGB_TRY(ws.right.ensure(KRa * block));
@@ -453,8 +435,14 @@ int run_kpm2d(Operator* H, Operator* Ja, Operator* Jb, int64_t NC, int64_t NR, i
   // scales, then the per-vector maxima of the L and R blocks (column pairs)
   const size_t scale_bytes = (size_t)(2 * NR + 8) * sizeof(double);
   KPMGB_TRY(ws.scales.ensure(scale_bytes + (size_t)(KLa + KRa) * sizeof(unsigned)));
-  const size_t cs = contract_scratch_bytes(K, (int)KRa, (int)KLa, precision, opt.contraction);
-  KPMGB_TRY(ws.gemm.ensure(cs));
+  if (const int rc = ws.gemm.ensure(plan.scratch)) {
+    if (plan.range == 0) return rc;
+    // no memory for the digit planes: the FP64 kernel needs a few MB
+    clear_error();
+    plan.range = 0;
+    KPMGB_TRY(ws.gemm.ensure(
+        contract_scratch_bytes(K, (int)KRa, (int)KLa, split, 0, contract_sms())));
+  }
   KPMGB_TRY(ensure_sync(H, s));
   KPMGB_CUDA(cudaMemsetAsync(mu, 0, (size_t)NC * NC * sizeof(double2), s));
 
@@ -613,6 +601,7 @@ int run_kpm2d(Operator* H, Operator* Ja, Operator* Jb, int64_t NC, int64_t NR, i
       c.status = ws.sync.as<unsigned>() + 1;
       c.scratch = ws.gemm.ptr;
       c.scratch_bytes = ws.gemm.bytes;
+      c.range = plan.range;
       c.reuse_l = n1 > 0;  // same left block as the previous contraction of this rep
       c.colpair = colpair;
       c.maxR = colpair ? (right_resident ? maxR + n1 : maxR) : nullptr;

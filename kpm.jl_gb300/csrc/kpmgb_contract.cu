@@ -18,18 +18,17 @@
 
 #include <algorithm>
 
+#include "kpmgb_contract_plan.h"
 #include "kpmgb_internal.h"
 
 namespace kpmgb {
 
 int launch_contract_split(const ContractArgs& a, int precision, cudaStream_t s);
-size_t contract_split_scratch_bytes(int64_t K, int nr, int nl);
-size_t contract_planes8_bytes(int64_t K, int nr, int nl);
 int launch_contract_planes8(const ContractArgs& a, int precision, cudaStream_t s);
 
 namespace {
 
-constexpr int TM = 32, TN = 32, KC = 16;
+constexpr int TM = kSimtTile, TN = kSimtTile, KC = 16;
 
 template <bool FF>
 __device__ __forceinline__ double2 load_elem(const void* base, int64_t idx) {
@@ -141,7 +140,9 @@ __global__ void k_mn_sym(double2* mu, int NC) {
   }
 }
 
-int num_sms_c() {
+}  // namespace
+
+int contract_sms() {
   static int sms = [] {
     int dev = 0, n = 0;
     cudaGetDevice(&dev);
@@ -151,31 +152,10 @@ int num_sms_c() {
   return sms;
 }
 
-int slices_for(int64_t K, int nr, int nl) {
-  const int64_t tiles = (int64_t)((nr + TM - 1) / TM) * ((nl + TN - 1) / TN);
-  const int64_t want = (4LL * num_sms_c() + tiles - 1) / tiles;
-  const int64_t maxs = std::max<int64_t>(1, K / 1024);
-  return (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(want, maxs), 64));
-}
-
-}  // namespace
-
-size_t contract_scratch_bytes(int64_t K, int nr, int nl, int precision, int contraction) {
-  (void)precision;
-  if (contraction == KPMGB_CONTRACT_SPLIT) return contract_split_scratch_bytes(K, nr, nl);
-  // Bound over every sub-block nr' <= nr, nl' <= nl that a launch may use:
-  // slices * nr' * nl' <= (4 * SMs / tiles' + 1) * tiles' * TM * TN.
-  const size_t tiles = (size_t)((nr + TM - 1) / TM) * ((nl + TN - 1) / TN);
-  const size_t bound = (4 * (size_t)num_sms_c() + tiles) * TM * TN;
-  const size_t simt =
-      std::max(bound, (size_t)slices_for(K, nr, nl) * nr * nl) * sizeof(double2) + kContractGateBytes;
-  return std::max(simt, contract_planes8_bytes(K, nr, nl));
-}
-
 int launch_contract(const ContractArgs& a, int precision, int contraction, cudaStream_t s) {
   if (a.nr <= 0 || a.nl <= 0) return KPMGB_OK;
   if (contraction == KPMGB_CONTRACT_SPLIT) return launch_contract_split(a, precision, s);
-  const int S = slices_for(a.K, a.nr, a.nl);
+  const int S = simt_slices(a.K, a.nr, a.nl, contract_sms());
   const size_t bytes = (size_t)S * a.nr * a.nl * sizeof(double2) + kContractGateBytes;
   if (bytes > a.scratch_bytes) return fail(KPMGB_ERR_ALLOC, "contraction scratch too small");
   int64_t kslice = (a.K + S - 1) / S;
@@ -187,7 +167,7 @@ int launch_contract(const ContractArgs& a, int precision, int contraction, cudaS
   // The digit planes are the faster form at every size (K = 1024, NC = 8: 0.15
   // against 1.12 ms per kpm_2d call; K = 65536, NC = 128: 1.9 against 7.9 ms).
   const unsigned* need = nullptr;  // device word: the FP64 kernels below have to run
-  if (contract_planes8_bytes(a.K, a.nr, a.nl) <= a.scratch_bytes) {
+  if (a.range > 0) {
     need = reinterpret_cast<const unsigned*>(scratch);
     KPMGB_TRY(launch_contract_planes8(a, precision, s));
   }

@@ -384,20 +384,10 @@ int launch_vec_absmax(const void* vecs, int64_t K, int nvec, unsigned* out, cuda
   return KPMGB_OK;
 }
 
-size_t contract_split_scratch_bytes(int64_t K, int nr, int nl) {
-  // the largest plan over sub-blocks nr' <= nr, nl' <= nl is the full block's
-  // (plane sizes grow with nr, nl; partials within part_bound_bytes)
-  const TcPlan pl = plan_for<Planes5>(K, nr, nl);
-  const size_t part_bound = part_bound_bytes<Planes5>(pl);
-  return pl.a_bytes + pl.b_bytes + 2 * pl.exp_bytes + std::max(pl.part_bytes, part_bound) + 1024;
-}
-
 int launch_contract_split(const ContractArgs& a, int precision, cudaStream_t s) {
-  const TcPlan pl = plan_for<Planes5>(a.K, a.nr, a.nl);
-  const size_t part_bound = part_bound_bytes<Planes5>(pl);
-  const size_t need = pl.a_bytes + pl.b_bytes + 2 * pl.exp_bytes +
-                      std::max(pl.part_bytes, part_bound) + 1024;
-  if (need > a.scratch_bytes) return fail(KPMGB_ERR_ALLOC, "split contraction scratch too small");
+  const TcPlan pl = plan_for<Planes5>(a.K, a.nr, a.nl, contract_sms());
+  if (split_scratch_bytes(a.K, a.nr, a.nl, contract_sms()) > a.scratch_bytes)
+    return fail(KPMGB_ERR_ALLOC, "split contraction scratch too small");
   if (!a.status) return fail(KPMGB_ERR_ARGUMENT, "split contraction needs a status word");
   // Layout: the L (B) planes and exponents first, at offsets that depend only
   // on (K, nl), so a caller contracting several right blocks against the same

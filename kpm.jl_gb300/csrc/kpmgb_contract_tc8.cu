@@ -23,7 +23,8 @@
 // form reads first.
 //
 // The planes of a K range are laid out, multiplied and added to the moments
-// before those of the next, so they take at most kPlaneBytes of scratch.
+// before those of the next, in scratch that the call's budget bounds
+// (contract_range, kpmgb_contract_plan.h).
 #include <mutex>
 #include <type_traits>
 
@@ -35,11 +36,8 @@ namespace {
 
 using C8 = Planes8;
 constexpr int S8 = C8::kSlices;
-constexpr size_t kPlaneBytes = size_t(2) << 30;
 // largest entry squared against the mean square: beyond 32^2 the FP64 kernel
 constexpr float kPeak = 1024.f;
-constexpr size_t kGateBytes = kContractGateBytes;
-constexpr int kStatChunk = 8192;  // complex elements per block of the statistics
 
 template <bool FF>
 __device__ __forceinline__ double2 load_f64(const void* base, int64_t idx) {
@@ -66,6 +64,7 @@ struct VecStat {
 };
 constexpr unsigned kAnyRe = 1u << 15, kAnyIm = 1u << 31;
 static_assert(kStatChunk < kAnyRe, "counts and flags share a half word");
+static_assert(sizeof(VecStat) == kVecStatBytes, "size of the statistics in the scratch");
 
 __device__ __forceinline__ int exponent_of(unsigned long long bits) { return (int)(bits >> 52); }
 
@@ -270,47 +269,6 @@ __global__ void __launch_bounds__(256) k_slice_f64(const void* vecs, int64_t K, 
   }
 }
 
-size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
-
-// Complex elements per K range: the planes of nr + 2 nl rows within the size
-// of the vectors themselves, but at least 64 MiB and at most kPlaneBytes, in
-// whole exact chunks.
-int64_t range_for(int64_t K, int nr, int nl) {
-  const size_t most = std::min<size_t>(
-      kPlaneBytes, std::max<size_t>((size_t)64 << 20, (size_t)K * (nr + nl) * 16));
-  const size_t rows = (size_t)((nr + TC_M - 1) / TC_M * TC_M) +
-                      (size_t)((2 * nl + C8::kN - 1) / C8::kN * C8::kN);
-  const int64_t chunk = C8::kChunk * C8::KT / 2;  // complex elements
-  const int64_t fit = (int64_t)(most / (rows * S8 * 2 * 2)) / chunk * chunk;
-  const int64_t range = std::max<int64_t>(fit, 64 * chunk);
-  // equal ranges: the tiles of a short last one would leave SMs idle
-  const int64_t n = (K + range - 1) / range;
-  return std::min(K, ((K + n - 1) / n + chunk - 1) / chunk * chunk);
-}
-
-struct Layout8 {
-  TcPlan pl;
-  int64_t range;
-  int chunks;  // statistics blocks per vector
-  size_t b, a, expB, expA, stat, gate, part, bytes;
-};
-
-Layout8 layout_for(int64_t K, int nr, int nl) {
-  Layout8 l;
-  l.range = range_for(K, nr, nl);
-  l.pl = plan_for<C8>(l.range, nr, nl);
-  l.chunks = (int)((K + kStatChunk - 1) / kStatChunk);
-  l.gate = 0;
-  l.b = kGateBytes;
-  l.expB = l.b + align256(l.pl.b_bytes);
-  l.a = l.expB + align256((size_t)nl * sizeof(int));
-  l.expA = l.a + align256(l.pl.a_bytes);
-  l.stat = l.expA + align256((size_t)nr * sizeof(int));
-  l.part = l.stat + align256((size_t)(nr + nl) * l.chunks * sizeof(VecStat));
-  l.bytes = l.part + std::max(l.pl.part_bytes, part_bound_bytes<C8>(l.pl));
-  return l;
-}
-
 template <bool FF>
 int launch_planes(const ContractArgs& a, const Layout8& l, uint8_t* base, cudaStream_t s) {
   const TcPlan& pl = l.pl;
@@ -379,12 +337,12 @@ int launch_planes(const ContractArgs& a, const Layout8& l, uint8_t* base, cudaSt
 
 }  // namespace
 
-size_t contract_planes8_bytes(int64_t K, int nr, int nl) { return layout_for(K, nr, nl).bytes; }
-
 // The gate word (nonzero: the FP64 kernel has to run) is the first of scratch.
 int launch_contract_planes8(const ContractArgs& a, int precision, cudaStream_t s) {
   if (!a.status) return fail(KPMGB_ERR_ARGUMENT, "the contraction needs a status word");
-  const Layout8 l = layout_for(a.K, a.nr, a.nl);
+  const Layout8 l = layout8(a.K, a.nr, a.nl, a.range, contract_sms());
+  if (l.bytes > a.scratch_bytes)
+    return fail(KPMGB_ERR_ALLOC, "scratch too small for the contraction's digit planes");
   uint8_t* base = static_cast<uint8_t*>(a.scratch);
   return precision == KPMGB_PREC_FF ? launch_planes<true>(a, l, base, s)
                                     : launch_planes<false>(a, l, base, s);

@@ -305,6 +305,8 @@ struct ContractArgs {
   unsigned* status = nullptr;  // device status word (bounded-wait expiry)
   void* scratch = nullptr;
   size_t scratch_bytes = 0;
+  int64_t range = 0;      // double precision: K range of the digit planes, the
+                          // same for every block of a call (0: FP64 kernel)
   bool reuse_l = false;   // L (and scratch) unchanged since the previous call:
                           // the split form keeps its L digit planes
   bool colpair = false;   // float-float R and L in the column-pair layout (the
@@ -320,10 +322,7 @@ struct ContractArgs {
 int launch_vec_absmax(const void* vecs, int64_t K, int nvec, unsigned* out, cudaStream_t s);
 int launch_contract(const ContractArgs& a, int precision, int contraction,
                     cudaStream_t s);
-size_t contract_scratch_bytes(int64_t K, int nr, int nl, int precision, int contraction);
-// The double-precision contraction's device word at the start of its scratch
-// (nonzero: its vectors need the FP64 kernel), padded to the planes' alignment.
-constexpr size_t kContractGateBytes = 1024;
+int contract_sms();  // SM count that the contraction's plans are made for
 int launch_mn_sym(double2* mu, int NC, cudaStream_t s);
 
 // Cluster-resident recurrence (kpmgb_cluster.cu): one thread-block cluster

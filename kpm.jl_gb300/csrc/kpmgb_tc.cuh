@@ -1,7 +1,8 @@
-// The digit-plane contraction on the tensor cores (tcgen05): tile shapes,
-// PTX helpers, the GEMM kernel and its K splits, shared by the five-digit
-// split form (kpmgb_contract_tc.cu, where the scheme is described) and the
-// eight-digit double-precision form (kpmgb_contract_tc8.cu).
+// The digit-plane contraction on the tensor cores (tcgen05): PTX helpers and
+// the GEMM kernel, shared by the five-digit split form (kpmgb_contract_tc.cu,
+// where the scheme is described) and the eight-digit double-precision form
+// (kpmgb_contract_tc8.cu).  Tile shapes, K splits and scratch sizes:
+// kpmgb_contract_plan.h.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -10,46 +11,17 @@
 #include <algorithm>
 #include <cmath>
 
+#include "kpmgb_contract_plan.h"
 #include "kpmgb_internal.h"
 
 namespace kpmgb {
 
 namespace {
 
-constexpr int TC_M = 128;      // A rows per tile
 constexpr int TMEM_COLS = 512;  // 2 buffers of 256 columns
 constexpr int TMEM_BUF = 256;
 constexpr int kSpin = 1 << 22;
 constexpr int kThreadsTC = 192;  // 6 warps
-
-// Digit planes S per operand, B rows N per tile, K' elements KT per k-tile (a
-// pipeline stage), k-tiles CHUNK per exact chunk, STAGES in shared memory.
-template <int S, int N, int KT_, int CHUNK_, int STAGES_, int64_t MAXK>
-struct PlaneCfg {
-  static constexpr int kSlices = S;
-  static constexpr int kN = N;
-  static constexpr int KT = KT_;
-  static constexpr int kChunk = CHUNK_;
-  static constexpr int kStages = STAGES_;
-  static constexpr uint32_t kATile = TC_M * KT * 2;  // one plane
-  static constexpr uint32_t kBTile = N * KT * 2;
-  static constexpr uint32_t kAStage = kATile * S;
-  static constexpr uint32_t kBStage = kBTile * S;
-  static constexpr uint32_t kStage = kAStage + kBStage;
-  static constexpr int64_t kMaxKt = MAXK / KT;  // k-tiles per split: int64 headroom
-  static constexpr int kAcc = S <= 5 ? 1 : 2;    // int64 accumulators per output
-  // a row's entries are integers of scale 2^(kBits - e): |N| <= 2^kBits
-  static constexpr int kBits = S == 5 ? 39 : 62;
-  // value of plane 0's unit: 2^(e - kLead)
-  static constexpr int kLead = kBits - 8 * (S - 1);
-  static_assert(N * S <= 256 && (N * S) % 16 == 0 && N % 16 == 0,
-                "one MMA covers up to S B planes");
-  static_assert(KT % 16 == 0, "K steps of 16");
-};
-// Five digits (the split contraction): 40 KiB + 15 KiB per stage.
-using Planes5 = PlaneCfg<5, 48, 32, 8, 4, (int64_t)1 << 24>;
-// Eight digits (the double-precision contraction): 32 KiB + 8 KiB per stage.
-using Planes8 = PlaneCfg<8, 32, 16, 8, 5, (int64_t)1 << 20>;
 
 // --------------------------------------------------------------- PTX helpers
 __device__ __forceinline__ uint32_t saddr(const void* p) {
@@ -363,70 +335,6 @@ k_tc_reduce(const double* __restrict__ part, int nsplit, int nr, int nl, int n0,
     }
     __syncthreads();
   }
-}
-
-inline int sm_count() {
-  static int n = [] {
-    int dev = 0, v = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    return v > 0 ? v : 1;
-  }();
-  return n;
-}
-
-struct TcPlan {
-  int mtiles, ntiles, nsplit;
-  int64_t ktiles, kt_per_split;
-  size_t a_bytes, b_bytes, exp_bytes, part_bytes;
-};
-
-template <class C>
-TcPlan plan_for(int64_t K, int nr, int nl) {
-  TcPlan pl;
-  pl.mtiles = (nr + TC_M - 1) / TC_M;
-  pl.ntiles = (2 * nl + C::kN - 1) / C::kN;
-  pl.ktiles = (2 * K + C::KT - 1) / C::KT;
-  const int64_t tiles = (int64_t)pl.mtiles * pl.ntiles;
-  const int64_t S = sm_count();  // one CTA per SM (shared memory)
-  const int64_t kmax = std::max<int64_t>(1, pl.ktiles / (4 * C::kChunk));
-  int64_t want = std::max<int64_t>(1, (2 * S + tiles - 1) / tiles);
-  want = std::min<int64_t>(want, kmax);
-  // K splits: the count in [want, 4 want] (at most 8 S + tiles CTAs) whose
-  // grid fills its last wave best, i.e. the least waves per unit of work
-  // ceil(n tiles / S) / n; e.g. 64 tiles on 152 SMs: 19 splits (8 full
-  // waves) instead of 5 (2.1 waves run as 3)
-  int64_t best = want;
-  double best_cost = 1e300;
-  for (int64_t n = want; n <= std::min<int64_t>(4 * want, kmax); ++n) {
-    if (n * tiles > 8 * S + tiles) break;
-    const double cost = (double)((n * tiles + S - 1) / S) / (double)n;
-    if (cost < best_cost * (1.0 - 1e-9)) {
-      best_cost = cost;
-      best = n;
-    }
-  }
-  want = std::max(best, (pl.ktiles + C::kMaxKt - 1) / C::kMaxKt);
-  pl.kt_per_split = (pl.ktiles + want - 1) / want;
-  pl.kt_per_split = (pl.kt_per_split + C::kChunk - 1) / C::kChunk * C::kChunk;
-  pl.kt_per_split = std::min(pl.kt_per_split, C::kMaxKt);
-  pl.nsplit = (int)((pl.ktiles + pl.kt_per_split - 1) / pl.kt_per_split);
-  pl.a_bytes = (size_t)pl.mtiles * pl.ktiles * C::kAStage;
-  pl.b_bytes = (size_t)pl.ntiles * pl.ktiles * C::kBStage;
-  pl.exp_bytes = ((size_t)(nr + nl) * sizeof(int) + 255) & ~size_t(255);
-  pl.part_bytes = (size_t)pl.nsplit * nr * 2 * nl * sizeof(double);
-  return pl;
-}
-
-// Partials of a plan, bounded over its sub-blocks: the split count times the
-// tiles stays within 8*SMs + tiles, or the minimum split count that keeps a
-// split within C::kMaxKt k-tiles times the tiles.
-template <class C>
-size_t part_bound_bytes(const TcPlan& pl) {
-  const int64_t tiles = (int64_t)pl.mtiles * pl.ntiles;
-  const int64_t nmin = (pl.ktiles + C::kMaxKt - 1) / C::kMaxKt;
-  return (size_t)std::max<int64_t>(8 * sm_count() + tiles, nmin * tiles) * TC_M * C::kN *
-         sizeof(double);
 }
 
 }  // namespace
