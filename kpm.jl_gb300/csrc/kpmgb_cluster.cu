@@ -374,7 +374,10 @@ namespace {
 
 // Clusters of 1..16 CTAs that the device holds side by side with one CTA per
 // SM (clusters lie within one of its processing clusters, so 16 CTAs fit far
-// fewer times than SMs / 16).
+// fewer times than SMs / 16).  The first call on a device also allows every
+// form of the kernel the most shared memory and the largest clusters, for good:
+// the limits belong to the process, and a limit of one call's size would fail
+// a larger launch of another thread that had just set its own.
 const int* clusters_side_by_side() {
   static std::mutex mtx;
   static std::map<int, std::array<int, kMaxCluster + 1>> table;
@@ -386,8 +389,17 @@ const int* clusters_side_by_side() {
   std::array<int, kMaxCluster + 1> side{};
   const void* fn = cluster_fn<false, true>(true);
   constexpr int kOnePerSm = 120 * 1024;  // more than half of an SM's shared memory
-  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kOnePerSm);
-  cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  int optin = 0;
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  for (const bool cache : {false, true})
+    for (const void* f : {cluster_fn<false, false>(cache), cluster_fn<false, true>(cache),
+                          cluster_fn<true, false>(cache), cluster_fn<true, true>(cache)}) {
+      cudaFuncAttributes fa{};
+      cudaFuncGetAttributes(&fa, f);
+      cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           optin - (int)fa.sharedSizeBytes);
+      cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    }
   for (int cs = 1; cs <= kMaxCluster; ++cs) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)cs);
@@ -523,9 +535,6 @@ int launch_kpm1d_cluster(const DeviceCSR& H, int64_t NH, int NR, int64_t NC, boo
     return fail(KPMGB_ERR_ARGUMENT, "the cluster-resident kernel cannot run here: %s",
                 cudaGetErrorString(e));
   };
-  KPMGB_TRY(setup(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)));
-  if (cs > 8)
-    KPMGB_TRY(setup(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(NR * cs));
   cfg.blockDim = dim3((unsigned)threads);
