@@ -65,6 +65,14 @@ int DevBuf::ensure(size_t need) {
   return dev_alloc(need, &ptr, &bytes);
 }
 
+int DevBuf::ensure_some(size_t want, size_t least, size_t* got) {
+  *got = want;
+  if (ensure(want) == KPMGB_OK) return KPMGB_OK;
+  clear_error();
+  *got = least;
+  return ensure(least);
+}
+
 void DevBuf::release(bool device_idle) {
   dev_release(ptr, bytes, device_idle);
   ptr = nullptr;
@@ -216,15 +224,6 @@ int run_kpm1d(Operator* op, int64_t NC, int64_t NR, int64_t NH, const void* psi_
   }
   if (!psi_r || !mu) return fail(KPMGB_ERR_ARGUMENT, "null buffer");
   Workspace& ws = op->ws;
-  const size_t slot = (size_t)NH * (NR + (NR & 1)) * 16;  // whole column pairs
-  KPMGB_TRY(ws.slots.ensure(2 * slot));
-  if (lr) KPMGB_TRY(ws.bra.ensure(slot));
-  // scales: column factors of the ket and the bra, and their products
-  KPMGB_TRY(ws.scales.ensure((size_t)(3 * NR + 2) * sizeof(double)));
-  KPMGB_TRY(ensure_sync(op, s));
-  char* slots = ws.slots.as<char>();
-  void* sl[2] = {slots, slots + slot};
-  double* sc = ws.scales.as<double>();
   const bool ff = precision == KPMGB_PREC_FF;
   // kernel_variant 10: one thread-block cluster per probe column, the
   // recurrence resident in distributed shared memory.  Automatic selection
@@ -253,8 +252,27 @@ int run_kpm1d(Operator* op, int64_t NC, int64_t NR, int64_t NH, const void* psi_
   // Float-float calls with 2..128 columns on complex operators of at most 12
   // nonzeros per row keep them in the column-pair layout (k_step_ffcp;
   // KPMGB_COLPAIR=0 keeps the standard layout and k_step_ffc).
-  const bool colpair = colpair_on && ff && !auto_cluster && variant == 0 && real_dots &&
-                       colpair_step_applies(op->csr, (int)NR, lr ? DOT_LR1 : DOT_DOUBLING);
+  bool colpair = colpair_on && ff && !auto_cluster && variant == 0 && real_dots &&
+                 colpair_step_applies(op->csr, (int)NR, lr ? DOT_LR1 : DOT_DOUBLING);
+  // two slots and the bra; column pairs of an odd NR hold one column more
+  size_t slot = 0;
+  auto ensure_slots = [&]() -> int {
+    slot = (size_t)NH * (colpair ? NR + (NR & 1) : NR) * 16;
+    KPMGB_TRY(ws.slots.ensure(2 * slot));
+    return lr ? ws.bra.ensure(slot) : KPMGB_OK;
+  };
+  if (const int rc = ensure_slots()) {
+    if (!colpair || NR % 2 == 0) return rc;
+    clear_error();
+    colpair = false;
+    KPMGB_TRY(ensure_slots());
+  }
+  // scales: column factors of the ket and the bra, and their products
+  KPMGB_TRY(ws.scales.ensure((size_t)(3 * NR + 2) * sizeof(double)));
+  KPMGB_TRY(ensure_sync(op, s));
+  char* slots = ws.slots.as<char>();
+  void* sl[2] = {slots, slots + slot};
+  double* sc = ws.scales.as<double>();
   const int layout = paired ? VEC_PAIRED : colpair ? VEC_COLPAIR : VEC_STD;
   KPMGB_TRY(launch_load_block(psi_r, sl[0], NH, (int)NR, precision, sc, false, s, layout));
   if (lr)
@@ -333,9 +351,9 @@ int run_kpm1d(Operator* op, int64_t NC, int64_t NR, int64_t NH, const void* psi_
   a.shape = chosen_shape;
   a.paired = paired;
   a.colpair = colpair;
-  size_t held = 0;
-  KPMGB_TRY(recurrence_scratch_bytes(a, precision, NC, lr, &held));
-  KPMGB_TRY(ws.partials.ensure(std::max(ws.partials.bytes, held)));
+  size_t most = 0, least = 0, held = 0;
+  KPMGB_TRY(recurrence_scratch_bytes(a, precision, NC, lr, &most, &least));
+  KPMGB_TRY(ws.partials.ensure_some(most, least, &held));
   a.partials = ws.partials.ptr;
   auto recurrence = [&]() -> int {
     return launch_recurrence(a, precision, NC, lr, sl, held, m, s);
@@ -962,11 +980,15 @@ static int run_ensemble(kpmgb_operator h, int32_t nseg, const int64_t* seg, int6
   // partial dots, in the partials buffer
   const size_t meta = ((size_t)(nseg + 1) * sizeof(int64_t) + (size_t)nseg * sizeof(int) + 15) &
                       ~(size_t)15;
-  const bool packed_ok = ff && paired_on && packed_members_apply(op->csr, (int)nb_max);
-  const size_t step_scratch = std::max(
-      ensemble_step_scratch_bytes(seg, nseg, (int)nb_max, kEnsRowsMin),
-      packed_ok ? ensemble_packed_scratch_bytes(seg, nseg, (int)nb_max, kEnsPackedRowsMin) : 0);
-  KPMGB_TRY(ws.partials.ensure(std::max(meta + step_scratch, ws.partials.bytes)));
+  bool packed_ok = ff && paired_on && packed_members_apply(op->csr, (int)nb_max);
+  const size_t plain =
+      meta + ensemble_step_scratch_bytes(seg, nseg, (int)nb_max, kEnsRowsMin);
+  size_t most = plain, held = 0;
+  if (packed_ok)
+    most = std::max(plain, meta + ensemble_packed_scratch_bytes(seg, nseg, (int)nb_max,
+                                                                kEnsPackedRowsMin));
+  KPMGB_TRY(ws.partials.ensure_some(most, plain, &held));
+  packed_ok = packed_ok && held == most;
   KPMGB_TRY(ensure_sync(op, s));
   char* mp = ws.partials.as<char>();
   EnsembleArgs ea;

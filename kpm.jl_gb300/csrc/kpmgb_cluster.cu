@@ -557,9 +557,12 @@ int launch_kpm1d_cluster(const DeviceCSR& H, int64_t NH, int NR, int64_t NC, boo
   const int nd = lr ? 1 : 2;
   const size_t first_bytes = (size_t)G * 2 * NR * sizeof(double2);
   const size_t step_bytes = (size_t)G * nd * NR * sizeof(double2);
-  const int64_t hold = std::max<int64_t>(
+  const int64_t most = std::max<int64_t>(
       1, std::min<int64_t>(N - 1, (int64_t)(kSumBytes / step_bytes)));
-  KPMGB_TRY(sums.ensure(std::max(sums.bytes, first_bytes + (size_t)hold * step_bytes)));
+  size_t room = 0;
+  KPMGB_TRY(sums.ensure_some(first_bytes + (size_t)most * step_bytes, first_bytes + step_bytes,
+                             &room));
+  const int64_t hold = (int64_t)((room - first_bytes) / step_bytes);
   ClusterParams p;
   p.rowptr = H.rowptr;
   p.col = H.col;

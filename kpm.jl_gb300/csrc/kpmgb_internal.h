@@ -87,6 +87,9 @@ struct DevBuf {
   void* ptr = nullptr;
   size_t bytes = 0;  // capacity
   int ensure(size_t need);
+  // Grows to `want` bytes, or to `least` where memory does not hold that;
+  // *got: how many of them may be used.
+  int ensure_some(size_t want, size_t least, size_t* got);
   void release(bool device_idle = false);
   template <typename T>
   T* as() const { return static_cast<T*>(ptr); }
