@@ -162,8 +162,6 @@ int check_status(Operator* op, cudaStream_t s) {
   KPMGB_CUDA(cudaMemcpyAsync(&st, op->ws.sync.as<unsigned>() + 1, sizeof(unsigned),
                              cudaMemcpyDeviceToHost, s));
   KPMGB_CUDA(cudaStreamSynchronize(s));
-  if (st & STATUS_SCRATCH)
-    return fail(KPMGB_ERR_CUDA, "internal scratch buffer too small for the launch grid");
   if (st & STATUS_TIMEOUT)
     return fail(KPMGB_ERR_TIMEOUT, "a bounded wait inside a kernel expired (pipeline stalled)");
   if (st & STATUS_GROWTH)

@@ -130,14 +130,13 @@ enum StatusBits : unsigned {
   STATUS_NONFINITE = 1u,
   STATUS_GROWTH = 2u,
   STATUS_TIMEOUT = 4u,
-  STATUS_SCRATCH = 8u,
 };
 
 struct Workspace {
   DevBuf slots;      // recurrence vectors, row-major NH x NR (16 B elements)
   DevBuf bra;        // bra block for the l/r path
   DevBuf partials;   // per-block moment partial sums
-  DevBuf sync;       // [0] ticket counter, [1] status bits, [2..] spare
+  DevBuf sync;       // [1] status bits, [2..] barrier words, claimed members
   DevBuf scales;     // per-column scale factors (float-float path)
   DevBuf mu;         // moments on the device (host-variant staging)
   DevBuf psi_in;     // staging for host probe blocks
@@ -231,7 +230,7 @@ int launch_step(const StepArgs& a, int precision, cudaStream_t s);
 // The same for n independent steps without dots (equal NH and NR; no step
 // reads what another writes): one launch for as many of them as share a kernel.
 int launch_steps(const StepArgs* steps, int n, int precision, cudaStream_t s);
-// Whether float-float doubling steps of NR columns on H can run on packed
+// Whether float-float steps of NR columns on H with these dots can run on packed
 // FP32 pairs over the paired vector layout (StepArgs::paired).
 bool packed_step_applies(const DeviceCSR& H, int NR, int dot);
 // Whether float-float steps of NR columns on H with these dots can run on

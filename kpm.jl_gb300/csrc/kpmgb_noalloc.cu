@@ -156,8 +156,6 @@ extern "C" int kpmgb_kpm1d_noalloc(int64_t NH, const int32_t* rowptr, const int3
   unsigned status = 0;
   KPMGB_CUDA(cudaMemcpyAsync(&status, sync + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
   KPMGB_CUDA(cudaStreamSynchronize(s));
-  if (status & STATUS_SCRATCH)
-    return fail(KPMGB_ERR_CUDA, "the no-alloc scratch is too small for the launch grid");
   if (status & STATUS_TIMEOUT)
     return fail(KPMGB_ERR_TIMEOUT, "a bounded wait inside a kernel expired");
   if (status & STATUS_NONFINITE)

@@ -165,7 +165,6 @@ struct StepChoice {
   KernelFn fn = nullptr;
   int grid = 0;
   int threads = kThreads;
-  size_t smem = 0;
   int slots = 0;  // resident blocks where early launches depend on them, else 0
   int split = 1;  // parts of the columns
   int batch = kMaxBatch;  // steps without dots per launch
@@ -185,14 +184,13 @@ int launch_step_kernel(const StepChoice& c, int n, cudaStream_t s, const KBatch&
   const int blocks = c.grid * n * c.split;
   const bool early = c.slots == 0 || blocks >= c.slots || 2 * blocks <= c.slots;
   if (!on || !early) {
-    c.fn<<<grid, c.threads, c.smem, s>>>(p);
+    c.fn<<<grid, c.threads, 0, s>>>(p);
     KPMGB_LAUNCHED();
     return KPMGB_OK;
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3((unsigned)c.threads);
-  cfg.dynamicSmemBytes = c.smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -240,8 +238,8 @@ int grid_for(KernelFn fn, int64_t NH, int lpr, int split = 1) {
       1, std::min<int64_t>(tiles, (int64_t)per_sm * num_sms() / split));
 }
 
-// Grid of a packed step: resident blocks per SM (with its threads and
-// dynamic shared memory) times the SM count, capped by the row tiles.
+// Grid of a packed step: resident blocks per SM times the SM count, capped by
+// the row tiles.
 int grid_packed(const PackedStep& ps, int64_t NH) {
   static std::mutex m;
   static std::unordered_map<const void*, int> cache;
@@ -252,9 +250,7 @@ int grid_packed(const PackedStep& ps, int64_t NH) {
     if (it != cache.end()) {
       per_sm = it->second;
     } else {
-      if (ps.smem > 48 * 1024)
-        cudaFuncSetAttribute(ps.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ps.smem);
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ps.fn, ps.threads, ps.smem) !=
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ps.fn, ps.threads, 0) !=
           cudaSuccess)
         per_sm = 1;
       per_sm = std::max(per_sm, 1);
@@ -303,7 +299,7 @@ int choose_step(const StepArgs& a, int precision, int ncols, StepChoice* out) {
                               : PackedStep{};
     if (!ps.fn) return fail(KPMGB_ERR_CUDA, "internal: column-pair layout without its kernel");
     *out = StepChoice{ps.fn, grid_for(ps.fn, a.NH, kThreads / ps.rows_per_block, ps.split),
-                      ps.threads, ps.smem, 0, ps.split};
+                      ps.threads, 0, ps.split};
     return KPMGB_OK;
   }
   if (a.paired) {
@@ -313,7 +309,7 @@ int choose_step(const StepArgs& a, int precision, int ncols, StepChoice* out) {
                               ? select_packed_step(ncols, a.dot, real, H.max_row_nnz, H.ell_w, a.NH)
                               : PackedStep{};
     if (!ps.fn) return fail(KPMGB_ERR_CUDA, "internal: paired layout without the packed kernel");
-    *out = StepChoice{ps.fn, grid_packed(ps, a.NH), ps.threads, ps.smem, 0, ps.split};
+    *out = StepChoice{ps.fn, grid_packed(ps, a.NH), ps.threads, 0, ps.split};
     return KPMGB_OK;
   }
   if (a.variant == 11 && precision != KPMGB_PREC_FF)
@@ -708,6 +704,7 @@ int launch_member_recurrence(const DeviceCSR& H, int64_t NH, int NR, int64_t NC,
   p.c0 = 0;
   p.ncols = NR;
   p.bra = nullptr;
+  p.parts = c.split;
   p.blk = a.blk;
   p.vmax = nullptr;
   p.ell_col = H.ell_col;

@@ -847,12 +847,11 @@ int ffc_lanes(int ncols);
 // real operators, 2..128 columns, steps with dots, rows of 5..8 nonzeros,
 // vectors in the paired element layout (re.hi, im.hi, re.lo, im.lo).  The
 // kernel to launch for such a call of NH rows (fn = nullptr when none
-// applies): threads per block, dynamic shared memory, rows per block tile and
-// the parts of the columns (gridDim.y).
+// applies): threads per block, rows per block tile and the parts of the columns
+// (gridDim.y).
 struct PackedStep {
   KernelFn fn = nullptr;
   int threads = 0;
-  size_t smem = 0;
   int rows_per_block = 0;
   int split = 1;
 };

@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_step_ffpk(
   pdl_enter();
   constexpr int GROUPS = kThreads / 32;  // rows per block tile
   constexpr int CPL = 2;
-  // 33..63 columns: the second column slot of the lanes past the last column
+  // 49..63 columns: the second column slot of the lanes past the last column
   // is dead (no loads, stores or dots)
   bool live[CPL];
 #pragma unroll
