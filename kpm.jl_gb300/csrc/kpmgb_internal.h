@@ -203,6 +203,8 @@ struct StepArgs {
   void* y = nullptr;
   double alpha = 1.0;
   double beta = 0.0;
+  int c0 = 0, c1 = 0;        // columns of this step (c1 = 0: all of them)
+  int max_grid = 0;          // blocks that `partials` has room for (CSR kernels; 0: any)
   const void* bra = nullptr;
   int dot = DOT_NONE;
   void* partials = nullptr;   // per-block sums of the dots (step_partials_bytes;
@@ -248,8 +250,9 @@ int step_partials_bytes(const StepArgs& a, int precision, size_t* bytes);
 // A kpm_1d recurrence from slot[0] (slot[1] is overwritten): NC/2 doubling
 // steps, or NC - 1 bra/ket steps (lr), with all moments into m.mu.  `a` names
 // the operator, sizes, kernel and bra; a.partials holds `held` bytes, between
-// the two counts of recurrence_scratch_bytes (*least at least, the returned
-// count for the fewest finishing launches).
+// the two counts of recurrence_scratch_bytes (*least at least, one step's sums
+// of one launch's columns; the returned count for the fewest finishing
+// launches).
 int launch_recurrence(StepArgs a, int precision, int64_t NC, bool lr, void* const (&slot)[2],
                       size_t held, MomentArgs m, cudaStream_t s);
 int recurrence_scratch_bytes(const StepArgs& a, int precision, int64_t NC, bool lr,

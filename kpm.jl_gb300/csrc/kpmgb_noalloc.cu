@@ -6,7 +6,7 @@
 // not take the device-wide synchronisation cudaMalloc/cudaFree imply.  For
 // them this entry point takes every input and output as device memory the
 // caller already owns, and keeps its scratch (two recurrence slots, the
-// per-block moment partial sums and the reduction ticket) in one file-scope
+// per-block moment partial sums) in one file-scope
 // device array of fixed size, kNoAllocScratchBytes.  Every GPU that loads the
 // library holds that array until the process exits.
 //
@@ -131,7 +131,13 @@ extern "C" int kpmgb_kpm1d_noalloc(int64_t NH, const int32_t* rowptr, const int3
   a.NR = (int)NR;
   size_t most = 0, part = 0;
   KPMGB_TRY(recurrence_scratch_bytes(a, KPMGB_PREC_FP64, NC, false, &most, &part));
-  const size_t need = kSyncBytes + 2 * align256(slot) + align256(part);
+  const size_t slots = kSyncBytes + 2 * align256(slot);
+  if (slots + align256(part) > kNoAllocScratchBytes) {
+    // fewer blocks leave fewer sums: two per SM, as long as they fit
+    a.max_grid = 2 * contract_sms();
+    KPMGB_TRY(recurrence_scratch_bytes(a, KPMGB_PREC_FP64, NC, false, &most, &part));
+  }
+  const size_t need = slots + align256(part);
   if (need > kNoAllocScratchBytes)
     return fail(KPMGB_ERR_ARGUMENT,
                 "kpmgb_kpm1d_noalloc needs %zu bytes of scratch for NH=%lld, NR=%lld; its static "
@@ -151,7 +157,7 @@ extern "C" int kpmgb_kpm1d_noalloc(int64_t NH, const int32_t* rowptr, const int3
   MomentArgs m;
   m.mu = reinterpret_cast<double2*>(mu_all);
   m.status = sync + 1;
-  const size_t room = kNoAllocScratchBytes - kSyncBytes - 2 * align256(slot);
+  const size_t room = kNoAllocScratchBytes - slots;
   KPMGB_TRY(launch_recurrence(a, KPMGB_PREC_FP64, NC, false, sl, std::min(most, room), m, s));
   unsigned status = 0;
   KPMGB_CUDA(cudaMemcpyAsync(&status, sync + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, s));

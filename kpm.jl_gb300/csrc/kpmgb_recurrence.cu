@@ -346,6 +346,7 @@ int choose_step(const StepArgs& a, int precision, int ncols, StepChoice* out) {
   out->split = (ncols + width - 1) / width;
   if (precision == KPMGB_PREC_FF && sh.cpl > 2) out->batch = 1;
   out->grid = grid_for(out->fn, a.NH, sh.lpr, out->split);
+  if (a.max_grid > 0) out->grid = std::min(out->grid, a.max_grid);
   // The FP64 step of a complex operator is bound by each SM's FP64 pipe.  A
   // grid that leaves some of the resident slots free, but fewer than it needs,
   // gets its successor's first blocks all on the SMs with those slots when
@@ -355,6 +356,8 @@ int choose_step(const StepArgs& a, int precision, int ncols, StepChoice* out) {
   if (precision == KPMGB_PREC_FP64 && !real) out->slots = blocks_per_sm(out->fn) * num_sms();
   return KPMGB_OK;
 }
+
+int last_column(const StepArgs& a) { return a.c1 > 0 ? a.c1 : a.NR; }
 
 int num_dots(int dot) { return dot == DOT_NONE ? 0 : (dot == DOT_LR1 ? 1 : 2); }
 
@@ -428,8 +431,8 @@ __global__ void __launch_bounds__(256) k_finish_moments(FinishParams f) {
 int step_partials_bytes(const StepArgs& a, int precision, size_t* bytes) {
   *bytes = 0;
   const int W = cols_per_launch();
-  for (int c0 = 0; c0 < a.NR; c0 += W) {
-    const int ncols = std::min(W, a.NR - c0);
+  for (int c0 = a.c0; c0 < last_column(a); c0 += W) {
+    const int ncols = std::min(W, last_column(a) - c0);
     StepChoice c;
     KPMGB_TRY(choose_step(a, precision, ncols, &c));
     *bytes += partials_count(a, c, ncols) * sizeof(double2);
@@ -452,9 +455,9 @@ int launch_finish_moments(const StepArgs& a, int precision, int nsteps, const Mo
   f.ld = a.NR;
   f.m = m;
   const int W = cols_per_launch();
-  for (int c0 = 0; c0 < a.NR; c0 += W) {
+  for (int c0 = a.c0; c0 < last_column(a); c0 += W) {
     f.c0 = c0;
-    f.ncols = std::min(W, a.NR - c0);
+    f.ncols = std::min(W, last_column(a) - c0);
     StepChoice c;
     KPMGB_TRY(choose_step(a, precision, f.ncols, &c));
     f.G = c.grid;
@@ -492,10 +495,10 @@ int launch_steps(const StepArgs* steps, int n, int precision, cudaStream_t s) {
       return fail(KPMGB_ERR_CUDA, "internal: a step with dots needs its partial sums");
   }
   const int W = cols_per_launch();
-  const int NR = steps[0].NR;
+  const int end = last_column(steps[0]);
   double2* partials = static_cast<double2*>(steps[0].partials);  // steps with dots launch alone
-  for (int c0 = 0; c0 < NR; c0 += W) {
-    const int ncols = std::min(W, NR - c0);
+  for (int c0 = steps[0].c0; c0 < end; c0 += W) {
+    const int ncols = std::min(W, end - c0);
     StepChoice c;  // of the steps filled in so far
     KBatch batch;
     int held = 0;
@@ -573,7 +576,18 @@ int recurrence_scratch_bytes(const StepArgs& a0, int precision, int64_t NC, bool
   KPMGB_TRY(step_partials_bytes(later_step(a, lr), precision, &step));
   const size_t n = (size_t)std::max<int64_t>(1, later_steps(NC, lr));
   *bytes = std::max(first, step * std::max<size_t>(1, std::min(n, kHeldBytes / step)));
-  if (least) *least = std::max(first, step);
+  if (least) {
+    // one launch's columns at a time
+    *least = 0;
+    StepArgs b = later_step(a, lr);
+    for (a.c0 = 0; a.c0 < a.NR; a.c0 = a.c1) {
+      b.c0 = a.c0;
+      a.c1 = b.c1 = std::min(a.c0 + cols_per_launch(), a.NR);
+      KPMGB_TRY(step_partials_bytes(a, precision, &first));
+      KPMGB_TRY(step_partials_bytes(b, precision, &step));
+      *least = std::max(*least, std::max(first, step));
+    }
+  }
   return KPMGB_OK;
 }
 
@@ -586,12 +600,23 @@ int launch_recurrence(StepArgs a, int precision, int64_t NC, bool lr, void* cons
   a.y = slot[1];
   a.alpha = 1.0;
   a.beta = 0.0;
-  KPMGB_TRY(launch_step(a, precision, s));
   const double growth = m.growth_limit;
   m.mom = MOM_STORE;
   m.i0 = 0;
   m.growth_limit = 0.0;
-  KPMGB_TRY(launch_finish_moments(a, precision, 1, m, s));
+  // a step and its moments at once, in parts of the columns whose sums fit
+  auto step_alone = [&](StepArgs t) -> int {
+    size_t bytes = 0;
+    KPMGB_TRY(step_partials_bytes(t, precision, &bytes));
+    const int W = bytes <= held ? t.NR : cols_per_launch();
+    for (t.c0 = 0; t.c0 < t.NR; t.c0 = t.c1) {
+      t.c1 = std::min(t.c0 + W, t.NR);
+      KPMGB_TRY(launch_step(t, precision, s));
+      KPMGB_TRY(launch_finish_moments(t, precision, 1, m, s));
+    }
+    return KPMGB_OK;
+  };
+  KPMGB_TRY(step_alone(a));
   // alpha_n = 2 H alpha_{n-1} - alpha_{n-2} in place: doubling moments
   // mu_{2n-2}, mu_{2n-1} (src/moment.jl:460-487), or mu_n = <psil|alpha_n>
   // (src/moment.jl:540-549)
@@ -612,8 +637,13 @@ int launch_recurrence(StepArgs a, int precision, int64_t NC, bool lr, void* cons
     b.x = slot[ip];
     b.z = slot[ip ^ 1];
     b.y = slot[ip ^ 1];
-    KPMGB_TRY(launch_step(b, precision, s));
     ip ^= 1;
+    if (hold == 1) {
+      KPMGB_TRY(step_alone(b));
+      m.i0 += lr ? 1 : 2;
+      continue;
+    }
+    KPMGB_TRY(launch_step(b, precision, s));
     if (++n == hold || i + 1 == later) {
       b.partials = base;
       KPMGB_TRY(launch_finish_moments(b, precision, (int)n, m, s));
