@@ -37,11 +37,14 @@ namespace {
 using namespace step;
 
 // --------------------------------------------------------------- dispatch
-// 9..12 columns: FP64 takes four lanes of three columns, which leaves none of
-// its scarce FP64 lanes idle (NH = 262144, 12 columns 106 us per step against
-// the 144 of 16 lanes), float-float too in steps without dots (kpm_2d of a
-// square 360x360, 64 moments, 12 columns 9.4 ms, 16 lanes 12.9); with dots it
-// takes 16 lanes (more rows in flight).
+// 9..12 columns: four lanes of three columns, which leave no lane idle (FP64
+// NH = 262144, 12 columns 106 us per step against the 144 of 16 lanes; kpm_2d of
+// a square 360x360, float-float, 64 moments, 12 columns 9.4 ms, 16 lanes 12.9).
+// Float-float steps with dots take 16 lanes, more rows in flight, below 40000
+// rows (9 real entries, 12 columns: 2000 rows 7.6 us against 12.0, 20000 19.3
+// and 18.8, 40000 30.2 and 25.8, 250000 172 and 115; 19 entries 2000 8.8 and
+// 13.9, 250000 237 and 148; 5 complex entries 20000 15.1 and 17.8, 80000 39.5
+// and 35.3).
 // Lanes per row times columns per lane; a shape narrower than the launch runs
 // the columns in parts.  Idle lanes cost as much as live ones (FP64: the pipe
 // serves whole warps; float-float: the issue slots), so parts of 16 or 8 serve
@@ -57,7 +60,8 @@ Shape pick_shape(int ncols, int precision, int dot, int64_t NH) {
   if (ncols <= 2) return {2, 1};
   if (ncols <= 4) return {4, 1};
   if (ncols <= 8) return {8, 1};
-  if (ncols <= 12 && (precision == KPMGB_PREC_FP64 || dot == DOT_NONE)) return {4, 3};
+  if (ncols <= 12 && (precision == KPMGB_PREC_FP64 || dot == DOT_NONE || NH >= 40000))
+    return {4, 3};
   if (ncols <= 16) return {16, 1};
   Shape best = ncols <= 32 ? Shape{32, 1} : ncols <= 64 ? Shape{32, 2} : Shape{32, 4};
   int width = best.lpr * best.cpl;
