@@ -235,23 +235,25 @@ int run_kpm1d(Operator* op, int64_t NC, int64_t NR, int64_t NH, const void* psi_
   if (variant != 0 && variant != 1 && variant != 4 && variant != 6 && variant != 9 &&
       variant != 10 && variant != 11)
     return fail(KPMGB_ERR_ARGUMENT, "unknown kernel_variant %d", variant);
-  const bool auto_cluster =
-      variant == 0 && cluster_auto_on && cluster_is_faster(op->csr, NH, (int)NR, precision, lr);
   // Float-float calls with 2..128 columns on real operators of 5..8
   // nonzeros in the longest row keep their vectors in the paired element layout
   // and run every step on packed FP32 pairs (k_step_ffpk / k_step_ffpk1;
-  // KPMGB_PAIRED=0 keeps the standard layout and k_step_ffr).  The doubling
-  // steps of both layouts leave out Im<x|y>, which is 0 for a Hermitian H;
-  // other operators keep to the kernels that compute it.
+  // KPMGB_PAIRED=0 keeps the standard layout and k_step_ffr); on complex
+  // operators of at most 12 nonzeros per row they keep them in the column-pair
+  // layout (k_step_ffcp; KPMGB_COLPAIR=0 keeps the standard layout and
+  // k_step_ffc).  The doubling steps of both layouts leave out Im<x|y>, which
+  // is 0 for a Hermitian H; other operators keep to the kernels that compute it.
   const bool real_dots = lr || op->csr.hermitian || variant == 11;
-  const bool paired = paired_on && ff && !auto_cluster && real_dots &&
-                      (variant == 0 || (variant == 11 && !lr && NR >= 9 && NR <= 64)) &&
-                      packed_step_applies(op->csr, (int)NR, lr ? DOT_LR1 : DOT_DOUBLING);
-  // Float-float calls with 2..128 columns on complex operators of at most 12
-  // nonzeros per row keep them in the column-pair layout (k_step_ffcp;
-  // KPMGB_COLPAIR=0 keeps the standard layout and k_step_ffc).
-  bool colpair = colpair_on && ff && !auto_cluster && variant == 0 && real_dots &&
-                 colpair_step_applies(op->csr, (int)NR, lr ? DOT_LR1 : DOT_DOUBLING);
+  const int dots = lr ? DOT_LR1 : DOT_DOUBLING;
+  bool paired = paired_on && ff && real_dots &&
+                (variant == 0 || (variant == 11 && !lr && NR >= 9 && NR <= 64)) &&
+                packed_step_applies(op->csr, (int)NR, dots);
+  bool colpair = colpair_on && ff && variant == 0 && real_dots &&
+                 colpair_step_applies(op->csr, (int)NR, dots);
+  const bool auto_cluster =
+      variant == 0 && cluster_auto_on &&
+      cluster_is_faster(op->csr, NH, (int)NR, precision, lr, paired || colpair);
+  if (auto_cluster) paired = colpair = false;
   // two slots and the bra; column pairs of an odd NR hold one column more
   size_t slot = 0;
   auto ensure_slots = [&]() -> int {

@@ -466,41 +466,57 @@ bool cached_bytes(const DeviceCSR& H, bool ff, int64_t rows, size_t* bytes, int6
 
 }  // namespace
 
-// Whether one cluster launch is expected to beat a launch per step: both times
-// per step (us) from measurements on GB300 (2D lattices, 5 entries per real
-// row; Haldane, 10 per complex row), linear in the rows that the busiest SM
-// holds and in all rows x columns.  Measured, cluster / launches: FP64 real
-// NH = 1024, NR = 8 1.8 / 4.2; 4096, 12 3.8 / 7.2; 9216, 4 5.0 / 4.1; 16384, 4
-// 6.6 / 5.3; 16384, 12 10.2 / 15.8; float-float 4096, 12 2.2 / 3.5; 16384, 8
-// 4.1 / 4.4; 32761, 1 4.8 / 3.7; FP64 complex 2048, 8 4.7 / 6.6; 8192, 4 11.2 /
-// 6.6; float-float complex 8192, 4 3.8 / 4.3 (float-float real, 16384, 4
-// 3.0 / 4.0 and 32761, 4 4.8 / 4.5 with the packed step).  Rows whose operator does not fit
-// beside them, or more than 2048 on an SM, take launches (65536, 12 FP64 50 /
-// 34).
-bool cluster_is_faster(const DeviceCSR& H, int64_t NH, int NR, int precision, bool lr) {
+// Whether one cluster launch is expected to beat a launch per step: times per
+// step (us) fitted to 5208 measured calls on GB300 (300..32768 rows of 3..19
+// entries, 1..400 columns).  Cluster: linear in the rows that the busiest SM
+// holds and their entries, with the operator beside the slots (c) or read from
+// global memory (u).  Launches of at most 128 columns: the greater of the chain
+// of a row, longer with several columns per lane, and all rows x columns.
+// Measured, cluster / launches: FP64 real NH = 1024, NR = 8 1.8 / 4.2; 4096, 12
+// 3.8 / 7.2; 16384, 4 6.6 / 5.3; 2048, 129 22 / 31; complex 2048, 8 4.7 / 6.6;
+// 8192, 4 11.2 / 6.6; 2048, 12 with 15 entries 8.3 / 17; float-float real 4096,
+// 12 2.2 / 3.5; 32761, 1 4.8 / 3.7; 2048, 129 10.7 / 24.  Beyond 2048 rows on an
+// SM, or with the operator in global memory, the cluster only serves many
+// columns of few rows, where launches take several passes (doubling ones a
+// tenth more than the fit says).  Over those calls the choice costs 0.3 to 1% more than the faster of
+// the two.
+bool cluster_is_faster(const DeviceCSR& H, int64_t NH, int NR, int precision, bool lr, bool pairs) {
+  struct Times {
+    double c[3], u[3], chain[3], work[3];
+  };
+  static constexpr Times kFp64Real = {{2.1, 3.1e-3, 5.3e-4}, {1.2, 2.5e-3, 9.7e-4},
+                                      {3.6, 0.22, 0.16}, {4.0, 1.8e-5, 4.3e-6}};
+  static constexpr Times kFp64Complex = {{2.4, 3.3e-3, 1.7e-3}, {2.5, 3.3e-3, 1.7e-3},
+                                         {3.7, 0.36, 0.27}, {4.2, 1.8e-5, 8.1e-6}};
+  static constexpr Times kFfReal = {{2.3, 1.2e-3, 2.1e-4}, {1.3, 1.1e-3, 5.9e-4},
+                                    {4.0, 0.13, 0.19}, {4.3, 1.6e-5, 2.0e-6}};
+  static constexpr Times kFfComplex = {{2.4, 1.3e-3, 2.8e-4}, {1.7, 8.8e-4, 7.1e-4},
+                                       {4.3, 0.10, 0.17}, {4.7, 2.7e-5, 1.6e-6}};
+  // launches on packed pairs and column pairs
+  static constexpr double kPaired[2][3] = {{2.7, 0.07, 0.018}, {3.3, 2.9e-6, 1.6e-6}};
+  static constexpr double kColpair[2][3] = {{2.2, 0.27, 0.0}, {3.9, 1.4e-5, 5.1e-7}};
   const bool ff = precision == KPMGB_PREC_FF, real = H.is_real != 0;
   const ClusterShape shape = cluster_shape(NH, NR);
+  if (shape.cs < 1) return false;
   size_t bytes = 0;
   int64_t cap = 0;
-  if (shape.cs < 1 || shape.load > 2048 ||
-      !cached_bytes(H, ff, (NH + shape.cs - 1) / shape.cs, &bytes, &cap))
-    return false;
-  const double row = (double)H.nnz / (double)NH / (real ? 5.0 : 10.0);
-  const double load = row * (double)shape.load, work = row * (double)NH * NR;
-  double cluster, launches;
-  if (!ff) {
-    cluster = 2.2 + (real ? 0.0044 : 0.0165) * load;
-    launches = real ? std::max(4.1, 2.2 + 5.8e-5 * work) : std::max(6.4, 1.0 + 1.25e-4 * work);
-  } else {
-    cluster = real ? 1.6 + 0.0017 * load : 2.0 + 0.0038 * load;
-    if (real)
-      launches = packed_step_applies(H, NR, lr ? DOT_LR1 : DOT_DOUBLING)
-                     ? 2.7 + 1.15e-5 * work
-                     : 3.5 + 1.9e-5 * work;
-    else
-      launches = NR <= 8 ? 4.0 + 2.9e-5 * work : 2.8 + 2.4e-5 * work;
+  const bool cache = cached_bytes(H, ff, (NH + shape.cs - 1) / shape.cs, &bytes, &cap);
+  const Times& t = ff ? (real ? kFfReal : kFfComplex) : (real ? kFp64Real : kFp64Complex);
+  const double(&c)[3] = cache ? t.c : t.u;
+  const double(&chain)[3] = !pairs ? t.chain : real ? kPaired[0] : kColpair[0];
+  const double(&work)[3] = !pairs ? t.work : real ? kPaired[1] : kColpair[1];
+  const double w = (double)H.nnz / (double)NH;
+  const double cluster = c[0] + (double)shape.load * (c[1] + c[2] * w);
+  double launches = 0.0;
+  for (int c0 = 0; c0 < NR; c0 += step::kMaxCols) {
+    const int n = std::min(step::kMaxCols, NR - c0);
+    // a few last columns find theirs far apart in rows of many
+    const double apart = n < 8 && c0 > 0 ? 2.0 : 1.0;
+    launches += std::max(apart * (chain[0] + w * (chain[1] + chain[2] * ((n + 31) / 32 - 1))),
+                         work[0] + (double)NH * n * (work[1] + work[2] * w));
   }
-  return cluster < launches;
+  if (cache && shape.load <= 2048) return cluster < launches;
+  return NR > 64 && NH <= 8192 && cluster < (lr ? 1.0 : 1.1) * launches;
 }
 
 int launch_kpm1d_cluster(const DeviceCSR& H, int64_t NH, int NR, int64_t NC, bool lr,

@@ -337,8 +337,9 @@ int launch_mn_sym(double2* mu, int NC, cudaStream_t s);
 int launch_kpm1d_cluster(const DeviceCSR& H, int64_t NH, int NR, int64_t NC, bool lr,
                          int precision, void* const (&slots)[2], const void* bra, DevBuf& sums,
                          const MomentArgs& m, cudaStream_t s);
-// Whether that is expected to take less time than a launch per step.
-bool cluster_is_faster(const DeviceCSR& H, int64_t NH, int NR, int precision, bool lr);
+// Whether that is expected to take less time than a launch per step (pairs: on
+// packed pairs or column pairs).
+bool cluster_is_faster(const DeviceCSR& H, int64_t NH, int NR, int precision, bool lr, bool pairs);
 // Moments of nsteps steps from their sums, [step][G][nd][NR], as
 // launch_recurrence makes them from its block sums.
 int launch_finish_sums(const double2* sums, int G, int nd, int NR, int64_t nsteps,

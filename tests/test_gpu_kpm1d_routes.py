@@ -40,6 +40,17 @@ def _check(H, NR, precision, rng):
     assert np.abs(got - ko.kpm_1d_lr(H, 7, bra, psi)).max() < TOL[precision]
 
 
+@pytest.mark.parametrize("precision", ["fp64", "ff"])
+@pytest.mark.parametrize("complex_v", [False, True])
+@pytest.mark.parametrize("n,W,NR", [
+    (300, 19, 129), (1024, 5, 400), (2048, 7, 129), (2048, 19, 200), (2900, 15, 153),
+    (4096, 9, 129), (9001, 19, 7), (16384, 5, 6), (20000, 3, 12),
+])
+def test_schedules(n, W, NR, complex_v, precision):
+    rng = np.random.default_rng(n + W)
+    _check(_band(n, W, complex_v, rng), NR, precision, rng)
+
+
 @pytest.mark.parametrize("n", [39999, 40000, 40013])
 @pytest.mark.parametrize("W,complex_v", [(3, False), (9, False), (15, True), (19, True)])
 @pytest.mark.parametrize("NR", [9, 11, 12])
