@@ -173,8 +173,10 @@ inline int64_t contract_range(int64_t K, int nr, int nl, int sms, size_t limit) 
   const Layout8 one = layout8(K, nr, nl, kRangeChunk, sms);
   const size_t per_chunk = one.pl.a_bytes + one.pl.b_bytes;
   if (limit < one.bytes) return 0;
+  const size_t whole = (size_t)((K + kRangeChunk - 1) / kRangeChunk) * per_chunk;
   const size_t most = std::min<size_t>(
-      kPlaneBytes, std::max<size_t>((size_t)64 << 20, (size_t)K * (nr + nl) * 16));
+      kPlaneBytes,
+      std::max<size_t>({(size_t)64 << 20, (size_t)K * (nr + nl) * 16, whole / 8}));
   // what the other parts leave: those of one chunk first, then those of the
   // range that this allows (they grow with it)
   int64_t chunks = 1;

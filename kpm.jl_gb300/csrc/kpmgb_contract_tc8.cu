@@ -68,28 +68,64 @@ static_assert(sizeof(VecStat) == kVecStatBytes, "size of the statistics in the s
 
 __device__ __forceinline__ int exponent_of(unsigned long long bits) { return (int)(bits >> 52); }
 
-// |v| / 2^(ex - 1023) as a float with 23 bits of v (0 below 2^-40), for v of at
-// most exponent ex: integer operations only, the FP64 pipe stays out of it
-__device__ __forceinline__ float relative(double v, int ex) {
-  const unsigned long long b = abs_bits(v);
-  const int d = exponent_of(b) - ex;
-  return d < -40 || b == 0 ? 0.f : __int_as_float(((127 + d) << 23) | (int)((b >> 29) & 0x7fffff));
+// The magnitudes of an entry's parts as bits that order like them.  Float-float
+// parts stand for themselves by their leading float, which keeps the FP64
+// conversions (a third of the FP64 kernel's own time for a few vectors) out of
+// the statistics: |hi| < 2^e bounds hi + lo by 2^e as well.
+template <bool FF>
+struct Magnitude;
+template <>
+struct Magnitude<false> {
+  using T = unsigned long long;
+  static constexpr int kMant = 52;
+  static __device__ __forceinline__ void load(const void* base, int64_t i, T& re, T& im) {
+    const double2 v = __ldg(static_cast<const double2*>(base) + i);
+    re = abs_bits(v.x);
+    im = abs_bits(v.y);
+  }
+  static __device__ __forceinline__ unsigned long long peak(T b) { return b; }
+  static __device__ __forceinline__ int mantissa(T b) { return (int)((b >> 29) & 0x7fffff); }
+};
+template <>
+struct Magnitude<true> {
+  using T = unsigned;
+  static constexpr int kMant = 23;
+  static __device__ __forceinline__ void load(const void* base, int64_t i, T& re, T& im) {
+    const float4 v = __ldg(static_cast<const float4*>(base) + i);
+    re = __float_as_uint(v.x) & 0x7fffffffu;
+    im = __float_as_uint(v.z) & 0x7fffffffu;
+  }
+  static __device__ __forceinline__ unsigned long long peak(T b) {
+    return (unsigned long long)__double_as_longlong((double)__uint_as_float(b));
+  }
+  static __device__ __forceinline__ int mantissa(T b) { return (int)(b & 0x7fffff); }
+};
+
+// A magnitude over 2 to the power of exponent field ex, at least its own, as a
+// float with 23 bits (0 below 2^-40): integer operations only
+template <bool FF>
+__device__ __forceinline__ float relative(typename Magnitude<FF>::T b, int ex) {
+  const int d = (int)(b >> Magnitude<FF>::kMant) - ex;
+  return d < -40 || b == 0 ? 0.f : __int_as_float(((127 + d) << 23) | Magnitude<FF>::mantissa(b));
 }
 
 // stat[v][chunk]
 template <bool FF>
 __global__ void __launch_bounds__(256) k_vec_stat(const void* vecs, int64_t K, int chunks,
                                                   VecStat* stat) {
-  __shared__ unsigned long long rp[256];
+  using Mag = Magnitude<FF>;
+  using B = typename Mag::T;
+  __shared__ B rp[256];
   __shared__ float rs[256];
   __shared__ unsigned rl[256];
   const int v = blockIdx.y, tid = threadIdx.x;
   const int64_t k0 = (int64_t)blockIdx.x * kStatChunk, k1 = min(K, k0 + kStatChunk);
-  unsigned long long m = 0;
+  B m = 0;
 #pragma unroll 4
   for (int64_t k = k0 + tid; k < k1; k += 256) {
-    const double2 x = load_f64<FF>(vecs, (int64_t)v * K + k);
-    m = max(m, max(abs_bits(x.x), abs_bits(x.y)));
+    B re, im;
+    Mag::load(vecs, (int64_t)v * K + k, re, im);
+    m = max(m, max(re, im));
   }
   rp[tid] = m;
   __syncthreads();
@@ -97,18 +133,19 @@ __global__ void __launch_bounds__(256) k_vec_stat(const void* vecs, int64_t K, i
     if (tid < w) rp[tid] = max(rp[tid], rp[tid + w]);
     __syncthreads();
   }
-  const int ex = exponent_of(rp[0]);
+  const int ex = (int)(rp[0] >> Mag::kMant);
   float s = 0.f;
   unsigned large = 0;
   bool re_any = false, im_any = false;
 #pragma unroll 4
   for (int64_t k = k0 + tid; k < k1; k += 256) {
-    const double2 x = load_f64<FF>(vecs, (int64_t)v * K + k);
-    const float re = relative(x.x, ex), im = relative(x.y, ex);
+    B rb, ib;
+    Mag::load(vecs, (int64_t)v * K + k, rb, ib);
+    const float re = relative<FF>(rb, ex), im = relative<FF>(ib, ex);
     s = fmaf(re, re, fmaf(im, im, s));
     large += (re >= 0.03125f ? 1u : 0u) + (im >= 0.03125f ? 1u << 16 : 0u);
-    re_any |= abs_bits(x.x) != 0;
-    im_any |= abs_bits(x.y) != 0;
+    re_any |= rb != 0;
+    im_any |= ib != 0;
   }
   rs[tid] = s;
   rl[tid] = large;
@@ -121,7 +158,8 @@ __global__ void __launch_bounds__(256) k_vec_stat(const void* vecs, int64_t K, i
     }
     __syncthreads();
   }
-  if (tid == 0) stat[(size_t)v * chunks + blockIdx.x] = VecStat{rp[0], rs[0], rl[0] | any};
+  if (tid == 0)
+    stat[(size_t)v * chunks + blockIdx.x] = VecStat{Mag::peak(rp[0]), rs[0], rl[0] | any};
 }
 
 // exps[v]: max |component| < 2^e (0 for a zero vector); *fp64 set when a
@@ -157,7 +195,7 @@ __global__ void __launch_bounds__(32) k_vec_gate(const VecStat* stat, int chunks
   }
   if (lane == 0) {
     exps[v] = m == 0 ? 0 : max(ex, 1) - 1022;
-    const float mx = relative(__longlong_as_double((long long)m), ex);
+    const float mx = relative<false>(m, ex);
     const bool peaked = !(mx * mx * 2.f * (float)K <= kPeak * s);
     const bool uneven = ((any & kAnyRe) && 16 * re < 9 * K) || ((any & kAnyIm) && 16 * im < 9 * K);
     if (m != 0 && (ex == 0x7ff || peaked || uneven)) atomicOr(fp64, 1u);
