@@ -420,8 +420,9 @@ const int* clusters_side_by_side() {
 }
 
 struct ClusterShape {
-  int cs = 0;        // CTAs per cluster; 0: no cluster holds the rows
-  int64_t load = 0;  // rows of all columns on the busiest SM
+  int cs = 0;         // CTAs per cluster; 0: no cluster holds the rows
+  int64_t waves = 0;  // clusters that follow one another on the busiest SM
+  int64_t load = 0;   // their rows
 };
 
 int64_t max_rows_per_cta() {
@@ -440,11 +441,8 @@ ClusterShape cluster_shape(int64_t NH, int NR) {
   for (int k = 1; k <= kMaxCluster; ++k) {
     const int64_t r = (NH + k - 1) / k;
     if (r > max_rows || (k > 1 && r < 32) || side[k] < 1) continue;
-    const int64_t load = ((NR + side[k] - 1) / side[k]) * r;
-    if (s.cs == 0 || load < s.load) {
-      s.load = load;
-      s.cs = k;
-    }
+    const int64_t waves = (NR + side[k] - 1) / side[k];
+    if (s.cs == 0 || waves * r < s.load) s = ClusterShape{k, waves, waves * r};
   }
   return s;
 }
@@ -467,54 +465,60 @@ bool cached_bytes(const DeviceCSR& H, bool ff, int64_t rows, size_t* bytes, int6
 }  // namespace
 
 // Whether one cluster launch is expected to beat a launch per step: times per
-// step (us) fitted to 5208 measured calls on GB300 (300..32768 rows of 3..19
+// step (us) fitted to 6984 measured calls on GB300 (300..32768 rows of 3..19
 // entries, 1..400 columns).  Cluster: linear in the rows that the busiest SM
 // holds and their entries, with the operator beside the slots (c) or read from
 // global memory (u).  Launches of at most 128 columns: the greater of the chain
-// of a row, longer with several columns per lane, and all rows x columns.
-// Measured, cluster / launches: FP64 real NH = 1024, NR = 8 1.8 / 4.2; 4096, 12
-// 3.8 / 7.2; 16384, 4 6.6 / 5.3; 2048, 129 22 / 31; complex 2048, 8 4.7 / 6.6;
-// 8192, 4 11.2 / 6.6; 2048, 12 with 15 entries 8.3 / 17; float-float real 4096,
-// 12 2.2 / 3.5; 32761, 1 4.8 / 3.7; 2048, 129 10.7 / 24.  Beyond 2048 rows on an
-// SM, or with the operator in global memory, the cluster only serves many
-// columns of few rows, where launches take several passes (doubling ones a
-// tenth more than the fit says).  Over those calls the choice costs 0.3 to 1% more than the faster of
-// the two.
+// of a row, longer with several columns per lane, and all rows x columns, idle
+// lanes included.  Measured, cluster / launches: FP64 real NH = 1024, NR = 8
+// 1.8 / 4.2; 4096, 12 3.8 / 7.2; 16384, 4 6.6 / 5.3; 15876, 5 8.0 / 11.6; 2048,
+// 129 22 / 31; complex 2048, 8 4.7 / 6.6; 8192, 4 11.2 / 6.6; 2450, 11 6.8 /
+// 13.4; float-float real 4096, 12 2.2 / 3.5; 32761, 1 4.8 / 3.7; 2048, 129 10.7 /
+// 24.  Beyond 2048 rows on an SM, or with the operator in global memory, the
+// cluster only serves many columns of few rows, where launches take several
+// passes (doubling ones a tenth more than the fit says).  Over those calls the
+// choice costs 0.3 to 1.2% more than the faster of the two.
 bool cluster_is_faster(const DeviceCSR& H, int64_t NH, int NR, int precision, bool lr, bool pairs) {
-  struct Times {
-    double c[3], u[3], chain[3], work[3];
+  struct Cluster {
+    double c[4], u[4];  // chain, per row, per entry, each further wave
   };
-  static constexpr Times kFp64Real = {{2.1, 3.1e-3, 5.3e-4}, {1.2, 2.5e-3, 9.7e-4},
-                                      {3.6, 0.22, 0.16}, {4.0, 1.8e-5, 4.3e-6}};
-  static constexpr Times kFp64Complex = {{2.4, 3.3e-3, 1.7e-3}, {2.5, 3.3e-3, 1.7e-3},
-                                         {3.7, 0.36, 0.27}, {4.2, 1.8e-5, 8.1e-6}};
-  static constexpr Times kFfReal = {{2.3, 1.2e-3, 2.1e-4}, {1.3, 1.1e-3, 5.9e-4},
-                                    {4.0, 0.13, 0.19}, {4.3, 1.6e-5, 2.0e-6}};
-  static constexpr Times kFfComplex = {{2.4, 1.3e-3, 2.8e-4}, {1.7, 8.8e-4, 7.1e-4},
-                                       {4.3, 0.10, 0.17}, {4.7, 2.7e-5, 1.6e-6}};
-  // launches on packed pairs and column pairs
-  static constexpr double kPaired[2][3] = {{2.7, 0.07, 0.018}, {3.3, 2.9e-6, 1.6e-6}};
-  static constexpr double kColpair[2][3] = {{2.2, 0.27, 0.0}, {3.9, 1.4e-5, 5.1e-7}};
+  struct Launch {
+    double chain[3];  // once, per entry, per entry and further column of a lane
+    double work[3];   // once, per row x column, per entry x column
+    double lr;        // bra/ket steps, which take fewer dots, against doubling ones
+  };
+  static constexpr Cluster kCluster[2][2] = {
+      {{{2.2, 3.5e-3, 1.8e-3, 0.41}, {3.0, 2.9e-3, 1.7e-3, 0.5}},
+       {{2.0, 3.2e-3, 5.5e-4, 0.54}, {1.1, 2.3e-3, 9.8e-4, 0.51}}},
+      {{{2.3, 1.5e-3, 3.0e-4, 0.21}, {1.8, 7.4e-4, 7.2e-4, 0.87}},
+       {{2.2, 1.3e-3, 2.2e-4, 0.25}, {1.3, 1.0e-3, 5.9e-4, 0.61}}}};  // [float-float][real]
+  static constexpr Launch kCsr[2][2] = {
+      {{{3.7, 0.34, 0.30}, {4.0, 1.9e-5, 7.8e-6}, 0.94}, {{3.8, 0.20, 0.18}, {3.9, 1.8e-5, 4.2e-6}, 0.91}},
+      {{{4.5, 0.10, 0.15}, {5.0, 2.4e-5, 1.3e-6}, 0.92}, {{4.2, 0.12, 0.17}, {4.6, 1.3e-5, 1.8e-6}, 0.91}}};
+  static constexpr Launch kPairs[2] = {{{2.4, 0.25, 0.034}, {3.8, 1.4e-5, 5.3e-7}, 1.0},
+                                       {{0.84, 0.36, 0.049}, {3.3, 2.6e-6, 1.6e-6}, 0.98}};
   const bool ff = precision == KPMGB_PREC_FF, real = H.is_real != 0;
   const ClusterShape shape = cluster_shape(NH, NR);
   if (shape.cs < 1) return false;
   size_t bytes = 0;
   int64_t cap = 0;
   const bool cache = cached_bytes(H, ff, (NH + shape.cs - 1) / shape.cs, &bytes, &cap);
-  const Times& t = ff ? (real ? kFfReal : kFfComplex) : (real ? kFp64Real : kFp64Complex);
-  const double(&c)[3] = cache ? t.c : t.u;
-  const double(&chain)[3] = !pairs ? t.chain : real ? kPaired[0] : kColpair[0];
-  const double(&work)[3] = !pairs ? t.work : real ? kPaired[1] : kColpair[1];
   const double w = (double)H.nnz / (double)NH;
-  const double cluster = c[0] + (double)shape.load * (c[1] + c[2] * w);
+  const double(&c)[4] = cache ? kCluster[ff][real].c : kCluster[ff][real].u;
+  const double cluster = c[0] + (double)shape.load * (c[1] + c[2] * w) +
+                         c[3] * (double)(std::min<int64_t>(shape.waves, 4) - 1);
+  const Launch& l = pairs ? kPairs[real] : kCsr[ff][real];
   double launches = 0.0;
   for (int c0 = 0; c0 < NR; c0 += step::kMaxCols) {
     const int n = std::min(step::kMaxCols, NR - c0);
+    int held = 0, cpl = 1;
+    launch_columns(NH, n, precision, lr ? DOT_LR1 : DOT_DOUBLING, pairs, &held, &cpl);
     // a few last columns find theirs far apart in rows of many
     const double apart = n < 8 && c0 > 0 ? 2.0 : 1.0;
-    launches += std::max(apart * (chain[0] + w * (chain[1] + chain[2] * ((n + 31) / 32 - 1))),
-                         work[0] + (double)NH * n * (work[1] + work[2] * w));
+    launches += std::max(apart * (l.chain[0] + w * (l.chain[1] + l.chain[2] * (cpl - 1))),
+                         l.work[0] + (double)NH * held * (l.work[1] + l.work[2] * w));
   }
+  if (lr) launches *= l.lr;
   if (cache && shape.load <= 2048) return cluster < launches;
   return NR > 64 && NH <= 8192 && cluster < (lr ? 1.0 : 1.1) * launches;
 }

@@ -232,6 +232,9 @@ int launch_step(const StepArgs& a, int precision, cudaStream_t s);
 // The same for n independent steps without dots (equal NH and NR; no step
 // reads what another writes): one launch for as many of them as share a kernel.
 int launch_steps(const StepArgs* steps, int n, int precision, cudaStream_t s);
+// The columns that the lanes of a launch of ncols columns hold, idle ones
+// included, and the columns per lane (pairs: packed pairs or column pairs).
+void launch_columns(int64_t NH, int ncols, int precision, int dot, bool pairs, int* held, int* cpl);
 // Whether float-float steps of NR columns on H with these dots can run on packed
 // FP32 pairs over the paired vector layout (StepArgs::paired).
 bool packed_step_applies(const DeviceCSR& H, int NR, int dot);

@@ -274,6 +274,18 @@ bool colpair_step_applies(const DeviceCSR& H, int NR, int dot) {
          select_colpair_step(NR, dot, H.is_real != 0, H.ell_w, H.max_row_nnz, H.n).fn != nullptr;
 }
 
+void launch_columns(int64_t NH, int ncols, int precision, int dot, bool pairs, int* held, int* cpl) {
+  *cpl = 1;
+  if (pairs) {
+    *held = ncols <= 2 ? ncols : ncols <= 4 ? 4 : (ncols + 7) / 8 * 8;
+    return;
+  }
+  const Shape s = pick_shape(ncols, precision, dot, NH);
+  const int width = s.lpr * s.cpl;
+  *held = (ncols + width - 1) / width * width;
+  *cpl = s.cpl;
+}
+
 bool packed_step_applies(const DeviceCSR& H, int NR, int dot) {
   return NR <= cols_per_launch() &&
          select_packed_step(NR, dot, H.is_real != 0, H.max_row_nnz, H.ell_w, H.n).fn != nullptr;
