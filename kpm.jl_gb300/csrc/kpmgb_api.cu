@@ -364,7 +364,7 @@ int run_kpm1d(Operator* op, int64_t NC, int64_t NR, int64_t NH, const void* psi_
   std::string key;
   auto put = [&](const void* v, size_t n) { key.append(static_cast<const char*>(v), n); };
   const int64_t ints[] = {NC, NR, NH, precision, chosen_variant, chosen_shape, o->stability_check,
-                          lr ? 1 : 0, (int64_t)ws.partials.bytes};
+                          lr ? 1 : 0, layout, (int64_t)ws.partials.bytes};
   const void* ptrs[] = {mu, ws.slots.ptr, ws.bra.ptr, ws.scales.ptr, ws.partials.ptr, ws.sync.ptr,
                         op->csr.rowptr, op->csr.col, op->csr.val, op->csr.val_ff};
   put(ints, sizeof ints);
