@@ -59,9 +59,9 @@ extern "C" {
 /* kpm_2d contraction arithmetic (mu = R L^H over K = NH*NR). */
 #define KPMGB_CONTRACT_FP64 0  /* double precision: eight digit planes on
                                   the tensor cores (63 bits below the largest
-                                  entry of each vector) for vectors without
-                                  long ranges of small entries, FP64 FMAs for
-                                  calls with any other                       */
+                                  entry of each vector) where they round less
+                                  than FP64 FMAs would for every pair of the
+                                  call's vectors, else FP64 FMAs             */
 #define KPMGB_CONTRACT_SPLIT 1 /* BF16 slices on tcgen05, FP32 accumulate */
 
 /* moment_parity of kpm_2d (src/moment.jl:913-915, :1067-1069). */

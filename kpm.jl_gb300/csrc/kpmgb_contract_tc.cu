@@ -26,9 +26,8 @@
 // 36 plane pairs with i + j <= 7 feed eight accumulators, each exact over a
 // chunk of 128 K' elements ((l+1) 2^21 multiples of 2^-8l, l <= 7: at most
 // 2^24), folded into two int64 per output (levels 0-3 in units of 2^-24,
-// levels 4-7 in units of 2^-56).  What it drops is below 2^-64 of the row
-// maxima's product per K' element: against 64-bit sums it is nearer than FP64
-// FMAs, which round every partial sum.
+// levels 4-7 in units of 2^-56).  What it drops, and when it is nearer than FP64
+// FMAs: kpmgb_contract_tc8.cu.
 //
 // MMA shape: the five B planes of a stage lie one after another along N, so
 // A plane i meets B planes 0..4-i in ONE tcgen05.mma of N = 48 (5 - i)

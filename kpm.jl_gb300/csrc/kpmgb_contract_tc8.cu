@@ -7,20 +7,19 @@
 // entry becomes the integer N = round(v 2^(62-e)), |v| < 2^e over its row
 // (exact for entries within 2^-9 of the row maximum, within 2^-63 of it for
 // the rest), cut into eight balanced base-256 digits; the digit products of
-// i + j <= 7 add up exactly and the dropped ones stay below 2^-64 of the
-// product of the row maxima per term.  Entries below 2^-9 of their row's
-// maximum keep fewer bits than FP64, so the planes serve vectors in which such
-// entries cannot decide a sum; the others keep the FP64 kernel.  A vector
-// passes when its largest entry is within a factor 32 of its root mean square
-// and when, of its real parts and of its imaginary parts, 9 in 16 or more lie
-// within 2^-7 of that entry (or all are 0): any two such vectors share an
-// eighth of their sites with products of 2^-14 of the maxima's or more, whose
-// FP64 sum is rounded by more than the planes drop.  Random-phase probes and
-// what the recurrence makes of them pass (of a Gaussian vector nearly nine in
-// ten parts are that large); probes on single sites, wave packets, vectors
-// whose imaginary part is small throughout, infinities and NaN do not.
-// k_vec_gate decides on the device and sets a word that each kernel of either
-// form reads first.
+// i + j <= 7 add up exactly, the dropped ones are 2^-62 of 2^(eL + eR) per term
+// (root mean square).  FP64 FMAs round every partial sum: runs of n of them
+// cost more than that, unless the terms are far below the product of the
+// maxima.  So the planes serve a call when, for every pair of vectors, real and
+// imaginary part of the sum by themselves, the terms are large enough to make
+// the FP64 sum the worse one (k_pair_gate, from mean squares over chunks of
+// 8192 sites), and each chunk is evenly filled, 9 in 16 or more of its parts
+// within 2^-5 of its largest, so that its mean squares tell its terms
+// (k_vec_gate; at most one chunk in eight may be filled in part).  Random
+// probes and what the recurrence makes of them pass, halves that are 0 or small
+// as well; probes on single sites, wave packets, parts that are small
+// throughout, infinities and NaN do not and keep the FP64 kernel.  The decision
+// is a word on the device that each kernel of either form reads first.
 //
 // The planes of a K range are laid out, multiplied and added to the moments
 // before those of the next, in scratch that the call's budget bounds
@@ -36,8 +35,12 @@ namespace {
 
 using C8 = Planes8;
 constexpr int S8 = C8::kSlices;
-// largest entry squared against the mean square: beyond 32^2 the FP64 kernel
-constexpr float kPeak = 1024.f;
+// Rounding per product, root mean square, in units of 2^(eL + eR): of the
+// planes (digit products beyond i + j = 7: seven of two digits of 74 each at
+// 2^-76, and what to_integer rounds), and of a run of n FP64 FMAs over products
+// of root mean square 1, times the square root of n.
+constexpr double kPlaneNoise = 0x1p-62;
+constexpr double kRunNoise = 0.42 * 0x1p-54;
 
 template <bool FF>
 __device__ __forceinline__ double2 load_f64(const void* base, int64_t idx) {
@@ -53,20 +56,20 @@ __device__ __forceinline__ unsigned long long abs_bits(double v) {
   return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
 }
 
-// Largest |component| of a chunk (bits of a double), the chunk's sum of squares
-// in units of that component's power of two squared, and how many real parts
-// (low half of `large`) and imaginary parts reach 2^-5 of that power; kAnyRe,
-// kAnyIm: some are not 0.
+// A chunk's real parts: exponent field of the largest (of a double), sum of
+// squares in units of its power of two squared (0: all are 0), and how many
+// reach 2^-4 of that power; the same of its imaginary parts in the high halves.
 struct VecStat {
-  unsigned long long peak;
-  float sumsq;
-  unsigned large;
+  float re, im;
+  unsigned exps, large;
 };
-constexpr unsigned kAnyRe = 1u << 15, kAnyIm = 1u << 31;
-static_assert(kStatChunk < kAnyRe, "counts and flags share a half word");
 static_assert(sizeof(VecStat) == kVecStatBytes, "size of the statistics in the scratch");
-
-__device__ __forceinline__ int exponent_of(unsigned long long bits) { return (int)(bits >> 52); }
+// What k_vec_gate leaves in their place: mean squares over 2^2e of the vector.
+struct VecLevel {
+  float re, im;
+  float unused[2];
+};
+static_assert(sizeof(VecLevel) == sizeof(VecStat), "levels replace the statistics");
 
 // The magnitudes of an entry's parts as bits that order like them.  Float-float
 // parts stand for themselves by their leading float, which keeps the FP64
@@ -115,91 +118,140 @@ __global__ void __launch_bounds__(256) k_vec_stat(const void* vecs, int64_t K, i
                                                   VecStat* stat) {
   using Mag = Magnitude<FF>;
   using B = typename Mag::T;
-  __shared__ B rp[256];
-  __shared__ float rs[256];
-  __shared__ unsigned rl[256];
+  __shared__ B peak_re[256], peak_im[256];
+  __shared__ float sum_re[256], sum_im[256];
+  __shared__ unsigned count[256];
   const int v = blockIdx.y, tid = threadIdx.x;
   const int64_t k0 = (int64_t)blockIdx.x * kStatChunk, k1 = min(K, k0 + kStatChunk);
-  B m = 0;
+  B mr = 0, mi = 0;
 #pragma unroll 4
   for (int64_t k = k0 + tid; k < k1; k += 256) {
     B re, im;
     Mag::load(vecs, (int64_t)v * K + k, re, im);
-    m = max(m, max(re, im));
+    mr = max(mr, re);
+    mi = max(mi, im);
   }
-  rp[tid] = m;
+  peak_re[tid] = mr;
+  peak_im[tid] = mi;
   __syncthreads();
   for (int w = 128; w > 0; w >>= 1) {
-    if (tid < w) rp[tid] = max(rp[tid], rp[tid + w]);
+    if (tid < w) {
+      peak_re[tid] = max(peak_re[tid], peak_re[tid + w]);
+      peak_im[tid] = max(peak_im[tid], peak_im[tid + w]);
+    }
     __syncthreads();
   }
-  const int ex = (int)(rp[0] >> Mag::kMant);
-  float s = 0.f;
+  const int er = (int)(peak_re[0] >> Mag::kMant), ei = (int)(peak_im[0] >> Mag::kMant);
+  float sr = 0.f, si = 0.f;
   unsigned large = 0;
-  bool re_any = false, im_any = false;
 #pragma unroll 4
   for (int64_t k = k0 + tid; k < k1; k += 256) {
     B rb, ib;
     Mag::load(vecs, (int64_t)v * K + k, rb, ib);
-    const float re = relative<FF>(rb, ex), im = relative<FF>(ib, ex);
-    s = fmaf(re, re, fmaf(im, im, s));
-    large += (re >= 0.03125f ? 1u : 0u) + (im >= 0.03125f ? 1u << 16 : 0u);
-    re_any |= rb != 0;
-    im_any |= ib != 0;
+    const float re = relative<FF>(rb, er), im = relative<FF>(ib, ei);
+    sr = fmaf(re, re, sr);
+    si = fmaf(im, im, si);
+    large += (re >= 0.0625f ? 1u : 0u) + (im >= 0.0625f ? 1u << 16 : 0u);
   }
-  rs[tid] = s;
-  rl[tid] = large;
-  const unsigned any =
-      (__syncthreads_or(re_any) ? kAnyRe : 0u) | (__syncthreads_or(im_any) ? kAnyIm : 0u);
+  sum_re[tid] = sr;
+  sum_im[tid] = si;
+  count[tid] = large;
+  __syncthreads();
   for (int w = 128; w > 0; w >>= 1) {
     if (tid < w) {
-      rs[tid] += rs[tid + w];
-      rl[tid] += rl[tid + w];
+      sum_re[tid] += sum_re[tid + w];
+      sum_im[tid] += sum_im[tid + w];
+      count[tid] += count[tid + w];
     }
     __syncthreads();
   }
   if (tid == 0)
-    stat[(size_t)v * chunks + blockIdx.x] = VecStat{Mag::peak(rp[0]), rs[0], rl[0] | any};
+    stat[(size_t)v * chunks + blockIdx.x] =
+        VecStat{sum_re[0], sum_im[0],
+                (unsigned)(Mag::peak(peak_re[0]) >> 52) |
+                    (unsigned)(Mag::peak(peak_im[0]) >> 52) << 16,
+                count[0]};
 }
 
-// exps[v]: max |component| < 2^e (0 for a zero vector); *fp64 set when a
-// vector is not finite, too peaked or too unevenly spread
-__global__ void __launch_bounds__(32) k_vec_gate(const VecStat* stat, int chunks, int64_t K,
-                                                 int* exps, unsigned* fp64) {
+// The mean square of n parts over 2^2e, e one above the exponent field ex.
+__device__ __forceinline__ float level_of(float sumsq, int part_ex, int ex, int n) {
+  if (sumsq == 0.f) return 0.f;
+  return fmaxf(ldexpf(sumsq / (float)n, max(2 * (part_ex - ex) - 2, -200)), 1.18e-38f);
+}
+
+// exps[v]: max |part| < 2^e (0 for a zero vector); *fp64 set when a vector is
+// not finite or its chunks are unevenly filled; levels in place of the
+// statistics.  One warp per vector.
+__global__ void __launch_bounds__(32) k_vec_gate(VecStat* stat, int chunks, int64_t K, int nl,
+                                                 int* expL, int* expR, unsigned* fp64) {
   const int v = blockIdx.x, lane = threadIdx.x;
-  unsigned long long m = 0;
-  for (int c = lane; c < chunks; c += 32) m = max(m, stat[(size_t)v * chunks + c].peak);
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, off));
-  const int ex = exponent_of(m);
-  float s = 0.f;
-  // parts of 2^-6 of the vector's power or more: those of the chunks whose own
-  // power is at most one less (chunks of 8192 Gaussian entries all are)
-  long long re = 0, im = 0;
-  unsigned any = 0;
+  VecStat* const st = stat + (size_t)v * chunks;
+  int ex = 0;
+  for (int c = lane; c < chunks; c += 32)
+    ex = max(ex, (int)max(st[c].exps & 0xffffu, st[c].exps >> 16));
+  ex = __reduce_max_sync(0xffffffffu, ex);
+  int used = 0, thin = 0;  // chunks that hold parts, and unevenly
   for (int c = lane; c < chunks; c += 32) {
-    const VecStat t = stat[(size_t)v * chunks + c];
-    s += ldexpf(t.sumsq, 2 * max(exponent_of(t.peak) - ex, -80));
-    any |= t.large & (kAnyRe | kAnyIm);
-    if (exponent_of(t.peak) >= ex - 1) {
-      re += t.large & (kAnyRe - 1);
-      im += (t.large >> 16) & (kAnyRe - 1);
-    }
+    const VecStat t = st[c];
+    const int n = (int)min((int64_t)kStatChunk, K - (int64_t)c * kStatChunk);
+    // a short last chunk says little by itself
+    const bool judged = n == kStatChunk || chunks == 1;
+    const bool re = t.re != 0.f, im = t.im != 0.f;
+    used += re || im ? 1 : 0;
+    thin += judged && ((re && 16 * (int)(t.large & 0xffffu) < 9 * n) ||
+                       (im && 16 * (int)(t.large >> 16) < 9 * n))
+                ? 1
+                : 0;
+    reinterpret_cast<VecLevel*>(st)[c] =
+        VecLevel{level_of(t.re, (int)(t.exps & 0xffffu), ex, n),
+                 level_of(t.im, (int)(t.exps >> 16), ex, n), {0.f, 0.f}};
   }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    s += __shfl_xor_sync(0xffffffffu, s, off);
-    re += __shfl_xor_sync(0xffffffffu, re, off);
-    im += __shfl_xor_sync(0xffffffffu, im, off);
-    any |= __shfl_xor_sync(0xffffffffu, any, off);
-  }
+  used = __reduce_add_sync(0xffffffffu, used);
+  thin = __reduce_add_sync(0xffffffffu, thin);
   if (lane == 0) {
-    exps[v] = m == 0 ? 0 : max(ex, 1) - 1022;
-    const float mx = relative<false>(m, ex);
-    const bool peaked = !(mx * mx * 2.f * (float)K <= kPeak * s);
-    const bool uneven = ((any & kAnyRe) && 16 * re < 9 * K) || ((any & kAnyIm) && 16 * im < 9 * K);
-    if (m != 0 && (ex == 0x7ff || peaked || uneven)) atomicOr(fp64, 1u);
+    (v < nl ? expL + v : expR + (v - nl))[0] = used == 0 ? 0 : max(ex, 1) - 1022;
+    if (ex == 0x7ff || 8 * thin > used) atomicOr(fp64, 1u);
   }
+}
+
+// *fp64 set when a wanted pair's products are too small for the planes: the
+// mean square of the products over the sites where both vectors hold parts,
+// over 2^2(eL + eR), below `least`; for the real and the imaginary part of the
+// sum by itself.
+__global__ void __launch_bounds__(256) k_pair_gate(const VecLevel* level, int chunks, int64_t K,
+                                                   int nl, int nr, int n0, int m0, int parity,
+                                                   int nmax_row, float least, unsigned* fp64) {
+  __shared__ float2 sl[16][17], sr[16][17];
+  if (*fp64) return;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int b0 = blockIdx.x * 16, a0 = blockIdx.y * 16;
+  float re = 0.f, im = 0.f, nre = 0.f, nim = 0.f;
+  for (int c0 = 0; c0 < chunks; c0 += 16) {
+    const float2 zero = make_float2(0.f, 0.f);
+    auto at = [&](int64_t v, bool have) {
+      return have && c0 + tx < chunks
+                 ? *reinterpret_cast<const float2*>(level + v * chunks + c0 + tx)
+                 : zero;
+    };
+    sl[ty][tx] = at(b0 + ty, b0 + ty < nl);
+    sr[ty][tx] = at(nl + a0 + ty, a0 + ty < nr);
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const float2 l = sl[tx][u], r = sr[ty][u];
+      const float n = (float)max((int64_t)0, min((int64_t)kStatChunk, K - (int64_t)(c0 + u) * kStatChunk));
+      const float rr = l.x * r.x, ii = l.y * r.y, ri = l.x * r.y, ir = l.y * r.x;
+      re = fmaf(n, rr + ii, re);
+      im = fmaf(n, ri + ir, im);
+      nre += (l.x != 0.f && r.x != 0.f) || (l.y != 0.f && r.y != 0.f) ? n : 0.f;
+      nim += (l.x != 0.f && r.y != 0.f) || (l.y != 0.f && r.x != 0.f) ? n : 0.f;
+    }
+    __syncthreads();
+  }
+  const int n = n0 + a0 + ty, m = m0 + b0 + tx;
+  if (a0 + ty < nr && b0 + tx < nl && n < nmax_row && keep_parity(parity, n, m) &&
+      !(re >= least * nre && im >= least * nim))
+    atomicOr(fp64, 1u);
 }
 
 // round(v 2^(62-e)) for |v| < 2^e
@@ -317,19 +369,28 @@ int launch_planes(const ContractArgs& a, const Layout8& l, uint8_t* base, cudaSt
   unsigned* gate = reinterpret_cast<unsigned*>(base + l.gate);
   double* part = reinterpret_cast<double*>(base + l.part);
   KPMGB_CUDA(cudaMemsetAsync(gate, 0, sizeof(unsigned), s));
-  auto stats = [&](const void* vecs, int nvec, int* exps) -> int {
+  auto stats = [&](const void* vecs, int nvec, VecStat* out) -> int {
     for (int v0 = 0; v0 < nvec; v0 += 65535) {  // the grid's y limit
       const int nv = std::min(nvec - v0, 65535);
       const void* p = static_cast<const char*>(vecs) + (size_t)v0 * a.K * 16;
-      k_vec_stat<FF><<<dim3((unsigned)l.chunks, (unsigned)nv), 256, 0, s>>>(p, a.K, l.chunks, stat);
-      KPMGB_LAUNCHED();
-      k_vec_gate<<<(unsigned)nv, 32, 0, s>>>(stat, l.chunks, a.K, exps + v0, gate);
+      k_vec_stat<FF><<<dim3((unsigned)l.chunks, (unsigned)nv), 256, 0, s>>>(
+          p, a.K, l.chunks, out + (size_t)v0 * l.chunks);
       KPMGB_LAUNCHED();
     }
     return KPMGB_OK;
   };
-  KPMGB_TRY(stats(a.L, a.nl, expB));
-  KPMGB_TRY(stats(a.R, a.nr, expA));
+  KPMGB_TRY(stats(a.L, a.nl, stat));
+  KPMGB_TRY(stats(a.R, a.nr, stat + (size_t)a.nl * l.chunks));
+  k_vec_gate<<<(unsigned)(a.nl + a.nr), 32, 0, s>>>(stat, l.chunks, a.K, a.nl, expB, expA, gate);
+  KPMGB_LAUNCHED();
+  // a slice of the FP64 kernel adds at least this many products one by one
+  const int64_t run =
+      std::max<int64_t>(1, a.K / simt_slices(a.K, a.nr, a.nl, contract_sms()));
+  const float least = (float)(kPlaneNoise * kPlaneNoise / (kRunNoise * kRunNoise * (double)run));
+  k_pair_gate<<<dim3((unsigned)((a.nl + 15) / 16), (unsigned)((a.nr + 15) / 16)), 256, 0, s>>>(
+      reinterpret_cast<const VecLevel*>(stat), l.chunks, a.K, a.nl, a.nr, a.n0, a.m0, a.parity,
+      a.nmax_row, least, gate);
+  KPMGB_LAUNCHED();
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   constexpr int kSmem = (int)(C8::kStages * C8::kStage);

@@ -112,9 +112,10 @@ def kpm_1d(H, NC: int, NR: int, NH: int | None = None, *, psi_in=None, psi_in_l=
     ``kernel`` picks the recurrence kernel (``include/kpmgb.h``,
     ``kernel_variant``): ``"auto"`` (one thread-block-cluster launch per call
     for small operators, else per-step launches of the row-streaming kernels
-    -- on packed FP32 pairs for real operators with 2..64 columns,
-    float-float doubling -- where they apply, else of the register-gather
-    kernel), ``"gather"``,
+    -- on packed FP32 pairs for real operators, on column pairs for complex
+    ones, float-float with 2..128 columns -- where they apply, else of the
+    register-gather kernel; float-float doubling calls on an operator that is
+    not Hermitian take the kernels that keep the imaginary part), ``"gather"``,
     ``"padded"``, ``"streaming"``, ``"cluster"``, ``"single"``, ``"tune"``.
     ``use_graph`` replays the per-step launches from a CUDA graph.  With
     ``NR_parallel=False`` the columns run one call each, with the same

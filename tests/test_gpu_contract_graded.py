@@ -111,3 +111,35 @@ def test_zero_vectors():
     half = (np.arange(n) % 2).astype(complex)
     assert _moment(half, np.ones(n, complex)) == n // 2
     assert _moment(half, 1 - half) == 0
+
+
+def _halves(rng, n, left, right):
+    """Gaussian vectors whose halves have the given sizes."""
+    h = n // 2
+    out = []
+    for sizes in (left, right):
+        v = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+        v[:h] *= sizes[0]
+        v[h:] *= sizes[1]
+        out.append(v)
+    return out
+
+
+@pytest.mark.parametrize("n", [5000, 16384, 41003])
+@pytest.mark.parametrize("left,right", [((1, 1), (1, 1)), ((1, 0), (0.04, 1)), ((1, 0), (0, 1)),
+                                        ((1, 1e-9), (1e-9, 1)), ((1, 0.1), (0, 1))]
+                         + [((1, 2.0 ** -k), (2.0 ** -k, 1)) for k in (3, 5, 6, 7, 8, 9, 12)])
+def test_halves_of_different_size(n, left, right):
+    """Terms far below the product of the maxima: the sum is as near to the
+    exact one as FP64 sums over runs of 1024 products and more are."""
+    rng = np.random.default_rng(n)
+    pl, pr = _halves(rng, n, left, right)
+    got = _moment(pl, pr)
+    x, y = pl.astype(np.clongdouble), pr.astype(np.clongdouble)
+    for value, terms in zip((got.real, got.imag), _parts(x, y)):
+        exact = math.fsum(map(float, terms))
+        # root mean square 0.42 2^-54 sqrt(run) per product, twelve of them (the
+        # figure is measured to within 2), and the rounding of the sums' total
+        size = float(np.sqrt((terms.astype(float) ** 2).sum()))
+        bound = 12 * 0.42 * 2.0 ** -54 * math.sqrt(1024) * size + 16 * 2.0 ** -53 * abs(exact)
+        assert abs(value - exact) <= bound, (value, exact)
