@@ -683,6 +683,7 @@ int kpmgb_operator_create(int64_t n, int64_t nnz, const int64_t* colptr, const i
   // across calls (no page faults, and the upload runs at the copy kernel's
   // rate); larger operators use a buffer of their own.
   constexpr size_t kCachedStaging = size_t(64) << 20;
+  constexpr size_t kFlagBytes = 64;
   static std::mutex staging_mtx;
   static HostCSR staging_csr;
   static unsigned char* staging = nullptr;
@@ -692,18 +693,24 @@ int kpmgb_operator_create(int64_t n, int64_t nnz, const int64_t* colptr, const i
   HostCSR local;
   HostCSR* hcp = &local;
   unsigned char* dst = nullptr;
+  // k_check_hermitian's answer: written into the page-locked buffer by the
+  // kernel, or copied from the device for operators without one (memset, copy
+  // and kernel took 100 us of a small operator's 620)
+  unsigned own_flag = 0;
+  unsigned* differs = &own_flag;
   if (need <= kCachedStaging) {
     staging_lk.lock();
-    if (staging_cap < need) {
+    if (staging_cap < need + kFlagBytes) {
       if (staging) cudaFreeHost(staging);
       staging = nullptr;
       staging_cap = 0;
-      const size_t cap = std::max(need, size_t(4) << 20);
+      const size_t cap = std::max(need + kFlagBytes, size_t(4) << 20);
       if (cudaHostAlloc(&staging, cap, cudaHostAllocPortable) == cudaSuccess) staging_cap = cap;
       else cudaGetLastError();  // fall back to a pageable buffer
     }
     hcp = &staging_csr;
-    dst = staging_cap >= need ? staging : nullptr;
+    dst = staging_cap >= need + kFlagBytes ? staging : nullptr;
+    if (dst) differs = reinterpret_cast<unsigned*>(staging + staging_cap - kFlagBytes);
   }
   HostCSR& hc = *hcp;
   std::string err;
@@ -727,7 +734,7 @@ int kpmgb_operator_create(int64_t n, int64_t nnz, const int64_t* colptr, const i
   c.max_row_nnz = hc.max_row_nnz;
   c.rmax = hc.rmax;
   const int is_real = hc.is_real;
-  unsigned differs = 0;
+  *differs = 0;
   const size_t nz = (size_t)std::max<int64_t>(nnz, 1);
   // one device block: the converted arrays (laid out as the host buffer, so
   // one copy uploads them), then the arrays built on the device
@@ -770,19 +777,20 @@ int kpmgb_operator_create(int64_t n, int64_t nnz, const int64_t* colptr, const i
         CREATE_CUDA(cudaGetLastError());
       g_launches.fetch_add(1);
       c.ell_w = W;
-      unsigned* flag = reinterpret_cast<unsigned*>(base + off_flag);
-      CREATE_CUDA(cudaMemsetAsync(flag, 0, sizeof(unsigned), op->stream));
+      unsigned* flag = dst ? differs : reinterpret_cast<unsigned*>(base + off_flag);
+      if (!dst) CREATE_CUDA(cudaMemsetAsync(flag, 0, sizeof(unsigned), op->stream));
       k_check_hermitian<<<(unsigned)((n + 255) / 256), 256, 0, op->stream>>>(c.rowptr, c.col, c.val,
                                                                              (int)n, flag);
       g_launches.fetch_add(1);
       CREATE_CUDA(cudaGetLastError());
-      CREATE_CUDA(cudaMemcpyAsync(&differs, flag, sizeof(unsigned), cudaMemcpyDeviceToHost,
-                                  op->stream));
+      if (!dst)
+        CREATE_CUDA(cudaMemcpyAsync(differs, flag, sizeof(unsigned), cudaMemcpyDeviceToHost,
+                                    op->stream));
     }
   }
   // the host buffer is released on return: the copy must have completed
   CREATE_CUDA(cudaStreamSynchronize(op->stream));
-  c.hermitian = differs == 0;
+  c.hermitian = *static_cast<volatile unsigned*>(differs) == 0;
 #undef CREATE_CUDA
   *out = reinterpret_cast<kpmgb_operator>(op);
   return KPMGB_OK;
